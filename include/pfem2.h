@@ -335,9 +335,10 @@ pfem2_status pfem2_enable_stage_timing(pfem2_ctx* ctx, int32_t on);
 pfem2_status pfem2_get_stream(pfem2_ctx* ctx, void** stream);
 /* Sizes of the pressure solver's multigrid hierarchy after pfem2_setup
  * (diagnostics; no counterpart in the reference). out[0..3]: unknowns per
- * level; out[4..11]: stored nonzeros of R01, R02, the b3 contribution rows,
- * the level-0 prolongator, and the J1, Pt1, J2, Pt2 rows of all blocks'
- * coarse lists (halo rows counted once per block that evaluates them).
+ * level; out[4..11]: stored nonzeros of the restrictions to level 1 and from
+ * it to level 2, 0, the level-0 prolongator, the J1 and Pt1 rows of all
+ * blocks' level-1 lists (halo rows counted once per block that evaluates
+ * them), the dense rows of the two coarsest levels, 0.
  * All zero without a hierarchy. */
 #define PFEM2_N_SOLVER_SIZES 12
 pfem2_status pfem2_solver_sizes(pfem2_ctx* ctx, int64_t* out);

@@ -21,6 +21,12 @@ namespace pfem2 {
 
 namespace {
 
+// entries of J_1 and Pt_1 rows that a block may read for its level-1 halo per
+// iteration; above, x1 is formed by the owners in a phase of its own (about 3
+// us an iteration): 2D channels read 1.5-2k (no gain), the 10k-cell pipe 13k
+// (pressure solve 1.47 -> 1.01 ms) and the 131k-cell pipe 23k (4.85 -> 3.47 ms)
+constexpr size_t kHaloMax = 4096;
+
 struct Csr {
   int n = 0, m = 0;
   std::vector<int> ptr{0}, col;
@@ -228,6 +234,31 @@ int tile_aggregate(const Csr& A, const std::vector<int>& tile, int t0, int per, 
   return na;
 }
 
+// aggregates of aggregates: the graph of the tentative (piecewise-constant)
+// coarse operator aggregated again inside the tiles; the new count
+int merge_aggregates(const Csr& A, const std::vector<int>& tile, int na, std::vector<int>& agg) {
+  Csr P;
+  P.n = A.n;
+  P.m = na;
+  P.ptr.assign(A.n + 1, 0);
+  std::vector<int> ctile(na, -1), cagg;
+  for (int i = 0; i < A.n; ++i) {
+    if (agg[i] >= 0) {
+      P.col.push_back(agg[i]);
+      P.val.push_back(1.0);
+      ctile[agg[i]] = tile[i];
+    }
+    P.ptr[i + 1] = (int)P.col.size();
+  }
+  const Csr Ac = spgemm(transpose(P), spgemm(A, P));
+  const int nc = aggregate(Ac, ctile, cagg);
+  for (int k = 0; k < na; ++k)
+    if (cagg[k] < 0) return na;  // an aggregate without neighbours: keep the finer ones
+  for (int i = 0; i < A.n; ++i)
+    if (agg[i] >= 0) agg[i] = cagg[agg[i]];
+  return nc;
+}
+
 struct Level {
   Csr A, J, P, Pt2;
   std::vector<double> dinv;
@@ -272,14 +303,14 @@ bool spd_inverse(std::vector<double>& M, int n) {
 
 pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vector<int>& col,
                       const std::vector<int>& len, const std::vector<Tile>& tiles, const std::vector<int>& st0,
-                      const std::vector<int>& bt0, bool split, int coarse_max, MgHost& H) {
+                      const std::vector<int>& bt0, int coarse_max, MgHost& H) {
   const int ni = (int)c.inst.size(), T = (int)tiles.size(), G = (int)bt0.size() - 1;
-  H.split = split;
+  // M2 is dense: level 2 is coarsened further where a system would have more
+  // dofs than this (151 MB of FP32 rows per system, 4 GB over a batch)
+  const int n2_max = std::max(512, std::min(6144, (int)std::sqrt(1.0e9 / ni)));
   const std::vector<int>& sp = c.h_sl_ptr;
   std::vector<std::vector<Level>> sysL(ni);
   std::vector<std::vector<double>> Einv(ni);
-  std::vector<double> w0(ni);
-  H.j0.assign(c.nell, 0.0);
   for (int s = 0; s < ni; ++s) {
     const int v0 = c.inst[s].v_off, n0 = c.inst[s].nv_pad;
     std::vector<Level>& L = sysL[s];
@@ -338,7 +369,6 @@ pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vec
         break;
       }
       V.w = 4.0 / (3.0 * rho_dinv_a(V.A, V.dinv));
-      H.w.push_back(V.w);
       // J = 2 w D^-1 - w^2 D^-1 A D^-1
       V.J = V.A;
       for (int i = 0; i < n; ++i)
@@ -349,7 +379,12 @@ pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vec
       std::vector<int> agg;
       // the coarsest level: groups of tiles, at most coarse_max unknowns per system
       const int ntl = st0[s + 1] - st0[s], per = (ntl + coarse_max - 1) / coarse_max;
-      const int na = l < kMgLevels - 2 ? aggregate(V.A, V.tile, agg) : tile_aggregate(V.A, V.tile, st0[s], per, agg);
+      int na = l < kMgLevels - 2 ? aggregate(V.A, V.tile, agg) : tile_aggregate(V.A, V.tile, st0[s], per, agg);
+      while (l == 1 && na > n2_max) {
+        const int nc = merge_aggregates(V.A, V.tile, na, agg);
+        if (nc == na) break;
+        na = nc;
+      }
       if (na == 0) {
         set_error("amg: aggregation produced no coarse unknowns");
         return PFEM2_MESH_ERROR;
@@ -372,19 +407,7 @@ pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vec
       L[l + 1].A = spgemm(transpose(V.P), spgemm(V.A, V.P));
       L[l + 1].tile = ctile;
     }
-    w0[s] = L[0].w;
-    // J_0 on the SELL pattern
-    for (int i = 0; i < n0; ++i) {
-      const int row = v0 + i, sl = row / kSlice, lane = row % kSlice;
-      const double di = L[0].dinv[i], w = L[0].w;
-      for (int j = 0; j < len[sl]; ++j) {
-        const int e = sp[sl] + j * kSlice + lane;
-        const int cc = col[e] - v0;
-        double v = -w * w * di * A[e] * L[0].dinv[cc];
-        if (j == 0) v += 2.0 * w * di;
-        H.j0[e] = v;
-      }
-    }
+    H.w0.push_back(L[0].w);
   }
   // ---- global numbering: systems in order, dofs tile-ordered inside
   std::vector<std::vector<int>> goff(kMgLevels, std::vector<int>(ni + 1, 0));
@@ -416,41 +439,76 @@ pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vec
   };
   for (int s = 0; s < ni; ++s) {
     std::vector<Level>& L = sysL[s];
-    append_rows(transpose(L[0].Pt2), c.inst[s].v_off, H.r01_ptr, H.r01_col, H.r01_val);
-    if (split) {
-      append_rows(transpose(L[1].Pt2), goff[1][s], H.q2_ptr, H.q2_col, H.q2_val);
-    } else {
-      const Csr P01 = spgemm(L[0].Pt2, L[1].Pt2);
-      append_rows(transpose(P01), c.inst[s].v_off, H.r02_ptr, H.r02_col, H.r02_val);
-    }
-    H.sys_D3.push_back(L[3].A.n);
-    H.sys_off3.push_back(goff[3][s]);
-    H.sys_n2.push_back(L[2].A.n);
+    Csr R = transpose(L[0].Pt2);
+    for (size_t e = 0; e < R.col.size(); ++e) R.val[e] /= L[0].dinv[R.col[e]];
+    append_rows(R, c.inst[s].v_off, H.r1_ptr, H.r1_col, H.r1_val);
+    append_rows(transpose(L[1].Pt2), goff[1][s], H.q2_ptr, H.q2_col, H.q2_val);
+    const int n2 = L[2].A.n, n3 = L[3].A.n;
+    H.sys_n2.push_back(n2);
     H.sys_off2.push_back(goff[2][s]);
-    H.dmax = std::max(H.dmax, L[3].A.n);
+    // M2 = J_2 + (Pt_2 E^-1) Pt_2^T
+    const Csr& P = L[2].Pt2;
+    const size_t m0 = H.m2.size();
+    H.m2.resize(m0 + (size_t)n2 * n2, 0.0);
+    std::vector<double> t(n3);
+    for (int i = 0; i < n2; ++i) {
+      double* row = H.m2.data() + m0 + (size_t)i * n2;
+      std::fill(t.begin(), t.end(), 0.0);
+      for (int e = P.ptr[i]; e < P.ptr[i + 1]; ++e) {
+        const double v = P.val[e];
+        const double* E = Einv[s].data() + (size_t)P.col[e] * n3;
+        for (int d = 0; d < n3; ++d) t[d] += v * E[d];
+      }
+      for (int j = 0; j < n2; ++j) {
+        double v = 0.0;
+        for (int e = P.ptr[j]; e < P.ptr[j + 1]; ++e) v += t[P.col[e]] * P.val[e];
+        row[j] = v;
+      }
+      for (int e = L[2].J.ptr[i]; e < L[2].J.ptr[i + 1]; ++e) row[L[2].J.col[e]] += L[2].J.val[e];
+    }
   }
-  // the restriction not in use: empty rows
-  if (split) H.r02_ptr.assign(H.n[2] + 1, 0);
-  else H.q2_ptr.assign(H.n[2] + 1, 0);
   // ---- per-block lists
   std::vector<int> sys_of_tile(T);
   for (int s = 0; s < ni; ++s)
     for (int t = st0[s]; t < st0[s + 1]; ++t) sys_of_tile[t] = s;
-  std::vector<int> loc1(H.n[1], -1), loc2(H.n[2], -1), loc3(H.n[3], -1);
-  for (int l = 1; l <= 2; ++l) {
-    H.blk_s[l].assign(1, 0);
-    H.s_jptr[l].assign(1, 0);
-    H.s_pptr[l].assign(1, 0);
+  std::vector<int> loc1(H.n[1], -1);
+  // the level-1 halo each block's rows prolong from, and the entries of its
+  // J_1 and Pt_1 rows
+  std::vector<std::vector<int>> halo(G);
+  size_t nhalo = 0;
+  for (int b = 0; b < G; ++b) {
+    const int t_lo = bt0[b], t_hi = bt0[b + 1];
+    std::vector<int>& h = halo[b];
+    for (int t = t_lo; t < t_hi; ++t) {
+      const int s = sys_of_tile[t], v0 = c.inst[s].v_off;
+      const Csr& P = sysL[s][0].Pt2;
+      for (int e = P.ptr[tiles[t].s0 * kSlice - v0]; e < P.ptr[tiles[t].s1 * kSlice - v0]; ++e) {
+        const int g = goff[1][s] + P.col[e];
+        if ((g < H.toff[1][t_lo] || g >= H.toff[1][t_hi]) && loc1[g] != b) {
+          loc1[g] = b;
+          h.push_back(g);
+        }
+      }
+    }
+    std::sort(h.begin(), h.end());
+    for (int g : h) {
+      const int s = H.lsys[1][g], r = g - goff[1][s];
+      const Level& V = sysL[s][1];
+      nhalo += V.J.ptr[r + 1] - V.J.ptr[r] + V.Pt2.ptr[r + 1] - V.Pt2.ptr[r];
+    }
   }
-  H.blk_s3.assign(1, 0);
-  H.blk_e.assign(1, 0);
+  std::fill(loc1.begin(), loc1.end(), -1);
+  H.xsplit = nhalo > (size_t)G * kHaloMax;
+  H.blk_s1.assign(1, 0);
+  H.j1_ptr.assign(1, 0);
+  H.p1_ptr.assign(1, 0);
+  H.blk_m2.assign(1, 0);
+  H.m2_off.assign(H.n[2], 0);
   H.p0_ptr.assign(c.nslices + 1, 0);
   H.p0_len.assign(c.nslices, 0);
   std::vector<std::vector<int>> p0c(c.nslices);
   std::vector<std::vector<double>> p0v(c.nslices);
   for (int l = 1; l <= 2; ++l) H.lk[l].assign(H.n[l], 0);
-  std::vector<std::vector<int>> g3_rows(H.n[3]);
-  H.c3_blk.assign(1, 0);
   for (int b = 0; b < G; ++b) {
     const int t_lo = bt0[b], t_hi = bt0[b + 1];
     // systems of a block are consecutive; lists store the index among them
@@ -462,112 +520,34 @@ pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vec
       for (int s = sys_of_tile[t_lo]; s <= sys_of_tile[t_hi - 1]; ++s) n2 += sysL[s][2].A.n;
       H.b2max = std::max(H.b2max, n2);
     }
-    // contributions of the own level-2 rows to b3 = Pt2^T b2: one row per
-    // touched level-3 dof, columns = own level-2 rows (relative index)
-    {
-      const int o2lo = H.toff[2][t_lo], o2hi = H.toff[2][t_hi];
-      std::vector<std::pair<int, std::pair<int, double>>> ent;  // (level-3 dof, (own row, value))
-      for (int g = o2lo; g < o2hi; ++g) {
-        const int s = H.lsys[2][g], a = g - goff[2][s];
-        const Csr& P = sysL[s][2].Pt2;
-        for (int e = P.ptr[a]; e < P.ptr[a + 1]; ++e) ent.push_back({goff[3][s] + P.col[e], {g - o2lo, P.val[e]}});
-      }
-      std::stable_sort(ent.begin(), ent.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
-      for (size_t k = 0; k < ent.size(); ++k) {
-        if (k == 0 || ent[k].first != ent[k - 1].first) {
-          const int d = ent[k].first;
-          g3_rows[d].push_back((int)H.c3_lk.size());
-          H.c3_lk.push_back(H.lsys[3][d] - sys_first);
-          H.c3_ptr.push_back((int)H.c3_col.size());
-        }
-        H.c3_col.push_back(ent[k].second.first);
-        H.c3_val.push_back(ent[k].second.second);
-      }
-      H.c3_blk.push_back((int)H.c3_lk.size());
+    long long mo = 0;
+    for (int g = H.toff[2][t_lo]; g < H.toff[2][t_hi]; ++g) {
+      H.m2_off[g] = (int)mo;
+      mo += sysL[H.lsys[2][g]][2].A.n;
     }
-    // S1: own level-1 dofs, then the halo the level-0 prolongation reads
-    std::vector<int> S1, S2, S3;
+    H.blk_m2.push_back(H.blk_m2.back() + mo);
+    // own level-1 dofs, then the halo the level-0 prolongation reads
+    std::vector<int> S1;
     for (int g = H.toff[1][t_lo]; g < H.toff[1][t_hi]; ++g) S1.push_back(g);
-    std::vector<int> halo;
-    for (int t = t_lo; t < t_hi; ++t) {
-      const int s = sys_of_tile[t], v0 = c.inst[s].v_off;
-      const Csr& P = sysL[s][0].Pt2;
-      for (int row = tiles[t].s0 * kSlice; row < tiles[t].s1 * kSlice; ++row)
-        for (int e = P.ptr[row - v0]; e < P.ptr[row - v0 + 1]; ++e) {
-          const int g = goff[1][s] + P.col[e];
-          if (g < H.toff[1][t_lo] || g >= H.toff[1][t_hi]) halo.push_back(g);
-        }
-    }
-    std::sort(halo.begin(), halo.end());
-    halo.erase(std::unique(halo.begin(), halo.end()), halo.end());
-    S1.insert(S1.end(), halo.begin(), halo.end());
+    if (!H.xsplit) S1.insert(S1.end(), halo[b].begin(), halo[b].end());
     for (int k = 0; k < (int)S1.size(); ++k) loc1[S1[k]] = k;
     for (int g : S1) {
-      const int s = H.lsys[1][g];
-      const Csr& P = sysL[s][1].Pt2;
-      const int a = g - goff[1][s];
-      for (int e = P.ptr[a]; e < P.ptr[a + 1]; ++e) S2.push_back(goff[2][s] + P.col[e]);
-    }
-    std::sort(S2.begin(), S2.end());
-    S2.erase(std::unique(S2.begin(), S2.end()), S2.end());
-    for (int k = 0; k < (int)S2.size(); ++k) loc2[S2[k]] = k;
-    for (int g : S2) {
-      const int s = H.lsys[2][g];
-      const Csr& P = sysL[s][2].Pt2;
-      const int a = g - goff[2][s];
-      for (int e = P.ptr[a]; e < P.ptr[a + 1]; ++e) S3.push_back(goff[3][s] + P.col[e]);
-    }
-    std::sort(S3.begin(), S3.end());
-    S3.erase(std::unique(S3.begin(), S3.end()), S3.end());
-    for (int k = 0; k < (int)S3.size(); ++k) loc3[S3[k]] = k;
-    // level-1 and level-2 entries: J rows (global columns), Pt rows (local columns)
-    const std::vector<int>* Sl[3] = {nullptr, &S1, &S2};
-    std::vector<int>* locn[3] = {nullptr, &loc2, &loc3};
-    for (int l = 1; l <= 2; ++l) {
-      for (int g : *Sl[l]) {
-        const int s = H.lsys[l][g], a = g - goff[l][s];
-        const Level& V = sysL[s][l];
-        H.s_sys[l].push_back(s - sys_first);
-        for (int e = V.J.ptr[a]; e < V.J.ptr[a + 1]; ++e) {
-          // level 1: global ids into b1; level 2: the system's own index
-          // into the block's shared copy of b2
-          H.s_jcol[l].push_back((l == 1 ? goff[l][s] : 0) + V.J.col[e]);
-          H.s_jval[l].push_back(V.J.val[e]);
-        }
-        H.s_jptr[l].push_back((int)H.s_jcol[l].size());
-        for (int e = V.Pt2.ptr[a]; e < V.Pt2.ptr[a + 1]; ++e) {
-          H.s_pcol[l].push_back((*locn[l])[goff[l + 1][s] + V.Pt2.col[e]]);
-          H.s_pval[l].push_back(V.Pt2.val[e]);
-        }
-        H.s_pptr[l].push_back((int)H.s_pcol[l].size());
+      const int s = H.lsys[1][g], r = g - goff[1][s];
+      const Level& V = sysL[s][1];
+      H.s1_lk.push_back(s - sys_first);
+      for (int e = V.J.ptr[r]; e < V.J.ptr[r + 1]; ++e) {
+        H.j1_col.push_back(goff[1][s] + V.J.col[e]);
+        H.j1_val.push_back(V.J.val[e]);
       }
-      H.blk_s[l].push_back((int)H.s_sys[l].size());
+      H.j1_ptr.push_back((int)H.j1_col.size());
+      for (int e = V.Pt2.ptr[r]; e < V.Pt2.ptr[r + 1]; ++e) {
+        H.p1_col.push_back(goff[2][s] + V.Pt2.col[e]);
+        H.p1_val.push_back(V.Pt2.val[e]);
+      }
+      H.p1_ptr.push_back((int)H.p1_col.size());
     }
+    H.blk_s1.push_back((int)H.s1_lk.size());
     H.s1max = std::max(H.s1max, (int)S1.size());
-    H.s2max = std::max(H.s2max, (int)S2.size());
-    H.s3max = std::max(H.s3max, (int)S3.size());
-    // level-3 entries: the coarse-inverse rows of each system's entries,
-    // stored transposed ([d][entry]) so that the entries read consecutive
-    // shared-memory words
-    int eb = 0;
-    for (size_t a = 0; a < S3.size();) {
-      const int s = H.lsys[3][S3[a]], D = H.sys_D3[s];
-      size_t b = a;
-      while (b < S3.size() && H.lsys[3][S3[b]] == s) ++b;
-      const int n = (int)(b - a);
-      for (size_t j = a; j < b; ++j) {
-        H.s3_sys.push_back(s - sys_first);
-        H.s3_eoff.push_back(eb + (int)(j - a));
-        H.s3_estr.push_back(n);
-      }
-      for (int d = 0; d < D; ++d)
-        for (size_t j = a; j < b; ++j) H.s3_E.push_back((float)Einv[s][(size_t)(S3[j] - goff[3][s]) * D + d]);
-      eb += D * n;
-      a = b;
-    }
-    H.blk_s3.push_back((int)H.s3_sys.size());
-    H.blk_e.push_back((int)H.s3_E.size());
-    H.emax = std::max(H.emax, eb);
     // level-0 prolongation rows of the block's slices
     for (int t = t_lo; t < t_hi; ++t) {
       const int s = sys_of_tile[t], v0 = c.inst[s].v_off;
@@ -585,23 +565,14 @@ pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vec
           const int i = sl * kSlice + l - v0;
           for (int e = P.ptr[i]; e < P.ptr[i + 1]; ++e) {
             const int j = e - P.ptr[i];
-            p0c[sl][(size_t)j * kSlice + l] = loc1[goff[1][s] + P.col[e]];
+            const int g = goff[1][s] + P.col[e];
+            p0c[sl][(size_t)j * kSlice + l] = H.xsplit ? g : loc1[g];
             p0v[sl][(size_t)j * kSlice + l] = P.val[e];
           }
         }
       }
     }
     for (int g : S1) loc1[g] = -1;
-    for (int g : S2) loc2[g] = -1;
-    for (int g : S3) loc3[g] = -1;
-  }
-  H.c3_ptr.push_back((int)H.c3_col.size());
-  H.g3_ptr.assign(1, 0);
-  H.c3_pos.assign(H.c3_lk.size(), 0);
-  for (int d = 0; d < H.n[3]; ++d) {
-    int n = H.g3_ptr.back();
-    for (int r : g3_rows[d]) H.c3_pos[r] = n++;
-    H.g3_ptr.push_back(n);
   }
   for (int sl = 0; sl < c.nslices; ++sl) {
     H.p0_ptr[sl + 1] = H.p0_ptr[sl] + H.p0_len[sl] * kSlice;

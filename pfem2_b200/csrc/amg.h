@@ -28,60 +28,42 @@ struct MgHost {
   std::vector<int> toff[kMgLevels];       // [l][ntiles+1] first level-l dof of each tile (l >= 1)
   std::vector<int> lsys[kMgLevels];       // [l][n_l] system of each level-l dof (l >= 1)
   std::vector<int> lk[3];                 // [1..2][n_l] index of that system among its block's systems
-  // restrictions from level 0 (CSR over the rows of level l, global
-  // level-0 columns): R0l = (Pt_0 ... Pt_{l-1})^T, l = 1, 2; R02 only
-  // without the split restriction
-  std::vector<int> r01_ptr, r01_col, r02_ptr, r02_col;
-  std::vector<double> r01_val, r02_val;
-  // split restriction (large systems): b2 = Pt_1^T b1 in a phase of its
-  // own, CSR over the level-2 rows with global level-1 columns
-  bool split = false;
+  // Pt_0^T D (applied to D^-1 v), CSR over the level-1 rows with global
+  // level-0 columns
+  std::vector<int> r1_ptr, r1_col;
+  std::vector<double> r1_val;
+  // Pt_1^T, CSR over the level-2 rows with global level-1 columns
   std::vector<int> q2_ptr, q2_col;
   std::vector<double> q2_val;
-  // b3 = Pt_2^T b2 in two steps: every block adds up the contributions of
-  // its own level-2 rows to the level-3 dofs they touch (CSR rows c3,
-  // columns = own level-2 row - first own row, grouped per block by c3_blk,
-  // c3_lk = the dof's system among the block's systems) and stores row r at
-  // c3_pos[r]; the contributions of level-3 dof d are then the contiguous
-  // range [g3_ptr[d], g3_ptr[d+1]) of that array, in block order
-  std::vector<int> c3_blk, c3_ptr, c3_col, c3_lk, g3_ptr, c3_pos;
-  std::vector<double> c3_val;
-  // level-0 smoother J_0 on the SELL pattern of A
-  std::vector<double> j0;
+  // M2 = J_2 + Pt_2 E^-1 Pt_2^T, dense rows of the system's n2 columns in
+  // level-2 order: where each block's rows start, and each row's offset there
+  std::vector<double> m2;
+  std::vector<long long> blk_m2;          // [G+1]
+  std::vector<int> m2_off;                // [n2]
   // post-smoothed prolongator of level 0 on SELL slices; columns are the
-  // indices into the owning block's level-1 list
+  // indices into the owning block's level-1 list (global with xsplit)
   std::vector<int> p0_ptr, p0_len, p0_col;
   std::vector<double> p0_val;
-  // per-block lists of the level-1 and level-2 dofs a block evaluates
-  // (own dofs and the halo its prolongation reads): J rows (level 1:
-  // global columns; level 2: the system's level-2 index), Pt rows with
-  // columns into the block's next-level list
-  std::vector<int> blk_s[3];              // [1..2][G+1] list offsets; [0] unused
-  // (s_sys, s3_sys: index of the entry's system among the block's systems)
-  std::vector<int> s_sys[3], s_jptr[3], s_jcol[3], s_pptr[3], s_pcol[3];
-  std::vector<double> s_jval[3], s_pval[3];
-  // per-block level-3 list: system, and where its column of the block's
-  // transposed coarse-inverse rows starts (stride s3_estr)
-  std::vector<int> blk_s3, s3_sys, s3_eoff, s3_estr, blk_e;
-  std::vector<float> s3_E;
-  std::vector<int> sys_D3, sys_off3;      // coarse size and first level-3 dof per system
+  // per-block lists of the level-1 dofs a block evaluates (own dofs, then,
+  // unless xsplit, the halo its rows prolong from): system among the block's,
+  // J_1 rows with global level-1 columns, Pt_1 rows with global level-2 columns
+  bool xsplit = false;
+  std::vector<int> blk_s1, s1_lk, j1_ptr, j1_col, p1_ptr, p1_col;
+  std::vector<double> j1_val, p1_val;
   std::vector<int> sys_n2, sys_off2;      // level-2 size and first level-2 dof per system
-  int s1max = 0, s2max = 0, s3max = 0, emax = 0, dmax = 1;
+  std::vector<double> w0;                 // level-0 smoother weight per system
+  int s1max = 0;
   int b2max = 0;                          // level-2 dofs of the local systems of a block
-  // diagnostics
-  std::vector<double> w;                  // smoother weight per system and level
 };
 
 // Builds the hierarchy of every pressure system. A, col, len: host copy of
 // the eliminated FP64 pressure matrix in the context's SELL layout; tiles,
 // st0: the pressure solve's tiles and first tile per system; bt0: first
-// tile per block of the persistent grid; split: restrict to level 2 in a
-// phase of its own (b2 = Pt_1^T b1) instead of through the composite R02;
-// coarse_max: level-3 unknowns per system at most (groups of tiles share
-// one), which bounds the dense inverse rows a block holds in shared memory.
+// tile per block of the persistent grid; coarse_max: level-3 unknowns per
+// system at most (groups of tiles share one).
 pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vector<int>& col,
                       const std::vector<int>& len, const std::vector<Tile>& tiles, const std::vector<int>& st0,
-                      const std::vector<int>& bt0, bool split, int coarse_max, MgHost& out);
+                      const std::vector<int>& bt0, int coarse_max, MgHost& out);
 
 // In-place inverse of an SPD matrix (Cholesky, then L^-T L^-1); false if
 // the matrix is not SPD.

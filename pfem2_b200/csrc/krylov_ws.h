@@ -1,0 +1,203 @@
+// krylov_ws.h -- the Krylov workspace and the device helpers shared by the
+// Jacobi solver kernel (krylov.cu) and the multigrid CG kernel (mgcg.cu).
+#pragma once
+#include <string>
+#include <vector>
+
+#include "common.cuh"
+#include "ctx.h"
+
+namespace pfem2 {
+
+constexpr int kMaxLocalSys = 16;  // systems a block of a solver grid may own parts of
+
+// a read-only array seen either in global memory (base 0) or through a
+// staged shared-memory copy of its range [base, ...)
+template <typename T>
+struct SV {
+  const T* p;
+  int base;
+  __device__ __forceinline__ T operator[](int i) const { return p[i - base]; }
+};
+
+__device__ __forceinline__ float fma_r(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fma_r(double a, double b, double c) { return fma(a, b, c); }
+
+template <int GL, typename T>
+__device__ __forceinline__ T group_sum(T v) {
+#pragma unroll
+  for (int o = GL / 2; o > 0; o >>= 1) v += __shfl_xor_sync(PFEM2_FULL_MASK, v, o);
+  return v;
+}
+
+// acc + sum over the entries of a SELL row of val(ei) * x(col), in entry
+// order, with the loads of CH entries issued before their products are
+// accumulated (one memory round trip per CH entries instead of one per entry)
+template <typename T, int CH = 8, typename Cols, typename Val, typename X>
+__device__ __forceinline__ T sell_dot(T acc, Cols cols, int base, int len, int lane, Val val, X x) {
+  for (int j0 = 0; j0 < len; j0 += CH) {
+    T av[CH], xv[CH];
+#pragma unroll
+    for (int u = 0; u < CH; ++u) {
+      const int j = j0 + u;
+      if (j < len) {
+        const int ei = base + j * 32 + lane;
+        av[u] = val(ei);
+        xv[u] = x(cols[ei]);
+      } else {
+        av[u] = T(0);
+        xv[u] = T(0);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < CH; ++u) acc = fma_r(av[u], xv[u], acc);
+  }
+  return acc;
+}
+
+// x[col] from the shared mirror m of the block's own rows [own0, own0 +
+// nown) when there is one, else from global memory: one generic load, no
+// branch (plain loads see the other blocks' writes of the previous phase,
+// which the phase start's acquire ordered before them)
+template <typename R>
+__device__ __forceinline__ R ldm(const R* g, const R* m, int col, int own0, int nown) {
+  const unsigned o = (unsigned)(col - own0);
+  const R* src = (m != nullptr && o < (unsigned)nown) ? m + o : g + col;
+  return *src;
+}
+
+// acc + sum over CSR entries [k0, k1) of val(k) * x(col(k)), the lanes of a
+// group of GL taking every GL-th entry, loads issued CH entries at a time
+template <int GL, int CH, typename T, typename Cols, typename Val, typename X>
+__device__ __forceinline__ T csr_dot(T acc, int k0, int k1, int sub, Cols cols, Val val, X x) {
+  for (int kb = k0 + sub; kb < k1; kb += CH * GL) {
+    T av[CH], xv[CH];
+#pragma unroll
+    for (int u = 0; u < CH; ++u) {
+      const int k = kb + u * GL;
+      if (k < k1) {
+        av[u] = val[k];
+        xv[u] = x(cols[k]);
+      } else {
+        av[u] = T(0);
+        xv[u] = T(0);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < CH; ++u) acc = fma_r(av[u], xv[u], acc);
+  }
+  return acc;
+}
+
+// copies src[lo, hi) into shared memory at `cur` (16-byte aligned pieces)
+// and returns the view of that range; the caller syncs before reading it
+__device__ __forceinline__ size_t al16_dev(size_t b) { return (b + 15) & ~(size_t)15; }
+
+template <typename T>
+__device__ __forceinline__ SV<T> stage_range(unsigned char*& cur, const T* src, int lo, int hi) {
+  T* dst = reinterpret_cast<T*>(cur);
+  for (int i = threadIdx.x; i < hi - lo; i += blockDim.x) dst[i] = src[lo + i];
+  cur += ((size_t)(hi - lo) * sizeof(T) + 15) & ~(size_t)15;
+  return SV<T>{dst, lo};
+}
+
+template <typename T>
+__device__ __forceinline__ SV<T> maybe_stage(bool on, unsigned char*& cur, const T* src, int lo, int hi) {
+  return on ? stage_range(cur, src, lo, hi) : SV<T>{src, 0};
+}
+
+// Waits until system counter *cnt has reached target (release adds of the
+// blocks that own parts of the system); false after spin_limit polls or when
+// another block has flagged an error. The caller fences afterwards.
+__device__ __forceinline__ bool wait_count(const unsigned* cnt, unsigned target, const GridBarrier& gb) {
+  unsigned spins = 0;
+  while ((int)(ld_relaxed_u32(cnt) - target) < 0) {
+    if (++spins > gb.spin_limit || *(volatile int*)gb.err != 0) return false;
+    __nanosleep(20);
+  }
+  return true;
+}
+
+// ------------------------------------------------------------------ host
+struct MgWs;  // mgcg.cu
+
+struct KrylovWs {
+  // Jacobi solves, [0] pressure (without multigrid), [1] velocity components
+  Tile* tiles[2] = {};
+  int* sys_slot0[2] = {};
+  int* sys_owner[2] = {};
+  int* blk_t0[2] = {};
+  int* blk_sys[2] = {};
+  int* blk_sys_off[2] = {};
+  int* blk_sl[2] = {};
+  int ntiles[2] = {}, nsys[2] = {}, grid[2] = {};
+  int stage[2] = {0, 0};   // staged categories per phase
+  size_t smem[2] = {0, 0}; // dynamic shared memory per phase
+  int ntl_max[2] = {0, 0}, items_max[2] = {0, 0};  // per block: tiles, (tile, slice) items
+  size_t items_bytes[2] = {0, 0};                  // shared memory of the item partials and offsets
+  int nsum[2] = {2, 2};                            // partial sums per tile of each phase
+  bool bicg[2] = {false, false};                   // phase solved by BiCGStab
+  void *bz = nullptr, *bw = nullptr, *rh = nullptr, *bs = nullptr, *bt = nullptr, *bkt = nullptr;
+  void *cu = nullptr, *cwh = nullptr, *csh = nullptr, *cw = nullptr, *cs = nullptr;
+  int vel_minb = 2;  // resident blocks per SM of the velocity solves
+  MgWs* mg = nullptr;
+  void *e = nullptr, *r = nullptr, *q = nullptr, *p = nullptr;
+  double* r64 = nullptr;
+  double* part = nullptr;
+  unsigned* scount = nullptr;
+  int* active = nullptr;
+  int* out_it[3] = {};
+  double* out_res[3] = {};
+  double* out_tol[3] = {};
+  int* out_outer[3] = {};
+  std::vector<void*> allocs;            // every device allocation of the workspace
+};
+
+template <typename T>
+inline pfem2_status ws_alloc(KrylovWs* w, T** p, size_t n) {
+  *p = nullptr;
+  if (n == 0) n = 1;
+  PFEM2_CUDA(cudaMalloc((void**)p, sizeof(T) * n));
+  w->allocs.push_back(*p);
+  PFEM2_CUDA(cudaMemset(*p, 0, sizeof(T) * n));
+  return PFEM2_OK;
+}
+
+template <typename T>
+inline pfem2_status ws_upload(KrylovWs* w, T** p, const std::vector<T>& v) {
+  PFEM2_TRY(ws_alloc(w, p, v.size()));
+  if (!v.empty()) PFEM2_CUDA(cudaMemcpy(*p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice));
+  return PFEM2_OK;
+}
+
+// FP64 host values as the inner type R (float for the mixed path)
+inline pfem2_status ws_upload_r(KrylovWs* w, bool mixed, void** p, const std::vector<double>& v) {
+  if (mixed) {
+    std::vector<float> f(v.begin(), v.end());
+    float* d;
+    PFEM2_TRY(ws_upload(w, &d, f));
+    *p = d;
+  } else {
+    double* d;
+    PFEM2_TRY(ws_upload(w, &d, v));
+    *p = d;
+  }
+  return PFEM2_OK;
+}
+
+inline size_t al16(size_t b) { return (b + 15) & ~(size_t)15; }
+
+// shared-memory budget of a solver block (dynamic part) with MINB resident blocks per SM
+constexpr size_t smem_budget(int minb) { return minb == 1 ? 200 * 1024 : 108 * 1024; }
+
+// krylov.cu: resets a solve's shared state (counters, barrier, error word)
+pfem2_status krylov_init_solve(Ctx& c, int nsys);
+int krylov_max_iter(const Ctx& c);
+
+// mgcg.cu: the multigrid CG of the pressure systems
+pfem2_status mg_setup(Ctx& c);
+pfem2_status mg_solve(Ctx& c);
+void mg_free(KrylovWs* w);
+void mg_sizes(const KrylovWs* w, long long* out12);
+
+}  // namespace pfem2
