@@ -297,13 +297,11 @@ __device__ __forceinline__ bool grid_sync_ra(const GridBarrier& gb, unsigned& k)
   return s_ok != 0;
 }
 
-__device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned* p) {
+__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   unsigned v;
-  asm volatile("ld.relaxed.gpu.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-
-__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
 __device__ __forceinline__ void red_release_add_u32(unsigned* p, unsigned v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
@@ -314,6 +312,37 @@ __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(PFEM2_FULL_MASK, v, o);
   return v;
+}
+
+// Sums N values (N a power of two, at most 32) over a warp with N - 1
+// exchanges instead of N * 5: at each halving step a lane keeps one half of
+// its values, sends the other half to its partner and adds what it receives.
+// Afterwards the lane holds the warp total of value warp_sum_many_index<N>.
+template <int N, typename T>
+__device__ __forceinline__ T warp_sum_many(T (&v)[N], int lane) {
+#pragma unroll
+  for (int h = N / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const T send = up ? v[i] : v[i + h];
+      const T keep = up ? v[i + h] : v[i];
+      v[i] = keep + __shfl_xor_sync(PFEM2_FULL_MASK, send, o);
+    }
+  }
+  T r = v[0];
+#pragma unroll
+  for (int o = 16 / N; o > 0; o >>= 1) r += __shfl_xor_sync(PFEM2_FULL_MASK, r, o);
+  return r;
+}
+
+template <int N>
+__device__ __forceinline__ int warp_sum_many_index(int lane) {
+  int idx = 0;
+#pragma unroll
+  for (int h = N / 2, o = 16; h >= 1; h >>= 1, o >>= 1)
+    if (lane & o) idx += h;
+  return idx;
 }
 
 }  // namespace pfem2

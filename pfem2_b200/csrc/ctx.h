@@ -38,13 +38,10 @@ struct HostInst {
   std::vector<int> cells, fb;
 };
 
-// Krylov tile: a run of SELL slices of one system.
+// A run of SELL slices of one system: an aggregation domain of the multigrid.
 struct Tile {
-  int sys;        // system id inside the phase
-  int comp;       // component slot (vector block)
-  int s0, s1;     // slice range
-  int slot;       // partial-sum slot (the slots of a system are contiguous)
-  int lk;         // index of the system among the systems of the tile's block
+  int sys;
+  int s0, s1;
 };
 
 struct Ctx {
@@ -157,11 +154,7 @@ struct Ctx {
   // Krylov workspace
   void* kws = nullptr;
   size_t kws_bytes = 0;
-  Tile* d_tiles[2] = {};      // [0] 1 component phase, [1] dim component phase
-  int ntiles[2] = {};
-  int tile_slices = 0;         // Krylov tile size in slices (0 = automatic)
   double* sys_scalars = nullptr;
-  double* tile_part = nullptr;
   int* d_sysinfo = nullptr;
   unsigned* barrier = nullptr;   // count, gen
   int* d_err = nullptr;         // abort flag of the running solve (reset per launch)
@@ -172,9 +165,6 @@ struct Ctx {
   // a wait timed out: the device state is not trusted, stepping calls
   // return PFEM2_BAD_STATE until the context is destroyed
   bool failed = false;
-  int coop_blocks = 0;
-  int solve_threads = 256;
-  int solve_blocks_per_sm = 1;  // persistent Krylov grid: blocks per SM
   long long mg_wide_min = 262144;  // rows from which one pressure system runs two blocks per SM
   bool two_level = true;        // pressure: multigrid preconditioner (else Jacobi)
   bool vel_bicg = false;        // velocity systems solved by BiCGStab (else CG)

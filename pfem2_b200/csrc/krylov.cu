@@ -9,16 +9,32 @@
 // (deal.II SolverControl(max_iter, tol), cylinder2D/cylinder2D.cc:736-779).
 //
 // The work between two synchronisation points is a "phase". A phase ends
-// with every tile publishing its partial sums and a release add on its
-// system's counter; the next phase starts once the counters of the block's
-// running systems show every tile of those systems done (a per-system
-// barrier: the instances of a batch do not wait for each other). Every
-// block that owns tiles of a system computes that system's scalars itself,
-// from the per-tile partial sums of the previous phase, in a fixed order:
-// no block publishes scalars and no phase waits for a finalizer.
+// with every block publishing its partial sums and a release add on the
+// counters of its systems; the next phase starts once the counters of the
+// block's running systems show every block of those systems done (a
+// per-system barrier: the instances of a batch do not wait for each other).
+// Every block computes its systems' scalars itself, from the partial sums of
+// the previous phase in a fixed order: no block publishes scalars and no
+// phase waits for a finalizer.
 //
-// CG takes one phase per iteration (one reduction), BiCGStab two; see the
-// decisions below.
+// BiCGStab (right-preconditioned, van der Vorst 1992) takes two phases per
+// iteration, CG one (single reduction, Chronopoulos and Gear 1989). A
+// restart costs one phase more: the FP64 residual r64 = b - A64 (x + e) is
+// formed with BiCGStab's pending e += omega K^-1 s on the fly, and the first
+// phase of the next cycle reads its start vector from r64 at the columns.
+// The vectors that a product gathers are packed four to a row (V4), so that
+// an entry costs one vector load instead of two to four.
+//
+// What bounds it: on the 52k-row channel the wait for the slowest block and
+// the dependent loads after it (a phase is about 2.5 us of waiting, sums and
+// publishing and 2 us of work), on the 131k-cell pipe the gathers and the
+// matrix from L2. A block owns a contiguous run of slices with all their
+// components, cut to equal lengths, and a warp takes one (slice, component)
+// at a time. Measured against tiles of 8 slices per component (some blocks
+// held two, others one), separate vectors, generic pointers and three phases
+// per restart, prediction and correction take per step: 52k channel FP32 0.45
+// ms instead of 0.86, FP64 0.59 instead of 1.03; 16 channels 1.38 instead of
+// 2.43; 10k pipe FP64 1.63 instead of 2.39; 131k pipe 3.6 instead of 7.7.
 //
 // The iterate is split x + e: e accumulates in the inner type R (FP32 for
 // the mixed path, FP64 for the plain path); once the recurrence residual
@@ -27,57 +43,76 @@
 // from the true residual. A system is done when the FP64 residual is <= tol.
 #include <algorithm>
 #include <cmath>
-#include <cstdlib>
-#include <cstdio>
+#include <cstring>
 #include <vector>
 
 #include "krylov_ws.h"
 
 namespace pfem2 {
 
-constexpr int kSolveThreads = 384;  // 12 warps
-constexpr int kWarps = kSolveThreads / 32;
+template <int MINB> struct SolveThreads { static constexpr int value = MINB == 1 ? 768 : 384; };
+static int solve_threads(int minb) { return minb == 1 ? SolveThreads<1>::value : SolveThreads<2>::value; }
 
-enum { S_OUT_A = 0, S_OUT_B = 1, S_A = 2, S_B = 3, S_DONE = 4, S_C0 = 5, S_C1 = 6 };
+enum { S_OUT_A = 0, S_OUT_B, S_A, S_B, S_C1, S_DONE };
 enum {
-  ACT_NONE = 0, ACT_OUT_A = 1, ACT_OUT_B = 2, ACT_OUT_DONE = 3,
-  ACT_P1 = 4,  // BiCGStab: finish the previous step, y = K^-1 p, v = A y
-  ACT_P2 = 5,  // BiCGStab: e += alpha y, s = r - alpha v, t = A K^-1 s
-  ACT_BF = 6,  // BiCGStab: e += omega K^-1 s before a reliable update
-  ACT_C0 = 7,  // CG: w = A u after a restart
-  ACT_C1 = 8   // CG: one iteration in one phase (single reduction)
+  ACT_NONE = 0,
+  ACT_OUT_A = 1,   // FP64 residual
+  ACT_FINISH = 2,  // x += e
+  ACT_P1 = 3,      // BiCGStab: finish the previous step, y = K^-1 p, v = A y
+  ACT_P2 = 4,      // BiCGStab: e += alpha y, s = r - alpha v, t = A K^-1 s
+  ACT_C0 = 5,      // CG: restart, w = A u
+  ACT_C1 = 6       // CG: one iteration in one phase (single reduction)
 };
-// partial sums per tile: CG uses 3, BiCGStab 5 (and the FP64 residual
-// phase |r|^2 and |b|^2)
+// partial sums per block and system: CG uses 3, BiCGStab 5 (and the FP64
+// residual phase |r|^2 and |b|^2)
 constexpr int kMaxSums = 5;
 
-constexpr int kMaxBlockTiles = 64;
+// What a block keeps in shared memory (template parameter SM, the most that
+// fits; every phase start's GPU-scope acquire invalidates L1, so what is read
+// from global memory costs an L2 round trip per phase). Known at compile time:
+// generic pointers made the solves 15-20% slower.
+//   1  the own rows of the vectors that no product gathers, the slices' pointers
+//   2  and the SELL columns
+//   3  and the SELL values of every component (once where they share a matrix)
 
-// categories of per-block static data copied into shared memory at kernel
-// start (every phase start's GPU-scope acquire invalidates L1, so static
-// indices read from global memory would cost an L2 round trip per phase)
-enum {
-  ST_L0META = 1,  // slice pointers / lengths of the block's slice range
-  ST_L0COL = 2    // SELL columns of that range
-};
+// the gathered vectors of a row: BiCGStab zr = K^-1 r, w = K^-1 v, y, kt =
+// K^-1 t; CG u = K^-1 r, wh = K^-1 w, sh = K^-1 s
+template <typename R> struct V4;
+template <> struct __align__(16) V4<float> { float a, b, c, d; };
+template <> struct __align__(32) V4<double> { double a, b, c, d; };
+
+__device__ __forceinline__ V4<float> ld4(const V4<float>* p) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  return V4<float>{v.x, v.y, v.z, v.w};
+}
+__device__ __forceinline__ V4<double> ld4(const V4<double>* p) {
+  const double2 v = reinterpret_cast<const double2*>(p)[0], w = reinterpret_cast<const double2*>(p)[1];
+  return V4<double>{v.x, v.y, w.x, w.y};
+}
+__device__ __forceinline__ void ld2(const V4<float>* p, float& a, float& b) {
+  const float2 v = *reinterpret_cast<const float2*>(p);
+  a = v.x;
+  b = v.y;
+}
+__device__ __forceinline__ void ld2(const V4<double>* p, double& a, double& b) {
+  const double2 v = *reinterpret_cast<const double2*>(p);
+  a = v.x;
+  b = v.y;
+}
 
 template <typename R> struct SolveArgs {
-  int ncomp, ninst, nsys, ntiles, nv;
-  const Tile* tiles;
-  const int* sys_slot0;   // [nsys+1] first partial slot of each system
-  const int* sys_owner;   // [nsys] block that reports the system's result
-  const int* blk_t0;      // [grid+1] first tile of each block
-  const int* blk_sys;     // systems of each block, at blk_sys_off[b]
-  const int* blk_sys_off;
-  const int* blk_sl;      // [2 grid] slice range [s0, s1) of each block's tiles
-  const int* sl_ptr;
-  const int* sl_len;
-  const int* sl_col;
+  int ncomp, ninst, nv;
+  const int *blk_inst, *blk_inst_off;  // instances of each block, at blk_inst_off[b]
+  const int *blk_slot;                 // per blk_inst entry: the block's partial slot (component 0)
+  const int *sys_slot0;                // [nsys+1] partial slots of each system
+  const int *blk_sl;                   // [grid+1] first slice
+  const int *slk;                      // [nslices] local instance of each slice (in its block)
+  const int *sl_ptr, *sl_len, *sl_col;
   const double* A64[3];
   const R* Ain[3];
   const R* dinv[3];
-  int stage;              // ST_* categories staged in shared memory
-  int ntl_max, items_max; // per block: tiles, (tile, slice) work items
+  int share;              // the components share one matrix
+  int items_max;
   double* x[3];
   const double* b[3];
   const unsigned char* isd[3];
@@ -85,21 +120,15 @@ template <typename R> struct SolveArgs {
   const double* tol_i;   // per instance
   const double* rtol_i;  // per instance: stop at max(tol, rtol |b|)
   const int* maxit_i;    // per instance
-  int nsum;              // partial sums per tile (3, or kMaxSums for BiCGStab)
   int bicg;              // BiCGStab instead of CG
-  // BiCGStab vectors (nv entries per component slot): zr = K^-1 r, y and
-  // w = K^-1 v double buffered (parity L.par; y in p), the shadow residual
-  // rh, s, t and kt = K^-1 t; v in q, r in r's first buffer
-  R *bz, *bw, *rh, *bs, *bt, *bkt;
-  // CG with one reduction per iteration: u = D^-1 r, wh = D^-1 w and
-  // sh = D^-1 s double buffered (parity L.par), w = A u and s = A p on the
-  // own rows only; p in p's first buffer, r in r's first buffer
-  R *cu, *cwh, *csh, *cw, *cs;
-  // workspace per component slot, nv entries each; r and p: 2 buffers
-  R *e, *r, *p, *q;
+  V4<R>* pk;             // [2 parities][ncomp][nv]
+  // own rows only, [ncomp][nv]: BiCGStab shadow residual, s, t, v; CG w, s, p
+  R *rh, *s, *t, *v;
+  R *e, *r;
   double* r64;
-  double* part;          // [2 parities][2 sums][ntiles slots]
-  unsigned* scount;      // [nsys][32]: per-system count of tile phases published (one 128-byte line each, zeroed per launch)
+  double* part;          // [2 parities][kMaxSums][nslots]
+  int nslots;
+  unsigned* scount;      // [nsys][32]: per-system count of block phases published (one 128-byte line each, zeroed per launch)
   int* active;
   int* out_it;           // [nsys] iterations
   double* out_res;       // [nsys] final residual norm
@@ -111,115 +140,218 @@ template <typename R> struct SolveArgs {
 };
 
 struct LocalSys {
-  int sys, state, it, outer, par, first, owner, maxit, act, chk;
-  int t0, t1;                       // partial slots of the system
-  double tol, rtol, intol, res, rz_prev, alpha, beta;
-  double omega;                     // BiCGStab (rz_prev holds rho = (rh, r))
+  int sys, state, act, it, outer, par, first, pend, maxit, slot;
+  int s0, s1;                       // partial slots of the system
+  double tol, rtol, intol, res, rz_prev, alpha, beta, omega, irv;
   double sum[kMaxSums];
 };
 
-template <typename R, int MINB>
-__global__ void __launch_bounds__(kSolveThreads, MINB) k_krylov(SolveArgs<R> a) {
+// sum of a partial array over the slots [t0, t1) by one warp, in a fixed order
+__device__ __forceinline__ double slot_sum(const double* part, int t0, int t1, int lane) {
+  double s = 0.0;
+  for (int tb = t0; tb < t1; tb += 320) {
+    double v[10];
+#pragma unroll
+    for (int u = 0; u < 10; ++u) {
+      const int t = tb + u * 32 + lane;
+      v[u] = t < t1 ? __ldcg(part + t) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 10; ++u) s += v[u];
+  }
+  return warp_sum(s);
+}
+
+// partial sums that a step needs from its system's previous phase
+__device__ __forceinline__ int sums_of(int state) {
+  return state == S_A ? 5 : state == S_C1 ? 3 : state == S_OUT_B ? 2 : state == S_B ? 1 : 0;
+}
+
+// the next step of a system from the sums of its previous phase (one thread;
+// identical in every block of the system)
+__device__ __forceinline__ void decide(LocalSys& L, bool bicg, double eta) {
+  const double* s = L.sum;
+  switch (L.state) {
+    case S_OUT_A:
+      L.act = ACT_OUT_A;
+      L.state = S_OUT_B;
+      break;
+    case S_OUT_B:
+      L.res = sqrt(s[0]);
+      // the first FP64 residual also summed |b|^2: the relative tolerance
+      if (L.outer == 0) L.tol = fmax(L.tol, L.rtol * sqrt(s[1]));
+      L.outer += 1;
+      if (L.res <= L.tol || L.it >= L.maxit || (bicg && L.outer > L.maxit) || !(L.res == L.res)) {
+        L.act = ACT_FINISH;
+        L.state = S_DONE;
+      } else {
+        L.intol = fmax(eta * L.res, 0.5 * L.tol);
+        L.first = 1;
+        L.beta = 0.0;
+        L.rz_prev = L.res * L.res;  // BiCGStab: rho = (rh, r) with rh = r
+        L.act = bicg ? ACT_P1 : ACT_C0;
+        L.state = bicg ? S_B : S_C1;
+      }
+      break;
+    case S_A: {
+      // BiCGStab after P2: (t,s), (t,t), (rh,s), (rh,t), (s,s)
+      // (one division deep: beta = (rho / rho_prev) (alpha / omega) with
+      // alpha / rho_prev = 1 / (rh, v))
+      const double om = s[1] > 0.0 ? s[0] / s[1] : 0.0, iom = s[1] / s[0];
+      const double rr = s[4] - 2.0 * om * s[0] + om * om * s[1];  // |s - omega t|^2
+      const double rho = s[2] - om * s[3];
+      L.omega = om;
+      L.it += 1;
+      if (!(om != 0.0) || !(rho != 0.0) || rr <= L.intol * L.intol || L.it >= L.maxit || !(rr == rr)) {
+        L.pend = 1;  // x += omega K^-1 s is folded into the FP64 residual
+        L.act = ACT_OUT_A;
+        L.state = S_OUT_B;
+      } else {
+        L.beta = rho * L.irv * iom;
+        L.rz_prev = rho;
+        L.act = ACT_P1;
+        L.state = S_B;
+      }
+      break;
+    }
+    case S_B: {
+      const double rv = s[0];  // (rh, v)
+      L.first = 0;
+      L.pend = 0;
+      if (!(rv != 0.0) || !(rv == rv)) {
+        L.act = ACT_OUT_A;  // breakdown: restart from the FP64 residual
+        L.state = S_OUT_B;
+      } else {
+        L.irv = 1.0 / rv;
+        L.alpha = L.rz_prev / rv;
+        L.act = ACT_P2;
+        L.state = S_A;
+      }
+      break;
+    }
+    case S_C1: {
+      // CG: (r, u), (w, u), (r, r) of the previous phase; beta = gamma /
+      // gamma_old, alpha = gamma / (delta - beta gamma / alpha_old)
+      const double g = s[0], dl = s[1], rr = s[2];
+      if (L.first == 1) {
+        L.first = 2;
+        L.alpha = dl != 0.0 ? g / dl : 0.0;
+        L.beta = 0.0;
+        L.rz_prev = g;
+        L.act = ACT_C1;
+      } else {
+        L.first = 0;
+        L.it += 1;
+        const double be = L.rz_prev != 0.0 ? g / L.rz_prev : 0.0;
+        const double den = dl - (L.alpha != 0.0 ? be * g / L.alpha : 0.0);
+        if (rr <= L.intol * L.intol || L.it >= L.maxit || !(rr == rr) || !(den > 0.0)) {
+          L.act = ACT_OUT_A;  // reliable update in FP64
+          L.state = S_OUT_B;
+        } else {
+          L.beta = be;
+          L.alpha = g / den;
+          L.rz_prev = g;
+          L.act = ACT_C1;
+        }
+      }
+      break;
+    }
+    default:
+      L.act = ACT_NONE;
+      break;
+  }
+}
+
+template <typename R, int MINB, int SM>
+__global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(SolveArgs<R> a) {
+  constexpr int kSolveThreads = SolveThreads<MINB>::value, kWarps = kSolveThreads / 32;
   extern __shared__ __align__(16) unsigned char dyn_smem[];
-  // entries of a SELL row (and of a long restriction row) whose loads are
-  // issued together: more with one block per SM, which has the registers;
-  // with two, nine: a Q1 row of 9 entries (2D) in one round of loads and one
-  // of 27 (3D) in three (eight took two and four: channel velocity solves
-  // 0.64 -> 0.61 ms, pipe 31.0 -> 26.9 ms per step)
-  constexpr int CH = MINB == 1 ? 16 : 9;
-  constexpr int NSMAX = kMaxSums;
-  const int NS = a.nsum;
+  // entries of a SELL row whose loads are issued together: a Q1 row of 9 (2D)
+  // in one round, one of 27 (3D) in three; with FP64 the registers hold five
+  constexpr int CH = sizeof(R) == 8 ? 5 : 9;
   __shared__ LocalSys ls[kMaxLocalSys];
-  __shared__ Tile stile[kMaxBlockTiles];
-  __shared__ int s_nls;
+  __shared__ int s_err;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t nv = (size_t)a.nv;
-  const int t_lo = a.blk_t0[blockIdx.x], t_hi = a.blk_t0[blockIdx.x + 1];
-  const int ntl = t_hi - t_lo;
-  const bool tiles_staged = ntl <= kMaxBlockTiles;
+  const int NC = a.ncomp;
+  const int io = a.blk_inst_off[blockIdx.x];
+  const int nls = min((a.blk_inst_off[blockIdx.x + 1] - io) * NC, kMaxLocalSys);
+  const int bs0 = a.blk_sl[blockIdx.x], bs1 = a.blk_sl[blockIdx.x + 1];
+  const int nitems = (bs1 - bs0) * NC, own0 = bs0 * 32;
+  const int NS = a.bicg ? kMaxSums : 3;
   unsigned bar_gen = 0;
 
-  // ---- local systems of this block
-  if (threadIdx.x == 0) {
-    const int o = a.blk_sys_off[blockIdx.x];
-    int n = a.blk_sys_off[blockIdx.x + 1] - o;
-    if (n > kMaxLocalSys) n = kMaxLocalSys;  // the host guarantees n <= kMaxLocalSys
-    s_nls = n;
-    for (int k = 0; k < n; ++k) {
-      LocalSys& L = ls[k];
-      const int s = a.blk_sys[o + k], inst = s % a.ninst;
-      L.sys = s;
-      L.state = S_OUT_A;
-      L.it = L.outer = L.par = L.chk = 0;
-      L.first = 1;
-      L.owner = a.sys_owner[s] == (int)blockIdx.x;
-      L.t0 = a.sys_slot0[s];
-      L.t1 = a.sys_slot0[s + 1];
-      L.maxit = a.maxit_i[inst];
-      L.tol = a.tol_i[inst];
-      L.rtol = a.rtol_i[inst];
-      L.intol = 0.5 * L.tol;
-      L.res = L.rz_prev = L.alpha = L.beta = L.omega = 0.0;
-      for (int q = 0; q < kMaxSums; ++q) L.sum[q] = 0.0;
-      L.act = ACT_NONE;
-    }
-  }
-  if (tiles_staged)
-    for (int i = threadIdx.x; i < ntl; i += kSolveThreads) stile[i] = a.tiles[t_lo + i];
-  __syncthreads();
-  const int nls = s_nls;
-  auto tile_at = [&](int t) -> Tile { return tiles_staged ? stile[t - t_lo] : a.tiles[t]; };
-
-  // ---- level-0 work items: (tile, slice) pairs in tile order; item0[t] is
-  // the first item of local tile t. Every item's partial sums go to spart,
-  // then each tile sums its items in order (deterministic).
+  // ---- shared memory: the items' partial sums, then the staged static data
   double* spart = reinterpret_cast<double*>(dyn_smem);
-  int* item0 = reinterpret_cast<int*>(dyn_smem + al16_dev((size_t)a.items_max * NS * sizeof(double)));
-  if (threadIdx.x == 0) {
-    int n = 0;
-    for (int t = 0; t < ntl; ++t) {
-      item0[t] = n;
-      const Tile T = tile_at(t_lo + t);
-      n += T.s1 - T.s0;
-    }
-    item0[ntl] = n;
+  unsigned char* cur = dyn_smem + al16_dev((size_t)a.items_max * NS * sizeof(double));
+  // own rows of the vectors that no product gathers: by item in shared memory
+  R *ve, *vr, *vs, *vt, *vv, *vh;
+  const int *SLp, *SLl, *SLk, *SLc;  // by slice - bs0; columns by entry - e0
+  const R *A0, *A1, *A2;
+  const int e0 = a.sl_ptr[bs0], ne = a.sl_ptr[bs1] - e0;
+  if constexpr (SM >= 1) {
+    const int n = a.items_max * 32;
+    ve = reinterpret_cast<R*>(cur);
+    vr = ve + n;
+    vs = ve + 2 * n;
+    vt = ve + 3 * n;
+    vv = ve + 4 * n;
+    vh = ve + 5 * n;
+    cur += al16_dev((size_t)6 * n * sizeof(R));
+    SLp = stage_copy(cur, a.sl_ptr + bs0, bs1 - bs0);
+    SLl = stage_copy(cur, a.sl_len + bs0, bs1 - bs0);
+    SLk = stage_copy(cur, a.slk + bs0, bs1 - bs0);
+  } else {
+    ve = a.e;
+    vr = a.r;
+    vs = a.s;
+    vt = a.t;
+    vv = a.v;
+    vh = a.rh;
+    SLp = a.sl_ptr + bs0;
+    SLl = a.sl_len + bs0;
+    SLk = a.slk + bs0;
   }
-  __syncthreads();
-  const int nitems = item0[ntl];
-  // local tile of item `it` (binary search; tiles are few)
-  auto item_tile = [&](int it) -> int {
-    int lo = 0, hi = ntl - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (item0[mid] <= it) lo = mid;
-      else hi = mid - 1;
-    }
-    return lo;
-  };
-  unsigned char* dyn_rest =
-      dyn_smem + al16_dev((size_t)a.items_max * NS * sizeof(double)) + al16_dev((size_t)(a.ntl_max + 1) * sizeof(int));
+  if constexpr (SM >= 2) SLc = stage_copy(cur, a.sl_col + e0, ne);
+  else SLc = a.sl_col + e0;
+  if constexpr (SM >= 3) {
+    A0 = stage_copy(cur, a.Ain[0] + e0, ne);
+    A1 = a.share || NC < 2 ? A0 : stage_copy(cur, a.Ain[1] + e0, ne);
+    A2 = a.share || NC < 3 ? A0 : stage_copy(cur, a.Ain[2] + e0, ne);
+  } else {
+    A0 = a.Ain[0] + e0;
+    A1 = a.Ain[1] + e0;
+    A2 = a.Ain[2] + e0;
+  }
 
-  // ---- shared memory: the staged static data
-  unsigned char* cur = dyn_rest;
-  const int bs0 = a.blk_sl[2 * blockIdx.x], bs1 = a.blk_sl[2 * blockIdx.x + 1];
-  const SV<int> SLp = maybe_stage<int>(a.stage & ST_L0META, cur, a.sl_ptr, bs0, bs1 + 1);
-  const SV<int> SLl = maybe_stage<int>(a.stage & ST_L0META, cur, a.sl_len, bs0, bs1);
-  const SV<int> SLc = maybe_stage<int>(a.stage & ST_L0COL, cur, a.sl_col, a.sl_ptr[bs0], a.sl_ptr[bs1]);
-  // ---- init: Dirichlet values preset in x, e = 0, p = 0
-  for (int it = warp; it < nitems; it += kWarps) {
-    const int tl = item_tile(it);
-    const Tile T = tile_at(t_lo + tl);
-    const int k = T.comp;
-    {
-      const int sl = T.s0 + (it - item0[tl]);
-      const int row = sl * 32 + lane;
+  // ---- local systems: component k of local instance i is system i NC + k
+  if (threadIdx.x == 0) s_err = 0;
+  for (int l = threadIdx.x; l < nls; l += kSolveThreads) {
+    LocalSys& L = ls[l];
+    const int inst = a.blk_inst[io + l / NC], s = (l % NC) * a.ninst + inst;
+    L.sys = s;
+    L.state = S_OUT_A;
+    L.act = ACT_NONE;
+    L.it = L.outer = L.par = L.pend = 0;
+    L.first = 1;
+    L.s0 = a.sys_slot0[s];
+    L.s1 = a.sys_slot0[s + 1];
+    L.slot = L.s0 + a.blk_slot[io + l / NC];
+    L.maxit = a.maxit_i[inst];
+    L.tol = a.tol_i[inst];
+    L.rtol = a.rtol_i[inst];
+    L.intol = 0.5 * L.tol;
+    L.res = L.rz_prev = L.alpha = L.beta = L.omega = L.irv = 0.0;
+  }
+  // ---- init: Dirichlet values preset in x, e = 0
+  for (int k = 0; k < NC; ++k)
+    for (int i = threadIdx.x; i < (bs1 - bs0) * 32; i += kSolveThreads) {
+      const int row = own0 + i;
       if (a.isd[k][row]) a.x[k][row] = a.g[k] ? a.g[k][row] : 0.0;
       a.e[k * nv + row] = R(0);
-      a.p[(2 * k) * nv + row] = R(0);
-      a.p[(2 * k + 1) * nv + row] = R(0);
     }
-  }
-  __shared__ int s_stop;
+  if (SM >= 1)
+    for (int i = threadIdx.x; i < nitems * 32; i += kSolveThreads) ve[i] = R(0);
   if (!grid_sync_ra(a.gb, bar_gen)) return;
 
   for (int iter = 0;; ++iter) {
@@ -227,405 +359,234 @@ __global__ void __launch_bounds__(kSolveThreads, MINB) k_krylov(SolveArgs<R> a) 
       if (threadIdx.x == 0) atomicCAS(a.gb.err, 0, 2);
       break;
     }
-    const double* prev = a.part + (size_t)((iter + 1) & 1) * a.ntiles * NS;
-    // ---- wait for the previous phase of the block's running systems: every
-    // tile adds 1 to its system's counter with a release add once its phase
-    // is written, so iter x (tiles of the system) means that every tile of
-    // the system has finished phase iter - 1; lane k of warp 0 polls local
-    // system k, then an acquire fence (and the block barrier) orders
-    // everything those blocks wrote before this phase's reads. Blocks of
-    // other systems are not waited for.
-    if (warp == 0) {
-      bool stop = true;
-      for (int k = 0; k < nls; ++k) stop &= ls[k].state == S_DONE;
-      if (!stop && iter > 0) {
-        const bool mine = lane < nls && ls[lane].state != S_DONE;
-        const unsigned target = mine ? (unsigned)iter * (unsigned)(ls[lane].t1 - ls[lane].t0) : 0u;
-        const unsigned* cnt = a.scount + (size_t)(mine ? ls[lane].sys : 0) * 32;
-        unsigned spins = 0;
-        for (;;) {
-          const bool ok = !mine || (int)(ld_relaxed_u32(cnt) - target) >= 0;
-          if (__all_sync(PFEM2_FULL_MASK, ok)) {
-            fence_acq_rel_gpu();
-            break;
-          }
-          if (__any_sync(PFEM2_FULL_MASK, ++spins > a.gb.spin_limit || *(volatile int*)a.gb.err != 0)) {
-            if (lane == 0) atomicCAS(a.gb.err, 0, 1);
-            stop = true;
-            break;
-          }
-          __nanosleep(20);
+    // ---- phase start: every block of a system adds 1 to its counter once
+    // its phase is written, so iter x (blocks of the system) means that all
+    // have finished phase iter - 1; the acquire orders what they wrote before
+    // this phase's reads. A warp per (local system, sum) waits and sums that
+    // phase's partials, then a thread per system takes the next step.
+    const double* prev = a.part + (size_t)((iter + 1) & 1) * kMaxSums * a.nslots;
+    for (int t = warp; t < nls * kMaxSums; t += kWarps) {
+      // (the first sums of all systems first)
+      const int q = t / nls, l = t - q * nls;
+      const LocalSys& L = ls[l];
+      if (L.state == S_DONE || iter == 0 || (q > 0 && q >= sums_of(L.state))) continue;
+      if (!wait_count(a.scount + (size_t)L.sys * 32, (unsigned)iter * (unsigned)(L.s1 - L.s0), a.gb)) {
+        if (lane == 0) {
+          atomicCAS(a.gb.err, 0, 1);
+          s_err = 1;
         }
+        break;
       }
-      if (lane == 0) s_stop = stop;
-    }
-    __syncthreads();
-    if (s_stop) break;
-    // the sums of the previous phase's partials: warp q sums partial q of
-    // every local system over its tiles in a fixed order (lane l adds tiles
-    // l, l + 32, ..., then the warp sum), all sums in one round of loads
-    if (warp < NS) {
-      const int q = warp;
-      for (int k = 0; k < nls; ++k) {
-        const int st = ls[k].state;
-        if (st == S_DONE || st == S_OUT_A) continue;
-        const int t0 = ls[k].t0, t1 = ls[k].t1;
-        const double* pq = prev + (size_t)q * a.ntiles;
-        double sq = 0.0;
-        for (int tb = t0; tb < t1; tb += 256) {
-          double v[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int t = tb + u * 32 + lane;
-            v[u] = t < t1 ? __ldcg(pq + t) : 0.0;
-          }
-#pragma unroll
-          for (int u = 0; u < 8; ++u) sq += v[u];
-        }
-        sq = warp_sum(sq);
-        if (lane == 0) ls[k].sum[q] = sq;
+      if (q < sums_of(L.state)) {
+        const double s = slot_sum(prev + (size_t)q * a.nslots, L.s0, L.s1, lane);
+        if (lane == 0) ls[l].sum[q] = s;
       }
     }
     __syncthreads();
-    // ---- decisions (thread 0; identical in every block owning the system)
-    if (threadIdx.x == 0) {
-      for (int k = 0; k < nls; ++k) {
-        LocalSys& L = ls[k];
-        int act = ACT_NONE;
-        // the first FP64 residual phase also summed |b|^2: the relative tolerance
-        if (L.state == S_OUT_B && L.outer == 0) L.tol = fmax(L.tol, L.rtol * sqrt(L.sum[1]));
-        if (a.bicg) {
-          // BiCGStab with the Jacobi preconditioner K (right-preconditioned,
-          // van der Vorst 1992) over the phases OUT_A (FP64 residual),
-          // OUT_B (restart: r = rh = r64, zr = K^-1 r), then P1 / P2 per
-          // iteration; BF completes the iterate before a reliable update
-          switch (L.state) {
-            case S_OUT_A:
-              act = ACT_OUT_A;
-              L.state = S_OUT_B;
-              break;
-            case S_OUT_B:
-              L.res = sqrt(L.sum[0]);
-              L.outer += 1;
-              if (L.res <= L.tol || L.it >= L.maxit || L.outer > L.maxit || !(L.res == L.res)) {
-                act = ACT_OUT_DONE;
-                L.state = S_DONE;
-              } else {
-                L.intol = fmax(a.eta * L.res, 0.5 * L.tol);
-                L.first = 1;
-                L.rz_prev = L.res * L.res;  // rho = (rh, r) with rh = r
-                act = ACT_OUT_B;
-                L.state = S_A;
-              }
-              break;
-            case S_A:
-              if (L.first) {
-                L.beta = 0.0;
-                act = ACT_P1;
-                L.state = S_B;
-              } else {
-                // sums of P2: (t,s), (t,t), (rh,s), (rh,t), (s,s)
-                const double ts = L.sum[0], tt = L.sum[1], rs = L.sum[2], rt = L.sum[3], ss = L.sum[4];
-                const double om = tt > 0.0 ? ts / tt : 0.0;
-                const double rr = sqrt(fmax(ss - 2.0 * om * ts + om * om * tt, 0.0));
-                const double rho = rs - om * rt;
-                L.omega = om;
-                L.it += 1;
-                if (!(om != 0.0) || !(rho != 0.0) || rr <= L.intol || L.it >= L.maxit || !(rr == rr)) {
-                  act = ACT_BF;  // x += omega K^-1 s, then a reliable update
-                  L.state = S_OUT_A;
-                } else {
-                  L.beta = (rho / L.rz_prev) * (L.alpha / om);
-                  L.rz_prev = rho;
-                  act = ACT_P1;
-                  L.state = S_B;
-                }
-              }
-              break;
-            case S_B: {
-              const double rv = L.sum[0];  // (rh, v)
-              L.first = 0;
-              if (!(rv != 0.0) || !(rv == rv)) {
-                act = ACT_OUT_A;  // breakdown: restart from the FP64 residual
-                L.state = S_OUT_B;
-              } else {
-                L.alpha = L.rz_prev / rv;
-                act = ACT_P2;
-                L.state = S_A;
-              }
-              break;
-            }
-            default:
-              break;
-          }
-        } else {
-          // CG with one reduction per iteration (Chronopoulos and
-          // Gear 1989): u = D^-1 r, w = A u, gamma = (r, u), delta = (w, u);
-          // beta = gamma / gamma_old, alpha = gamma / (delta - beta gamma /
-          // alpha_old); p = u + beta p, s = w + beta s (= A p), x += alpha p,
-          // r -= alpha s. One phase per iteration (C1), the w = A u of a
-          // restart in a phase of its own (C0).
-          switch (L.state) {
-            case S_OUT_A:
-              act = ACT_OUT_A;
-              L.state = S_OUT_B;
-              break;
-            case S_OUT_B:
-              L.res = sqrt(L.sum[0]);
-              L.outer += 1;
-              if (L.res <= L.tol || L.it >= L.maxit || !(L.res == L.res)) {
-                act = ACT_OUT_DONE;
-                L.state = S_DONE;
-              } else {
-                L.intol = fmax(a.eta * L.res, 0.5 * L.tol);
-                L.chk = 0;
-                act = ACT_OUT_B;
-                L.state = S_C0;
-              }
-              break;
-            case S_C0:
-              act = ACT_C0;
-              L.state = S_C1;
-              break;
-            case S_C1: {
-              // sums of the previous phase: (r, u), (w, u), (r, r)
-              const double g = L.sum[0], dl = L.sum[1], rr = sqrt(L.sum[2]);
-              if (!L.chk) {
-                L.alpha = dl != 0.0 ? g / dl : 0.0;
-                L.beta = 0.0;
-                L.rz_prev = g;
-                act = ACT_C1;
-              } else {
-                L.it += 1;
-                const double be = L.rz_prev != 0.0 ? g / L.rz_prev : 0.0;
-                const double den = dl - (L.alpha != 0.0 ? be * g / L.alpha : 0.0);
-                if (rr <= L.intol || L.it >= L.maxit || !(rr == rr) || !(den > 0.0)) {
-                  act = ACT_OUT_A;  // reliable update in FP64
-                  L.state = S_OUT_B;
-                } else {
-                  L.beta = be;
-                  L.alpha = g / den;
-                  L.rz_prev = g;
-                  act = ACT_C1;
-                }
-              }
-              break;
-            }
-            default:
-              break;
-          }
-        }
-        L.act = act;
-      }
-    }
+    if (threadIdx.x < nls) decide(ls[threadIdx.x], a.bicg != 0, a.eta);
     __syncthreads();
-    // ---- level-0 work on the own (tile, slice) items, a warp per item
+    if (s_err) break;
+    bool any = false;
+    for (int l = 0; l < nls; ++l) any |= ls[l].act != ACT_NONE;
+    if (!any) break;  // every local system is done
+    // ---- the block's (slice, component) items, a warp per item
     for (int it = warp; it < nitems; it += kWarps) {
-      const int tl = item_tile(it);
-      const Tile T = tile_at(t_lo + tl);
-      const int sl = T.s0 + (it - item0[tl]);
-      const int k = T.comp;
-      const LocalSys& L = ls[T.lk];
+      const int sl = bs0 + it / NC, k = it % NC;
+      const LocalSys& L = ls[SLk[sl - bs0] * NC + k];
       const int act = L.act;
       if (act == ACT_NONE) continue;
       double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0, v4 = 0.0;
+      const int row = sl * 32 + lane;
+      const size_t g0 = k * nv + row, o = SM >= 1 ? (size_t)(it * 32 + lane) : g0;
+      const int p0 = SLp[sl - bs0] - e0, len = SLl[sl - bs0];
       const R* dinv = a.dinv[k];
-      R* e = a.e + k * nv;
-      R* r = a.r + (2 * k) * nv;
-      R* q = a.q + k * nv;
-      double* r64 = a.r64 + k * nv;
+      const R* A = k == 0 ? A0 : (k == 1 ? A1 : A2);
+      const auto aval = [&](int ei) { return A[ei]; };
+      const double* r64 = a.r64 + k * nv;
+      const V4<R>* pk = a.pk + (size_t)(L.par * NC + k) * nv;
+      V4<R>* pn = a.pk + (size_t)((L.par ^ 1) * NC + k) * nv;
       if (act == ACT_OUT_A) {
-        const double* A = a.A64[k];
+        const double* A64 = a.A64[k] + e0;
         const double* xk = a.x[k];
-        {
-          const int row = sl * 32 + lane;
-          const double acc = sell_dot<double, CH>(
-              0.0, SLc, SLp[sl], SLl[sl], lane, [&](int ei) { return A[ei]; },
-              [&](int col) { return __ldcg(xk + col) + (double)__ldcg(e + col); });
-          const double bb = a.b[k][row];
-          const double rr = bb - acc;
-          r64[row] = rr;
-          v0 += rr * rr;
-          v1 += bb * bb;
-        }
-      } else if (act == ACT_OUT_B || act == ACT_OUT_DONE) {
-        {
-          const int row = sl * 32 + lane;
-          a.x[k][row] += (double)e[row];
-          e[row] = R(0);
-          if (act == ACT_OUT_B) {
-            const R rr = R(r64[row]);
-            r[row] = rr;
-            if (a.bicg) {
-              a.rh[k * nv + row] = rr;
-              a.bz[(2 * k + L.par) * nv + row] = rr * dinv[row];
-            } else {
-              a.cu[(2 * k + L.par) * nv + row] = rr * dinv[row];
-            }
+        const R* e = a.e + k * nv;
+        const bool pend = L.pend != 0;
+        const R al = R(L.alpha), om = R(L.omega);
+        const double bb = a.b[k][row];
+        const double acc = sell_dot<double, CH>(0.0, SLc, p0, len, lane, [&](int ei) { return A64[ei]; }, [&](int j) {
+          R ee = __ldcg(e + j);
+          if (pend) {
+            R zr, w;
+            ld2(pk + j, zr, w);
+            ee = fma_r(om, fma_r(-al, w, zr), ee);  // the last step's omega K^-1 s
           }
+          return __ldcg(xk + j) + (double)ee;
+        });
+        const double rr = bb - acc;
+        a.r64[g0] = rr;
+        v0 = rr * rr;
+        v1 = bb * bb;
+      } else if (act == ACT_FINISH) {
+        R ee = ve[o];
+        if (L.pend) {
+          R zr, w;
+          ld2(pk + row, zr, w);
+          ee = fma_r(R(L.omega), fma_r(-R(L.alpha), w, zr), ee);
         }
-      } else if (act == ACT_C0) {
-        // w = A u, wh = D^-1 w after a restart; (r, u), (w, u), (r, r)
-        const int row = sl * 32 + lane;
-        const R* u = a.cu + (2 * k + L.par) * nv;
-        const R* A = a.Ain[k];
-        const R w = sell_dot<R, CH>(R(0), SLc, SLp[sl], SLl[sl], lane, [&](int ei) { return A[ei]; },
-                                    [&](int j) { return u[j]; });
-        a.cw[k * nv + row] = w;
-        a.cwh[(2 * k + L.par) * nv + row] = w * dinv[row];
-        const double rr = (double)r[row], uu = (double)u[row];
-        v0 += rr * uu;
-        v1 += (double)w * uu;
-        v2 += rr * rr;
-      } else if (act == ACT_C1) {
-        // p = u + beta p, s = w + beta s, sh = wh + beta sh, e += alpha p,
-        // r -= alpha s, u' = u - alpha sh (= D^-1 r'), w' = A u' with u'
-        // formed on the fly at the columns from u, wh and the old sh, wh' =
-        // D^-1 w'; (r', u'), (w', u'), (r', r'). The first iteration after a
-        // restart has p = u, s = w, sh = wh.
-        const int row = sl * 32 + lane;
-        const bool first = L.chk == 0;
-        const R al = R(L.alpha), be = R(L.beta);
-        const R* uo = a.cu + (2 * k + L.par) * nv;
-        const R* who = a.cwh + (2 * k + L.par) * nv;
-        const R* sho = a.csh + (2 * k + L.par) * nv;
-        const auto unew = [&](int j) -> R {
-          const R sh = first ? who[j] : fma_r(be, sho[j], who[j]);
-          return fma_r(-al, sh, uo[j]);
-        };
-        R* pk = a.p + (2 * k) * nv;
-        R* sk = a.cs + k * nv;
-        const R sh = first ? who[row] : fma_r(be, sho[row], who[row]);
-        const R pp = first ? uo[row] : fma_r(be, pk[row], uo[row]);
-        const R ss = first ? a.cw[k * nv + row] : fma_r(be, sk[row], a.cw[k * nv + row]);
-        pk[row] = pp;
-        sk[row] = ss;
-        e[row] = fma_r(al, pp, e[row]);
-        const R rn = fma_r(-al, ss, r[row]);
-        r[row] = rn;
-        const R un = unew(row);
-        const R* A = a.Ain[k];
-        const R w = sell_dot<R, CH>(R(0), SLc, SLp[sl], SLl[sl], lane, [&](int ei) { return A[ei]; }, unew);
-        a.csh[(2 * k + (L.par ^ 1)) * nv + row] = sh;
-        a.cu[(2 * k + (L.par ^ 1)) * nv + row] = un;
-        a.cwh[(2 * k + (L.par ^ 1)) * nv + row] = w * dinv[row];
-        a.cw[k * nv + row] = w;
-        v0 += (double)rn * (double)un;
-        v1 += (double)w * (double)un;
-        v2 += (double)rn * (double)rn;
+        a.x[k][row] += (double)ee;
+        continue;
       } else if (act == ACT_P1) {
         // y' = zr' + beta (y - omega w), zr' = zr - alpha w - omega kt the
-        // preconditioned new residual (first step after a restart: y' = zr),
+        // preconditioned new residual (after a restart y' = zr' = K^-1 r64),
         // v = A y' with y' formed on the fly at the columns, w' = K^-1 v
-        const int row = sl * 32 + lane;
-        const bool first = L.first != 0;
-        const R al = R(L.alpha), om = R(L.omega), be = R(L.beta);
-        const R* zo = a.bz + (2 * k + L.par) * nv;
-        const R* wo = a.bw + (2 * k + L.par) * nv;
-        const R* yo = a.p + (2 * k + L.par) * nv;
-        const R* kt = a.bkt + k * nv;
-        const auto ynew = [&](int j) -> R {
-          if (first) return zo[j];
-          const R zr = fma_r(-om, kt[j], fma_r(-al, wo[j], zo[j]));
-          return fma_r(be, fma_r(-om, wo[j], yo[j]), zr);
-        };
-        R zr_row = zo[row];
-        if (!first) {
-          const R zs = fma_r(-al, wo[row], zo[row]);
-          e[row] = fma_r(om, zs, e[row]);
-          r[row] = fma_r(-om, a.bt[k * nv + row], a.bs[k * nv + row]);
-          zr_row = fma_r(-om, kt[row], zs);
+        // (own-row loads first: a warp issues in order, so that their round
+        // trip and the gathers' are one)
+        R yrow, zr_row, acc;
+        const R di = dinv[row];
+        const R e_old = ve[o];
+        if (L.first) {
+          const R rr = R(__ldcg(r64 + row));
+          const double xo = a.x[k][row];
+          R zr = R(0), w = R(0);
+          if (L.pend) ld2(pk + row, zr, w);
+          acc = sell_dot<R, CH>(R(0), SLc, p0, len, lane, aval, [&](int j) { return R(__ldcg(r64 + j)) * dinv[j]; });
+          const R ee = L.pend ? fma_r(R(L.omega), fma_r(-R(L.alpha), w, zr), e_old) : e_old;
+          a.x[k][row] = xo + (double)ee;
+          ve[o] = R(0);
+          if (SM >= 1) a.e[g0] = R(0);
+          vr[o] = rr;
+          vh[o] = rr;
+          yrow = zr_row = rr * di;
+          v0 = (double)rr * (double)acc;
+        } else {
+          const R al = R(L.alpha), om = R(L.omega), be = R(L.beta);
+          const auto ynew = [&](const V4<R>& g) {
+            const R zr = fma_r(-om, g.d, fma_r(-al, g.b, g.a));
+            return fma_r(be, fma_r(-om, g.b, g.c), zr);
+          };
+          const V4<R> g = ld4(pk + row);
+          const R t_old = vt[o], s_old = vs[o], rh = vh[o];
+          acc = sell_dot<R, CH>(R(0), SLc, p0, len, lane, aval, [&](int j) { return ynew(ld4(pk + j)); });
+          const R zs = fma_r(-al, g.b, g.a);
+          const R ee = fma_r(om, zs, e_old);
+          ve[o] = ee;
+          if (SM >= 1) a.e[g0] = ee;  // read by the FP64 residual at its columns
+          vr[o] = fma_r(-om, t_old, s_old);
+          zr_row = fma_r(-om, g.d, zs);
+          yrow = ynew(g);
+          v0 = (double)rh * (double)acc;
         }
-        const R yrow = ynew(row);
-        const R* A = a.Ain[k];
-        const R acc = sell_dot<R, CH>(R(0), SLc, SLp[sl], SLl[sl], lane, [&](int ei) { return A[ei]; }, ynew);
-        a.bz[(2 * k + (L.par ^ 1)) * nv + row] = zr_row;
-        a.p[(2 * k + (L.par ^ 1)) * nv + row] = yrow;
-        a.bw[(2 * k + (L.par ^ 1)) * nv + row] = acc * dinv[row];
-        q[row] = acc;
-        v0 += (double)a.rh[k * nv + row] * (double)acc;
+        pn[row] = V4<R>{zr_row, acc * di, yrow, R(0)};
+        vv[o] = acc;
       } else if (act == ACT_P2) {
         // e += alpha y, s = r - alpha v, t = A K^-1 s (K^-1 s = zr - alpha w
         // formed on the fly), kt = K^-1 t; sums (t,s) (t,t) (rh,s) (rh,t) (s,s)
-        const int row = sl * 32 + lane;
         const R al = R(L.alpha);
-        const R* zc = a.bz + (2 * k + L.par) * nv;
-        const R* wc = a.bw + (2 * k + L.par) * nv;
-        e[row] = fma_r(al, a.p[(2 * k + L.par) * nv + row], e[row]);
-        const R sv = fma_r(-al, q[row], r[row]);
-        const R* A = a.Ain[k];
-        const R tv = sell_dot<R, CH>(R(0), SLc, SLp[sl], SLl[sl], lane, [&](int ei) { return A[ei]; },
-                                     [&](int j) { return fma_r(-al, wc[j], zc[j]); });
-        a.bs[k * nv + row] = sv;
-        a.bt[k * nv + row] = tv;
-        a.bkt[k * nv + row] = tv * dinv[row];
-        const double rh = (double)a.rh[k * nv + row];
-        v0 += (double)tv * (double)sv;
-        v1 += (double)tv * (double)tv;
-        v2 += rh * (double)sv;
-        v3 += rh * (double)tv;
-        v4 += (double)sv * (double)sv;
-      } else if (act == ACT_BF) {
-        // the last step's x += omega K^-1 s (K^-1 s = zr - alpha w)
-        const int row = sl * 32 + lane;
-        const R zs = fma_r(-R(L.alpha), a.bw[(2 * k + L.par) * nv + row], a.bz[(2 * k + L.par) * nv + row]);
-        e[row] = fma_r(R(L.omega), zs, e[row]);
+        const R y = pk[row].c, e_old = ve[o], v_old = vv[o], r_old = vr[o], di = dinv[row];
+        const double rh = (double)vh[o];
+        const R tv = sell_dot<R, CH>(R(0), SLc, p0, len, lane, aval, [&](int j) {
+          R zr, w;
+          ld2(pk + j, zr, w);
+          return fma_r(-al, w, zr);
+        });
+        const R sv = fma_r(-al, v_old, r_old);
+        const R ee = fma_r(al, y, e_old);
+        ve[o] = ee;
+        if (SM >= 1) a.e[g0] = ee;
+        vs[o] = sv;
+        vt[o] = tv;
+        const_cast<V4<R>*>(pk)[row].d = tv * di;
+        v0 = (double)tv * (double)sv;
+        v1 = (double)tv * (double)tv;
+        v2 = rh * (double)sv;
+        v3 = rh * (double)tv;
+        v4 = (double)sv * (double)sv;
+      } else if (act == ACT_C0) {
+        // restart: u = K^-1 r64, w = A u, wh = K^-1 w; (r, u), (w, u), (r, r)
+        const R e_old = ve[o], rr = R(__ldcg(r64 + row)), di = dinv[row], u = rr * di;
+        const double xo = a.x[k][row];
+        const R w = sell_dot<R, CH>(R(0), SLc, p0, len, lane, aval, [&](int j) { return R(__ldcg(r64 + j)) * dinv[j]; });
+        a.x[k][row] = xo + (double)e_old;
+        ve[o] = R(0);
+        if (SM >= 1) a.e[g0] = R(0);
+        vr[o] = rr;
+        vv[o] = w;
+        pn[row] = V4<R>{u, w * di, R(0), R(0)};
+        v0 = (double)rr * (double)u;
+        v1 = (double)w * (double)u;
+        v2 = (double)rr * (double)rr;
+      } else {
+        // C1: p = u + beta p, s = w + beta s, sh = wh + beta sh, e += alpha p,
+        // r -= alpha s, u' = u - alpha sh (= K^-1 r'), w' = A u' with u'
+        // formed on the fly at the columns, wh' = K^-1 w'; (r', u'), (w', u'),
+        // (r', r'). The first iteration after a restart has p = u, s = w, sh = wh.
+        const bool first = L.first != 0;
+        const R al = R(L.alpha), be = R(L.beta);
+        const auto shn = [&](const V4<R>& g) { return first ? g.b : fma_r(be, g.c, g.b); };
+        const V4<R> g = ld4(pk + row);
+        const R p_old = vt[o], s_old = vs[o], w_old = vv[o], e_old = ve[o], r_old = vr[o], di = dinv[row];
+        const R w = sell_dot<R, CH>(R(0), SLc, p0, len, lane, aval, [&](int j) {
+          const V4<R> h = ld4(pk + j);
+          return fma_r(-al, shn(h), h.a);
+        });
+        const R sh = shn(g), un = fma_r(-al, sh, g.a);
+        const R pp = first ? g.a : fma_r(be, p_old, g.a);
+        const R ss = first ? w_old : fma_r(be, s_old, w_old);
+        const R rn = fma_r(-al, ss, r_old);
+        vt[o] = pp;
+        vs[o] = ss;
+        const R ee = fma_r(al, pp, e_old);
+        ve[o] = ee;
+        if (SM >= 1) a.e[g0] = ee;
+        vr[o] = rn;
+        pn[row] = V4<R>{un, w * di, sh, R(0)};
+        vv[o] = w;
+        v0 = (double)rn * (double)un;
+        v1 = (double)w * (double)un;
+        v2 = (double)rn * (double)rn;
       }
       // the item's partial sums (warp order is fixed: deterministic)
-      v0 = warp_sum(v0);
-      v1 = warp_sum(v1);
-      if (lane == 0) {
-        spart[NS * it] = v0;
-        spart[NS * it + 1] = v1;
-      }
-      if (NSMAX > 2 && NS > 2) {
-        const double vx[3] = {warp_sum(v2), NS > 3 ? warp_sum(v3) : 0.0, NS > 4 ? warp_sum(v4) : 0.0};
-        if (lane == 0)
-#pragma unroll
-          for (int q = 2; q < NSMAX; ++q)
-            if (q < NS) spart[NS * it + q] = vx[q - 2];
+      double* sp = spart + (size_t)NS * it;
+      if (act == ACT_P2) {
+        double v[8] = {v0, v1, v2, v3, v4, 0.0, 0.0, 0.0};
+        const double tot = warp_sum_many<8, double>(v, lane);
+        const int q = warp_sum_many_index<8>(lane);
+        if ((lane & 3) == 0 && q < kMaxSums) sp[q] = tot;
+      } else if (act == ACT_P1) {
+        v0 = warp_sum(v0);
+        if (lane == 0) sp[0] = v0;
+      } else {
+        double v[4] = {v0, v1, v2, 0.0};
+        const double tot = warp_sum_many<4, double>(v, lane);
+        const int q = warp_sum_many_index<4>(lane);
+        if ((lane & 7) == 0 && q < 3) sp[q] = tot;
       }
     }
     __syncthreads();
-    // per tile: its items' partials in order, into this phase's parity buffer
-    // and the tile's count on its system's counter (a release add: after
-    // the block barrier above it publishes every write of the block in this
-    // phase)
-    for (int tl = threadIdx.x; tl < ntl; tl += kSolveThreads) {
-      const Tile T = tile_at(t_lo + tl);
-      if (ls[T.lk].act != ACT_NONE) {
-        double sm[NSMAX];
-#pragma unroll
-        for (int q = 0; q < NSMAX; ++q) sm[q] = 0.0;
-        for (int it = item0[tl]; it < item0[tl + 1]; ++it) {
-#pragma unroll
-          for (int q = 0; q < NSMAX; ++q)
-            if (q < NS) sm[q] += spart[NS * it + q];
-        }
-        double* dst = a.part + (size_t)(iter & 1) * a.ntiles * NS + T.slot;
-#pragma unroll
-        for (int q = 0; q < NSMAX; ++q)
-          if (q < NS) dst[(size_t)q * a.ntiles] = sm[q];
+    // ---- publish, a warp per local system: the block's partial sums (items
+    // in a fixed order) into this phase's parity, then a release add on the
+    // system's counter, which after the block barrier above covers every
+    // write of the block's phase
+    for (int l = warp; l < nls; l += kWarps) {
+      LocalSys& L = ls[l];
+      const int act = L.act, k = l % NC, il = l / NC;
+      const int ns = act == ACT_P2 ? kMaxSums : act == ACT_P1 ? 1 : act == ACT_NONE || act == ACT_FINISH ? 0 : 3;
+      if (lane < ns) {  // lane q adds up sum q
+        double s = 0.0;
+        for (int j = 0; j < bs1 - bs0; ++j)
+          if (SLk[j] == il) s += spart[(size_t)NS * (j * NC + k) + lane];
+        a.part[((size_t)(iter & 1) * kMaxSums + lane) * a.nslots + L.slot] = s;
       }
-      red_release_add_u32(a.scount + (size_t)T.sys * 32, 1u);
-    }
-    // ---- bookkeeping
-    if (threadIdx.x == 0) {
-      for (int k = 0; k < nls; ++k) {
-        LocalSys& L = ls[k];
-        if (L.act == ACT_P1) L.par ^= 1;
-        if (L.act == ACT_C1) {
-          L.par ^= 1;
-          L.chk = 1;
-        }
-        if (L.act == ACT_OUT_DONE && L.owner) {
+      __syncwarp();
+      if (lane == 0) {
+        red_release_add_u32(a.scount + (size_t)L.sys * 32, 1u);
+        if (act == ACT_P1 || act == ACT_C0 || act == ACT_C1) L.par ^= 1;
+        if (act == ACT_FINISH && L.slot == L.s0) {
           a.out_it[L.sys] = L.it;
           a.out_res[L.sys] = L.res;
           a.out_tol[L.sys] = L.tol;
           a.out_outer[L.sys] = L.outer;
           atomicSub(a.active, 1);
         }
-        L.act = ACT_NONE;
       }
     }
   }
@@ -633,19 +594,25 @@ __global__ void __launch_bounds__(kSolveThreads, MINB) k_krylov(SolveArgs<R> a) 
 
 // ------------------------------------------------------------------ host
 template <typename R, int MINB>
-static int occupancy(size_t smem) {
-  int occ = 0;
-  // one process-wide upper bound, so contexts with different systems coexist
-  cudaFuncSetAttribute((const void*)k_krylov<R, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem_budget(MINB));
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_krylov<R, MINB>, kSolveThreads, smem) != cudaSuccess)
-    return 0;
-  return occ;
+static const void* kernel_of(int sm) {
+  return sm == 0   ? (const void*)k_krylov<R, MINB, 0>
+         : sm == 1 ? (const void*)k_krylov<R, MINB, 1>
+         : sm == 2 ? (const void*)k_krylov<R, MINB, 2>
+                   : (const void*)k_krylov<R, MINB, 3>;
 }
 
-static int occupancy_any(bool mixed, int minb, size_t smem) {
-  if (minb == 1) return mixed ? occupancy<float, 1>(smem) : occupancy<double, 1>(smem);
-  return mixed ? occupancy<float, 2>(smem) : occupancy<double, 2>(smem);
+template <typename R>
+static const void* kernel_of(int minb, int sm) {
+  return minb == 1 ? kernel_of<R, 1>(sm) : kernel_of<R, 2>(sm);
+}
+
+static int occupancy(bool mixed, int minb, int sm, size_t smem) {
+  const void* k = mixed ? kernel_of<float>(minb, sm) : kernel_of<double>(minb, sm);
+  int occ = 0;
+  // one process-wide upper bound, so contexts with different systems coexist
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_budget(minb));
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, solve_threads(minb), smem) != cudaSuccess) return 0;
+  return occ;
 }
 
 void krylov_free(Ctx& c) {
@@ -660,182 +627,118 @@ void krylov_free(Ctx& c) {
 pfem2_status krylov_setup(Ctx& c) {
   KrylovWs* w = new KrylovWs();
   c.kws = w;
-  // the velocity solves: two blocks per SM hide more latency, one has fewer
-  // blocks to wait for at every phase and the registers of the SM share
-  w->vel_minb = c.tune.vel_blocks_per_sm ? c.tune.vel_blocks_per_sm : 2;
-  c.tune.vel_blocks_per_sm = w->vel_minb;
   const int dim = c.dim, ni = (int)c.inst.size();
-  const size_t nv = c.nv;
-  const int bps = std::max(1, c.solve_blocks_per_sm);
-  int maxtiles = 0, maxsys = 0;
+  // slices per block: one block per SM, but at least four slices (channel of
+  // 1k rows, FP64: 0.49 ms per step with four, 0.53 with six, 0.48 with two;
+  // 13k rows: 0.48 with four, 0.53 with two)
+  const int ts_auto = std::max(4, (c.nslices + c.num_sms - 1) / c.num_sms);
+  // the velocity solves of one system: a block of 768 threads per SM, so that
+  // few blocks are waited for (52k channel: prediction and correction 0.45 ms
+  // per step against 0.55 with two blocks of 384; 131k pipe 3.58 against
+  // 3.77), unless 12 warps hold its items in one round; a batch takes two of
+  // 384, whose instances wait less for each other (16 channels: 1.38 against
+  // 1.44 ms)
+  w->vel_minb = c.tune.vel_blocks_per_sm ? c.tune.vel_blocks_per_sm : (ni > 1 || ts_auto * dim <= 12 ? 2 : 1);
+  c.tune.vel_blocks_per_sm = w->vel_minb;
+  const size_t nv = c.nv, rs = c.kmixed ? sizeof(float) : sizeof(double);
+  int maxslots = 0;
   // phase 0: the pressure systems where the multigrid is not used
   for (int ph = c.two_level ? 1 : 0; ph < 2; ++ph) {
     const int ncomp = ph == 0 ? 1 : dim;
-    const int nsys = ncomp * ni;
-    std::vector<Tile> tiles;
-    if (ph == 0) {
-      // pressure: about one tile per SM for a single system, tiles of about
-      // 8 slices in a batch
-      const int dcap = ni == 1 ? 160 : 96;
-      const int nb = c.num_sms;
-      long long tot_sl = 0;
-      for (int i = 0; i < ni; ++i) tot_sl += c.inst[i].nv_pad / kSlice;
-      for (int i = 0; i < ni; ++i) {
-        const int sl0 = c.inst[i].v_off / kSlice, nsl = c.inst[i].nv_pad / kSlice;
-        const long long share = ni == 1 ? std::max<long long>(1, (long long)nb * nsl / tot_sl) : (nsl + 7) / 8;
-        int D = (int)std::min<long long>(std::min<long long>(share, dcap), nsl);
-        const int sps = (nsl + D - 1) / D;
-        for (int a = 0; a < nsl; a += sps) tiles.push_back(Tile{i, 0, sl0 + a, sl0 + std::min(nsl, a + sps), 0, 0});
-      }
-    } else {
-      // velocity components: tiles ordered (instance, slice run, component)
-      // so that the slices of a block form one contiguous range
-      const long long slices = (long long)c.nslices * ncomp;
-      const long long target = 4LL * bps * c.num_sms;
-      int ts = (int)std::max<long long>(8, (slices + target - 1) / target);
-      if (c.tune.vel_tile_slices > 0) ts = c.tune.vel_tile_slices;
-      c.tune.vel_tile_slices = ts;
-      for (int i = 0; i < ni; ++i) {
-        const int sl0 = c.inst[i].v_off / kSlice, sl1 = (c.inst[i].v_off + c.inst[i].nv_pad) / kSlice;
-        for (int a = sl0; a < sl1; a += ts)
-          for (int k = 0; k < ncomp; ++k) tiles.push_back(Tile{k * ni + i, k, a, std::min(sl1, a + ts), 0, 0});
-      }
-    }
-    const int T = (int)tiles.size();
-    // partial slots: the tiles of a system, contiguous
-    std::vector<int> slot0(nsys + 1, 0), cnt(nsys, 0);
-    for (const Tile& t : tiles) slot0[t.sys + 1]++;
-    for (int s = 0; s < nsys; ++s) slot0[s + 1] += slot0[s];
-    std::vector<int> owner(nsys, -1);
     const int minb = ph == 0 ? 2 : w->vel_minb;
-    const int occ = std::min(minb, occupancy_any(c.kmixed, minb, 0));
+    const int occ = std::min(minb, occupancy(c.kmixed, minb, 0, 0));
     if (occ < 1) {
       set_error("krylov: the solver kernel cannot be resident");
       return PFEM2_CUDA_ERROR;
     }
-    const int G = std::min(T, occ * c.num_sms);
-    std::vector<int> bt0(G + 1), bsys_off(1, 0), bsys, bsl(2 * G, 0);
-    // split the tile sequence where the running slice count crosses
-    // b / G of the total (a tile goes to the block holding its midpoint):
-    // blocks get equal work when tiles differ in size
-    {
-      std::vector<long long> pre(T + 1, 0);
-      for (int u = 0; u < T; ++u) pre[u + 1] = pre[u] + (tiles[u].s1 - tiles[u].s0);
-      bt0[0] = 0;
-      int t = 0;
-      for (int b = 1; b < G; ++b) {
-        const long long goal = pre[T] * b / G;
-        while (t < T && 2 * pre[t] + (pre[t + 1] - pre[t]) < 2 * goal) ++t;
-        // every block keeps at least one tile and leaves one for each later block
-        t = std::min(std::max(t, bt0[b - 1] + 1), T - (G - b));
-        bt0[b] = t;
-      }
-      bt0[G] = T;
+    // every block takes the same run of slices with all their components
+    int ts = ni > 1 || ph == 0 ? 4 : ts_auto;
+    if (ph == 1) {
+      if (c.tune.vel_tile_slices > 0) ts = c.tune.vel_tile_slices;
+      c.tune.vel_tile_slices = ts;
     }
-    size_t meta = 0, col = 0;
-    int ntl_max = 0, items_max = 0;
-    for (int b = 0; b < G; ++b) {
-      std::vector<int> lst;
-      int s0 = 1 << 30, s1 = -1, items = 0;
-      ntl_max = std::max(ntl_max, bt0[b + 1] - bt0[b]);
-      for (int t = bt0[b]; t < bt0[b + 1]; ++t) items += tiles[t].s1 - tiles[t].s0;
-      items_max = std::max(items_max, items);
-      for (int t = bt0[b]; t < bt0[b + 1]; ++t) {
-        Tile& tl = tiles[t];
-        int k = (int)(std::find(lst.begin(), lst.end(), tl.sys) - lst.begin());
-        if (k == (int)lst.size()) lst.push_back(tl.sys);
-        tl.lk = k;
-        tl.slot = slot0[tl.sys] + cnt[tl.sys]++;
-        if (owner[tl.sys] < 0) owner[tl.sys] = b;
-        s0 = std::min(s0, tl.s0);
-        s1 = std::max(s1, tl.s1);
+    const int G = std::max(1, std::min(occ * c.num_sms, (c.nslices + ts - 1) / ts));
+    std::vector<int> bsl(G + 1), binst, binst_off(1, 0), bslot, cnt(ni, 0), slot0(ncomp * ni + 1, 0), slk(c.nslices, 0);
+    for (int b = 0; b <= G; ++b) bsl[b] = (int)((long long)c.nslices * b / G);
+    w->items_max[ph] = 0;
+    size_t meta = 0, ne = 0;
+    for (int b = 0, i = 0; b < G; ++b) {
+      const int s0 = bsl[b], s1 = bsl[b + 1];
+      while ((c.inst[i].v_off + c.inst[i].nv_pad) / kSlice <= s0) ++i;
+      int last = i - 1;
+      for (int sl = s0, j = i; sl < s1; ++sl) {
+        while ((c.inst[j].v_off + c.inst[j].nv_pad) / kSlice <= sl) ++j;
+        for (; last < j; ++last) {
+          binst.push_back(last + 1);
+          bslot.push_back(cnt[last + 1]++);
+        }
+        slk[sl] = j - i;
       }
-      if ((int)lst.size() > kMaxLocalSys) {
+      binst_off.push_back((int)binst.size());
+      if ((binst_off[b + 1] - binst_off[b]) * ncomp > kMaxLocalSys) {
         set_error("krylov: more than 16 systems would share one block (instances too small for the batch)");
         return PFEM2_INVALID_ARG;
       }
-      bsys.insert(bsys.end(), lst.begin(), lst.end());
-      bsys_off.push_back((int)bsys.size());
-      if (s1 < s0) s0 = s1 = 0;
-      // the block's tiles are ordered so that their slices form one range
-      bsl[2 * b] = s0;
-      bsl[2 * b + 1] = s1;
-      meta = std::max(meta, al16(4 * (size_t)(s1 - s0 + 1)) + al16(4 * (size_t)(s1 - s0)));
-      col = std::max(col, al16(4 * (size_t)(c.h_sl_ptr[s1] - c.h_sl_ptr[s0])));
+      w->items_max[ph] = std::max(w->items_max[ph], (s1 - s0) * ncomp);
+      meta = std::max(meta, 3 * al16(4 * (size_t)(s1 - s0)));
+      ne = std::max(ne, (size_t)(c.h_sl_ptr[s1] - c.h_sl_ptr[s0]));
     }
-    w->ntl_max[ph] = ntl_max;
-    w->items_max[ph] = items_max;
-    w->bicg[ph] = ph == 0 ? c.p_bicg : c.vel_bicg;
-    // BiCGStab 5 sums, CG 3 (one reduction per iteration)
-    w->nsum[ph] = w->bicg[ph] ? kMaxSums : 3;
-    w->items_bytes[ph] =
-        al16(sizeof(double) * w->nsum[ph] * (size_t)items_max) + al16(sizeof(int) * (size_t)(ntl_max + 1));
-    w->smem[ph] = w->items_bytes[ph];
-    if (w->smem[ph] + meta <= smem_budget(minb)) {
-      w->stage[ph] |= ST_L0META;
-      w->smem[ph] += meta;
-    }
-    if (w->smem[ph] + col <= smem_budget(minb)) {
-      w->stage[ph] |= ST_L0COL;
-      w->smem[ph] += col;
-    }
-    if (occupancy_any(c.kmixed, minb, w->smem[ph]) * c.num_sms < G) {
-      w->stage[ph] = 0;
-      w->smem[ph] = w->items_bytes[ph];
-    }
-    w->ntiles[ph] = T;
-    w->nsys[ph] = nsys;
+    for (int k = 0; k < ncomp; ++k)
+      for (int i = 0; i < ni; ++i) slot0[k * ni + i + 1] = slot0[k * ni + i] + cnt[i];
+    w->nslots[ph] = slot0.back();
+    maxslots = std::max(maxslots, w->nslots[ph]);
     w->grid[ph] = G;
-    PFEM2_TRY(ws_upload(w, &w->tiles[ph], tiles));
-    PFEM2_TRY(ws_upload(w, &w->sys_slot0[ph], slot0));
-    PFEM2_TRY(ws_upload(w, &w->sys_owner[ph], owner));
-    PFEM2_TRY(ws_upload(w, &w->blk_t0[ph], bt0));
-    PFEM2_TRY(ws_upload(w, &w->blk_sys[ph], bsys));
-    PFEM2_TRY(ws_upload(w, &w->blk_sys_off[ph], bsys_off));
+    w->bicg[ph] = ph == 0 ? c.p_bicg : c.vel_bicg;
+    w->st_meta[ph] = meta;
+    w->st_entries[ph] = ne;
+    PFEM2_TRY(ws_upload(w, &w->blk_inst[ph], binst));
+    PFEM2_TRY(ws_upload(w, &w->blk_inst_off[ph], binst_off));
+    PFEM2_TRY(ws_upload(w, &w->blk_slot[ph], bslot));
     PFEM2_TRY(ws_upload(w, &w->blk_sl[ph], bsl));
-    maxtiles = std::max(maxtiles, T);
-    maxsys = std::max(maxsys, nsys);
+    PFEM2_TRY(ws_upload(w, &w->sys_slot0[ph], slot0));
+    PFEM2_TRY(ws_upload(w, &w->slk[ph], slk));
   }
-  if (c.kmixed) {
-    float *e, *r, *q, *p;
-    PFEM2_TRY(ws_alloc(w, &e, nv * dim));
-    PFEM2_TRY(ws_alloc(w, &r, 2 * nv * dim));
-    PFEM2_TRY(ws_alloc(w, &q, nv * dim));
-    PFEM2_TRY(ws_alloc(w, &p, 2 * nv * dim));
-    w->e = e; w->r = r; w->q = q; w->p = p;
-  } else {
-    double *e, *r, *q, *p;
-    PFEM2_TRY(ws_alloc(w, &e, nv * dim));
-    PFEM2_TRY(ws_alloc(w, &r, 2 * nv * dim));
-    PFEM2_TRY(ws_alloc(w, &q, nv * dim));
-    PFEM2_TRY(ws_alloc(w, &p, 2 * nv * dim));
-    w->e = e; w->r = r; w->q = q; w->p = p;
-  }
-  PFEM2_TRY(ws_alloc(w, &w->r64, nv * dim));
-  PFEM2_TRY(ws_alloc(w, &w->part, 2 * (size_t)kMaxSums * maxtiles));
+  // systems whose components have the same Dirichlet rows share the mass matrix
+  w->mass_share = true;
   {
-    // single-reduction Jacobi CG vectors: u, wh, sh double buffered, w, s
-    const size_t rs = c.kmixed ? sizeof(float) : sizeof(double);
-    unsigned char* b[5];
-    const size_t n[5] = {2 * nv * dim, 2 * nv * dim, 2 * nv * dim, nv * dim, nv * dim};
-    for (int k = 0; k < 5; ++k) PFEM2_TRY(ws_alloc(w, &b[k], n[k] * rs));
-    w->cu = b[0]; w->cwh = b[1]; w->csh = b[2]; w->cw = b[3]; w->cs = b[4];
+    std::vector<unsigned char> d0(nv), dk(nv);
+    PFEM2_CUDA(cudaMemcpy(d0.data(), c.isdir[0], nv, cudaMemcpyDeviceToHost));
+    for (int k = 1; k < dim; ++k) {
+      PFEM2_CUDA(cudaMemcpy(dk.data(), c.isdir[k], nv, cudaMemcpyDeviceToHost));
+      w->mass_share = w->mass_share && d0 == dk;
+    }
   }
-  if (c.vel_bicg || c.p_bicg) {
-    // BiCGStab vectors: zr and w double buffered, rh, s, t, kt
-    const size_t rs = c.kmixed ? sizeof(float) : sizeof(double);
-    unsigned char* b[6];
-    const size_t n[6] = {2 * nv * dim, 2 * nv * dim, nv * dim, nv * dim, nv * dim, nv * dim};
-    for (int k = 0; k < 6; ++k) PFEM2_TRY(ws_alloc(w, &b[k], n[k] * rs));
-    w->bz = b[0]; w->bw = b[1]; w->rh = b[2]; w->bs = b[3]; w->bt = b[4]; w->bkt = b[5];
-  }
-  PFEM2_TRY(ws_alloc(w, &w->scount, 32 * (size_t)maxsys));
+  unsigned char* b[7];
+  const size_t n[7] = {2 * 4 * nv * dim, nv * dim, nv * dim, nv * dim, nv * dim, nv * dim, nv * dim};
+  for (int k = 0; k < 7; ++k) PFEM2_TRY(ws_alloc(w, &b[k], n[k] * rs));
+  w->pk = b[0]; w->e = b[1]; w->r = b[2]; w->v = b[3]; w->s = b[4]; w->t = b[5]; w->rh = b[6];
+  PFEM2_TRY(ws_alloc(w, &w->r64, nv * dim));
+  PFEM2_TRY(ws_alloc(w, &w->part, 2 * (size_t)kMaxSums * maxslots));
+  PFEM2_TRY(ws_alloc(w, &w->scount, 32 * (size_t)dim * ni));
   PFEM2_TRY(ws_alloc(w, &w->active, 1));
   for (int k = 0; k < 3; ++k) {
-    PFEM2_TRY(ws_alloc(w, &w->out_it[k], maxsys));
-    PFEM2_TRY(ws_alloc(w, &w->out_res[k], maxsys));
-    PFEM2_TRY(ws_alloc(w, &w->out_tol[k], maxsys));
-    PFEM2_TRY(ws_alloc(w, &w->out_outer[k], maxsys));
+    PFEM2_TRY(ws_alloc(w, &w->out_it[k], dim * ni));
+    PFEM2_TRY(ws_alloc(w, &w->out_res[k], dim * ni));
+    PFEM2_TRY(ws_alloc(w, &w->out_tol[k], dim * ni));
+    PFEM2_TRY(ws_alloc(w, &w->out_outer[k], dim * ni));
+  }
+  // shared memory per solve (0 prediction, 1 pressure, 2 correction)
+  for (int which = 0; which < 3; ++which) {
+    const int ph = which == 1 ? 0 : 1;
+    if (which == 1 && c.two_level) continue;
+    const int minb = ph == 0 ? 2 : w->vel_minb, ncomp = ph == 0 ? 1 : dim;
+    const int nmat = which == 2 && w->mass_share ? 1 : ncomp;
+    size_t smem = al16(sizeof(double) * (w->bicg[ph] ? kMaxSums : 3) * (size_t)w->items_max[ph]);
+    const size_t level[3] = {al16(6 * 32 * rs * (size_t)w->items_max[ph]) + w->st_meta[ph],
+                             al16(4 * w->st_entries[ph]), nmat * al16(rs * w->st_entries[ph])};
+    int sm = 0;
+    while (sm < 3 && smem + level[sm] <= smem_budget(minb)) smem += level[sm++];
+    if (occupancy(c.kmixed, minb, sm, smem) * c.num_sms < w->grid[ph]) {
+      set_error("krylov: the solver grid cannot be resident");
+      return PFEM2_CUDA_ERROR;
+    }
+    w->sm[which] = sm;
+    w->smem[which] = smem;
   }
   return PFEM2_OK;
 }
@@ -884,25 +787,21 @@ static pfem2_status solve_impl(Ctx& c, int which) {
   SolveArgs<R> a{};
   a.ncomp = ncomp;
   a.ninst = ni;
-  a.nsys = w->nsys[ph];
-  a.ntiles = w->ntiles[ph];
   a.nv = c.nv;
-  a.tiles = w->tiles[ph];
+  a.blk_inst = w->blk_inst[ph];
+  a.blk_inst_off = w->blk_inst_off[ph];
+  a.blk_slot = w->blk_slot[ph];
   a.sys_slot0 = w->sys_slot0[ph];
-  a.sys_owner = w->sys_owner[ph];
-  a.blk_t0 = w->blk_t0[ph];
-  a.blk_sys = w->blk_sys[ph];
-  a.blk_sys_off = w->blk_sys_off[ph];
   a.blk_sl = w->blk_sl[ph];
-  a.stage = w->stage[ph];
-  a.ntl_max = w->ntl_max[ph];
+  a.slk = w->slk[ph];
   a.items_max = w->items_max[ph];
   a.sl_ptr = c.sl_ptr;
   a.sl_len = c.sl_len;
   a.sl_col = c.sl_col;
+  a.share = which == 2 && w->mass_share;
   for (int k = 0; k < 3; ++k) {
     const int kk = k < ncomp ? k : 0;
-    const int mtx = which == 0 ? kk : (which == 1 ? 3 : 4 + kk);
+    const int mtx = which == 0 ? kk : (which == 1 ? 3 : 4 + (a.share ? 0 : kk));
     a.A64[k] = c.A64[mtx];
     a.Ain[k] = c.kmixed ? (const R*)c.A32[mtx] : (const R*)c.A64[mtx];
     a.dinv[k] = c.kmixed ? (const R*)c.dinv32[mtx] : (const R*)c.dinv64[mtx];
@@ -926,13 +825,13 @@ static pfem2_status solve_impl(Ctx& c, int which) {
   a.tol_i = (const double*)c.sys_scalars + (which == 1 ? ni : 0);
   a.rtol_i = (const double*)c.sys_scalars + 2 * ni + (which == 1 ? ni : 0);
   a.bicg = w->bicg[ph] ? 1 : 0;
-  a.nsum = w->nsum[ph];
-  a.bz = (R*)w->bz; a.bw = (R*)w->bw; a.rh = (R*)w->rh; a.bs = (R*)w->bs; a.bt = (R*)w->bt; a.bkt = (R*)w->bkt;
-  a.cu = (R*)w->cu; a.cwh = (R*)w->cwh; a.csh = (R*)w->csh; a.cw = (R*)w->cw; a.cs = (R*)w->cs;
+  a.pk = (V4<R>*)w->pk;
+  a.rh = (R*)w->rh; a.s = (R*)w->s; a.t = (R*)w->t; a.v = (R*)w->v;
   a.maxit_i = c.d_sysinfo;
-  a.e = (R*)w->e; a.r = (R*)w->r; a.q = (R*)w->q; a.p = (R*)w->p;
+  a.e = (R*)w->e; a.r = (R*)w->r;
   a.r64 = w->r64;
   a.part = w->part;
+  a.nslots = w->nslots[ph];
   a.scount = w->scount;
   a.active = w->active;
   a.out_it = w->out_it[which];
@@ -940,17 +839,18 @@ static pfem2_status solve_impl(Ctx& c, int which) {
   a.out_tol = w->out_tol[which];
   a.out_outer = w->out_outer[which];
   a.eta = c.kmixed ? c.refine_eta : 0.0;
-  // phases per iteration, and BiCGStab's restarts (three phases each, at most max_iter)
+  // phases per iteration, and the restarts (one phase more, at most max_iter)
   a.iter_cap = (a.bicg ? 5 : 4) * krylov_max_iter(c) + 256;
   a.gb.count = c.barrier;
   a.gb.gen = c.barrier + 1;
   a.gb.err = c.d_err;
   a.gb.spin_limit = c.spin_limit;
-  PFEM2_TRY(krylov_init_solve(c, a.nsys));
+  PFEM2_TRY(krylov_init_solve(c, ncomp * ni));
   void* args[] = {&a};
   // the velocity solves at vel_minb blocks per SM, a pressure solve at two
-  const void* kern = (ph == 1 && w->vel_minb == 1) ? (const void*)k_krylov<R, 1> : (const void*)k_krylov<R, 2>;
-  PFEM2_CUDA(cudaLaunchCooperativeKernel(kern, dim3(w->grid[ph]), dim3(kSolveThreads), args, w->smem[ph], c.stream));
+  const int minb = ph == 0 ? 2 : w->vel_minb;
+  PFEM2_CUDA(cudaLaunchCooperativeKernel(kernel_of<R>(minb, w->sm[which]), dim3(w->grid[ph]), dim3(solve_threads(minb)), args, w->smem[which],
+                                         c.stream));
   c.launches++;
   return PFEM2_OK;
 }

@@ -101,17 +101,26 @@ __device__ __forceinline__ SV<T> stage_range(unsigned char*& cur, const T* src, 
   return SV<T>{dst, lo};
 }
 
+// the same without a base: element i of the copy is src[i]
+template <typename T>
+__device__ __forceinline__ const T* stage_copy(unsigned char*& cur, const T* src, int n) {
+  T* dst = reinterpret_cast<T*>(cur);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
+  cur += al16_dev((size_t)n * sizeof(T));
+  return dst;
+}
+
 template <typename T>
 __device__ __forceinline__ SV<T> maybe_stage(bool on, unsigned char*& cur, const T* src, int lo, int hi) {
   return on ? stage_range(cur, src, lo, hi) : SV<T>{src, 0};
 }
 
-// Waits until system counter *cnt has reached target (release adds of the
-// blocks that own parts of the system); false after spin_limit polls or when
-// another block has flagged an error. The caller fences afterwards.
+// Waits (acquire) until system counter *cnt has reached target (release adds
+// of the blocks that own parts of the system); false after spin_limit polls
+// or when another block has flagged an error.
 __device__ __forceinline__ bool wait_count(const unsigned* cnt, unsigned target, const GridBarrier& gb) {
   unsigned spins = 0;
-  while ((int)(ld_relaxed_u32(cnt) - target) < 0) {
+  while ((int)(ld_acquire_u32(cnt) - target) < 0) {
     if (++spins > gb.spin_limit || *(volatile int*)gb.err != 0) return false;
     __nanosleep(20);
   }
@@ -123,25 +132,17 @@ struct MgWs;  // mgcg.cu
 
 struct KrylovWs {
   // Jacobi solves, [0] pressure (without multigrid), [1] velocity components
-  Tile* tiles[2] = {};
-  int* sys_slot0[2] = {};
-  int* sys_owner[2] = {};
-  int* blk_t0[2] = {};
-  int* blk_sys[2] = {};
-  int* blk_sys_off[2] = {};
-  int* blk_sl[2] = {};
-  int ntiles[2] = {}, nsys[2] = {}, grid[2] = {};
-  int stage[2] = {0, 0};   // staged categories per phase
-  size_t smem[2] = {0, 0}; // dynamic shared memory per phase
-  int ntl_max[2] = {0, 0}, items_max[2] = {0, 0};  // per block: tiles, (tile, slice) items
-  size_t items_bytes[2] = {0, 0};                  // shared memory of the item partials and offsets
-  int nsum[2] = {2, 2};                            // partial sums per tile of each phase
+  int *blk_inst[2] = {}, *blk_inst_off[2] = {}, *blk_slot[2] = {}, *blk_sl[2] = {}, *sys_slot0[2] = {}, *slk[2] = {};
+  int grid[2] = {}, nslots[2] = {}, items_max[2] = {};
+  size_t st_meta[2] = {}, st_entries[2] = {};      // per block: static index bytes, SELL entries
   bool bicg[2] = {false, false};                   // phase solved by BiCGStab
-  void *bz = nullptr, *bw = nullptr, *rh = nullptr, *bs = nullptr, *bt = nullptr, *bkt = nullptr;
-  void *cu = nullptr, *cwh = nullptr, *csh = nullptr, *cw = nullptr, *cs = nullptr;
+  bool mass_share = false;                         // the components' mass matrices are equal
+  int sm[3] = {};                                  // what is kept in shared memory per solve
+  size_t smem[3] = {};                             // dynamic shared memory per solve
+  void *pk = nullptr, *rh = nullptr, *s = nullptr, *t = nullptr, *v = nullptr;
   int vel_minb = 2;  // resident blocks per SM of the velocity solves
   MgWs* mg = nullptr;
-  void *e = nullptr, *r = nullptr, *q = nullptr, *p = nullptr;
+  void *e = nullptr, *r = nullptr;
   double* r64 = nullptr;
   double* part = nullptr;
   unsigned* scount = nullptr;

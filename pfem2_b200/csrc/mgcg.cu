@@ -275,8 +275,8 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
     // ---- phase start, a warp per local system: every block that owns part
     // of the system adds 1 to its counter once its phase is written, so iter
     // x (blocks of the system) means that all have finished phase iter - 1;
-    // the acquire fence (and the block barrier) orders what they wrote before
-    // this phase's reads. Then the sums the next step needs, and the step
+    // the acquire (and the block barrier) orders what they wrote before this
+    // phase's reads. Then the sums the next step needs, and the step
     // itself (identical in every block that owns part of the system). Warps
     // without a system come here from the work after publishing.
     MgAct* const sa = sact[iter & 1];
@@ -297,7 +297,6 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
           }
           continue;
         }
-        fence_acq_rel_gpu();
       }
       int next = st + 1;  // T_B .. T_A are in phase order
       switch (st) {
@@ -463,6 +462,7 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
       const int o = it * 32 + lane, row = own0 + o;
       double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
       if (act == DO_A) {
+        const R di = a.dinv[row];
         const R acc = sell_dot<R, CH>(R(0), SLc, SLp[sl], SLl[sl], lane, [&](int ei) { return SLa[ei]; },
                                       [&](int col) { return ldm(a.z, mz, col, own0, nown); });
         const R be = R(L.beta);
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
         }
         mq[o] = qq;
         mp[o] = pp;
-        const R dd = a.dinv[row] * qq;
+        const R dd = di * qq;
         a.dq[row] = dd;
         if (mdq) mdq[o] = dd;
         v0 = (double)pp * (double)qq;
@@ -498,10 +498,10 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
         if (mz) mz[o] = acc;
         v0 = (double)mr[o] * (double)acc;
       } else if (act == DO_OUT_A) {
+        const double bb = a.b[row];
         const double acc = sell_dot<double, CH>(
             0.0, SLc, SLp[sl], SLl[sl], lane, [&](int ei) { return a.A64[ei]; },
             [&](int col) { return __ldcg(a.x + col) + (double)ldm(a.e, me, col, own0, nown); });
-        const double bb = a.b[row];
         const double rr = bb - acc;
         a.r64[row] = rr;
         v0 = rr * rr;
@@ -518,18 +518,14 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
         }
         continue;
       }
-#pragma unroll
-      for (int s = 16; s > 0; s >>= 1) {
-        v0 += __shfl_xor_sync(PFEM2_FULL_MASK, v0, s);
-        v1 += __shfl_xor_sync(PFEM2_FULL_MASK, v1, s);
-        v2 += __shfl_xor_sync(PFEM2_FULL_MASK, v2, s);
-        v3 += __shfl_xor_sync(PFEM2_FULL_MASK, v3, s);
-      }
-      if (lane == 0) {
-        spart[kMgSums * it] = v0;
-        spart[kMgSums * it + 1] = v1;
-        spart[kMgSums * it + 2] = v2;
-        spart[kMgSums * it + 3] = v3;
+      if (act == DO_UZ) {
+        v0 = warp_sum(v0);
+        if (lane == 0) spart[kMgSums * it] = v0;
+      } else {
+        double v[4] = {v0, v1, v2, v3};
+        const double tot = warp_sum_many<4, double>(v, lane);
+        const int q = warp_sum_many_index<4>(lane);
+        if ((lane & 7) == 0) spart[kMgSums * it + q] = tot;
       }
     }
     __syncthreads();
@@ -539,28 +535,14 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
     for (int k = warp; k < nls; k += NW) {
       const MgSys& L = ls[k];
       const int act = sa[k].act;
-      if (act == DO_A || act == DO_UZ || act == DO_OUT_A) {
-        double s[kMgSums] = {0.0, 0.0, 0.0, 0.0};
-        for (int it = L.it0 + lane; it < L.it1; it += 32)
-#pragma unroll
-          for (int q = 0; q < kMgSums; ++q) s[q] += spart[kMgSums * it + q];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-          for (int q = 0; q < kMgSums; ++q) s[q] += __shfl_xor_sync(PFEM2_FULL_MASK, s[q], o);
-        if (lane == 0) {
-          double* dst = a.part + L.slot;
-          if (act == DO_UZ) {
-            dst[6 * (size_t)a.nslots] = s[0];
-          } else if (act == DO_A) {
-#pragma unroll
-            for (int q = 0; q < kMgSums; ++q) dst[(2 + q) * (size_t)a.nslots] = s[q];
-          } else {
-            dst[0] = s[0];
-            dst[a.nslots] = s[1];
-          }
-        }
+      const int ns = act == DO_A ? 4 : act == DO_OUT_A ? 2 : act == DO_UZ ? 1 : 0;
+      if (lane < ns) {  // lane q adds up sum q
+        double s = 0.0;
+        for (int it = L.it0; it < L.it1; ++it) s += spart[kMgSums * it + lane];
+        const int row = (act == DO_A ? 2 : act == DO_UZ ? 6 : 0) + lane;
+        a.part[(size_t)row * a.nslots + L.slot] = s;
       }
+      __syncwarp();
       if (lane == 0) {
         red_release_add_u32(a.scount + (size_t)L.sys * 32, 1u);
         if (act == DO_FINISH && L.owner) {
@@ -581,10 +563,10 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
         const MgAct& L = sa[SLk[sl]];
         if (L.act != DO_B2 || L.stop) continue;
         const int o = it * 32 + lane;
+        const R di = a.dinv[own0 + o], w = R(ls[SLk[sl]].w);
         const R acc = sell_dot<R, CH>(R(0), SLc, SLp[sl], SLl[sl], lane, [&](int ei) { return SLa[ei]; },
                                       [&](int col) { return ldm(a.dq, mdq, col, own0, nown); });
-        const R w = R(ls[SLk[sl]].w);
-        const R jq = w * fma_r(-w * a.dinv[own0 + o], acc, R(2) * ldq[o]);
+        const R jq = w * fma_r(-w * di, acc, R(2) * ldq[o]);
         mj[o] = L.restart ? jq : fma_r(-R(L.alpha), jq, mj[o]);
       }
     }
@@ -669,7 +651,7 @@ pfem2_status mg_setup(Ctx& c) {
     const long long share = ni == 1 ? std::max(1, nb) : (nsl + 7) / 8;
     const int D = (int)std::min<long long>(std::min<long long>(share, dcap), nsl);
     const int sps = (nsl + D - 1) / D;
-    for (int t = 0; t < nsl; t += sps) tiles.push_back(Tile{i, 0, sl0 + t, sl0 + std::min(nsl, t + sps), 0, 0});
+    for (int t = 0; t < nsl; t += sps) tiles.push_back(Tile{i, sl0 + t, sl0 + std::min(nsl, t + sps)});
     st0.push_back((int)tiles.size());
   }
   const int T = (int)tiles.size(), G = std::min(T, nb);
@@ -880,7 +862,7 @@ pfem2_status mg_solve_impl(Ctx& c) {
   a.maxit_i = c.d_sysinfo;
   a.z = (R*)m->z; a.dq = (R*)m->dq; a.jr = (R*)m->jr;
   a.c1 = (R*)m->c1; a.b1 = (R*)m->b1; a.x1 = (R*)m->x1; a.b2 = (R*)m->b2; a.x2 = (R*)m->x2;
-  a.p = (R*)w->p; a.q = (R*)w->q; a.r = (R*)w->r; a.e = (R*)w->e;
+  a.p = (R*)w->s; a.q = (R*)w->v; a.r = (R*)w->r; a.e = (R*)w->e;
   a.r64 = w->r64;
   a.part = m->part;
   a.nslots = m->nslots;

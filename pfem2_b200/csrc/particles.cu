@@ -865,37 +865,6 @@ __device__ __forceinline__ void proj_add(ProjAcc<DIM, R>& acc, const R* x, const
   }
 }
 
-// Sums N values (N a power of two, at most 32) over a warp with N - 1
-// exchanges instead of N * 5: at each halving step a lane keeps one half of
-// its values, sends the other half to its partner and adds what it receives.
-// Afterwards the lane holds the warp total of value warp_sum_many_index<N>.
-template <int N, typename T>
-__device__ __forceinline__ T warp_sum_many(T (&v)[N], int lane) {
-#pragma unroll
-  for (int h = N / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
-    const bool up = (lane & o) != 0;
-#pragma unroll
-    for (int i = 0; i < h; ++i) {
-      const T send = up ? v[i] : v[i + h];
-      const T keep = up ? v[i + h] : v[i];
-      v[i] = keep + __shfl_xor_sync(PFEM2_FULL_MASK, send, o);
-    }
-  }
-  T r = v[0];
-#pragma unroll
-  for (int o = 16 / N; o > 0; o >>= 1) r += __shfl_xor_sync(PFEM2_FULL_MASK, r, o);
-  return r;
-}
-
-template <int N>
-__device__ __forceinline__ int warp_sum_many_index(int lane) {
-  int idx = 0;
-#pragma unroll
-  for (int h = N / 2, o = 16; h >= 1; h >>= 1, o >>= 1)
-    if (lane & o) idx += h;
-  return idx;
-}
-
 template <int DIM, typename R>
 __device__ __forceinline__ void proj_store(ProjAcc<DIM, R>& acc, R* __restrict__ partial, int c, int lane) {
   constexpr int K = Dims<DIM>::NV * (DIM + 1);
