@@ -546,11 +546,14 @@ static pfem2_status do_setup(Ctx& c) {
   if (c.moving) PFEM2_TRY(ale_setup(c));
   if (!c.cfg.particles_only) {
     PFEM2_TRY(krylov_setup(c));
+    PFEM2_CUDA(cudaDeviceSynchronize());  // the copies so far are on the default stream
     PFEM2_TRY(assemble_matrices(c));
     PFEM2_CUDA(cudaStreamSynchronize(c.stream));
     PFEM2_TRY(krylov_setup_precond(c));
   }
   PFEM2_CUDA(cudaGetLastError());
+  // the copies and fills of the setup are on the default stream, the steps on c.stream
+  PFEM2_CUDA(cudaDeviceSynchronize());
   c.setup_done = true;
   return PFEM2_OK;
 }
@@ -590,7 +593,7 @@ static pfem2_status check_counters(Ctx& c, bool sync) {
   c.stats.n_far_movers_last_move = cnt[CNT_FAR];
   // the error flags are read once: clear them for the passes to come
   if (cnt[CNT_LIST_OVERFLOW] | cnt[CNT_CAP_OVERFLOW] | cnt[CNT_FAR_OVERFLOW] | cnt[CNT_SCAN_TIMEOUT])
-    PFEM2_CUDA(cudaMemset(c.d_counters + CNT_N_STATS, 0, sizeof(int) * (CNT_N - CNT_N_STATS)));
+    PFEM2_CUDA(cudaMemsetAsync(c.d_counters + CNT_N_STATS, 0, sizeof(int) * (CNT_N - CNT_N_STATS), c.stream));
   if (cnt[CNT_LIST_OVERFLOW]) {
     set_error("rebin: more incoming particles than the per-cell capacity (particles_per_cell_max)");
     return PFEM2_PARTICLE_OVERFLOW;
@@ -864,7 +867,8 @@ pfem2_status pfem2_seed(pfem2_ctx* x, int32_t instance, const uint32_t q[3], uin
     }
   for (auto& in : c.inst)
     if (in.q[0] == 0) { set_error("every instance needs particles: seed all instances"); return PFEM2_BAD_STATE; }
-  PFEM2_CUDA(cudaMemcpy(c.d_inst, c.h_inst.data(), sizeof(DevInst) * c.h_inst.size(), cudaMemcpyHostToDevice));
+  PFEM2_CUDA(cudaMemcpyAsync(c.d_inst, c.h_inst.data(), sizeof(DevInst) * c.h_inst.size(), cudaMemcpyHostToDevice,
+                             c.stream));
   size_t total = 0;
   for (auto& in : c.inst) total += (size_t)in.nc * in.q[0] * in.q[1] * in.q[2];
   PFEM2_TRY(alloc_particles(c, total));

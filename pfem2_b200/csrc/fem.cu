@@ -578,7 +578,7 @@ pfem2_status launch_loads(Ctx& c, int instance, int patch, double* out_dev) {
     Ctx::LoadFaces e{instance, patch, (int)h.size(), nullptr};
     if (e.n > 0) {
       PFEM2_CUDA(cudaMalloc(&e.d, sizeof(int) * h.size()));
-      PFEM2_CUDA(cudaMemcpy(e.d, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice));
+      PFEM2_CUDA(cudaMemcpyAsync(e.d, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice, c.stream));
     }
     c.load_faces.push_back(e);
     lf = &c.load_faces.back();

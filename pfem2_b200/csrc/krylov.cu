@@ -911,8 +911,8 @@ pfem2_status krylov_read_stats(Ctx& c) {
   PFEM2_CUDA(cudaMemcpy(&sticky, c.d_err_sticky, sizeof(int), cudaMemcpyDeviceToHost));
   if (err > 0 && err < 8) sticky |= 1 << err;
   if (sticky) {
-    PFEM2_CUDA(cudaMemset(c.d_err_sticky, 0, sizeof(int)));
-    PFEM2_CUDA(cudaMemset(c.d_err, 0, sizeof(int)));
+    PFEM2_CUDA(cudaMemsetAsync(c.d_err_sticky, 0, sizeof(int), c.stream));
+    PFEM2_CUDA(cudaMemsetAsync(c.d_err, 0, sizeof(int), c.stream));
   }
   if (sticky & 2) {
     set_error("krylov: a wait for the other blocks timed out");

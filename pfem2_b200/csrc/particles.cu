@@ -1545,10 +1545,12 @@ static pfem2_status set_impl(Ctx& c, const int* counts, const int* cell, const d
   PFEM2_CUDA(cudaMalloc(&dcell, sizeof(int) * nn));
   PFEM2_CUDA(cudaMalloc(&dxi, sizeof(double) * nn * DIM));
   PFEM2_CUDA(cudaMalloc(&du, sizeof(double) * nn * DIM));
-  PFEM2_CUDA(cudaMemcpy(dpos, pos.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-  PFEM2_CUDA(cudaMemcpy(dcell, gcell.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-  PFEM2_CUDA(cudaMemcpy(dxi, xi, sizeof(double) * n * DIM, cudaMemcpyHostToDevice));
-  PFEM2_CUDA(cudaMemcpy(du, u, sizeof(double) * n * DIM, cudaMemcpyHostToDevice));
+  // (on the context's stream, which does not wait for the default stream's
+  // copies: those may still be in flight when the call returns)
+  PFEM2_CUDA(cudaMemcpyAsync(dpos, pos.data(), sizeof(int) * n, cudaMemcpyHostToDevice, c.stream));
+  PFEM2_CUDA(cudaMemcpyAsync(dcell, gcell.data(), sizeof(int) * n, cudaMemcpyHostToDevice, c.stream));
+  PFEM2_CUDA(cudaMemcpyAsync(dxi, xi, sizeof(double) * n * DIM, cudaMemcpyHostToDevice, c.stream));
+  PFEM2_CUDA(cudaMemcpyAsync(du, u, sizeof(double) * n * DIM, cudaMemcpyHostToDevice, c.stream));
   if (n) {
     k_unpack_in<DIM, R><<<grid_for(c, n, 256), 256, 0, c.stream>>>((int)n, dpos, dcell, dxi, du, c.pcell[b],
                                                                  (R*)c.pxi[b], (R*)c.pu[b], (size_t)c.pcap);
