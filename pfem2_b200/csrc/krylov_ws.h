@@ -11,15 +11,6 @@ namespace pfem2 {
 
 constexpr int kMaxLocalSys = 16;  // systems a block of a solver grid may own parts of
 
-// a read-only array seen either in global memory (base 0) or through a
-// staged shared-memory copy of its range [base, ...)
-template <typename T>
-struct SV {
-  const T* p;
-  int base;
-  __device__ __forceinline__ T operator[](int i) const { return p[i - base]; }
-};
-
 __device__ __forceinline__ float fma_r(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double fma_r(double a, double b, double c) { return fma(a, b, c); }
 
@@ -55,17 +46,6 @@ __device__ __forceinline__ T sell_dot(T acc, Cols cols, int base, int len, int l
   return acc;
 }
 
-// x[col] from the shared mirror m of the block's own rows [own0, own0 +
-// nown) when there is one, else from global memory: one generic load, no
-// branch (plain loads see the other blocks' writes of the previous phase,
-// which the phase start's acquire ordered before them)
-template <typename R>
-__device__ __forceinline__ R ldm(const R* g, const R* m, int col, int own0, int nown) {
-  const unsigned o = (unsigned)(col - own0);
-  const R* src = (m != nullptr && o < (unsigned)nown) ? m + o : g + col;
-  return *src;
-}
-
 // acc + sum over CSR entries [k0, k1) of val(k) * x(col(k)), the lanes of a
 // group of GL taking every GL-th entry, loads issued CH entries at a time
 template <int GL, int CH, typename T, typename Cols, typename Val, typename X>
@@ -89,30 +69,16 @@ __device__ __forceinline__ T csr_dot(T acc, int k0, int k1, int sub, Cols cols, 
   return acc;
 }
 
-// copies src[lo, hi) into shared memory at `cur` (16-byte aligned pieces)
-// and returns the view of that range; the caller syncs before reading it
 __device__ __forceinline__ size_t al16_dev(size_t b) { return (b + 15) & ~(size_t)15; }
 
-template <typename T>
-__device__ __forceinline__ SV<T> stage_range(unsigned char*& cur, const T* src, int lo, int hi) {
-  T* dst = reinterpret_cast<T*>(cur);
-  for (int i = threadIdx.x; i < hi - lo; i += blockDim.x) dst[i] = src[lo + i];
-  cur += ((size_t)(hi - lo) * sizeof(T) + 15) & ~(size_t)15;
-  return SV<T>{dst, lo};
-}
-
-// the same without a base: element i of the copy is src[i]
+// copies src[0, n) into shared memory at `cur` (16-byte aligned pieces); the
+// caller syncs before reading it
 template <typename T>
 __device__ __forceinline__ const T* stage_copy(unsigned char*& cur, const T* src, int n) {
   T* dst = reinterpret_cast<T*>(cur);
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
   cur += al16_dev((size_t)n * sizeof(T));
   return dst;
-}
-
-template <typename T>
-__device__ __forceinline__ SV<T> maybe_stage(bool on, unsigned char*& cur, const T* src, int lo, int hi) {
-  return on ? stage_range(cur, src, lo, hi) : SV<T>{src, 0};
 }
 
 // Waits (acquire) until system counter *cnt has reached target (release adds

@@ -36,9 +36,9 @@
 //
 // Against the form before it (r' = r - alpha q restricted on the fly from two
 // gathered vectors, J2, E^-1 and Pt2 evaluated by every block for its whole
-// halo, barriers between the levels of one phase) an iteration takes 25 us
-// instead of 40 on the channel with disk (52k rows, FP32), 31 instead of 270
-// on a 10k-cell pipe (FP64), 75 instead of 420 on a 131k-cell pipe and 58
+// halo, barriers between the levels of one phase) an iteration takes 17 us
+// instead of 40 on the channel with disk (52k rows, FP32), 24 instead of 270
+// on a 10k-cell pipe (FP64), 47 instead of 420 on a 131k-cell pipe and 53
 // instead of 147 on a batch of 16 channels (282k rows).
 #include <algorithm>
 #include <cmath>
@@ -55,21 +55,25 @@ constexpr int kMgSums = 4;  // partial sums of a phase at most
 enum { T_OUT_A = 0, T_OUT_B, T_B, T_B2, T_X2, T_X1, T_UZ, T_A, T_DONE };
 enum { DO_NONE = 0, DO_OUT_A, DO_OUT_B, DO_FINISH, DO_B, DO_B2, DO_X2, DO_X1, DO_UZ, DO_A };
 
-// static data copied into shared memory at kernel start while the budget
-// lasts (every phase start's acquire invalidates L1, so static operands read
-// from global memory cost an L2 round trip per phase), in this order
+// What a block keeps in shared memory: bits of the template parameter SM (every
+// phase start's acquire invalidates L1, so static operands read from global
+// memory cost an L2 round trip per phase). Known at compile time: through
+// generic pointers a solve took 0.92 ms instead of 0.78 on the 52k channel and
+// 3.4 instead of 2.2 on the 131k pipe.
 enum {
-  SG_META = 1,   // row pointers and local system indices
-  SG_OWN = 2,    // the block's own rows of z, p, q, r, e, dq and J0 r
-  SG_COL = 4,    // SELL columns
-  SG_A = 8,      // SELL values
-  SG_M2 = 16,    // rows of M2
-  SG_Q2 = 32,    // Pt1^T
-  SG_P0 = 64,    // Pt0
-  SG_P1 = 128,   // Pt1 of the level-1 list
-  SG_J1 = 256,   // J1 of the level-1 list
-  SG_R1 = 512    // Pt0^T D
+  SG_OWN = 1,    // the block's own rows of z, p, q, r, e, dq, J0 r, 1 / D; row pointers and local systems
+  SG_COL = 2,    // SELL columns
+  SG_M2 = 4,     // rows of M2
+  SG_Q2 = 8,     // Pt1^T
+  SG_A = 16,     // SELL values
+  SG_P0 = 32,    // Pt0
+  SG_P1 = 64,    // Pt1 of the level-1 list
+  SG_J1 = 128,   // J1 of the level-1 list
+  SG_R1 = 256    // Pt0^T D
 };
+// the combinations compiled, largest first: everything (52k rows FP32), all but
+// the restriction (FP64), the vectors and small operators, nothing
+constexpr int kMgMask[] = {511, 255, 15, 0};
 
 template <typename R> struct MgArgs {
   int nv, nsys, ninst;
@@ -98,7 +102,7 @@ template <typename R> struct MgArgs {
   const R *j1_val, *p1_val;
   const int *sys_n2, *sys_off2;
   const double* sys_w;               // level-0 smoother weight
-  int stage, items_max, s1max, b2max;
+  int items_max, s1max, b2max;
   double* x;
   const double *b, *g;
   const unsigned char* isd;
@@ -156,7 +160,13 @@ __device__ __forceinline__ void slot_sums(const double* part, int stride, int t0
     for (int q = 0; q < N; ++q) s[q] += __shfl_xor_sync(PFEM2_FULL_MASK, s[q], o);
 }
 
-template <typename R, int NT, int MINB>
+template <bool ON, typename T>
+__device__ __forceinline__ const T* place(unsigned char*& cur, const T* src, int n) {
+  if constexpr (ON) return stage_copy(cur, src, n);
+  else return src;
+}
+
+template <typename R, int NT, int MINB, int SM>
 __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int NW = NT / 32;
@@ -184,47 +194,63 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
   const int o1lo = a.blk_o1[blockIdx.x], o1hi = a.blk_o1[blockIdx.x + 1];
   const int o2lo = a.blk_o2[blockIdx.x], o2hi = a.blk_o2[blockIdx.x + 1];
   const int s1lo = a.blk_s1[blockIdx.x], s1hi = a.blk_s1[blockIdx.x + 1];
-  const bool sm = a.stage & SG_META;
-  const SV<int> SLp = maybe_stage<int>(sm, cur, a.sl_ptr, bs0, bs1 + 1);
-  const SV<int> SLl = maybe_stage<int>(sm, cur, a.sl_len, bs0, bs1);
-  const SV<int> SLk = maybe_stage<int>(sm, cur, a.slk, bs0, bs1);
-  const SV<int> P0p = maybe_stage<int>(sm, cur, a.p0_ptr, bs0, bs1 + 1);
-  const SV<int> P0l = maybe_stage<int>(sm, cur, a.p0_len, bs0, bs1);
-  const SV<int> K1 = maybe_stage<int>(sm, cur, a.lk1, o1lo, o1hi);
-  const SV<int> R1p = maybe_stage<int>(sm, cur, a.r1_ptr, o1lo, o1hi + 1);
-  const SV<int> K2 = maybe_stage<int>(sm, cur, a.lk2, o2lo, o2hi);
-  const SV<int> Q2p = maybe_stage<int>(sm, cur, a.q2_ptr, o2lo, o2hi + 1);
-  const SV<int> M2o = maybe_stage<int>(sm, cur, a.m2_off, o2lo, o2hi);
-  const SV<int> S1k = maybe_stage<int>(sm, cur, a.s1_lk, s1lo, s1hi);
-  const SV<int> J1p = maybe_stage<int>(sm, cur, a.j1_ptr, s1lo, s1hi + 1);
-  const SV<int> P1p = maybe_stage<int>(sm, cur, a.p1_ptr, s1lo, s1hi + 1);
-  R *mz = nullptr, *mp = a.p + own0, *mq = a.q + own0, *mr = a.r + own0, *me = nullptr, *mdq = nullptr,
-    *mj = a.jr + own0;
-  if (a.stage & SG_OWN) {
-    R* m = reinterpret_cast<R*>(cur);
-    mz = m;
-    mp = m + nown;
-    mq = m + 2 * nown;
-    mr = m + 3 * nown;
-    me = m + 4 * nown;
-    mdq = m + 5 * nown;
-    mj = m + 6 * nown;
+  // (pointers by slice - bs0, level-1 dof - o1lo, level-2 dof - o2lo, level-1
+  // list entry - s1lo; columns and values by entry - first entry)
+  constexpr bool OWN = SM & SG_OWN;
+  const int no1 = o1hi - o1lo, no2 = o2hi - o2lo, ns1 = s1hi - s1lo;
+  const int* const SLp = place<OWN>(cur, a.sl_ptr + bs0, nitems + 1);
+  const int* const SLl = place<OWN>(cur, a.sl_len + bs0, nitems);
+  const int* const SLk = place<OWN>(cur, a.slk + bs0, nitems);
+  const int* const P0p = place<OWN>(cur, a.p0_ptr + bs0, nitems + 1);
+  const int* const P0l = place<OWN>(cur, a.p0_len + bs0, nitems);
+  const int* const K1 = place<OWN>(cur, a.lk1 + o1lo, no1);
+  const int* const R1p = place<OWN>(cur, a.r1_ptr + o1lo, no1 + 1);
+  const int* const K2 = place<OWN>(cur, a.lk2 + o2lo, no2);
+  const int* const Q2p = place<OWN>(cur, a.q2_ptr + o2lo, no2 + 1);
+  const int* const M2o = place<OWN>(cur, a.m2_off + o2lo, no2);
+  const int* const S1k = place<OWN>(cur, a.s1_lk + s1lo, ns1);
+  const int* const J1p = place<OWN>(cur, a.j1_ptr + s1lo, ns1 + 1);
+  const int* const P1p = place<OWN>(cur, a.p1_ptr + s1lo, ns1 + 1);
+  const R* const di0 = place<OWN>(cur, a.dinv + own0, nown);
+  R *lz, *mp, *mq, *mr, *le, *ldq, *mj;
+  if constexpr (OWN) {
+    lz = reinterpret_cast<R*>(cur);
+    mp = lz + nown;
+    mq = lz + 2 * nown;
+    mr = lz + 3 * nown;
+    le = lz + 4 * nown;
+    ldq = lz + 5 * nown;
+    mj = lz + 6 * nown;
     cur += al16_dev((size_t)7 * nown * sizeof(R));
+  } else {
+    lz = a.z + own0;
+    mp = a.p + own0;
+    mq = a.q + own0;
+    mr = a.r + own0;
+    le = a.e + own0;
+    ldq = a.dq + own0;
+    mj = a.jr + own0;
   }
-  const SV<int> SLc = maybe_stage<int>(a.stage & SG_COL, cur, a.sl_col, a.sl_ptr[bs0], a.sl_ptr[bs1]);
-  const SV<R> SLa = maybe_stage<R>(a.stage & SG_A, cur, a.A, a.sl_ptr[bs0], a.sl_ptr[bs1]);
+  const int e0 = a.sl_ptr[bs0], ne = a.sl_ptr[bs1] - e0;
+  const int* const SLc = place<(SM & SG_COL) != 0>(cur, a.sl_col + e0, ne);
   const long long m2lo = a.blk_m2[blockIdx.x];
-  const SV<R> M2 = maybe_stage<R>(a.stage & SG_M2, cur, a.m2 + m2lo, 0, (int)(a.blk_m2[blockIdx.x + 1] - m2lo));
-  const SV<int> Q2c = maybe_stage<int>(a.stage & SG_Q2, cur, a.q2_col, a.q2_ptr[o2lo], a.q2_ptr[o2hi]);
-  const SV<R> Q2v = maybe_stage<R>(a.stage & SG_Q2, cur, a.q2_val, a.q2_ptr[o2lo], a.q2_ptr[o2hi]);
-  const SV<int> P0c = maybe_stage<int>(a.stage & SG_P0, cur, a.p0_col, a.p0_ptr[bs0], a.p0_ptr[bs1]);
-  const SV<R> P0v = maybe_stage<R>(a.stage & SG_P0, cur, a.p0_val, a.p0_ptr[bs0], a.p0_ptr[bs1]);
-  const SV<int> P1c = maybe_stage<int>(a.stage & SG_P1, cur, a.p1_col, a.p1_ptr[s1lo], a.p1_ptr[s1hi]);
-  const SV<R> P1v = maybe_stage<R>(a.stage & SG_P1, cur, a.p1_val, a.p1_ptr[s1lo], a.p1_ptr[s1hi]);
-  const SV<int> J1c = maybe_stage<int>(a.stage & SG_J1, cur, a.j1_col, a.j1_ptr[s1lo], a.j1_ptr[s1hi]);
-  const SV<R> J1v = maybe_stage<R>(a.stage & SG_J1, cur, a.j1_val, a.j1_ptr[s1lo], a.j1_ptr[s1hi]);
-  const SV<int> R1c = maybe_stage<int>(a.stage & SG_R1, cur, a.r1_col, a.r1_ptr[o1lo], a.r1_ptr[o1hi]);
-  const SV<R> R1v = maybe_stage<R>(a.stage & SG_R1, cur, a.r1_val, a.r1_ptr[o1lo], a.r1_ptr[o1hi]);
+  const R* const M2 = place<(SM & SG_M2) != 0>(cur, a.m2 + m2lo, (int)(a.blk_m2[blockIdx.x + 1] - m2lo));
+  const int q20 = a.q2_ptr[o2lo], nq2 = a.q2_ptr[o2hi] - q20;
+  const int* const Q2c = place<(SM & SG_Q2) != 0>(cur, a.q2_col + q20, nq2);
+  const R* const Q2v = place<(SM & SG_Q2) != 0>(cur, a.q2_val + q20, nq2);
+  const R* const SLa = place<(SM & SG_A) != 0>(cur, a.A + e0, ne);
+  const int p00 = a.p0_ptr[bs0], np0 = a.p0_ptr[bs1] - p00;
+  const int* const P0c = place<(SM & SG_P0) != 0>(cur, a.p0_col + p00, np0);
+  const R* const P0v = place<(SM & SG_P0) != 0>(cur, a.p0_val + p00, np0);
+  const int p10 = a.p1_ptr[s1lo], np1 = a.p1_ptr[s1hi] - p10;
+  const int* const P1c = place<(SM & SG_P1) != 0>(cur, a.p1_col + p10, np1);
+  const R* const P1v = place<(SM & SG_P1) != 0>(cur, a.p1_val + p10, np1);
+  const int j10 = a.j1_ptr[s1lo], nj1 = a.j1_ptr[s1hi] - j10;
+  const int* const J1c = place<(SM & SG_J1) != 0>(cur, a.j1_col + j10, nj1);
+  const R* const J1v = place<(SM & SG_J1) != 0>(cur, a.j1_val + j10, nj1);
+  const int r10 = a.r1_ptr[o1lo], nr1 = a.r1_ptr[o1hi] - r10;
+  const int* const R1c = place<(SM & SG_R1) != 0>(cur, a.r1_col + r10, nr1);
+  const R* const R1v = place<(SM & SG_R1) != 0>(cur, a.r1_val + r10, nr1);
 
   // ---- local systems (consecutive), their items, own level-2 offsets
   if (threadIdx.x == 0) {
@@ -260,11 +286,8 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
     const int row = own0 + i;
     if (a.isd[row]) a.x[row] = a.g ? a.g[row] : 0.0;
     a.e[row] = R(0);
-    if (me) me[i] = R(0);
+    if (OWN) le[i] = R(0);
   }
-  R* const le = me ? me : a.e + own0;
-  R* const lz = mz ? mz : a.z + own0;
-  R* const ldq = mdq ? mdq : a.dq + own0;
   if (!grid_sync_ra(a.gb, bar_gen)) return;
 
   for (int iter = 0;; ++iter) {
@@ -385,11 +408,11 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
         const int sub = threadIdx.x % GL, grp = threadIdx.x / GL;
         for (int base = o1lo; base < o1hi; base += NG) {
           const int i = base + grp;
-          const bool on = i < o1hi && sa[K1[i]].act == DO_B;
+          const bool on = i < o1hi && sa[K1[i - o1lo]].act == DO_B;
           R acc = R(0);
           if (on)
-            acc = csr_dot<GL, 8, R>(acc, R1p[i], R1p[i + 1], sub, R1c, R1v,
-                                    [&](int j) { return ldm(a.dq, mdq, j, own0, nown); });
+            acc = csr_dot<GL, 8, R>(acc, R1p[i - o1lo] - r10, R1p[i - o1lo + 1] - r10, sub, R1c, R1v,
+                                    [&](int j) { return a.dq[j]; });
           acc = group_sum<GL>(acc);
           if (on && sub == 0) a.c1[i] = acc;
         }
@@ -399,14 +422,14 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
     }
     if (acts & (1u << DO_B2)) {
       for (int i = o2lo + warp; i < o2hi; i += NW) {
-        const MgAct& L = sa[K2[i]];
+        const MgAct& L = sa[K2[i - o2lo]];
         if (L.act != DO_B2 || L.stop) continue;
-        R acc = csr_dot<32, CH, R>(R(0), Q2p[i], Q2p[i + 1], lane, Q2c, Q2v, [&](int c) { return __ldcg(a.c1 + c); });
+        R acc = csr_dot<32, CH, R>(R(0), Q2p[i - o2lo] - q20, Q2p[i - o2lo + 1] - q20, lane, Q2c, Q2v, [&](int c) { return __ldcg(a.c1 + c); });
         acc = warp_sum(acc);
         if (lane == 0) a.b2[i] = L.restart ? acc : fma_r(-R(L.alpha), acc, a.b2[i]);
       }
       for (int i = o1hi - 1 - (int)threadIdx.x; i >= o1lo; i -= NT) {
-        const MgAct& L = sa[K1[i]];
+        const MgAct& L = sa[K1[i - o1lo]];
         if (L.act != DO_B2 || L.stop) continue;
         a.b1[i] = L.restart ? a.c1[i] : fma_r(-R(L.alpha), a.c1[i], a.b1[i]);
       }
@@ -418,10 +441,10 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
       }
       __syncthreads();
       for (int i = o2lo + warp; i < o2hi; i += NW) {
-        const MgSys& L = ls[K2[i]];
-        if (sa[K2[i]].act != DO_X2) continue;
+        const MgSys& L = ls[K2[i - o2lo]];
+        if (sa[K2[i - o2lo]].act != DO_X2) continue;
         const R* bb = sb2 + L.b2off;
-        const int m0 = M2o[i], n2 = L.n2;
+        const int m0 = M2o[i - o2lo], n2 = L.n2;
         R acc = R(0);
         for (int d0 = lane; d0 < n2; d0 += 256) {
           R mv[8];
@@ -442,8 +465,8 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
       for (int base = s1lo; base < s1hi; base += NG) {
         const int j = base + grp;
         R acc = R(0);
-        const bool on = j < s1hi && sa[S1k[j]].act == want;
-        if (on) acc = csr_dot<GL, 8, R>(acc, P1p[j], P1p[j + 1], sub, P1c, P1v, [&](int c) { return __ldcg(a.x2 + c); });
+        const bool on = j < s1hi && sa[S1k[j - s1lo]].act == want;
+        if (on) acc = csr_dot<GL, 8, R>(acc, P1p[j - s1lo] - p10, P1p[j - s1lo + 1] - p10, sub, P1c, P1v, [&](int c) { return __ldcg(a.x2 + c); });
         acc = group_sum<GL>(acc);
         if (on && sub == 0) {
           acc += sx1[j - s1lo];
@@ -455,16 +478,15 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
     }
     // ---- level-0 rows, a warp per slice
     for (int it = warp; it < nitems; it += NW) {
-      const int sl = bs0 + it;
-      const MgAct& L = sa[SLk[sl]];
+      const MgAct& L = sa[SLk[it]];
       const int act = L.act;
       if (act == DO_NONE || act == DO_B || act == DO_X2 || act == DO_X1) continue;
-      const int o = it * 32 + lane, row = own0 + o;
+      const int o = it * 32 + lane, row = own0 + o, c0 = SLp[it] - e0, len = SLl[it];
       double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
       if (act == DO_A) {
-        const R di = a.dinv[row];
-        const R acc = sell_dot<R, CH>(R(0), SLc, SLp[sl], SLl[sl], lane, [&](int ei) { return SLa[ei]; },
-                                      [&](int col) { return ldm(a.z, mz, col, own0, nown); });
+        const R di = di0[o];
+        const R acc = sell_dot<R, CH>(R(0), SLc, c0, len, lane, [&](int ei) { return SLa[ei]; },
+                                      [&](int col) { return a.z[col]; });
         const R be = R(L.beta);
         R qq = acc, pp = lz[o];
         if (!L.first) {
@@ -475,7 +497,7 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
         mp[o] = pp;
         const R dd = di * qq;
         a.dq[row] = dd;
-        if (mdq) mdq[o] = dd;
+        if (OWN) ldq[o] = dd;
         v0 = (double)pp * (double)qq;
         v1 = (double)mr[o] * (double)qq;
         v2 = (double)qq * (double)qq;
@@ -486,22 +508,23 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
           const R ee = fma_r(al, mp[o], le[o]);
           le[o] = ee;
           mr[o] = fma_r(-al, mq[o], mr[o]);
-          if (me && L.stop) a.e[row] = ee;
+          if (OWN && L.stop) a.e[row] = ee;
         }
         continue;
       } else if (act == DO_UZ) {
-        const R acc = a.xsplit ? sell_dot<R, CH>(mj[o], P0c, P0p[sl], P0l[sl], lane, [&](int ei) { return P0v[ei]; },
-                                                 [&](int col) { return __ldcg(a.x1 + col); })
-                               : sell_dot<R, CH>(mj[o], P0c, P0p[sl], P0l[sl], lane, [&](int ei) { return P0v[ei]; },
+        const int p0 = P0p[it] - p00, pl = P0l[it];
+        const R acc = a.xsplit ? sell_dot<R, CH>(mj[o], P0c, p0, pl, lane, [&](int ei) { return P0v[ei]; },
+                                                 [&](int col) { return a.x1[col]; })
+                               : sell_dot<R, CH>(mj[o], P0c, p0, pl, lane, [&](int ei) { return P0v[ei]; },
                                                  [&](int col) { return sx1[col]; });
         a.z[row] = acc;
-        if (mz) mz[o] = acc;
+        if (OWN) lz[o] = acc;
         v0 = (double)mr[o] * (double)acc;
       } else if (act == DO_OUT_A) {
         const double bb = a.b[row];
         const double acc = sell_dot<double, CH>(
-            0.0, SLc, SLp[sl], SLl[sl], lane, [&](int ei) { return a.A64[ei]; },
-            [&](int col) { return __ldcg(a.x + col) + (double)ldm(a.e, me, col, own0, nown); });
+            0.0, SLc, c0, len, lane, [&](int ei) { return a.A64[e0 + ei]; },
+            [&](int col) { return __ldcg(a.x + col) + (double)__ldcg(a.e + col); });
         const double rr = bb - acc;
         a.r64[row] = rr;
         v0 = rr * rr;
@@ -512,9 +535,9 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
         if (act == DO_OUT_B) {
           const R rr = R(a.r64[row]);
           mr[o] = rr;
-          const R dd = a.dinv[row] * rr;
+          const R dd = di0[o] * rr;
           a.dq[row] = dd;
-          if (mdq) mdq[o] = dd;
+          if (OWN) ldq[o] = dd;
         }
         continue;
       }
@@ -559,13 +582,12 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
     const int w0 = nls < NW / 4 ? nls : 0;
     if ((acts & (1u << DO_B2)) && warp >= w0) {
       for (int it = warp - w0; it < nitems; it += NW - w0) {
-        const int sl = bs0 + it;
-        const MgAct& L = sa[SLk[sl]];
+        const MgAct& L = sa[SLk[it]];
         if (L.act != DO_B2 || L.stop) continue;
         const int o = it * 32 + lane;
-        const R di = a.dinv[own0 + o], w = R(ls[SLk[sl]].w);
-        const R acc = sell_dot<R, CH>(R(0), SLc, SLp[sl], SLl[sl], lane, [&](int ei) { return SLa[ei]; },
-                                      [&](int col) { return ldm(a.dq, mdq, col, own0, nown); });
+        const R di = di0[o], w = R(ls[SLk[it]].w);
+        const R acc = sell_dot<R, CH>(R(0), SLc, SLp[it] - e0, SLl[it], lane, [&](int ei) { return SLa[ei]; },
+                                      [&](int col) { return a.dq[col]; });
         const R jq = w * fma_r(-w * di, acc, R(2) * ldq[o]);
         mj[o] = L.restart ? jq : fma_r(-R(L.alpha), jq, mj[o]);
       }
@@ -577,8 +599,8 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
       for (int base = s1lo; base < s1hi; base += NG) {
         const int j = base + grp;
         R acc = R(0);
-        const bool on = j < s1hi && sa[S1k[j]].act == DO_X2;
-        if (on) acc = csr_dot<GL, 8, R>(acc, J1p[j], J1p[j + 1], sub, J1c, J1v, [&](int c) { return __ldcg(a.b1 + c); });
+        const bool on = j < s1hi && sa[S1k[j - s1lo]].act == DO_X2;
+        if (on) acc = csr_dot<GL, 8, R>(acc, J1p[j - s1lo] - j10, J1p[j - s1lo + 1] - j10, sub, J1c, J1v, [&](int c) { return __ldcg(a.b1 + c); });
         acc = group_sum<GL>(acc);
         if (on && sub == 0) sx1[j - s1lo] = acc;
       }
@@ -590,7 +612,7 @@ __global__ void __launch_bounds__(NT, MINB) k_mgcg(MgArgs<R> a) {
 
 // ------------------------------------------------------------------ host
 struct MgWs {
-  int minb = 1, grid = 0, nsys = 0, nslots = 0, stage = 0;
+  int minb = 1, grid = 0, nsys = 0, nslots = 0, mask = 0;  // mask: index into kMgMask
   size_t smem = 0;
   bool wide = false, xsplit = false;
   int items_max = 0, s1max = 0, b2max = 0;
@@ -618,12 +640,19 @@ namespace {
 
 constexpr int mg_threads(int minb) { return minb == 1 ? 512 : 384; }
 
-template <typename R>
-const void* mg_kernel(int minb) {
-  return minb == 1 ? (const void*)k_mgcg<R, mg_threads(1), 1> : (const void*)k_mgcg<R, mg_threads(2), 2>;
+template <typename R, int MINB>
+const void* mg_kernel(int mask) {
+  constexpr int NT = mg_threads(MINB);
+  return mask == 0   ? (const void*)k_mgcg<R, NT, MINB, kMgMask[0]>
+         : mask == 1 ? (const void*)k_mgcg<R, NT, MINB, kMgMask[1]>
+         : mask == 2 ? (const void*)k_mgcg<R, NT, MINB, kMgMask[2]>
+                     : (const void*)k_mgcg<R, NT, MINB, kMgMask[3]>;
 }
 
-const void* mg_kernel_any(bool mixed, int minb) { return mixed ? mg_kernel<float>(minb) : mg_kernel<double>(minb); }
+template <typename R>
+const void* mg_kernel(int minb, int mask) {
+  return minb == 1 ? mg_kernel<R, 1>(mask) : mg_kernel<R, 2>(mask);
+}
 
 }  // namespace
 
@@ -711,7 +740,7 @@ pfem2_status mg_setup(Ctx& c) {
   // the budget lasts (maximum over blocks; the kernel stages the same pieces)
   const size_t rs = c.kmixed ? sizeof(float) : sizeof(double), i4 = 4;
   size_t smem = al16(sizeof(double) * kMgSums * m->items_max) + al16(rs * m->s1max) + al16(rs * m->b2max);
-  constexpr int NC = 10;
+  constexpr int NC = 9;
   size_t cat[NC] = {};
   for (int b = 0; b < G; ++b) {
     const int s0 = bsl[2 * b], s1 = bsl[2 * b + 1], ns = s1 - s0;
@@ -722,12 +751,12 @@ pfem2_status mg_setup(Ctx& c) {
     const size_t nj = H.j1_ptr[l1] - H.j1_ptr[l0], np = H.p1_ptr[l1] - H.p1_ptr[l0];
     const size_t nr = H.r1_ptr[bo1[b + 1]] - H.r1_ptr[bo1[b]];
     const size_t v[NC] = {2 * al16(i4 * (ns + 1)) + 3 * al16(i4 * ns) + al16(i4 * n1) + al16(i4 * (n1 + 1)) +
-                              2 * al16(i4 * n2) + al16(i4 * (n2 + 1)) + al16(i4 * nl) + 2 * al16(i4 * (nl + 1)),
-                          al16(rs * 7 * 32 * ns),
+                              2 * al16(i4 * n2) + al16(i4 * (n2 + 1)) + al16(i4 * nl) + 2 * al16(i4 * (nl + 1)) +
+                              al16(rs * 32 * ns) + al16(rs * 7 * 32 * ns),
                           al16(i4 * ne),
-                          al16(rs * ne),
                           al16(rs * nm),
                           al16(i4 * nq) + al16(rs * nq),
+                          al16(rs * ne),
                           al16(i4 * np0) + al16(rs * np0),
                           al16(i4 * np) + al16(rs * np),
                           al16(i4 * nj) + al16(rs * nj),
@@ -739,17 +768,20 @@ pfem2_status mg_setup(Ctx& c) {
     set_error("krylov: the pressure multigrid's per-block data exceed shared memory");
     return PFEM2_INVALID_ARG;
   }
-  for (int k = 0; k < NC; ++k)
-    if (smem + cat[k] <= budget) {
-      m->stage |= 1 << k;
-      smem += cat[k];
+  for (m->mask = 0;; ++m->mask) {
+    size_t need = smem;
+    for (int k = 0; k < NC; ++k)
+      if (kMgMask[m->mask] >> k & 1) need += cat[k];
+    if (need <= budget) {
+      m->smem = need;
+      break;
     }
-  m->smem = smem;
-  const void* kern = mg_kernel_any(c.kmixed, m->minb);
+  }
+  const void* kern = c.kmixed ? mg_kernel<float>(m->minb, m->mask) : mg_kernel<double>(m->minb, m->mask);
   // one process-wide upper bound, so contexts with different hierarchies coexist
   PFEM2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
   int occ = 0;
-  PFEM2_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, mg_threads(m->minb), smem));
+  PFEM2_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, mg_threads(m->minb), m->smem));
   if (occ * c.num_sms < G) {
     set_error("krylov: the multigrid solver grid cannot be resident");
     return PFEM2_CUDA_ERROR;
@@ -849,7 +881,6 @@ pfem2_status mg_solve_impl(Ctx& c) {
   a.j1_ptr = m->j1_ptr; a.j1_col = m->j1_col; a.j1_val = (const R*)m->j1_val;
   a.p1_ptr = m->p1_ptr; a.p1_col = m->p1_col; a.p1_val = (const R*)m->p1_val;
   a.sys_n2 = m->sys_n2; a.sys_off2 = m->sys_off2; a.sys_w = m->sys_w;
-  a.stage = m->stage;
   a.items_max = m->items_max;
   a.s1max = m->s1max;
   a.b2max = m->b2max;
@@ -881,7 +912,7 @@ pfem2_status mg_solve_impl(Ctx& c) {
   a.gb.spin_limit = c.spin_limit;
   PFEM2_TRY(krylov_init_solve(c, a.nsys));
   void* args[] = {&a};
-  PFEM2_CUDA(cudaLaunchCooperativeKernel(mg_kernel<R>(m->minb), dim3(m->grid), dim3(mg_threads(m->minb)), args,
+  PFEM2_CUDA(cudaLaunchCooperativeKernel(mg_kernel<R>(m->minb, m->mask), dim3(m->grid), dim3(mg_threads(m->minb)), args,
                                          m->smem, c.stream));
   c.launches++;
   return PFEM2_OK;
