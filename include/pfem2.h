@@ -191,9 +191,9 @@ typedef struct {
    * (0 = PFEM2_FP32_DEFAULT). Ignored by PFEM2_PREC_FP64. */
   int32_t fp32_stages;
   /* 1: the mesh moves (pfem2_mesh_elasticity / pfem2_move_mesh, 2D, one
-   * instance): the matrices are reassembled every step and the pressure is
-   * solved without the multigrid hierarchy, which is built once on the host
-   * (CG with Jacobi, or BiCGStab with Jacobi as p_solver says). */
+   * instance): the matrices are reassembled every step; the pressure's
+   * multigrid hierarchy stays that of the mesh at pfem2_setup (CG), or the
+   * pressure is solved by BiCGStab with Jacobi, as p_solver says. */
   int32_t moving_mesh;
   int32_t pad_;
 } pfem2_config;

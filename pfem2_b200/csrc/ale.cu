@@ -7,14 +7,17 @@
 // per-cell records, and the particles' relocation in the moved mesh
 // (sort_particles_into_subdomains_and_cells, then check_empty_cells).
 //
-// The elasticity system couples the dim displacement components: its
-// dim x dim blocks live on the scalar SELL pattern (entry 0 of a row is the
-// diagonal), assembled node-centric like the flow matrices (a thread owns a
-// row and sums its cells in ascending order: deterministic, no atomics),
-// Dirichlet rows and columns eliminated symmetrically, then solved by one
-// persistent cooperative CG kernel (Jacobi, FP64) with two grid barriers per
-// iteration and per-block partial sums that every block adds in the same
-// order, so that all blocks take the same decisions.
+// The elasticity system couples the dim displacement components. It is one
+// scalar system of dim x nv rows, components one after the other, on slices
+// of its own: slice c nslices + s holds rows c nv + 32 s ..., with the entries
+// of the scalar pattern's slice s once per column component. Assembly is
+// node-centric like the flow matrices (a thread owns a vertex' rows and sums
+// its cells in ascending order: deterministic, no atomics), Dirichlet rows and
+// columns are eliminated symmetrically, and the flow's Jacobi CG kernel solves
+// it (krylov.cu, FP64, one reduction per iteration, one thread-block cluster
+// for small meshes): 8.2 us per
+// iteration on a mesh of 8k cells against 11.6 with two reductions and a grid
+// barrier after each.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -25,28 +28,31 @@
 
 namespace pfem2 {
 
-constexpr int kAleThreads = 256;
-
 __device__ __forceinline__ int ale_entry(const int* __restrict__ sl_ptr, int row, int j) {
   return sl_ptr[row >> 5] + j * 32 + (row & 31);
 }
 
-// K[ci * DIM + cj][(a, b)] += sum over the cells around a and their QGauss(2)
-// points of (lambda d_ci N_a d_cj N_b + mu d_cj N_a d_ci N_b
+// entry e of vertex row `row` in the scalar pattern, row component a, column
+// component b (nell entries in the scalar pattern)
+template <int DIM>
+__device__ __forceinline__ size_t el_entry(const int* __restrict__ sl_ptr, const int* __restrict__ sl_len, int nell,
+                                           int row, int e, int a, int b) {
+  const int s = row >> 5, p = sl_ptr[s];
+  return (size_t)DIM * ((size_t)a * nell + p) + (size_t)b * sl_len[s] * 32 + (e - p);
+}
+
+// K[(a, ci), (b, cj)] += sum over the cells around vertex a and their
+// QGauss(2) points of (lambda d_ci N_a d_cj N_b + mu d_cj N_a d_ci N_b
 // + delta_ci,cj mu grad N_a . grad N_b) JxW
 template <int DIM>
-__global__ void __launch_bounds__(128) k_elastic_assemble(int nv, const int* __restrict__ v2c_ptr,
+__global__ void __launch_bounds__(128) k_elastic_assemble(int nv, int nell, const int* __restrict__ v2c_ptr,
                                                           const int* __restrict__ v2c_cell,
                                                           const unsigned char* __restrict__ v2c_loc,
-                                                          const int* __restrict__ inc_slot, const double* __restrict__ X,
+                                                          const int* __restrict__ inc_slot, const int* __restrict__ sl_ptr,
+                                                          const int* __restrict__ sl_len, const double* __restrict__ X,
                                                           const int* __restrict__ cv, double lambda, double mu,
-                                                          double* __restrict__ K0, double* __restrict__ K1,
-                                                          double* __restrict__ K2, double* __restrict__ K3,
-                                                          double* __restrict__ K4, double* __restrict__ K5,
-                                                          double* __restrict__ K6, double* __restrict__ K7,
-                                                          double* __restrict__ K8) {
+                                                          double* __restrict__ K) {
   constexpr int NV = Dims<DIM>::NV;
-  double* K[9] = {K0, K1, K2, K3, K4, K5, K6, K7, K8};
   for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < nv; row += gridDim.x * blockDim.x) {
     for (int k = v2c_ptr[row]; k < v2c_ptr[row + 1]; ++k) {
       const int c = v2c_cell[k], la = v2c_loc[k];
@@ -69,7 +75,7 @@ __global__ void __launch_bounds__(128) k_elastic_assemble(int nv, const int* __r
             for (int cj = 0; cj < DIM; ++cj) {
               double v = lambda * q.G[la][ci] * q.G[lb][cj] + mu * q.G[la][cj] * q.G[lb][ci];
               if (ci == cj) v += mu * gg;
-              K[ci * DIM + cj][e] += v * q.JxW;
+              K[el_entry<DIM>(sl_ptr, sl_len, nell, row, e, ci, cj)] += v * q.JxW;
             }
         }
       }
@@ -82,17 +88,14 @@ __global__ void __launch_bounds__(128) k_elastic_assemble(int nv, const int* __r
 // blocks' diagonal (1 where it is 0: padding rows) and gets rhs = K_aa g_a;
 // a free row moves its constrained columns to the right-hand side
 template <int DIM>
-__global__ void k_elastic_eliminate(int nv, const int* __restrict__ sl_ptr, const int* __restrict__ sl_len,
-                                    const int* __restrict__ sl_col, double* __restrict__ K0, double* __restrict__ K1,
-                                    double* __restrict__ K2, double* __restrict__ K3, double* __restrict__ K4,
-                                    double* __restrict__ K5, double* __restrict__ K6, double* __restrict__ K7,
-                                    double* __restrict__ K8, const unsigned char* __restrict__ fix,
-                                    const double* __restrict__ g, double* __restrict__ rhs,
-                                    double* __restrict__ dinv) {
-  double* K[9] = {K0, K1, K2, K3, K4, K5, K6, K7, K8};
+__global__ void k_elastic_eliminate(int nv, int nell, const int* __restrict__ sl_ptr, const int* __restrict__ sl_len,
+                                    const int* __restrict__ sl_col, double* __restrict__ K,
+                                    const unsigned char* __restrict__ fix, const double* __restrict__ g,
+                                    double* __restrict__ rhs, double* __restrict__ dinv) {
   for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < nv; row += gridDim.x * blockDim.x) {
     const int len = sl_len[row >> 5];
     const int e0 = ale_entry(sl_ptr, row, 0);
+    const auto at = [&](int e, int a, int b) -> double& { return K[el_entry<DIM>(sl_ptr, sl_len, nell, row, e, a, b)]; };
     if (fix[row]) {
       for (int j = 0; j < len; ++j) {
         const int e = ale_entry(sl_ptr, row, j);
@@ -101,11 +104,11 @@ __global__ void k_elastic_eliminate(int nv, const int* __restrict__ sl_ptr, cons
         for (int a = 0; a < DIM; ++a)
 #pragma unroll
           for (int b = 0; b < DIM; ++b)
-            if (!(diag && a == b)) K[a * DIM + b][e] = 0.0;
+            if (!(diag && a == b)) at(e, a, b) = 0.0;
       }
 #pragma unroll
       for (int a = 0; a < DIM; ++a) {
-        double& d = K[a * DIM + a][e0];
+        double& d = at(e0, a, a);
         if (d == 0.0) d = 1.0;
         rhs[(size_t)a * nv + row] = d * g[(size_t)a * nv + row];
         dinv[(size_t)a * nv + row] = 1.0 / d;
@@ -122,207 +125,16 @@ __global__ void k_elastic_eliminate(int nv, const int* __restrict__ sl_ptr, cons
         for (int a = 0; a < DIM; ++a)
 #pragma unroll
           for (int b = 0; b < DIM; ++b) {
-            s[a] -= K[a * DIM + b][e] * g[(size_t)b * nv + col];
-            K[a * DIM + b][e] = 0.0;
+            s[a] -= at(e, a, b) * g[(size_t)b * nv + col];
+            at(e, a, b) = 0.0;
           }
       }
 #pragma unroll
       for (int a = 0; a < DIM; ++a) {
         rhs[(size_t)a * nv + row] = s[a];
-        dinv[(size_t)a * nv + row] = 1.0 / K[a * DIM + a][e0];
+        dinv[(size_t)a * nv + row] = 1.0 / at(e0, a, a);
       }
     }
-  }
-}
-
-struct ElasticArgs {
-  int nv, maxit;
-  double tol, rtol;
-  const int *sl_ptr, *sl_len, *sl_col;
-  const double* K[9];
-  const double *rhs, *dinv, *g;
-  const unsigned char* fix;
-  double *x, *r, *z, *q, *p;  // p: 2 buffers of [dim][nv]
-  double* part;               // [2][grid][4]
-  int* out;                   // iterations, converged
-  double* res;                // final residual, tolerance
-  GridBarrier gb;
-};
-
-// block sum of NS values in a fixed order (warp shuffles, then warp 0)
-template <int NS>
-__device__ __forceinline__ void block_sums(double* v, double* out) {
-  __shared__ double sh[kAleThreads / 32][NS];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-  for (int k = 0; k < NS; ++k) v[k] = warp_sum(v[k]);
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < NS; ++k) sh[warp][k] = v[k];
-  __syncthreads();
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int k = 0; k < NS; ++k) {
-      double s = 0.0;
-      for (int w = 0; w < kAleThreads / 32; ++w) s += sh[w][k];
-      out[k] = s;
-    }
-  __syncthreads();
-}
-
-// every block adds the blocks' partials in block order (same result in all)
-template <int NS>
-__device__ __forceinline__ void grid_sums(const double* part, double* out) {
-  __shared__ double sh[NS];
-  if (threadIdx.x < 32) {
-    double s[NS];
-#pragma unroll
-    for (int k = 0; k < NS; ++k) s[k] = 0.0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += 32)
-#pragma unroll
-      for (int k = 0; k < NS; ++k) s[k] += __ldcg(part + (size_t)b * 4 + k);
-#pragma unroll
-    for (int k = 0; k < NS; ++k) s[k] = warp_sum(s[k]);
-    if (threadIdx.x == 0)
-#pragma unroll
-      for (int k = 0; k < NS; ++k) sh[k] = s[k];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < NS; ++k) out[k] = sh[k];
-  __syncthreads();
-}
-
-// y_a(row) = sum_b sum_entries K_ab x_b(col), x_b(col) given by the functor
-template <int DIM, typename XF>
-__device__ __forceinline__ void kmul_row(const ElasticArgs& a, int row, XF xf, double* y) {
-  const int len = a.sl_len[row >> 5];
-#pragma unroll
-  for (int c = 0; c < DIM; ++c) y[c] = 0.0;
-  for (int j = 0; j < len; ++j) {
-    const int e = ale_entry(a.sl_ptr, row, j);
-    const int col = a.sl_col[e];
-    double xv[DIM];
-#pragma unroll
-    for (int b = 0; b < DIM; ++b) xv[b] = xf(b, col);
-#pragma unroll
-    for (int c = 0; c < DIM; ++c)
-#pragma unroll
-      for (int b = 0; b < DIM; ++b) y[c] += a.K[c * DIM + b][e] * xv[b];
-  }
-}
-
-// The partial sums of consecutive reductions alternate between two buffers
-// of [grid][4]: a block writes reduction k + 1 while slower blocks may still
-// read reduction k, and reduction k + 2 only after the barrier that all of
-// them passed after reading k.
-template <int DIM>
-__global__ void __launch_bounds__(kAleThreads) k_elastic_cg(ElasticArgs a) {
-  const size_t nv = (size_t)a.nv;
-  const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gstride = gridDim.x * blockDim.x;
-  unsigned bar = 0;
-  int red = 0;  // reductions so far (buffer parity)
-  auto publish = [&](const double* v, int ns) {
-    if (threadIdx.x == 0)
-      for (int k = 0; k < ns; ++k) a.part[(size_t)(red & 1) * gridDim.x * 4 + blockIdx.x * 4 + k] = v[k];
-  };
-  auto buf = [&]() { return a.part + (size_t)(red & 1) * gridDim.x * 4; };
-  // x0 = g on the constrained vertices, 0 elsewhere
-  for (int row = gtid; row < a.nv; row += gstride)
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) a.x[c * nv + row] = a.fix[row] ? a.g[c * nv + row] : 0.0;
-  if (!grid_sync_ra(a.gb, bar)) return;
-  // r = b - K x0, z = D^-1 r; |r|^2, |b|^2, (r, z)
-  double s0[3];
-  {
-    double v[3] = {0.0, 0.0, 0.0};
-    for (int row = gtid; row < a.nv; row += gstride) {
-      double y[DIM];
-      kmul_row<DIM>(a, row, [&](int b, int col) { return __ldcg(a.x + b * nv + col); }, y);
-#pragma unroll
-      for (int c = 0; c < DIM; ++c) {
-        const double bb = a.rhs[c * nv + row], rr = bb - y[c];
-        const double zz = rr * a.dinv[c * nv + row];
-        a.r[c * nv + row] = rr;
-        a.z[c * nv + row] = zz;
-        v[0] += rr * rr;
-        v[1] += bb * bb;
-        v[2] += rr * zz;
-      }
-    }
-    double out[3];
-    block_sums<3>(v, out);
-    publish(out, 3);
-  }
-  if (!grid_sync_ra(a.gb, bar)) return;
-  grid_sums<3>(buf(), s0);
-  ++red;
-  const double tol = fmax(a.tol, a.rtol * sqrt(s0[1]));
-  double res = sqrt(s0[0]), rho = s0[2], beta = 0.0;
-  int it = 0, par = 0;
-  bool ok = res <= tol;
-  while (!ok && it < a.maxit) {
-    // A: p' = z + beta p (formed on the fly at the columns), q = K p', (p', q)
-    const double* po = a.p + (size_t)par * DIM * nv;
-    double* pn = a.p + (size_t)(par ^ 1) * DIM * nv;
-    {
-      double v[1] = {0.0};
-      for (int row = gtid; row < a.nv; row += gstride) {
-        double y[DIM];
-        kmul_row<DIM>(a, row,
-                      [&](int b, int col) { return fma(beta, __ldcg(po + b * nv + col), __ldcg(a.z + b * nv + col)); }, y);
-#pragma unroll
-        for (int c = 0; c < DIM; ++c) {
-          const double pp = fma(beta, po[c * nv + row], a.z[c * nv + row]);
-          pn[c * nv + row] = pp;
-          a.q[c * nv + row] = y[c];
-          v[0] += pp * y[c];
-        }
-      }
-      double out[1];
-      block_sums<1>(v, out);
-      publish(out, 1);
-    }
-    if (!grid_sync_ra(a.gb, bar)) return;
-    double pq[1];
-    grid_sums<1>(buf(), pq);
-    ++red;
-    const double alpha = pq[0] != 0.0 ? rho / pq[0] : 0.0;
-    // B: x += alpha p', r -= alpha q, z = D^-1 r, (r, z), (r, r)
-    {
-      double v[2] = {0.0, 0.0};
-      for (int row = gtid; row < a.nv; row += gstride)
-#pragma unroll
-        for (int c = 0; c < DIM; ++c) {
-          const size_t i = c * nv + row;
-          a.x[i] = fma(alpha, pn[i], a.x[i]);
-          const double rr = fma(-alpha, a.q[i], a.r[i]);
-          const double zz = rr * a.dinv[i];
-          a.r[i] = rr;
-          a.z[i] = zz;
-          v[0] += rr * zz;
-          v[1] += rr * rr;
-        }
-      double out[2];
-      block_sums<2>(v, out);
-      publish(out, 2);
-    }
-    if (!grid_sync_ra(a.gb, bar)) return;
-    double rz[2];
-    grid_sums<2>(buf(), rz);
-    ++red;
-    ++it;
-    res = sqrt(rz[1]);
-    ok = res <= tol || !(res == res);
-    beta = rho != 0.0 ? rz[0] / rho : 0.0;
-    rho = rz[0];
-    par ^= 1;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    a.out[0] = it;
-    a.out[1] = res <= tol ? 1 : 0;
-    a.res[0] = res;
-    a.res[1] = tol;
   }
 }
 
@@ -416,33 +228,41 @@ __global__ void k_v2c_dir(int nv, const double* __restrict__ X, const int* __res
 }
 
 static pfem2_status ale_alloc(Ctx& c) {
-  if (c.ale_vec) return PFEM2_OK;
+  if (c.ale_x) return PFEM2_OK;
   const size_t nv = c.nv, dim = c.dim;
   auto al = [&](void** p, size_t bytes) -> pfem2_status {
     PFEM2_CUDA(cudaMalloc(p, bytes));
     PFEM2_CUDA(cudaMemset(*p, 0, bytes));
     return PFEM2_OK;
   };
-  for (int k = 0; k < c.dim * c.dim; ++k) PFEM2_TRY(al((void**)&c.ale_K[k], sizeof(double) * c.nell));
-  PFEM2_TRY(al((void**)&c.ale_fix, nv));
+  PFEM2_TRY(al((void**)&c.ale_K, sizeof(double) * dim * dim * c.nell));
+  PFEM2_TRY(al((void**)&c.ale_fix, dim * nv));
   PFEM2_TRY(al((void**)&c.ale_g, sizeof(double) * dim * nv));
   PFEM2_TRY(al((void**)&c.ale_rhs, sizeof(double) * dim * nv));
   PFEM2_TRY(al((void**)&c.ale_dinv, sizeof(double) * dim * nv));
-  PFEM2_TRY(al((void**)&c.ale_vec, sizeof(double) * 6 * dim * nv));
+  PFEM2_TRY(al((void**)&c.ale_x, sizeof(double) * dim * nv));
   PFEM2_TRY(al((void**)&c.ale_new, sizeof(double) * 4 * nv));
-  PFEM2_TRY(al((void**)&c.ale_out, sizeof(int) * 2));
-  PFEM2_TRY(al((void**)&c.ale_res, sizeof(double) * 2));
   PFEM2_TRY(al((void**)&c.ale_flag, sizeof(int)));
-  // the CG's persistent grid: every block resident
-  int occ = 0;
-  const void* k = c.dim == 2 ? (const void*)k_elastic_cg<2> : (const void*)k_elastic_cg<3>;
-  PFEM2_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, kAleThreads, 0));
-  if (occ < 1) {
-    set_error("moving mesh: the elasticity solver cannot be resident");
-    return PFEM2_CUDA_ERROR;
-  }
-  c.ale_grid = (int)std::min<long long>((long long)occ * c.num_sms, std::max<long long>(1, (c.nv + kAleThreads - 1) / kAleThreads));
-  PFEM2_TRY(al((void**)&c.ale_part, sizeof(double) * 2 * 4 * c.ale_grid));
+  // the system's own slices (see the head of this file)
+  std::vector<int> len(c.nslices), col(c.nell), slp(1, 0), sll, slc((size_t)dim * dim * c.nell);
+  PFEM2_CUDA(cudaMemcpy(len.data(), c.sl_len, sizeof(int) * c.nslices, cudaMemcpyDeviceToHost));
+  PFEM2_CUDA(cudaMemcpy(col.data(), c.sl_col, sizeof(int) * c.nell, cudaMemcpyDeviceToHost));
+  for (size_t a = 0; a < dim; ++a)
+    for (int s = 0; s < c.nslices; ++s) {
+      const int n = len[s] * kSlice, p = c.h_sl_ptr[s];
+      for (size_t b = 0; b < dim; ++b)
+        for (int e = 0; e < n; ++e) slc[slp.back() + b * n + e] = (int)(b * nv) + col[p + e];
+      sll.push_back((int)dim * len[s]);
+      slp.push_back(slp.back() + (int)dim * n);
+    }
+  PFEM2_TRY(al((void**)&c.ale_slp, sizeof(int) * slp.size()));
+  PFEM2_TRY(al((void**)&c.ale_sll, sizeof(int) * sll.size()));
+  PFEM2_TRY(al((void**)&c.ale_slc, sizeof(int) * slc.size()));
+  PFEM2_CUDA(cudaMemcpy(c.ale_slp, slp.data(), sizeof(int) * slp.size(), cudaMemcpyHostToDevice));
+  PFEM2_CUDA(cudaMemcpy(c.ale_sll, sll.data(), sizeof(int) * sll.size(), cudaMemcpyHostToDevice));
+  PFEM2_CUDA(cudaMemcpy(c.ale_slc, slc.data(), sizeof(int) * slc.size(), cudaMemcpyHostToDevice));
+  PFEM2_TRY(krylov_elastic_setup(c, slp));
+  PFEM2_CUDA(cudaDeviceSynchronize());  // (these copies are on the default stream)
   return PFEM2_OK;
 }
 
@@ -463,12 +283,10 @@ pfem2_status ale_setup(Ctx& c) {
 }
 
 void ale_free(Ctx& c) {
-  void* p[] = {c.ale_bnd, c.ale_fix, c.ale_g, c.ale_rhs, c.ale_dinv, c.ale_vec, c.ale_part,
-               c.ale_out, c.ale_res, c.ale_xphys, c.ale_new, c.ale_flag};
+  void* p[] = {c.ale_bnd, c.ale_fix, c.ale_g,     c.ale_rhs, c.ale_dinv, c.ale_x,   c.ale_K,
+               c.ale_slp, c.ale_sll, c.ale_slc, c.ale_xphys, c.ale_new, c.ale_flag};
   for (void* q : p)
     if (q) cudaFree(q);
-  for (int k = 0; k < 9; ++k)
-    if (c.ale_K[k]) cudaFree(c.ale_K[k]);
 }
 
 pfem2_status ale_elasticity(Ctx& c, const pfem2_elasticity& e, const double* body_disp, int* iters, double* res) {
@@ -476,7 +294,7 @@ pfem2_status ale_elasticity(Ctx& c, const pfem2_elasticity& e, const double* bod
   const int dim = c.dim, NV = 1 << dim, NF = 2 * dim;
   const size_t nv = c.nv;
   // constrained vertices: fixed boundaries (zero) and the body; padding rows
-  std::vector<unsigned char> fix(nv, 0);
+  std::vector<unsigned char> fix(dim * nv, 0);  // (the same per component)
   std::vector<double> g(dim * nv, 0.0);
   for (const HostInst& in : c.inst) {
     for (int k = in.nv; k < in.nv_pad; ++k) fix[in.v_off + k] = 1;
@@ -494,78 +312,42 @@ pfem2_status ale_elasticity(Ctx& c, const pfem2_elasticity& e, const double* bod
           }
       }
   }
-  PFEM2_CUDA(cudaMemcpyAsync(c.ale_fix, fix.data(), nv, cudaMemcpyHostToDevice, c.stream));
+  for (int d = 1; d < dim; ++d) std::copy(fix.begin(), fix.begin() + nv, fix.begin() + (size_t)d * nv);
+  PFEM2_CUDA(cudaMemcpyAsync(c.ale_fix, fix.data(), dim * nv, cudaMemcpyHostToDevice, c.stream));
   PFEM2_CUDA(cudaMemcpyAsync(c.ale_g, g.data(), sizeof(double) * dim * nv, cudaMemcpyHostToDevice, c.stream));
-  for (int k = 0; k < dim * dim; ++k) PFEM2_CUDA(cudaMemsetAsync(c.ale_K[k], 0, sizeof(double) * c.nell, c.stream));
-  double** K = c.ale_K;
-  const int grid = grid_for(c, c.nv, 128, 8);
-  if (dim == 2)
-    k_elastic_assemble<2><<<grid, 128, 0, c.stream>>>(c.nv, c.v2c_ptr, c.v2c_cell, c.v2c_loc, c.inc_slot, c.X, c.cv,
-                                                      e.lambda, e.mu, K[0], K[1], K[2], K[3], K[4], K[5], K[6], K[7],
-                                                      K[8]);
-  else
-    k_elastic_assemble<3><<<grid, 128, 0, c.stream>>>(c.nv, c.v2c_ptr, c.v2c_cell, c.v2c_loc, c.inc_slot, c.X, c.cv,
-                                                      e.lambda, e.mu, K[0], K[1], K[2], K[3], K[4], K[5], K[6], K[7],
-                                                      K[8]);
-  const int g2 = grid_for(c, c.nv, 256, 8);
-  if (dim == 2)
-    k_elastic_eliminate<2><<<g2, 256, 0, c.stream>>>(c.nv, c.sl_ptr, c.sl_len, c.sl_col, K[0], K[1], K[2], K[3], K[4],
-                                                     K[5], K[6], K[7], K[8], c.ale_fix, c.ale_g, c.ale_rhs, c.ale_dinv);
-  else
-    k_elastic_eliminate<3><<<g2, 256, 0, c.stream>>>(c.nv, c.sl_ptr, c.sl_len, c.sl_col, K[0], K[1], K[2], K[3], K[4],
-                                                     K[5], K[6], K[7], K[8], c.ale_fix, c.ale_g, c.ale_rhs, c.ale_dinv);
+  PFEM2_CUDA(cudaMemsetAsync(c.ale_K, 0, sizeof(double) * dim * dim * c.nell, c.stream));
+  PFEM2_CUDA(cudaMemsetAsync(c.ale_x, 0, sizeof(double) * dim * nv, c.stream));  // x0 = g on the constrained rows, else 0
+  const int grid = grid_for(c, c.nv, 128, 8), g2 = grid_for(c, c.nv, 256, 8);
+  if (dim == 2) {
+    k_elastic_assemble<2><<<grid, 128, 0, c.stream>>>(c.nv, c.nell, c.v2c_ptr, c.v2c_cell, c.v2c_loc, c.inc_slot,
+                                                      c.sl_ptr, c.sl_len, c.X, c.cv, e.lambda, e.mu, c.ale_K);
+    k_elastic_eliminate<2><<<g2, 256, 0, c.stream>>>(c.nv, c.nell, c.sl_ptr, c.sl_len, c.sl_col, c.ale_K, c.ale_fix,
+                                                     c.ale_g, c.ale_rhs, c.ale_dinv);
+  } else {
+    k_elastic_assemble<3><<<grid, 128, 0, c.stream>>>(c.nv, c.nell, c.v2c_ptr, c.v2c_cell, c.v2c_loc, c.inc_slot,
+                                                      c.sl_ptr, c.sl_len, c.X, c.cv, e.lambda, e.mu, c.ale_K);
+    k_elastic_eliminate<3><<<g2, 256, 0, c.stream>>>(c.nv, c.nell, c.sl_ptr, c.sl_len, c.sl_col, c.ale_K, c.ale_fix,
+                                                     c.ale_g, c.ale_rhs, c.ale_dinv);
+  }
   c.launches += 2;
-  ElasticArgs a{};
-  a.nv = c.nv;
-  a.maxit = e.max_iter > 0 ? e.max_iter : 10000;
-  a.tol = e.tol;
-  a.rtol = e.rtol;
-  a.sl_ptr = c.sl_ptr;
-  a.sl_len = c.sl_len;
-  a.sl_col = c.sl_col;
-  for (int k = 0; k < 9; ++k) a.K[k] = K[k];
-  a.rhs = c.ale_rhs;
-  a.dinv = c.ale_dinv;
-  a.g = c.ale_g;
-  a.fix = c.ale_fix;
-  const size_t blk = (size_t)dim * nv;
-  a.x = c.ale_vec;
-  a.r = c.ale_vec + blk;
-  a.z = c.ale_vec + 2 * blk;
-  a.q = c.ale_vec + 3 * blk;
-  a.p = c.ale_vec + 4 * blk;
-  a.part = c.ale_part;
-  a.out = c.ale_out;
-  a.res = c.ale_res;
-  a.gb.count = c.barrier;
-  a.gb.gen = c.barrier + 1;
-  a.gb.err = c.d_err;
-  a.gb.spin_limit = c.spin_limit;
-  PFEM2_CUDA(cudaMemsetAsync(c.barrier, 0, 2 * sizeof(unsigned), c.stream));
-  PFEM2_CUDA(cudaMemsetAsync(c.d_err, 0, sizeof(int), c.stream));
-  PFEM2_CUDA(cudaMemsetAsync(c.ale_out, 0, 2 * sizeof(int), c.stream));
-  void* args[] = {&a};
-  const void* kern = dim == 2 ? (const void*)k_elastic_cg<2> : (const void*)k_elastic_cg<3>;
-  PFEM2_CUDA(cudaLaunchCooperativeKernel(kern, dim3(c.ale_grid), dim3(kAleThreads), args, 0, c.stream));
-  c.launches++;
+  const ElasticSystem E{c.ale_slp, c.ale_sll, c.ale_slc, c.ale_K, c.ale_dinv, c.ale_rhs, c.ale_g, c.ale_fix, c.ale_x};
+  PFEM2_TRY(krylov_elastic_solve(c, E, e.tol, e.rtol, e.max_iter > 0 ? e.max_iter : 10000));
   // the displacement into the fields
   for (int d = 0; d < dim; ++d)
-    PFEM2_CUDA(cudaMemcpyAsync(c.F[PFEM2_FIELD_DISP_X + d], a.x + (size_t)d * nv, sizeof(double) * nv,
+    PFEM2_CUDA(cudaMemcpyAsync(c.F[PFEM2_FIELD_DISP_X + d], c.ale_x + (size_t)d * nv, sizeof(double) * nv,
                                cudaMemcpyDeviceToDevice, c.stream));
-  int out[2] = {0, 0}, err = 0;
-  double rr[2] = {0.0, 0.0};
-  PFEM2_CUDA(cudaMemcpyAsync(out, c.ale_out, sizeof(out), cudaMemcpyDeviceToHost, c.stream));
-  PFEM2_CUDA(cudaMemcpyAsync(rr, c.ale_res, sizeof(rr), cudaMemcpyDeviceToHost, c.stream));
+  int it = 0, err = 0;
+  double rr = 0.0, tol = 0.0;
   PFEM2_CUDA(cudaMemcpyAsync(&err, c.d_err, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-  PFEM2_CUDA(cudaStreamSynchronize(c.stream));
-  if (iters) *iters = out[0];
-  if (res) *res = rr[0];
+  PFEM2_TRY(krylov_elastic_read(c, &it, &rr, &tol));
+  if (iters) *iters = it;
+  if (res) *res = rr;
   if (err) {
     set_error("mesh elasticity: a wait of the solver timed out");
     c.failed = true;
     return PFEM2_TIMEOUT;
   }
-  if (!out[1]) {
+  if (!(rr <= tol)) {
     set_error("mesh elasticity: the CG did not converge within max_iter");
     return PFEM2_NOT_CONVERGED;
   }

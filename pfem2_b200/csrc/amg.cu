@@ -407,7 +407,7 @@ pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vec
       L[l + 1].A = spgemm(transpose(V.P), spgemm(V.A, V.P));
       L[l + 1].tile = ctile;
     }
-    H.w0.push_back(L[0].w);
+    H.w0.push_back(c.moving ? std::min(L[0].w, 0.49) : L[0].w);
   }
   // ---- global numbering: systems in order, dofs tile-ordered inside
   std::vector<std::vector<int>> goff(kMgLevels, std::vector<int>(ni + 1, 0));
@@ -440,7 +440,8 @@ pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vec
   for (int s = 0; s < ni; ++s) {
     std::vector<Level>& L = sysL[s];
     Csr R = transpose(L[0].Pt2);
-    for (size_t e = 0; e < R.col.size(); ++e) R.val[e] /= L[0].dinv[R.col[e]];
+    if (!c.moving)
+      for (size_t e = 0; e < R.col.size(); ++e) R.val[e] /= L[0].dinv[R.col[e]];
     append_rows(R, c.inst[s].v_off, H.r1_ptr, H.r1_col, H.r1_val);
     append_rows(transpose(L[1].Pt2), goff[1][s], H.q2_ptr, H.q2_col, H.q2_val);
     const int n2 = L[2].A.n, n3 = L[3].A.n;

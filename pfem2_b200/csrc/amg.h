@@ -28,8 +28,8 @@ struct MgHost {
   std::vector<int> toff[kMgLevels];       // [l][ntiles+1] first level-l dof of each tile (l >= 1)
   std::vector<int> lsys[kMgLevels];       // [l][n_l] system of each level-l dof (l >= 1)
   std::vector<int> lk[3];                 // [1..2][n_l] index of that system among its block's systems
-  // Pt_0^T D (applied to D^-1 v), CSR over the level-1 rows with global
-  // level-0 columns
+  // Pt_0^T D (applied to D^-1 v; Pt_0^T on a moving mesh), CSR over the
+  // level-1 rows with global level-0 columns
   std::vector<int> r1_ptr, r1_col;
   std::vector<double> r1_val;
   // Pt_1^T, CSR over the level-2 rows with global level-1 columns
@@ -51,7 +51,7 @@ struct MgHost {
   std::vector<int> blk_s1, s1_lk, j1_ptr, j1_col, p1_ptr, p1_col;
   std::vector<double> j1_val, p1_val;
   std::vector<int> sys_n2, sys_off2;      // level-2 size and first level-2 dof per system
-  std::vector<double> w0;                 // level-0 smoother weight per system
+  std::vector<double> w0;                 // level-0 smoother weight per system (at most 0.49 on a moving mesh)
   int s1max = 0;
   int b2max = 0;                          // level-2 dofs of the local systems of a block
 };

@@ -405,12 +405,11 @@ static pfem2_status do_setup(Ctx& c) {
   if (c.p_bicg) c.two_level = false;
   if (c.moving) {
     // the matrices follow the mesh: reassembled every step; the multigrid
-    // hierarchy (built once on the host) is not used
+    // hierarchy stays that of the mesh at setup
     if (c.inst.size() != 1 || c.dim != 2 || c.cfg.particles_only) {
       set_error("moving_mesh: one 2D instance with the FEM");
       return PFEM2_INVALID_ARG;
     }
-    c.two_level = false;
     c.inst[0].cs.reassemble_every_step = 1;
   }
   // instance table

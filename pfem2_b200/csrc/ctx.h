@@ -172,26 +172,23 @@ struct Ctx {
   double refine_eta = 1e-3;     // mixed: inner residual reduction per FP64 refinement
 
   // moving mesh (pfem2_config.moving_mesh): boundary vertices, the
-  // elasticity blocks K[a * dim + b] on the SELL pattern, constraint table,
-  // right-hand side / inverse diagonal ([dim][nv]), CG vectors, particle
-  // positions before a move ([dim][pcap] FP64), reinterpolated fields, and
-  // the device status word of the mesh kernels (1: a cell turned inside out)
+  // elasticity system (slices of its own, ale.cu), constraint table, right-
+  // hand side / inverse diagonal / solution ([dim][nv]), particle positions
+  // before a move ([dim][pcap] FP64), reinterpolated fields, and the device
+  // status word of the mesh kernels (1: a cell turned inside out)
   bool moving = false;
   unsigned char* ale_bnd = nullptr;
-  double* ale_K[9] = {};
+  double* ale_K = nullptr;     // [dim * dim * nell]
+  int *ale_slp = nullptr, *ale_sll = nullptr, *ale_slc = nullptr;
   unsigned char* ale_fix = nullptr;
   double* ale_g = nullptr;
   double* ale_rhs = nullptr;
   double* ale_dinv = nullptr;
-  double* ale_vec = nullptr;   // x, r, z, q, p[2]: 6 [dim][nv] blocks
-  double* ale_part = nullptr;  // [2][grid][4] partial sums of the CG
-  int* ale_out = nullptr;      // [2] iterations, converged; ale_res: residual and tolerance
-  double* ale_res = nullptr;
+  double* ale_x = nullptr;
   double* ale_xphys = nullptr;
   size_t ale_xphys_cap = 0;
   double* ale_new = nullptr;   // [4][nv]
   int* ale_flag = nullptr;
-  int ale_grid = 0;
 
   // launch shapes: as set by the caller (0 = automatic) and as resolved at
   // setup (caller, else the tuning cache, else by size)
@@ -291,5 +288,15 @@ void krylov_free(Ctx& c);
 pfem2_status krylov_solve(Ctx& c, int which);
 pfem2_status krylov_read_stats(Ctx& c);
 void krylov_sizes(Ctx& c, long long* out12);
+// the mesh elasticity's system (FP64): dim x nv rows, components one after the other
+struct ElasticSystem {
+  const int *sl_ptr, *sl_len, *sl_col;
+  const double *A, *dinv, *rhs, *g;
+  const unsigned char* isd;
+  double* x;
+};
+pfem2_status krylov_elastic_setup(Ctx& c, const std::vector<int>& slp);
+pfem2_status krylov_elastic_solve(Ctx& c, const ElasticSystem& E, double tol, double rtol, int maxit);
+pfem2_status krylov_elastic_read(Ctx& c, int* it, double* res, double* tol);
 
 }  // namespace pfem2

@@ -66,6 +66,12 @@ enum {
 // partial sums per block and system: CG uses 3, BiCGStab 5 (and the FP64
 // residual phase |r|^2 and |b|^2)
 constexpr int kMaxSums = 5;
+constexpr int kClusterMax = 16;  // blocks of a cluster
+// items (slices x components) up to which one cluster solves: above, the 16
+// SMs' work outweighs the cheaper barrier (1k channel FP64, 70 items:
+// prediction and correction 0.49 -> 0.38 ms per step; 8k cells, 520 items:
+// 0.45 -> 0.63)
+constexpr int kClusterItems = 300;
 
 // What a block keeps in shared memory (template parameter SM, the most that
 // fits; every phase start's GPU-scope acquire invalidates L1, so what is read
@@ -135,6 +141,7 @@ template <typename R> struct SolveArgs {
   double* out_tol;       // [nsys] tolerance the system was solved to
   int* out_outer;        // [nsys] FP64 residual evaluations
   double eta;
+  int trust;             // stop on the recurrence residual (CG), without the FP64 check
   int iter_cap;
   GridBarrier gb;
 };
@@ -169,7 +176,7 @@ __device__ __forceinline__ int sums_of(int state) {
 
 // the next step of a system from the sums of its previous phase (one thread;
 // identical in every block of the system)
-__device__ __forceinline__ void decide(LocalSys& L, bool bicg, double eta) {
+__device__ __forceinline__ void decide(LocalSys& L, bool bicg, bool trust, double eta) {
   const double* s = L.sum;
   switch (L.state) {
     case S_OUT_A:
@@ -185,7 +192,7 @@ __device__ __forceinline__ void decide(LocalSys& L, bool bicg, double eta) {
         L.act = ACT_FINISH;
         L.state = S_DONE;
       } else {
-        L.intol = fmax(eta * L.res, 0.5 * L.tol);
+        L.intol = trust ? L.tol : fmax(eta * L.res, 0.5 * L.tol);
         L.first = 1;
         L.beta = 0.0;
         L.rz_prev = L.res * L.res;  // BiCGStab: rho = (rh, r) with rh = r
@@ -245,8 +252,9 @@ __device__ __forceinline__ void decide(LocalSys& L, bool bicg, double eta) {
         const double be = L.rz_prev != 0.0 ? g / L.rz_prev : 0.0;
         const double den = dl - (L.alpha != 0.0 ? be * g / L.alpha : 0.0);
         if (rr <= L.intol * L.intol || L.it >= L.maxit || !(rr == rr) || !(den > 0.0)) {
-          L.act = ACT_OUT_A;  // reliable update in FP64
-          L.state = S_OUT_B;
+          L.act = trust ? ACT_FINISH : ACT_OUT_A;  // reliable update in FP64
+          L.state = trust ? S_DONE : S_OUT_B;
+          if (trust) L.res = sqrt(rr);
         } else {
           L.beta = be;
           L.alpha = g / den;
@@ -262,7 +270,24 @@ __device__ __forceinline__ void decide(LocalSys& L, bool bicg, double eta) {
   }
 }
 
-template <typename R, int MINB, int SM>
+// CL: the grid is one thread-block cluster. The blocks then exchange their
+// partial sums through each other's shared memory and meet at the cluster's
+// hardware barrier (about 0.5 us) instead of publishing to and polling
+// counters in L2 (about 2 us a phase): small systems, whose phases are short.
+__device__ __forceinline__ void cluster_sync_ra() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// stores v at the address that p has in the shared memory of block `rank` of the cluster
+__device__ __forceinline__ void st_cluster(double* p, unsigned rank, double v) {
+  const unsigned addr = (unsigned)__cvta_generic_to_shared(p);
+  unsigned remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote), "d"(v) : "memory");
+}
+
+template <typename R, int MINB, int SM, bool CL>
 __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(SolveArgs<R> a) {
   constexpr int kSolveThreads = SolveThreads<MINB>::value, kWarps = kSolveThreads / 32;
   extern __shared__ __align__(16) unsigned char dyn_smem[];
@@ -271,6 +296,7 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
   constexpr int CH = sizeof(R) == 8 ? 5 : 9;
   __shared__ LocalSys ls[kMaxLocalSys];
   __shared__ int s_err;
+  __shared__ double s_pub[CL ? 2 * 3 * kMaxSums * kClusterMax : 1];  // [parity][system][sum][block]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t nv = (size_t)a.nv;
   const int NC = a.ncomp;
@@ -352,7 +378,8 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
     }
   if (SM >= 1)
     for (int i = threadIdx.x; i < nitems * 32; i += kSolveThreads) ve[i] = R(0);
-  if (!grid_sync_ra(a.gb, bar_gen)) return;
+  if constexpr (CL) cluster_sync_ra();
+  else if (!grid_sync_ra(a.gb, bar_gen)) return;
 
   for (int iter = 0;; ++iter) {
     if (iter >= a.iter_cap) {
@@ -364,27 +391,42 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
     // have finished phase iter - 1; the acquire orders what they wrote before
     // this phase's reads. A warp per (local system, sum) waits and sums that
     // phase's partials, then a thread per system takes the next step.
-    const double* prev = a.part + (size_t)((iter + 1) & 1) * kMaxSums * a.nslots;
-    for (int t = warp; t < nls * kMaxSums; t += kWarps) {
-      // (the first sums of all systems first)
-      const int q = t / nls, l = t - q * nls;
-      const LocalSys& L = ls[l];
-      if (L.state == S_DONE || iter == 0 || (q > 0 && q >= sums_of(L.state))) continue;
-      if (!wait_count(a.scount + (size_t)L.sys * 32, (unsigned)iter * (unsigned)(L.s1 - L.s0), a.gb)) {
-        if (lane == 0) {
-          atomicCAS(a.gb.err, 0, 1);
-          s_err = 1;
+    if constexpr (CL) {
+      for (int l = warp; l < nls; l += kWarps) {
+        LocalSys& L = ls[l];
+        if (iter > 0 && lane < sums_of(L.state)) {
+          const double* v = s_pub + ((((iter + 1) & 1) * 3 + l) * kMaxSums + lane) * kClusterMax;
+          double t = 0.0;
+          for (int b = 0; b < (int)gridDim.x; ++b) t += v[b];
+          L.sum[lane] = t;
         }
-        break;
+        __syncwarp();
+        if (lane == 0) decide(L, a.bicg != 0, a.trust != 0, a.eta);
       }
-      if (q < sums_of(L.state)) {
-        const double s = slot_sum(prev + (size_t)q * a.nslots, L.s0, L.s1, lane);
-        if (lane == 0) ls[l].sum[q] = s;
+      __syncthreads();
+    } else {
+      const double* prev = a.part + (size_t)((iter + 1) & 1) * kMaxSums * a.nslots;
+      for (int t = warp; t < nls * kMaxSums; t += kWarps) {
+        // (the first sums of all systems first)
+        const int q = t / nls, l = t - q * nls;
+        const LocalSys& L = ls[l];
+        if (L.state == S_DONE || iter == 0 || (q > 0 && q >= sums_of(L.state))) continue;
+        if (!wait_count(a.scount + (size_t)L.sys * 32, (unsigned)iter * (unsigned)(L.s1 - L.s0), a.gb)) {
+          if (lane == 0) {
+            atomicCAS(a.gb.err, 0, 1);
+            s_err = 1;
+          }
+          break;
+        }
+        if (q < sums_of(L.state)) {
+          const double s = slot_sum(prev + (size_t)q * a.nslots, L.s0, L.s1, lane);
+          if (lane == 0) ls[l].sum[q] = s;
+        }
       }
+      __syncthreads();
+      if (threadIdx.x < nls) decide(ls[threadIdx.x], a.bicg != 0, a.trust != 0, a.eta);
+      __syncthreads();
     }
-    __syncthreads();
-    if (threadIdx.x < nls) decide(ls[threadIdx.x], a.bicg != 0, a.eta);
-    __syncthreads();
     if (s_err) break;
     bool any = false;
     for (int l = 0; l < nls; ++l) any |= ls[l].act != ACT_NONE;
@@ -570,15 +612,22 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
       LocalSys& L = ls[l];
       const int act = L.act, k = l % NC, il = l / NC;
       const int ns = act == ACT_P2 ? kMaxSums : act == ACT_P1 ? 1 : act == ACT_NONE || act == ACT_FINISH ? 0 : 3;
-      if (lane < ns) {  // lane q adds up sum q
-        double s = 0.0;
+      double s = 0.0;
+      if (lane < ns)  // lane q adds up sum q
         for (int j = 0; j < bs1 - bs0; ++j)
           if (SLk[j] == il) s += spart[(size_t)NS * (j * NC + k) + lane];
+      if constexpr (CL) {
+        for (int q = 0; q < ns; ++q) {
+          const double v = __shfl_sync(PFEM2_FULL_MASK, s, q);
+          if (lane < (int)gridDim.x)
+            st_cluster(s_pub + (((iter & 1) * 3 + l) * kMaxSums + q) * kClusterMax + blockIdx.x, lane, v);
+        }
+      } else if (lane < ns) {
         a.part[((size_t)(iter & 1) * kMaxSums + lane) * a.nslots + L.slot] = s;
       }
       __syncwarp();
       if (lane == 0) {
-        red_release_add_u32(a.scount + (size_t)L.sys * 32, 1u);
+        if (!CL) red_release_add_u32(a.scount + (size_t)L.sys * 32, 1u);
         if (act == ACT_P1 || act == ACT_C0 || act == ACT_C1) L.par ^= 1;
         if (act == ACT_FINISH && L.slot == L.s0) {
           a.out_it[L.sys] = L.it;
@@ -589,30 +638,198 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
         }
       }
     }
+    if constexpr (CL) cluster_sync_ra();
   }
 }
 
 // ------------------------------------------------------------------ host
 template <typename R, int MINB>
 static const void* kernel_of(int sm) {
-  return sm == 0   ? (const void*)k_krylov<R, MINB, 0>
-         : sm == 1 ? (const void*)k_krylov<R, MINB, 1>
-         : sm == 2 ? (const void*)k_krylov<R, MINB, 2>
-                   : (const void*)k_krylov<R, MINB, 3>;
+  return sm == 0   ? (const void*)k_krylov<R, MINB, 0, false>
+         : sm == 1 ? (const void*)k_krylov<R, MINB, 1, false>
+         : sm == 2 ? (const void*)k_krylov<R, MINB, 2, false>
+                   : (const void*)k_krylov<R, MINB, 3, false>;
 }
 
 template <typename R>
-static const void* kernel_of(int minb, int sm) {
+static const void* kernel_of(int minb, int sm, bool cluster) {
+  if (cluster) return sm == 2 ? (const void*)k_krylov<R, 1, 2, true> : (const void*)k_krylov<R, 1, 3, true>;
   return minb == 1 ? kernel_of<R, 1>(sm) : kernel_of<R, 2>(sm);
 }
 
+static const void* kernel_of(bool mixed, int minb, int sm, bool cluster) {
+  return mixed ? kernel_of<float>(minb, sm, cluster) : kernel_of<double>(minb, sm, cluster);
+}
+
 static int occupancy(bool mixed, int minb, int sm, size_t smem) {
-  const void* k = mixed ? kernel_of<float>(minb, sm) : kernel_of<double>(minb, sm);
+  const void* k = kernel_of(mixed, minb, sm, false);
   int occ = 0;
   // one process-wide upper bound, so contexts with different systems coexist
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_budget(minb));
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, solve_threads(minb), smem) != cudaSuccess) return 0;
   return occ;
+}
+
+static void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& at, int grid, size_t smem, cudaStream_t st) {
+  cfg = cudaLaunchConfig_t{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(solve_threads(1));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = grid;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+}
+
+// whether the device can hold one cluster of `grid` such blocks
+static bool cluster_fits(bool mixed, int sm, int grid, size_t smem) {
+  const void* k = kernel_of(mixed, 1, sm, true);
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at;
+  cluster_config(cfg, at, grid, smem, 0);
+  int n = 0;
+  const bool ok =
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_budget(1)) == cudaSuccess &&
+      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+      cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n >= 1;
+  if (!ok) cudaGetLastError();
+  return ok;
+}
+
+// shared memory of a block and what it holds; sm < 0: not even its partial sums fit
+static size_t plan_smem(const JacobiPlan& P, size_t rs, int minb, int nmat, int& sm) {
+  size_t smem = al16(sizeof(double) * (P.bicg ? kMaxSums : 3) * (size_t)P.items_max);
+  const size_t level[3] = {al16(6 * 32 * rs * (size_t)P.items_max) + P.st_meta, al16(4 * P.st_entries),
+                           nmat * al16(rs * P.st_entries)};
+  sm = 0;
+  while (sm < 3 && smem + level[sm] <= smem_budget(minb)) smem += level[sm++];
+  return smem;
+}
+
+// the blocks' slice runs: G equal runs of the slices, whose instances are
+// given by their slice offsets ioff (ascending, ioff.back() = all)
+static pfem2_status plan_runs(JacobiPlan& P, std::vector<int> (&up)[6], const std::vector<int>& ioff,
+                              const std::vector<int>& slp, int ncomp, int G) {
+  const int ni = (int)ioff.size() - 1, ns = ioff.back();
+  std::vector<int>&bsl = up[0], &binst = up[1], &binst_off = up[2], &bslot = up[3], &slot0 = up[4], &slk = up[5];
+  std::vector<int> cnt(ni, 0);
+  bsl.assign(G + 1, 0);
+  binst.clear();
+  bslot.clear();
+  binst_off.assign(1, 0);
+  slot0.assign(ncomp * ni + 1, 0);
+  slk.assign(ns, 0);
+  for (int b = 0; b <= G; ++b) bsl[b] = (int)((long long)ns * b / G);
+  P.grid = G;
+  P.items_max = 0;
+  P.st_meta = P.st_entries = 0;
+  for (int b = 0, i = 0; b < G; ++b) {
+    const int s0 = bsl[b], s1 = bsl[b + 1];
+    while (ioff[i + 1] <= s0) ++i;
+    int last = i - 1;
+    for (int sl = s0, j = i; sl < s1; ++sl) {
+      while (ioff[j + 1] <= sl) ++j;
+      for (; last < j; ++last) {
+        binst.push_back(last + 1);
+        bslot.push_back(cnt[last + 1]++);
+      }
+      slk[sl] = j - i;
+    }
+    binst_off.push_back((int)binst.size());
+    if ((binst_off[b + 1] - binst_off[b]) * ncomp > kMaxLocalSys) {
+      set_error("krylov: more than 16 systems would share one block (instances too small for the batch)");
+      return PFEM2_INVALID_ARG;
+    }
+    P.items_max = std::max(P.items_max, (s1 - s0) * ncomp);
+    P.st_meta = std::max(P.st_meta, 3 * al16(4 * (size_t)(s1 - s0)));
+    P.st_entries = std::max(P.st_entries, (size_t)(slp[s1] - slp[s0]));
+  }
+  for (int k = 0; k < ncomp; ++k)
+    for (int i = 0; i < ni; ++i) slot0[k * ni + i + 1] = slot0[k * ni + i] + cnt[i];
+  P.nslots = slot0.back();
+  return PFEM2_OK;
+}
+
+// Partition of a solve: one cluster where the systems are small, else blocks
+// of at least `ts` slices, minb to an SM (0: by size). mixed: the inner type.
+static pfem2_status plan_build(Ctx& c, KrylovWs* w, JacobiPlan& P, bool mixed, const std::vector<int>& ioff,
+                               const std::vector<int>& slp, int ncomp, int nmat, int minb, int ts, bool try_cluster) {
+  const int ni = (int)ioff.size() - 1, ns = ioff.back();
+  const size_t rs = mixed ? sizeof(float) : sizeof(double);
+  std::vector<int> up[6];
+  P.cluster = false;
+  if (try_cluster && ni == 1 && ns * ncomp <= kClusterItems) {
+    int G = 1;
+    while (2 * G <= kClusterMax && 4 * G <= ns) G *= 2;
+    PFEM2_TRY(plan_runs(P, up, ioff, slp, ncomp, G));
+    const size_t smem = plan_smem(P, rs, 1, nmat, P.sm);
+    if (P.sm >= 2 && cluster_fits(mixed, P.sm, G, smem)) {
+      P.cluster = true;
+      P.minb = 1;
+    }
+  }
+  if (!P.cluster) {
+    // one block per SM, but at least four slices in each (channel of 1k rows,
+    // FP64: 0.49 ms per step with four, 0.53 with six, 0.48 with two; 13k
+    // rows: 0.48 with four, 0.53 with two)
+    const int ts_auto = std::max(4, (ns + c.num_sms - 1) / c.num_sms);
+    // one system: a block of 768 threads per SM, so that few blocks are waited
+    // for (52k channel: prediction and correction 0.45 ms per step against
+    // 0.55 with two blocks of 384; 131k pipe 3.58 against 3.77), unless 12
+    // warps hold its items in one round; a batch takes two of 384, whose
+    // instances wait less for each other (16 channels: 1.38 against 1.44 ms)
+    P.minb = minb ? minb : (ni > 1 || ts_auto * ncomp <= 12 ? 2 : 1);
+    if (!ts) ts = ni > 1 ? 4 : ts_auto;
+    const int occ = std::min(P.minb, occupancy(mixed, P.minb, 0, 0));
+    if (occ < 1) {
+      set_error("krylov: the solver kernel cannot be resident");
+      return PFEM2_CUDA_ERROR;
+    }
+    PFEM2_TRY(plan_runs(P, up, ioff, slp, ncomp, std::max(1, std::min(occ * c.num_sms, (ns + ts - 1) / ts))));
+  }
+  P.ts = (ns + P.grid - 1) / P.grid;
+  int** dst[6] = {&P.blk_sl, &P.blk_inst, &P.blk_inst_off, &P.blk_slot, &P.sys_slot0, &P.slk};
+  for (int k = 0; k < 6; ++k) PFEM2_TRY(ws_upload(w, dst[k], up[k]));
+  return PFEM2_OK;
+}
+
+template <typename R>
+static void plan_args(const KrylovWs* w, const JacobiPlan& P, SolveArgs<R>& a) {
+  a.blk_inst = P.blk_inst;
+  a.blk_inst_off = P.blk_inst_off;
+  a.blk_slot = P.blk_slot;
+  a.sys_slot0 = P.sys_slot0;
+  a.blk_sl = P.blk_sl;
+  a.slk = P.slk;
+  a.items_max = P.items_max;
+  a.nslots = P.nslots;
+  a.bicg = P.bicg;
+  a.scount = w->scount;
+  a.active = w->active;
+}
+
+template <typename R>
+static pfem2_status plan_launch(Ctx& c, const JacobiPlan& P, SolveArgs<R>& a, int nmat) {
+  a.gb.count = c.barrier;
+  a.gb.gen = c.barrier + 1;
+  a.gb.err = c.d_err;
+  a.gb.spin_limit = c.spin_limit;
+  int sm = 0;
+  const size_t smem = plan_smem(P, sizeof(R), P.minb, nmat, sm);
+  const void* kern = kernel_of<R>(P.minb, sm, P.cluster);
+  void* args[] = {&a};
+  if (P.cluster) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at;
+    cluster_config(cfg, at, P.grid, smem, c.stream);
+    PFEM2_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
+  } else {
+    PFEM2_CUDA(cudaLaunchCooperativeKernel(kern, dim3(P.grid), dim3(solve_threads(P.minb)), args, smem, c.stream));
+  }
+  c.launches++;
+  return PFEM2_OK;
 }
 
 void krylov_free(Ctx& c) {
@@ -628,75 +845,22 @@ pfem2_status krylov_setup(Ctx& c) {
   KrylovWs* w = new KrylovWs();
   c.kws = w;
   const int dim = c.dim, ni = (int)c.inst.size();
-  // slices per block: one block per SM, but at least four slices (channel of
-  // 1k rows, FP64: 0.49 ms per step with four, 0.53 with six, 0.48 with two;
-  // 13k rows: 0.48 with four, 0.53 with two)
-  const int ts_auto = std::max(4, (c.nslices + c.num_sms - 1) / c.num_sms);
-  // the velocity solves of one system: a block of 768 threads per SM, so that
-  // few blocks are waited for (52k channel: prediction and correction 0.45 ms
-  // per step against 0.55 with two blocks of 384; 131k pipe 3.58 against
-  // 3.77), unless 12 warps hold its items in one round; a batch takes two of
-  // 384, whose instances wait less for each other (16 channels: 1.38 against
-  // 1.44 ms)
-  w->vel_minb = c.tune.vel_blocks_per_sm ? c.tune.vel_blocks_per_sm : (ni > 1 || ts_auto * dim <= 12 ? 2 : 1);
-  c.tune.vel_blocks_per_sm = w->vel_minb;
   const size_t nv = c.nv, rs = c.kmixed ? sizeof(float) : sizeof(double);
+  std::vector<int> ioff(1, 0);
+  for (const HostInst& in : c.inst) ioff.push_back((in.v_off + in.nv_pad) / kSlice);
   int maxslots = 0;
-  // phase 0: the pressure systems where the multigrid is not used
+  // plan 0: the pressure systems where the multigrid is not used
   for (int ph = c.two_level ? 1 : 0; ph < 2; ++ph) {
-    const int ncomp = ph == 0 ? 1 : dim;
-    const int minb = ph == 0 ? 2 : w->vel_minb;
-    const int occ = std::min(minb, occupancy(c.kmixed, minb, 0, 0));
-    if (occ < 1) {
-      set_error("krylov: the solver kernel cannot be resident");
-      return PFEM2_CUDA_ERROR;
-    }
-    // every block takes the same run of slices with all their components
-    int ts = ni > 1 || ph == 0 ? 4 : ts_auto;
+    JacobiPlan& P = w->plan[ph];
+    P.bicg = ph == 0 ? c.p_bicg : c.vel_bicg;
+    const bool tuned = ph == 1 && (c.tune.vel_blocks_per_sm || c.tune.vel_tile_slices);
+    PFEM2_TRY(plan_build(c, w, P, c.kmixed, ioff, c.h_sl_ptr, ph == 0 ? 1 : dim, ph == 0 ? 1 : dim,
+                         ph == 0 ? 0 : c.tune.vel_blocks_per_sm, ph == 0 ? 0 : c.tune.vel_tile_slices, !tuned));
+    maxslots = std::max(maxslots, P.nslots);
     if (ph == 1) {
-      if (c.tune.vel_tile_slices > 0) ts = c.tune.vel_tile_slices;
-      c.tune.vel_tile_slices = ts;
+      if (!c.tune.vel_blocks_per_sm) c.tune.vel_blocks_per_sm = P.minb;
+      if (!c.tune.vel_tile_slices) c.tune.vel_tile_slices = P.ts;
     }
-    const int G = std::max(1, std::min(occ * c.num_sms, (c.nslices + ts - 1) / ts));
-    std::vector<int> bsl(G + 1), binst, binst_off(1, 0), bslot, cnt(ni, 0), slot0(ncomp * ni + 1, 0), slk(c.nslices, 0);
-    for (int b = 0; b <= G; ++b) bsl[b] = (int)((long long)c.nslices * b / G);
-    w->items_max[ph] = 0;
-    size_t meta = 0, ne = 0;
-    for (int b = 0, i = 0; b < G; ++b) {
-      const int s0 = bsl[b], s1 = bsl[b + 1];
-      while ((c.inst[i].v_off + c.inst[i].nv_pad) / kSlice <= s0) ++i;
-      int last = i - 1;
-      for (int sl = s0, j = i; sl < s1; ++sl) {
-        while ((c.inst[j].v_off + c.inst[j].nv_pad) / kSlice <= sl) ++j;
-        for (; last < j; ++last) {
-          binst.push_back(last + 1);
-          bslot.push_back(cnt[last + 1]++);
-        }
-        slk[sl] = j - i;
-      }
-      binst_off.push_back((int)binst.size());
-      if ((binst_off[b + 1] - binst_off[b]) * ncomp > kMaxLocalSys) {
-        set_error("krylov: more than 16 systems would share one block (instances too small for the batch)");
-        return PFEM2_INVALID_ARG;
-      }
-      w->items_max[ph] = std::max(w->items_max[ph], (s1 - s0) * ncomp);
-      meta = std::max(meta, 3 * al16(4 * (size_t)(s1 - s0)));
-      ne = std::max(ne, (size_t)(c.h_sl_ptr[s1] - c.h_sl_ptr[s0]));
-    }
-    for (int k = 0; k < ncomp; ++k)
-      for (int i = 0; i < ni; ++i) slot0[k * ni + i + 1] = slot0[k * ni + i] + cnt[i];
-    w->nslots[ph] = slot0.back();
-    maxslots = std::max(maxslots, w->nslots[ph]);
-    w->grid[ph] = G;
-    w->bicg[ph] = ph == 0 ? c.p_bicg : c.vel_bicg;
-    w->st_meta[ph] = meta;
-    w->st_entries[ph] = ne;
-    PFEM2_TRY(ws_upload(w, &w->blk_inst[ph], binst));
-    PFEM2_TRY(ws_upload(w, &w->blk_inst_off[ph], binst_off));
-    PFEM2_TRY(ws_upload(w, &w->blk_slot[ph], bslot));
-    PFEM2_TRY(ws_upload(w, &w->blk_sl[ph], bsl));
-    PFEM2_TRY(ws_upload(w, &w->sys_slot0[ph], slot0));
-    PFEM2_TRY(ws_upload(w, &w->slk[ph], slk));
   }
   // systems whose components have the same Dirichlet rows share the mass matrix
   w->mass_share = true;
@@ -722,24 +886,100 @@ pfem2_status krylov_setup(Ctx& c) {
     PFEM2_TRY(ws_alloc(w, &w->out_tol[k], dim * ni));
     PFEM2_TRY(ws_alloc(w, &w->out_outer[k], dim * ni));
   }
-  // shared memory per solve (0 prediction, 1 pressure, 2 correction)
+  // residency of the grids with their shared memory (a cluster's is checked with its plan)
   for (int which = 0; which < 3; ++which) {
-    const int ph = which == 1 ? 0 : 1;
-    if (which == 1 && c.two_level) continue;
-    const int minb = ph == 0 ? 2 : w->vel_minb, ncomp = ph == 0 ? 1 : dim;
-    const int nmat = which == 2 && w->mass_share ? 1 : ncomp;
-    size_t smem = al16(sizeof(double) * (w->bicg[ph] ? kMaxSums : 3) * (size_t)w->items_max[ph]);
-    const size_t level[3] = {al16(6 * 32 * rs * (size_t)w->items_max[ph]) + w->st_meta[ph],
-                             al16(4 * w->st_entries[ph]), nmat * al16(rs * w->st_entries[ph])};
+    const JacobiPlan& P = w->plan[which == 1 ? 0 : 1];
+    if ((which == 1 && c.two_level) || P.cluster) continue;
     int sm = 0;
-    while (sm < 3 && smem + level[sm] <= smem_budget(minb)) smem += level[sm++];
-    if (occupancy(c.kmixed, minb, sm, smem) * c.num_sms < w->grid[ph]) {
+    const size_t smem = plan_smem(P, rs, P.minb, which == 1 || (which == 2 && w->mass_share) ? 1 : dim, sm);
+    if (occupancy(c.kmixed, P.minb, sm, smem) * c.num_sms < P.grid) {
       set_error("krylov: the solver grid cannot be resident");
       return PFEM2_CUDA_ERROR;
     }
-    w->sm[which] = sm;
-    w->smem[which] = smem;
   }
+  // (a cluster keeps the same operands in shared memory in every solve)
+  return PFEM2_OK;
+}
+
+// Plan and vectors of the mesh elasticity (moving contexts, first use): one
+// FP64 system of dim x nv rows whose components follow each other, on slices
+// of its own (ale.cu).
+pfem2_status krylov_elastic_setup(Ctx& c, const std::vector<int>& slp) {
+  KrylovWs* w = (KrylovWs*)c.kws;
+  JacobiPlan& P = w->elastic;
+  const std::vector<int> ioff = {0, (int)slp.size() - 1};
+  const size_t n = (size_t)c.nv * c.dim;
+  P.bicg = false;
+  PFEM2_TRY(plan_build(c, w, P, false, ioff, slp, 1, 1, 0, 0, true));
+  double** v[] = {&w->el_pk, &w->el_e, &w->el_r, &w->el_v, &w->el_s, &w->el_t, &w->el_r64, &w->el_part, &w->el_res};
+  const size_t m[] = {2 * 4 * n, n, n, n, n, n, n, 2 * (size_t)kMaxSums * P.nslots, 4};
+  for (int k = 0; k < 9; ++k) PFEM2_TRY(ws_alloc(w, v[k], m[k]));
+  PFEM2_TRY(ws_alloc(w, &w->el_int, 3));
+  int sm = 0;
+  const size_t smem = plan_smem(P, sizeof(double), P.minb, 1, sm);
+  if (!P.cluster && occupancy(false, P.minb, sm, smem) * c.num_sms < P.grid) {
+    set_error("moving mesh: the elasticity solver cannot be resident");
+    return PFEM2_CUDA_ERROR;
+  }
+  return PFEM2_OK;
+}
+
+// CG (Jacobi, FP64) on that system; stops on the recurrence residual. el_res:
+// tol, rtol, residual, tolerance; el_int: max_iter, iterations, spare.
+pfem2_status krylov_elastic_solve(Ctx& c, const ElasticSystem& E, double tol, double rtol, int maxit) {
+  KrylovWs* w = (KrylovWs*)c.kws;
+  const JacobiPlan& P = w->elastic;
+  const double tr[4] = {tol, rtol, 0.0, 0.0};
+  const int mi[3] = {maxit, 0, 0};
+  PFEM2_CUDA(cudaMemcpyAsync(w->el_res, tr, sizeof(tr), cudaMemcpyHostToDevice, c.stream));
+  PFEM2_CUDA(cudaMemcpyAsync(w->el_int, mi, sizeof(mi), cudaMemcpyHostToDevice, c.stream));
+  SolveArgs<double> a{};
+  plan_args(w, P, a);
+  a.ncomp = a.ninst = 1;
+  a.nv = c.nv * c.dim;
+  a.sl_ptr = E.sl_ptr;
+  a.sl_len = E.sl_len;
+  a.sl_col = E.sl_col;
+  a.share = 1;
+  for (int k = 0; k < 3; ++k) {
+    a.A64[k] = a.Ain[k] = E.A;
+    a.dinv[k] = E.dinv;
+    a.x[k] = E.x;
+    a.b[k] = E.rhs;
+    a.isd[k] = E.isd;
+    a.g[k] = E.g;
+  }
+  a.tol_i = w->el_res;
+  a.rtol_i = w->el_res + 1;
+  a.maxit_i = w->el_int;
+  a.pk = (V4<double>*)w->el_pk;
+  a.e = w->el_e;
+  a.r = w->el_r;
+  a.v = w->el_v;
+  a.s = w->el_s;
+  a.t = a.rh = w->el_t;
+  a.r64 = w->el_r64;
+  a.part = w->el_part;
+  a.out_it = w->el_int + 1;
+  a.out_outer = w->el_int + 2;
+  a.out_res = w->el_res + 2;
+  a.out_tol = w->el_res + 3;
+  a.trust = 1;
+  a.iter_cap = 2 * maxit + 64;
+  PFEM2_TRY(krylov_init_solve(c, 1));
+  return plan_launch(c, P, a, 1);
+}
+
+pfem2_status krylov_elastic_read(Ctx& c, int* it, double* res, double* tol) {
+  KrylovWs* w = (KrylovWs*)c.kws;
+  int mi[3];
+  double tr[4];
+  PFEM2_CUDA(cudaMemcpyAsync(mi, w->el_int, sizeof(mi), cudaMemcpyDeviceToHost, c.stream));
+  PFEM2_CUDA(cudaMemcpyAsync(tr, w->el_res, sizeof(tr), cudaMemcpyDeviceToHost, c.stream));
+  PFEM2_CUDA(cudaStreamSynchronize(c.stream));
+  *it = mi[1];
+  *res = tr[2];
+  *tol = tr[3];
   return PFEM2_OK;
 }
 
@@ -781,20 +1021,14 @@ int krylov_max_iter(const Ctx& c) {
 template <typename R>
 static pfem2_status solve_impl(Ctx& c, int which) {
   KrylovWs* w = (KrylovWs*)c.kws;
-  const int ph = which == 1 ? 0 : 1;
+  const JacobiPlan& P = w->plan[which == 1 ? 0 : 1];
   const int ncomp = which == 1 ? 1 : c.dim;
   const int ni = (int)c.inst.size();
   SolveArgs<R> a{};
   a.ncomp = ncomp;
   a.ninst = ni;
   a.nv = c.nv;
-  a.blk_inst = w->blk_inst[ph];
-  a.blk_inst_off = w->blk_inst_off[ph];
-  a.blk_slot = w->blk_slot[ph];
-  a.sys_slot0 = w->sys_slot0[ph];
-  a.blk_sl = w->blk_sl[ph];
-  a.slk = w->slk[ph];
-  a.items_max = w->items_max[ph];
+  plan_args(w, P, a);
   a.sl_ptr = c.sl_ptr;
   a.sl_len = c.sl_len;
   a.sl_col = c.sl_col;
@@ -824,16 +1058,12 @@ static pfem2_status solve_impl(Ctx& c, int which) {
   }
   a.tol_i = (const double*)c.sys_scalars + (which == 1 ? ni : 0);
   a.rtol_i = (const double*)c.sys_scalars + 2 * ni + (which == 1 ? ni : 0);
-  a.bicg = w->bicg[ph] ? 1 : 0;
   a.pk = (V4<R>*)w->pk;
   a.rh = (R*)w->rh; a.s = (R*)w->s; a.t = (R*)w->t; a.v = (R*)w->v;
   a.maxit_i = c.d_sysinfo;
   a.e = (R*)w->e; a.r = (R*)w->r;
   a.r64 = w->r64;
   a.part = w->part;
-  a.nslots = w->nslots[ph];
-  a.scount = w->scount;
-  a.active = w->active;
   a.out_it = w->out_it[which];
   a.out_res = w->out_res[which];
   a.out_tol = w->out_tol[which];
@@ -841,18 +1071,8 @@ static pfem2_status solve_impl(Ctx& c, int which) {
   a.eta = c.kmixed ? c.refine_eta : 0.0;
   // phases per iteration, and the restarts (one phase more, at most max_iter)
   a.iter_cap = (a.bicg ? 5 : 4) * krylov_max_iter(c) + 256;
-  a.gb.count = c.barrier;
-  a.gb.gen = c.barrier + 1;
-  a.gb.err = c.d_err;
-  a.gb.spin_limit = c.spin_limit;
   PFEM2_TRY(krylov_init_solve(c, ncomp * ni));
-  void* args[] = {&a};
-  // the velocity solves at vel_minb blocks per SM, a pressure solve at two
-  const int minb = ph == 0 ? 2 : w->vel_minb;
-  PFEM2_CUDA(cudaLaunchCooperativeKernel(kernel_of<R>(minb, w->sm[which]), dim3(w->grid[ph]), dim3(solve_threads(minb)), args, w->smem[which],
-                                         c.stream));
-  c.launches++;
-  return PFEM2_OK;
+  return plan_launch(c, P, a, P.cluster || !a.share ? ncomp : 1);
 }
 
 pfem2_status krylov_solve(Ctx& c, int which) {

@@ -96,17 +96,24 @@ __device__ __forceinline__ bool wait_count(const unsigned* cnt, unsigned target,
 // ------------------------------------------------------------------ host
 struct MgWs;  // mgcg.cu
 
+// partition of a Jacobi solve over its grid
+struct JacobiPlan {
+  int *blk_inst = nullptr, *blk_inst_off = nullptr, *blk_slot = nullptr, *blk_sl = nullptr, *sys_slot0 = nullptr,
+      *slk = nullptr;
+  int grid = 0, nslots = 0, items_max = 0, minb = 2, ts = 0;
+  int sm = 0;                                      // cluster: what a block keeps in shared memory
+  bool cluster = false, bicg = false;
+  size_t st_meta = 0, st_entries = 0;              // per block: static index bytes, SELL entries
+};
+
 struct KrylovWs {
-  // Jacobi solves, [0] pressure (without multigrid), [1] velocity components
-  int *blk_inst[2] = {}, *blk_inst_off[2] = {}, *blk_slot[2] = {}, *blk_sl[2] = {}, *sys_slot0[2] = {}, *slk[2] = {};
-  int grid[2] = {}, nslots[2] = {}, items_max[2] = {};
-  size_t st_meta[2] = {}, st_entries[2] = {};      // per block: static index bytes, SELL entries
-  bool bicg[2] = {false, false};                   // phase solved by BiCGStab
+  JacobiPlan plan[2];                              // [0] pressure (without multigrid), [1] velocity components
+  JacobiPlan elastic;                              // mesh elasticity
+  double *el_pk = nullptr, *el_e = nullptr, *el_r = nullptr, *el_v = nullptr, *el_s = nullptr, *el_t = nullptr,
+         *el_r64 = nullptr, *el_part = nullptr, *el_res = nullptr;
+  int* el_int = nullptr;
   bool mass_share = false;                         // the components' mass matrices are equal
-  int sm[3] = {};                                  // what is kept in shared memory per solve
-  size_t smem[3] = {};                             // dynamic shared memory per solve
   void *pk = nullptr, *rh = nullptr, *s = nullptr, *t = nullptr, *v = nullptr;
-  int vel_minb = 2;  // resident blocks per SM of the velocity solves
   MgWs* mg = nullptr;
   void *e = nullptr, *r = nullptr;
   double* r64 = nullptr;
