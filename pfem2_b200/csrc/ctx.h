@@ -15,6 +15,9 @@ constexpr int kSlice = 32;          // SELL slice height (rows per warp)
 constexpr int kMaxPatch = 32;       // max cells around a vertex
 constexpr int kMaxRing = 64;        // max cells sharing a vertex with a cell
 constexpr int kNumSys = 7;          // pred x,y,z, pressure, mass x,y,z
+// re-sort: list entries stored per cell (a longer list lies in the overflow part), cells of a tile of its scan
+constexpr int kListStride = 64, kScanTile = 2048;
+constexpr int kMoverMax = 256;      // longest mover list of a cell (ranked in as many ints of shared memory)
 constexpr int kFarMax = 16384;      // far-mover list capacity (sorted in 128 KB of shared memory)
 
 // Per-instance parameters visible to kernels.
@@ -42,6 +45,14 @@ struct HostInst {
 struct Tile {
   int sys;
   int s0, s1;
+};
+
+// particles that changed cell within the 1-ring of their old cell, by new
+// cell, in no order: a cell's list holds the first cap, cnt counts them all
+struct Movers {
+  int* cnt = nullptr;   // [nc], reset before each advection
+  int* list = nullptr;  // [nc][cap]
+  int cap = 0;
 };
 
 struct Ctx {
@@ -78,8 +89,7 @@ struct Ctx {
   void* cell_geo = nullptr;   // [nc] CellGeo<dim, Real>: local frame, inverse Jacobian, affine flag
   int* ring_ptr = nullptr;
   int* ring_cell = nullptr;
-  int* ring_rev = nullptr;       // [ring entry (c, k)] position of c in the ring of ring_cell[k]
-  unsigned* dest_mask = nullptr; // [nc] per old cell: ring positions that received movers (reset per advection)
+  Movers movers;                 // of the last advection, by new cell
   DevInst* d_inst = nullptr;
   std::vector<DevInst> h_inst;
 
@@ -140,7 +150,10 @@ struct Ctx {
   // the environment variable PFEM2_ADVECT_SPLIT_MIN overrides it at creation
   long long adv_split_min = 0;
   int* cell_start[2] = {};
-  unsigned long long* rebin_tiles = nullptr;  // ticket + status words of the rebin's single-pass scan
+  unsigned long long* rebin_tiles = nullptr;  // ticket + status words of the re-sort's scan, overflow fill count
+  int* rebin_cnt = nullptr;                   // [nc] particles of each cell after the re-sort
+  int* rebin_pos = nullptr;                   // [nc] where a list longer than the stride lies in the overflow part
+  int* rebin_list = nullptr;                  // [nc][kListStride] lists, then pcap entries of overflow
   int* d_np = nullptr;       // [2] particle count of buffer 0/1
   int far_cap = 0;
   unsigned long long* far_keys = nullptr;

@@ -17,6 +17,7 @@
 //                   (:723-772), with the projection partials fused in
 //   k_project_*     distribute_particle_velocities_to_grid (:858-918)
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 
@@ -27,16 +28,17 @@ namespace pfem2 {
 
 constexpr int kRebinWarps = 8;
 constexpr int kMaxBuckets = 256;
-// resident rebin blocks per SM the registers are capped for: the kernel is
-// bound by dependent loads, so resident warps pay more than registers; in 2D
-// FP32 six blocks (48 warps) measured 17% faster than the four that 64
-// registers allowed, in 3D FP32 four blocks 36% faster than uncapped; with
-// FP64 particles five blocks in 2D (0.186 -> 0.110 ms on the 52k-cell
-// channel against two uncapped, 96 registers) and three in 3D (3.15 -> 1.61
-// ms on the 442k-cell pipe against one, 181 registers)
+// Resident blocks per SM that the re-sort kernels' registers are capped for.
+// Both wait for dependent loads, so resident warps pay until the spilled
+// registers' traffic (every store reaches the L2) outweighs them. Re-sort of
+// the 1M-cell FP32 mesh with 6 / 5 blocks (gather / write) 1.04 ms; 6 / 6:
+// 1.66, 4 / 4: 1.15, 8 / 5: 1.06; 201k-cell FP64 mesh with 6 / 4 0.240 ms,
+// 4 / 4: 0.262, 3 / 4: 0.301; 131k-cell pipe, FP32 particles, 4 / 3 0.367 ms,
+// 3 / 3: 0.435, 4 / 4: 0.53; 10k-cell pipe, FP64, 3 / 2 0.038 ms, 4 / 3: 0.053.
 template <int DIM, typename R>
 struct RebinMinBlocks {
-  static constexpr int value = sizeof(R) == 4 ? (DIM == 2 ? 6 : 4) : (DIM == 2 ? 5 : 3);
+  static constexpr int gather = sizeof(R) == 4 ? (DIM == 2 ? 6 : 4) : (DIM == 2 ? 6 : 3);
+  static constexpr int write = sizeof(R) == 4 ? (DIM == 2 ? 5 : 3) : (DIM == 2 ? 4 : 2);
 };
 
 // ------------------------------------------------------------------ seed
@@ -408,22 +410,21 @@ __device__ __forceinline__ int advect_steps(int c0, R* x, R dts, int s0, int& s_
 __device__ __forceinline__ void advect_record(int p, int c0, int c, const int* __restrict__ ring_ptr,
                                               const int* __restrict__ ring_cell,
                                               unsigned long long* __restrict__ far_keys, int far_cap,
-                                              int* __restrict__ counters, unsigned* __restrict__ dest_mask) {
+                                              int* __restrict__ counters, const Movers mv) {
   if (c < 0) {
     atomicAdd(counters + CNT_DELETED, 1);
   } else if (c != c0) {
-    // a particle that left the 1-ring of its old cell goes to the far list;
-    // one that stays in it marks its destination (bit = ring position) in
-    // the old cell's mask, so that the re-sort scans only segments that send
-    // particles to a cell
+    // a particle that stays in the 1-ring of its old cell goes to the mover
+    // list of its new cell; one that left it to the far list, and its place
+    // in the mover list, drawn before the ring is searched, stays empty
+    const int k = atomicAdd(mv.cnt + c, 1);
     bool near = false;
-    const int r0 = __ldg(ring_ptr + c0);
-    for (int rr = r0; rr < __ldg(ring_ptr + c0 + 1); ++rr)
+    for (int rr = __ldg(ring_ptr + c0); rr < __ldg(ring_ptr + c0 + 1); ++rr)
       if (__ldg(ring_cell + rr) == c) {
         near = true;
-        atomicOr(dest_mask + c0, rr - r0 < 32 ? 1u << (rr - r0) : 0xffffffffu);
         break;
       }
+    if (k < mv.cap) mv.list[(size_t)c * mv.cap + k] = near ? p : INT_MAX;
     if (!near) {
       int slot = atomicAdd(counters + CNT_FAR, 1);
       if (slot < far_cap) far_keys[slot] = ((unsigned long long)(unsigned)c << 32) | (unsigned)p;
@@ -442,7 +443,7 @@ __global__ void __launch_bounds__(256, AdvectMinBlocks<DIM, R>::value) k_advect_
     const R* __restrict__ Vr, const R* __restrict__ dVr, int nv, int S, const DevInst* __restrict__ inst,
     const int* __restrict__ cell_inst, const int* __restrict__ v2c_ptr, const int* __restrict__ v2c_cell,
     const R* __restrict__ v2c_dir, const int* __restrict__ ring_ptr, const int* __restrict__ ring_cell,
-    unsigned long long* __restrict__ far_keys, int far_cap, int* __restrict__ counters, unsigned* __restrict__ dest_mask) {
+    unsigned long long* __restrict__ far_keys, int far_cap, int* __restrict__ counters, const Movers mv) {
   constexpr int NV = Dims<DIM>::NV;
   const int n = min(*d_np, (int)cap);
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
@@ -468,7 +469,7 @@ __global__ void __launch_bounds__(256, AdvectMinBlocks<DIM, R>::value) k_advect_
     int s_left = 0;
     int c = advect_steps<DIM, R, true>(c0, x, dts, 0, s_left, S, geo, cv, Vr, nv, v2c_ptr, v2c_cell, v2c_dir);
     if (c < 0) c = -1;
-    advect_record(p, c0, c, ring_ptr, ring_cell, far_keys, far_cap, counters, dest_mask);
+    advect_record(p, c0, c, ring_ptr, ring_cell, far_keys, far_cap, counters, mv);
     newcell[p] = c;
 #pragma unroll
     for (int d = 0; d < DIM; ++d) xi[d * cap + p] = x[d];
@@ -494,7 +495,7 @@ __global__ void __launch_bounds__(kAdvThreads, AdvectMinBlocks<DIM, R>::value) k
     const R* __restrict__ Vr, const R* __restrict__ dVr, int nv, int S, const DevInst* __restrict__ inst,
     const int* __restrict__ cell_inst, const int* __restrict__ v2c_ptr, const int* __restrict__ v2c_cell,
     const R* __restrict__ v2c_dir, const int* __restrict__ ring_ptr, const int* __restrict__ ring_cell,
-    unsigned long long* __restrict__ far_keys, int far_cap, int* __restrict__ counters, unsigned* __restrict__ dest_mask) {
+    unsigned long long* __restrict__ far_keys, int far_cap, int* __restrict__ counters, const Movers mv) {
   constexpr int NV = Dims<DIM>::NV;
   constexpr int NW = kAdvThreads / 32;
   constexpr int QN = 64;  // below 32 left over + 32 appended
@@ -506,22 +507,42 @@ __global__ void __launch_bounds__(kAdvThreads, AdvectMinBlocks<DIM, R>::value) k
   const int lo = min(n, (int)blockIdx.x * chunk), hi = min(n, lo + chunk);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int nq = 0;  // the warp's queued particles (uniform over the warp)
+  // 2D: a slice's records are loaded while the one before it is worked on
+  // (32M FP32 particles: 1.16 -> 1.09 ms; the FP64 3D kernel, at its register
+  // limit, 1.27 -> 1.31 ms on the 131k-cell pipe)
+  constexpr bool AHEAD = DIM == 2;
+  int c_next = 0;
+  R x_next[DIM], u_next[DIM];
+  const auto fetch = [&](int p) {
+    if (p < hi) {
+      c_next = cell[p];
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) {
+        x_next[d] = xi[d * cap + p];
+        if (FUSE) u_next[d] = u[d * cap + p];
+      }
+    }
+  };
+  if (AHEAD) fetch(lo + warp * 32 + lane);
   for (int base = lo + warp * 32;; base += kAdvThreads) {
     const bool more = base < hi;  // uniform over the warp
     if (more) {
       const int p = base + lane;
       bool leave = false;
-      int s_left = 0, c0 = 0;
-      R x[DIM];
+      int s_left = 0;
+      if (!AHEAD) fetch(p);
+      const int c0 = c_next;
+      R x[DIM], up[DIM];
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) {
+        x[d] = x_next[d];
+        up[d] = u_next[d];
+      }
+      if (AHEAD) fetch(p + kAdvThreads);
       if (p < hi) {
-        c0 = cell[p];
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) x[d] = xi[d * cap + p];
         if (FUSE) {
-          R N[NV], up[DIM];
+          R N[NV];
           shape_values<DIM, R>(x, N);
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) up[d] = u[d * cap + p];
 #pragma unroll
           for (int v = 0; v < NV; ++v) {
             const int g = __ldg(cv + (size_t)c0 * NV + v);
@@ -567,7 +588,7 @@ __global__ void __launch_bounds__(kAdvThreads, AdvectMinBlocks<DIM, R>::value) k
         int c = advect_steps<DIM, R, true>(c0, x, dts, (int)q_s[warp][k], s_left, S, geo, cv, Vr, nv, v2c_ptr,
                                            v2c_cell, v2c_dir);
         if (c < 0) c = -1;
-        advect_record(p, c0, c, ring_ptr, ring_cell, far_keys, far_cap, counters, dest_mask);
+        advect_record(p, c0, c, ring_ptr, ring_cell, far_keys, far_cap, counters, mv);
         newcell[p] = c;
 #pragma unroll
         for (int d = 0; d < DIM; ++d) xi[d * cap + p] = x[d];
@@ -616,7 +637,7 @@ __global__ void __launch_bounds__(256) k_relocate(
     const int* __restrict__ v2c_ptr, const int* __restrict__ v2c_cell, const R* __restrict__ v2c_dir,
     const double* __restrict__ xphys, const int* __restrict__ ring_ptr, const int* __restrict__ ring_cell,
     unsigned long long* __restrict__ far_keys, int far_cap, int* __restrict__ counters,
-    unsigned* __restrict__ dest_mask) {
+    const Movers mv) {
   constexpr int NV = Dims<DIM>::NV;
   const int n = min(*d_np, (int)cap);
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
@@ -644,7 +665,7 @@ __global__ void __launch_bounds__(256) k_relocate(
       for (int v = 0; v < NV; ++v) gvx[v] = __ldg(cv + (size_t)c0 * NV + v);
       if (!locate_from<DIM, R>(c, G, L, x0, xo, xn, uf, x, gvx, geo, v2c_ptr, v2c_cell, v2c_dir)) c = -1;
     }
-    advect_record(p, c0, c, ring_ptr, ring_cell, far_keys, far_cap, counters, dest_mask);
+    advect_record(p, c0, c, ring_ptr, ring_cell, far_keys, far_cap, counters, mv);
     newcell[p] = c;
     if (c >= 0)
 #pragma unroll
@@ -725,11 +746,11 @@ template <int DIM, typename R>
 static pfem2_status relocate_impl(Ctx& c, const double* xphys) {
   const int b = c.cur;
   PFEM2_CUDA(cudaMemsetAsync(c.d_counters, 0, sizeof(int) * CNT_N_STATS, c.stream));
-  PFEM2_CUDA(cudaMemsetAsync(c.dest_mask, 0, sizeof(unsigned) * c.nc, c.stream));
+  PFEM2_CUDA(cudaMemsetAsync(c.movers.cnt, 0, sizeof(int) * c.nc, c.stream));
   k_relocate<DIM, R><<<grid_for(c, c.pcap, 256, 8), 256, 0, c.stream>>>(
       c.pcell[b], (R*)c.pxi[b], c.newcell, (size_t)c.pcap, c.d_np + b, (const CellGeo<DIM, R>*)c.cell_geo, c.cv,
       c.v2c_ptr, c.v2c_cell, (const R*)c.v2c_dir_r, xphys, c.ring_ptr, c.ring_cell, c.far_keys, c.far_cap,
-      c.d_counters, c.dest_mask);
+      c.d_counters, c.movers);
   k_far_sort<<<1, 1024, sizeof(unsigned long long) * c.far_cap, c.stream>>>(c.far_keys, c.d_counters, c.far_cap);
   c.launches += 2;
   return PFEM2_OK;
@@ -801,13 +822,13 @@ static pfem2_status advect_impl(Ctx& c, bool fuse) {
           c.pcell[b], (R*)c.pxi[b], (R*)c.pu[b], c.newcell, (size_t)c.pcap, c.d_np + b,
           (const CellGeo<DIM, R>*)c.cell_geo, c.cv, (const R*)c.Vr, (const R*)c.dVr, c.nv, S, c.d_inst, c.cell_inst,
           c.v2c_ptr, c.v2c_cell, (const R*)c.v2c_dir_r, c.ring_ptr, c.ring_cell, c.far_keys, c.far_cap, c.d_counters,
-          c.dest_mask);
+          c.movers);
     else
       k_advect_one<DIM, R, false><<<grid, 256, 0, c.stream>>>(
           c.pcell[b], (R*)c.pxi[b], (R*)c.pu[b], c.newcell, (size_t)c.pcap, c.d_np + b,
           (const CellGeo<DIM, R>*)c.cell_geo, c.cv, (const R*)c.Vr, (const R*)c.dVr, c.nv, S, c.d_inst, c.cell_inst,
           c.v2c_ptr, c.v2c_cell, (const R*)c.v2c_dir_r, c.ring_ptr, c.ring_cell, c.far_keys, c.far_cap, c.d_counters,
-          c.dest_mask);
+          c.movers);
     c.launches++;
   } else {
     // the queue kernel's blocks walk contiguous chunks
@@ -817,13 +838,13 @@ static pfem2_status advect_impl(Ctx& c, bool fuse) {
           c.pcell[b], (R*)c.pxi[b], (R*)c.pu[b], c.newcell, (size_t)c.pcap, c.d_np + b,
           (const CellGeo<DIM, R>*)c.cell_geo, c.cv, (const R*)c.Vr, (const R*)c.dVr, c.nv, S, c.d_inst, c.cell_inst,
           c.v2c_ptr, c.v2c_cell, (const R*)c.v2c_dir_r, c.ring_ptr, c.ring_cell, c.far_keys, c.far_cap, c.d_counters,
-          c.dest_mask);
+          c.movers);
     else
       k_advect_q<DIM, R, false><<<grid, kAdvThreads, 0, c.stream>>>(
           c.pcell[b], (R*)c.pxi[b], (R*)c.pu[b], c.newcell, (size_t)c.pcap, c.d_np + b,
           (const CellGeo<DIM, R>*)c.cell_geo, c.cv, (const R*)c.Vr, (const R*)c.dVr, c.nv, S, c.d_inst, c.cell_inst,
           c.v2c_ptr, c.v2c_cell, (const R*)c.v2c_dir_r, c.ring_ptr, c.ring_cell, c.far_keys, c.far_cap, c.d_counters,
-          c.dest_mask);
+          c.movers);
     c.launches++;
   }
   k_far_sort<<<1, 1024, sizeof(unsigned long long) * c.far_cap, c.stream>>>(c.far_keys, c.d_counters, c.far_cap);
@@ -833,17 +854,16 @@ static pfem2_status advect_impl(Ctx& c, bool fuse) {
 
 pfem2_status launch_advect(Ctx& c, bool fuse) {
   PFEM2_CUDA(cudaMemsetAsync(c.d_counters, 0, sizeof(int) * CNT_N_STATS, c.stream));
-  PFEM2_CUDA(cudaMemsetAsync(c.dest_mask, 0, sizeof(unsigned) * c.nc, c.stream));
+  PFEM2_CUDA(cudaMemsetAsync(c.movers.cnt, 0, sizeof(int) * c.nc, c.stream));
   if (c.dim == 2) return c.pmixed ? advect_impl<2, float>(c, fuse) : advect_impl<2, double>(c, fuse);
   return c.pmixed ? advect_impl<3, float>(c, fuse) : advect_impl<3, double>(c, fuse);
 }
 
 // ----------------------------------------------------------------- rebin
-// One warp per target cell. Pass 0 counts, pass 1 writes. The incoming
-// particles of cell c are gathered from the old segments of the cells
-// sharing a vertex with c (ascending cell id, segment order), so the
-// result is a stable sort by cell of the old storage order; particles that
-// left that 1-ring come from the sorted far list and are merged by index.
+// One warp per target cell. The incoming particles of cell c are its stayers,
+// the movers that advection listed for it and particles from beyond its 1-ring
+// in the sorted far list, in ascending old index, so the result is a stable
+// sort by cell of the old storage order.
 // With CHECK the per-sub-cell counts are walked in that order: a particle
 // whose bucket already holds MAX_PARTICLES_PER_CELL_PART is removed, and
 // every empty sub-cell receives one particle at its centre, appended in
@@ -886,7 +906,7 @@ __device__ __forceinline__ void proj_store(ProjAcc<DIM, R>& acc, R* __restrict__
 // For FP32 coordinates xi * q is exact in FP64, so that happens only when
 // it is an integer; for FP64 coordinates a relative 1e-12 decides.
 template <typename R>
-__device__ __forceinline__ int sub_bucket_fp64(R xr, double h, int q) {
+__device__ __forceinline__ int sub_bucket_fp64(R xr, const double& h, int q) {
   const double xi = (double)xr;
   double t = xi * (double)q;
   if (sizeof(R) == 4) {
@@ -900,7 +920,7 @@ __device__ __forceinline__ int sub_bucket_fp64(R xr, double h, int q) {
 }
 
 template <typename R>
-__device__ __forceinline__ int sub_bucket(R xr, double h, int q) {
+__device__ __forceinline__ int sub_bucket(R xr, const double& h, int q) {
   return sub_bucket_fp64<R>(xr, h, q);
 }
 
@@ -911,7 +931,7 @@ __device__ __forceinline__ int sub_bucket(R xr, double h, int q) {
 // as for 0, 1 and anything outside (0, 1)). Same results as the FP64 form,
 // with integer instructions only.
 template <>
-__device__ __forceinline__ int sub_bucket<float>(float xr, double h, int q) {
+__device__ __forceinline__ int sub_bucket<float>(float xr, const double& h, int q) {
   const unsigned b = __float_as_uint(xr);
   if (b - 1u < 0x3f7fffffu) {  // 0 < xi < 1 (positive, below the bits of 1.0f)
     const int e = (int)(b >> 23);
@@ -949,107 +969,98 @@ __device__ __forceinline__ int far_lower_bound(const unsigned long long* keys, i
   return lo;
 }
 
-// status words of the single-pass scan over tiles of kRebinWarps cells:
-// bits 62-63 = 1 (tile aggregate known) or 2 (inclusive prefix known), the
-// low bits the value
-constexpr unsigned long long kTileAgg = 1ull << 62, kTilePre = 2ull << 62, kTileVal = (1ull << 62) - 1;
+// The re-sort runs as three kernels. k_rebin_gather: a warp per target cell
+// gathers and checks its incoming particles and stores their list and count.
+// k_rebin_scan: exclusive sums of the counts. k_rebin_write: a warp per cell
+// copies its particles to their new place with the projection partials. No
+// warp waits for another, except in the scan (0.013 ms for 1M cells). As one
+// kernel, where a block of eight cells looked back over the blocks before it
+// for its offset, the ticket, the look-back and the block barriers cost more
+// than the lists' way through memory. All are bound by dependent loads and by
+// issue (gather 560, write 340 warp instructions a cell of 28 FP32 particles,
+// 50% and 42% of the issue slots), not by bytes. 1M cells, 28M particles, FP32:
+// 1.73 -> 1.04 ms (1.51 with the mover lists alone); 201k cells, 3M particles,
+// FP64: 0.365 -> 0.240 ms; 52k cells, 1.7M, FP32: 0.147 -> 0.117 ms; 131k-cell
+// pipe, 3.5M, FP32: 0.575 -> 0.370 ms.
 
-// One pass: a block takes tiles of kRebinWarps consecutive target cells in
-// ticket order (an atomic counter, so a block waits only on tiles taken by
-// blocks already running), a warp per cell gathers and checks its incoming
-// particles into shared memory, the block publishes the tile's particle
-// count and finds its output offset by looking back over the previous
-// tiles' published counts (decoupled look-back; waits bounded, a timeout is
-// flagged in CNT_SCAN_TIMEOUT), then every warp writes its cell's particles,
-// its new_start entry and its projection partials.
-template <int DIM, typename R, bool CHECK, bool PROJ>
-__global__ void __launch_bounds__(kRebinWarps * 32, RebinMinBlocks<DIM, R>::value) k_rebin(
-    const int* __restrict__ old_start, const int* __restrict__ newcell, const R* __restrict__ oxi,
-    const R* __restrict__ ou, size_t cap, int* __restrict__ ncell, R* __restrict__ nxi, R* __restrict__ nu,
-    int* __restrict__ new_start, int* __restrict__ np_out, int nc, const int* __restrict__ ring_ptr,
-    const int* __restrict__ ring_cell, const int* __restrict__ ring_rev,
-    const unsigned* __restrict__ dest_mask, const unsigned long long* __restrict__ far_keys, int far_cap,
-    const DevInst* __restrict__ inst, const int* __restrict__ cell_inst, const int* __restrict__ cv,
-    const R* __restrict__ Vr, int nv, R* __restrict__ partial, int list_cap, int* __restrict__ counters,
-    unsigned long long* __restrict__ tiles, unsigned spin_limit) {
-  constexpr int NV = Dims<DIM>::NV;
+// Incoming particles of cell c in ascending old index, written to list by the
+// calling warp: the stayers are a run of the cell's old segment, the movers
+// come unordered from the cell's mover list and are ranked by comparing each
+// with all (scratch: kMaxBuckets ints, 16-byte aligned); movers from cells
+// before c precede the stayers, the others follow. Returns their number (the
+// entries beyond list_cap are dropped). A cell with more movers than its list
+// holds scans the old segments of its whole 1-ring.
+__device__ __forceinline__ int gather_incoming(int c, const int* __restrict__ old_start,
+                                               const int* __restrict__ newcell, int cap,
+                                               const int* __restrict__ ring_ptr, const int* __restrict__ ring_cell,
+                                               const Movers& mv, int* list, int* scratch, int list_cap) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = lanemask_lt();
+  const int nm = mv.cnt[c], sb = min(old_start[c], cap), se = min(old_start[c + 1], cap);
+  int m0 = lane < nm ? mv.list[(size_t)c * mv.cap + lane] : INT_MAX;
+  int v = sb + lane < se ? newcell[sb + lane] : -1;
+  int n = 0;
+  const auto append = [&](int p, bool in) {
+    const unsigned m = __ballot_sync(PFEM2_FULL_MASK, in);
+    const int pos = n + __popc(m & lt);
+    if (in && pos < list_cap) list[pos] = p;
+    n += __popc(m);
+  };
+  if (nm > mv.cap) {
+    for (int r = __ldg(ring_ptr + c); r < __ldg(ring_ptr + c + 1); ++r) {
+      const int s = __ldg(ring_cell + r);
+      const int e = min(old_start[s + 1], cap);
+      for (int base = min(old_start[s], cap); base < e; base += 32)
+        append(base + lane, base + lane < e && newcell[base + lane] == c);
+    }
+    return n;
+  }
+  int n_mv = __popc(__ballot_sync(PFEM2_FULL_MASK, m0 != INT_MAX));
+  if (nm > 0) scratch[lane] = m0;
+  n = __popc(__ballot_sync(PFEM2_FULL_MASK, m0 < sb));
+  for (int i = 32; i < nm; i += 32) {
+    const int m = i + lane < nm ? mv.list[(size_t)c * mv.cap + i + lane] : INT_MAX;
+    scratch[i + lane] = m;
+    n += __popc(__ballot_sync(PFEM2_FULL_MASK, m < sb));
+    n_mv += __popc(__ballot_sync(PFEM2_FULL_MASK, m != INT_MAX));
+  }
+  const int n_lo = n;
+  append(sb + lane, v == c);
+  for (int base = sb + 32; base < se; base += 32) {
+    v = base + lane < se ? newcell[base + lane] : -1;
+    append(base + lane, v == c);
+  }
+  __syncwarp();
+  const int n_stay = n - n_lo;
+  for (int i = lane; i < nm; i += 32) {
+    const int m = i < 32 ? m0 : scratch[i];
+    int rank = 0;
+    for (int k = 0; k < nm; k += 4) {
+      const int4 q = *reinterpret_cast<const int4*>(scratch + k);
+      rank += (q.x < m) + (q.y < m) + (q.z < m) + (q.w < m);
+    }
+    const int pos = rank < n_lo ? rank : rank + n_stay;
+    if (m != INT_MAX && pos < list_cap) list[pos] = m;
+  }
+  __syncwarp();
+  return n_mv + n_stay;
+}
+
+template <int DIM, typename R, bool CHECK>
+__global__ void __launch_bounds__(kRebinWarps * 32, RebinMinBlocks<DIM, R>::gather) k_rebin_gather(
+    const int* __restrict__ old_start, const int* __restrict__ newcell, const R* __restrict__ oxi, size_t cap, int nc,
+    const int* __restrict__ ring_ptr, const int* __restrict__ ring_cell, const Movers mv, const unsigned long long* __restrict__ far_keys, int far_cap,
+    const DevInst* __restrict__ inst, const int* __restrict__ cell_inst, int list_cap, int* __restrict__ counters,
+    int* __restrict__ cnt, int* __restrict__ glist, int* __restrict__ glist_pos, int* __restrict__ novf) {
   extern __shared__ int smem[];
-  __shared__ int s_tile, s_base;
-  __shared__ int s_cnt[kRebinWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int* list = smem + warp * (list_cap + kMaxBuckets);
-  int* bcnt = list + list_cap;
+  int* bcnt = smem + warp * kMaxBuckets;
+  int* list = smem + kRebinWarps * kMaxBuckets + warp * list_cap;
   const unsigned lt = lanemask_lt();
   int nfar = counters[CNT_FAR];
   if (nfar > far_cap) nfar = far_cap;
-  const int ntiles = (nc + kRebinWarps - 1) / kRebinWarps;
-  unsigned long long* status = tiles + 1;
-  for (;;) {
-    if (threadIdx.x == 0) s_tile = (int)atomicAdd(tiles, 1ull);
-    __syncthreads();
-    const int t = s_tile;
-    if (t >= ntiles) break;
-    const int c = t * kRebinWarps + warp;
-    int ntot = 0;
-    if (c < nc) {
-    // gather the incoming particles of c in (ring cell, segment) order: the
-    // ring's segment bounds are loaded across lanes, segments of neighbours
-    // that sent no particle to c (their destination masks) are dropped, then
-    // the first 32 new-cell ids of 8 remaining segments at a time, so the
-    // loads overlap
-    int n_in = 0;
-    const int r0 = __ldg(ring_ptr + c), nr = __ldg(ring_ptr + c + 1) - r0;
-    for (int kb = 0; kb < nr; kb += 32) {
-      int sb = 0, se = 0;
-      if (kb + lane < nr) {
-        const int s = __ldg(ring_cell + r0 + kb + lane);
-        sb = min(old_start[s], (int)cap);
-        se = min(old_start[s + 1], (int)cap);
-        if (s != c) {
-          const int rv = __ldg(ring_rev + r0 + kb + lane);
-          const unsigned m = dest_mask[s];
-          const bool sends = rv < 32 ? ((m >> rv) & 1u) != 0u : m != 0u;
-          if (!sends) se = sb;
-        }
-      }
-      unsigned act = __ballot_sync(PFEM2_FULL_MASK, se > sb);
-      while (act) {
-        int idx[8], v[8], bs[8], es[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          idx[j] = act ? __ffs(act) - 1 : -1;
-          act &= act ? act - 1u : 0u;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int src = idx[j] < 0 ? 0 : idx[j];
-          bs[j] = __shfl_sync(PFEM2_FULL_MASK, sb, src);
-          es[j] = __shfl_sync(PFEM2_FULL_MASK, se, src);
-          const int p = bs[j] + lane;
-          v[j] = (idx[j] >= 0 && p < es[j]) ? newcell[p] : -1;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (idx[j] < 0) break;
-          {
-            const int p = bs[j] + lane;
-            const bool pred = v[j] == c;
-            const unsigned m = __ballot_sync(PFEM2_FULL_MASK, pred);
-            const int pos = n_in + __popc(m & lt);
-            if (pred && pos < list_cap) list[pos] = p;
-            n_in += __popc(m);
-          }
-          for (int base = bs[j] + 32; base < es[j]; base += 32) {  // segments longer than a warp
-            const int p = base + lane;
-            const bool pred = p < es[j] && newcell[p] == c;
-            const unsigned m = __ballot_sync(PFEM2_FULL_MASK, pred);
-            const int pos = n_in + __popc(m & lt);
-            if (pred && pos < list_cap) list[pos] = p;
-            n_in += __popc(m);
-          }
-        }
-      }
-    }
+  for (int c = blockIdx.x * kRebinWarps + warp; c < nc; c += gridDim.x * kRebinWarps) {
+    int n_in = gather_incoming(c, old_start, newcell, (int)cap, ring_ptr, ring_cell, mv, list, bcnt, list_cap);
     if (nfar > 0) {
       const int lo = far_lower_bound(far_keys, nfar, (unsigned long long)(unsigned)c << 32);
       const int hi = far_lower_bound(far_keys, nfar, (unsigned long long)(unsigned)(c + 1) << 32);
@@ -1075,53 +1086,61 @@ __global__ void __launch_bounds__(kRebinWarps * 32, RebinMinBlocks<DIM, R>::valu
       if (lane == 0) atomicExch(counters + CNT_LIST_OVERFLOW, 1);
       n_in = list_cap;
     }
-    const DevInst& I = inst[__ldg(cell_inst + c)];
-    const int q0 = I.q[0], q1 = I.q[1], q2 = DIM == 3 ? I.q[2] : 1;
-    const int nb1 = q1 + 1, nb2 = q2 + 1;
-    const double h0 = I.h[0], h1 = I.h[1], h2 = I.h[2];
     int n_keep = n_in, n_new = 0;
     if (CHECK) {
-      const int nb = (q0 + 1) * nb1 * nb2;
-      for (int k = lane; k < nb; k += 32) bcnt[k] = 0;
-      __syncwarp();
+      const DevInst& I = inst[__ldg(cell_inst + c)];
+      const int q0 = I.q[0], q1 = I.q[1], q2 = DIM == 3 ? I.q[2] : 1;
+      const int nb1 = q1 + 1, nb2 = q2 + 1;
+      // one chunk of 32 particles needs no counts in shared memory, and up to
+      // 32 sub-cells fit a mask of the occupied ones
+      const int Q = q0 * q1 * q2;
+      const bool masked = Q <= 32, counts = n_in > 32 || !masked;
+      unsigned occupied = 0;
+      if (counts) {
+        const int nb = (q0 + 1) * nb1 * nb2;
+        for (int k = lane; k < nb; k += 32) bcnt[k] = 0;
+        __syncwarp();
+      }
       n_keep = 0;
       for (int base = 0; base < n_in; base += 32) {
         const int i = base + lane;
         const bool active = i < n_in;
         const int p = active ? list[i] : -1;
         int bi = -1;
+        unsigned bit = 0;
         if (active) {
-          const int b0 = sub_bucket<R>(oxi[p], h0, q0);
-          const int b1 = sub_bucket<R>(oxi[cap + p], h1, q1);
-          const int b2 = DIM == 3 ? sub_bucket<R>(oxi[2 * cap + p], h2, q2) : 0;
+          const int b0 = sub_bucket<R>(oxi[p], I.h[0], q0);
+          const int b1 = sub_bucket<R>(oxi[cap + p], I.h[1], q1);
+          const int b2 = DIM == 3 ? sub_bucket<R>(oxi[2 * cap + p], I.h[2], q2) : 0;
           bi = (b0 * nb1 + b1) * nb2 + b2;
+          if (masked && b0 < q0 && b1 < q1 && b2 < q2) bit = 1u << ((b0 * q1 + b1) * q2 + b2);
         }
+        occupied |= __reduce_or_sync(PFEM2_FULL_MASK, bit);
         const unsigned peers = __match_any_sync(PFEM2_FULL_MASK, bi);
-        bool keep = false;
         int prev = 0;
-        if (active) prev = bcnt[bi];
-        __syncwarp();
-        if (active) {
-          keep = prev + __popc(peers & lt) + 1 <= I.max_per_part;
-          if ((peers & lt) == 0) bcnt[bi] = prev + __popc(peers);
+        if (counts) {
+          if (active) prev = bcnt[bi];
+          __syncwarp();
+          if (active && (peers & lt) == 0) bcnt[bi] = prev + __popc(peers);
         }
+        const bool keep = active && prev + __popc(peers & lt) + 1 <= I.max_per_part;
         const unsigned km = __ballot_sync(PFEM2_FULL_MASK, keep);
         const int kpos = n_keep + __popc(km & lt);
         __syncwarp();
-        if (keep) list[kpos] = p;
+        if (keep && kpos != i) list[kpos] = p;  // kpos <= i: no particle is overwritten before it is read
         n_keep += __popc(km);
         __syncwarp();
       }
       // empty sub-cells -> new particles, (i,j,k) order
-      const int Q = q0 * q1 * q2;
       for (int base = 0; base < Q; base += 32) {
         const int t = base + lane;
         bool e = false;
-        if (t < Q) {
+        if (masked) {
+          e = t < Q && !((occupied >> lane) & 1u);
+        } else if (t < Q) {
           int ijk[3];
           sub_cell_ijk(t, q1, q2, I.qm, ijk);
-          const int i0 = ijk[0], i1 = ijk[1], i2 = ijk[2];
-          e = bcnt[(i0 * nb1 + i1) * nb2 + i2] == 0;
+          e = bcnt[(ijk[0] * nb1 + ijk[1]) * nb2 + ijk[2]] == 0;
         }
         const unsigned em = __ballot_sync(PFEM2_FULL_MASK, e);
         const int pos = n_keep + n_new + __popc(em & lt);
@@ -1132,161 +1151,242 @@ __global__ void __launch_bounds__(kRebinWarps * 32, RebinMinBlocks<DIM, R>::valu
         if (lane == 0) atomicExch(counters + CNT_LIST_OVERFLOW, 1);
         n_new = list_cap - n_keep;
       }
-      __syncwarp();
-    }
-      ntot = n_keep + n_new;
-      if (CHECK && lane == 0) {
+      if (lane == 0) {
         if (n_in - n_keep) atomicAdd(counters + CNT_REMOVED, n_in - n_keep);
         if (n_new) atomicAdd(counters + CNT_RESEEDED, n_new);
       }
     }
-    if (lane == 0) s_cnt[warp] = ntot;
-    __syncthreads();
-    if (warp == 0) {
-      unsigned long long agg = 0;
-      for (int w = 0; w < kRebinWarps; ++w) agg += (unsigned)s_cnt[w];
-      unsigned long long excl = 0;
-      if (t == 0) {
-        if (lane == 0) atomicExch(status, kTilePre | agg);
-      } else {
-        if (lane == 0) atomicExch(status + t, kTileAgg | agg);
-        // look back over windows of 32 predecessors (lane k reads tile
-        // j - k): the window ends at the nearest tile with a published
-        // prefix; the tiles before it must have published their aggregates
-        int j = t - 1;
-        unsigned spins = 0;
-        for (;;) {
-          const int k = j - lane;
-          const unsigned long long wd =
-              k >= 0 ? *(volatile const unsigned long long*)(status + k) : kTilePre;  // before tile 0: prefix 0
-          const unsigned pre = __ballot_sync(PFEM2_FULL_MASK, (wd >> 62) == 2);
-          const unsigned wait = __ballot_sync(PFEM2_FULL_MASK, (wd >> 62) == 0);
-          const int lp = pre ? __ffs(pre) - 1 : 31;
-          const unsigned upto = lp == 31 ? PFEM2_FULL_MASK : (2u << lp) - 1u;
-          if (wait & upto) {
-            if (++spins > spin_limit) {
-              if (lane == 0) atomicExch(counters + CNT_SCAN_TIMEOUT, 1);
-              break;
-            }
-            __nanosleep(32);
-            continue;
-          }
-          excl += warp_sum((unsigned long long)(lane <= lp ? (wd & kTileVal) : 0ull));
-          if (pre) break;
-          j -= 32;
-        }
-        if (lane == 0) atomicExch(status + t, kTilePre | ((excl + agg) & kTileVal));
-      }
-      if (lane == 0) s_base = (int)excl;
+    __syncwarp();
+    // the list and its length; the overflow part holds cap entries, enough
+    // for every list that fits the particle storage
+    const int n = n_keep + n_new;
+    int pos = -1;
+    int* dst = glist + (size_t)c * kListStride;
+    if (n > kListStride) {
+      if (lane == 0) pos = atomicAdd(novf, n);
+      pos = __shfl_sync(PFEM2_FULL_MASK, pos, 0);
+      if (pos < 0 || (size_t)pos + n > cap) pos = -1;
+      dst = glist + (size_t)nc * kListStride + pos;
     }
-    __syncthreads();
-    if (c < nc) {
-      int out = s_base;
-      for (int w = 0; w < warp; ++w) out += s_cnt[w];
-      if (lane == 0) {
-        new_start[c] = out;
-        if (c == nc - 1) {
-          new_start[nc] = out + ntot;
-          *np_out = out + ntot;
-        }
-      }
-      const DevInst& I = inst[__ldg(cell_inst + c)];
-      const int q1 = I.q[1], q2 = DIM == 3 ? I.q[2] : 1;
-      const double h0 = I.h[0], h1 = I.h[1], h2 = I.h[2];
-      ProjAcc<DIM, R> acc;
-      if (PROJ) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v)
-#pragma unroll
-          for (int k = 0; k <= DIM; ++k) acc.a[v][k] = R(0);
-      }
-      for (int j = lane; j < ntot; j += 32) {
-        const int code = list[j];
-        R x[DIM], uu[DIM];
-        if (code >= 0) {
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) {
-            x[d] = oxi[d * cap + code];
-            uu[d] = ou[d * cap + code];
-          }
-        } else {
-          const int t = -1 - code;
-          int id[3];
-          sub_cell_ijk(t, q1, q2, I.qm, id);
-          const double hh[3] = {h0, h1, h2};
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) x[d] = R((id[d] + 1.0 / 2) * hh[d]);
-          R N[NV];
-          shape_values<DIM, R>(x, N);
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) uu[d] = R(0);
-#pragma unroll
-          for (int v = 0; v < NV; ++v) {
-            const int g = __ldg(cv + (size_t)c * NV + v);
-#pragma unroll
-            for (int d = 0; d < DIM; ++d) uu[d] = uu[d] + N[v] * Vr[(size_t)d * nv + g];
-          }
-        }
-        const size_t o = (size_t)out + j;
-        if (o < cap) {
-          ncell[o] = c;
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) {
-            nxi[d * cap + o] = x[d];
-            nu[d * cap + o] = uu[d];
-          }
-        }
-        if (PROJ) proj_add<DIM, R>(acc, x, uu);
-      }
-      if (PROJ) proj_store<DIM, R>(acc, partial, c, lane);
+    if (n <= kListStride || pos >= 0)
+      for (int i = lane; i < n; i += 32) dst[i] = list[i];
+    if (lane == 0) {
+      cnt[c] = n;
+      if (n > kListStride) glist_pos[c] = pos;
     }
     __syncwarp();
-    __syncthreads();
+  }
+}
+
+// status words of the scan's tiles: bits 62-63 = 1 (tile aggregate known) or 2
+// (inclusive prefix known), the low bits the value
+constexpr unsigned long long kTileAgg = 1ull << 62, kTilePre = 2ull << 62, kTileVal = (1ull << 62) - 1;
+constexpr int kScanThreads = 256, kScanItems = kScanTile / kScanThreads;
+
+// new_start[c] = sum of the counts before cell c, new_start[nc] and *np_out =
+// their sum: one pass over tiles in ticket order (a block waits only on tiles
+// taken by blocks already running) with decoupled look-back; waits bounded, a
+// timeout is flagged in CNT_SCAN_TIMEOUT
+__global__ void __launch_bounds__(kScanThreads) k_rebin_scan(int nc, const int* __restrict__ cnt,
+                                                             int* __restrict__ new_start, int* __restrict__ np_out,
+                                                             int* __restrict__ counters,
+                                                             unsigned long long* __restrict__ tiles,
+                                                             unsigned spin_limit) {
+  __shared__ int s_tile, s_base, s_w[kScanThreads / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned long long* status = tiles + 1;
+  if (threadIdx.x == 0) s_tile = (int)atomicAdd(tiles, 1ull);
+  __syncthreads();
+  const int t = s_tile, c0 = t * kScanTile + threadIdx.x * kScanItems;
+  int v[kScanItems], sum = 0;
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) {
+    v[k] = c0 + k < nc ? cnt[c0 + k] : 0;
+    sum += v[k];
+  }
+  int inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(PFEM2_FULL_MASK, inc, o);
+    if (lane >= o) inc += y;
+  }
+  if (lane == 31) s_w[warp] = inc;
+  __syncthreads();
+  if (warp == 0) {
+    unsigned long long agg = 0;
+    for (int w = 0; w < kScanThreads / 32; ++w) agg += (unsigned)s_w[w];
+    unsigned long long excl = 0;
+    if (t == 0) {
+      if (lane == 0) atomicExch(status, kTilePre | agg);
+    } else {
+      if (lane == 0) atomicExch(status + t, kTileAgg | agg);
+      // look back over windows of 32 predecessors (lane k reads tile j - k):
+      // the window ends at the nearest tile with a published prefix; the
+      // tiles before it must have published their aggregates
+      int j = t - 1;
+      unsigned spins = 0;
+      for (;;) {
+        if (spins++ >= spin_limit) {
+          if (lane == 0) atomicExch(counters + CNT_SCAN_TIMEOUT, 1);
+          break;
+        }
+        const int k = j - lane;
+        const unsigned long long wd =
+            k >= 0 ? *(volatile const unsigned long long*)(status + k) : kTilePre;  // before tile 0: prefix 0
+        const unsigned pre = __ballot_sync(PFEM2_FULL_MASK, (wd >> 62) == 2);
+        const unsigned wait = __ballot_sync(PFEM2_FULL_MASK, (wd >> 62) == 0);
+        const int lp = pre ? __ffs(pre) - 1 : 31;
+        const unsigned upto = lp == 31 ? PFEM2_FULL_MASK : (2u << lp) - 1u;
+        if (wait & upto) {
+          __nanosleep(32);
+          continue;
+        }
+        excl += warp_sum((unsigned long long)(lane <= lp ? (wd & kTileVal) : 0ull));
+        if (pre) break;
+        j -= 32;
+      }
+      if (lane == 0) atomicExch(status + t, kTilePre | ((excl + agg) & kTileVal));
+    }
+    if (lane == 0) s_base = (int)excl;
+  }
+  __syncthreads();
+  int out = s_base + inc - sum;
+  for (int w = 0; w < warp; ++w) out += s_w[w];
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) {
+    if (c0 + k < nc) new_start[c0 + k] = out;
+    out += v[k];
+    if (c0 + k == nc - 1) {
+      new_start[nc] = out;
+      *np_out = out;
+    }
+  }
+}
+
+template <int DIM, typename R, bool PROJ>
+__global__ void __launch_bounds__(kRebinWarps * 32, RebinMinBlocks<DIM, R>::write) k_rebin_write(
+    const R* __restrict__ oxi, const R* __restrict__ ou, size_t cap, int* __restrict__ ncell, R* __restrict__ nxi,
+    R* __restrict__ nu, const int* __restrict__ new_start, int nc, const DevInst* __restrict__ inst,
+    const int* __restrict__ cell_inst, const int* __restrict__ cv, const R* __restrict__ Vr, int nv,
+    R* __restrict__ partial, const int* __restrict__ cnt, const int* __restrict__ glist,
+    const int* __restrict__ glist_pos) {
+  constexpr int NV = Dims<DIM>::NV;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the next cell's count, place and list are loaded while a cell is worked on
+  // (the list's entries from the count on are not used)
+  const int step = gridDim.x * kRebinWarps;
+  int n_next = 0, out_next = 0, code_next = 0;
+  const auto fetch = [&](int c) {
+    if (c < nc) {
+      n_next = cnt[c];
+      out_next = new_start[c];
+      code_next = glist[(size_t)c * kListStride + lane];
+    }
+  };
+  fetch(blockIdx.x * kRebinWarps + warp);
+  for (int c = blockIdx.x * kRebinWarps + warp; c < nc; c += step) {
+    const int n = n_next, out = out_next;
+    int code = code_next;
+    fetch(c + step);
+    const int* list = glist + (size_t)c * kListStride;
+    bool stored = true;
+    if (n > kListStride) {
+      const int pos = glist_pos[c];
+      stored = pos >= 0;  // else more particles than their storage holds (reported): any particle will do
+      list = glist + (size_t)nc * kListStride + max(pos, 0);
+      code = stored ? list[lane] : -1;
+    }
+    ProjAcc<DIM, R> acc;
+    if (PROJ) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+#pragma unroll
+        for (int k = 0; k <= DIM; ++k) acc.a[v][k] = R(0);
+    }
+    for (int j = lane; j < n; j += 32) {
+      if (j >= 32) code = stored ? list[j] : -1;
+      R x[DIM], uu[DIM];
+      if (code >= 0) {
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+          x[d] = oxi[d * cap + code];
+          uu[d] = ou[d * cap + code];
+        }
+      } else {
+        const DevInst& I = inst[__ldg(cell_inst + c)];
+        const int t = -1 - code;
+        int id[3];
+        sub_cell_ijk(t, I.q[1], DIM == 3 ? I.q[2] : 1, I.qm, id);
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) x[d] = R((id[d] + 1.0 / 2) * I.h[d]);
+        R N[NV];
+        shape_values<DIM, R>(x, N);
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) uu[d] = R(0);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          const int g = __ldg(cv + (size_t)c * NV + v);
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) uu[d] = uu[d] + N[v] * Vr[(size_t)d * nv + g];
+        }
+      }
+      const size_t o = (size_t)out + j;
+      if (o < cap) {
+        ncell[o] = c;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+          nxi[d * cap + o] = x[d];
+          nu[d * cap + o] = uu[d];
+        }
+      }
+      if (PROJ) proj_add<DIM, R>(acc, x, uu);
+    }
+    if (PROJ) proj_store<DIM, R>(acc, partial, c, lane);
   }
 }
 
 template <int DIM, typename R, bool CHECK, bool PROJ>
-static void rebin_launch(Ctx& c, const int* newcell) {
+static pfem2_status rebin_launch(Ctx& c, const int* newcell) {
   const int o = c.cur, nb = 1 - c.cur;
   const size_t smem = (size_t)kRebinWarps * (c.list_cap + kMaxBuckets) * sizeof(int);
-  const int ntiles = (c.nc + kRebinWarps - 1) / kRebinWarps;
-  const int grid = grid_for(c, (long long)c.nc * 32, kRebinWarps * 32, c.tune.rebin_blocks_per_sm);
-  cudaMemsetAsync(c.rebin_tiles, 0, sizeof(unsigned long long) * ((size_t)ntiles + 1), c.stream);
-  k_rebin<DIM, R, CHECK, PROJ><<<grid, kRebinWarps * 32, smem, c.stream>>>(
-      c.cell_start[o], newcell, (const R*)c.pxi[o], (const R*)c.pu[o], (size_t)c.pcap, c.pcell[nb], (R*)c.pxi[nb],
-      (R*)c.pu[nb], c.cell_start[nb], c.d_np + nb, c.nc, c.ring_ptr, c.ring_cell, c.ring_rev, c.dest_mask, c.far_keys,
-      c.far_cap, c.d_inst,
-      c.cell_inst, c.cv, (const R*)c.Vr, c.nv, (R*)c.partial, c.list_cap, c.d_counters, c.rebin_tiles,
-      c.spin_limit >> 2);
-  c.launches += 1;
+  const int ntiles = (c.nc + kScanTile - 1) / kScanTile;
+  // resident blocks only: a cell per warp at a time, the cells in turn
+  const int ggrid = grid_for(c, (long long)c.nc * 32, kRebinWarps * 32,
+                             std::min(c.tune.rebin_blocks_per_sm, RebinMinBlocks<DIM, R>::gather));
+  const int wgrid = grid_for(c, (long long)c.nc * 32, kRebinWarps * 32,
+                             std::min(c.tune.rebin_blocks_per_sm, RebinMinBlocks<DIM, R>::write));
+  PFEM2_CUDA(cudaFuncSetAttribute((const void*)k_rebin_gather<DIM, R, CHECK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)smem));
+  // ticket and status words of the scan, then the overflow part's fill count
+  PFEM2_CUDA(cudaMemsetAsync(c.rebin_tiles, 0, sizeof(unsigned long long) * ((size_t)ntiles + 2), c.stream));
+  int* novf = (int*)(c.rebin_tiles + ntiles + 1);
+  k_rebin_gather<DIM, R, CHECK><<<ggrid, kRebinWarps * 32, smem, c.stream>>>(
+      c.cell_start[o], newcell, (const R*)c.pxi[o], (size_t)c.pcap, c.nc, c.ring_ptr, c.ring_cell, c.movers,
+      c.far_keys, c.far_cap, c.d_inst, c.cell_inst, c.list_cap, c.d_counters, c.rebin_cnt, c.rebin_list,
+      c.rebin_pos, novf);
+  k_rebin_scan<<<ntiles, kScanThreads, 0, c.stream>>>(c.nc, c.rebin_cnt, c.cell_start[nb], c.d_np + nb, c.d_counters,
+                                                      c.rebin_tiles, c.spin_limit >> 2);
+  k_rebin_write<DIM, R, PROJ><<<wgrid, kRebinWarps * 32, 0, c.stream>>>(
+      (const R*)c.pxi[o], (const R*)c.pu[o], (size_t)c.pcap, c.pcell[nb], (R*)c.pxi[nb], (R*)c.pu[nb],
+      c.cell_start[nb], c.nc, c.d_inst, c.cell_inst, c.cv, (const R*)c.Vr, c.nv, (R*)c.partial, c.rebin_cnt,
+      c.rebin_list, c.rebin_pos);
+  c.launches += 3;
   c.cur = nb;
+  return PFEM2_OK;
 }
 
 template <int DIM, typename R>
 static pfem2_status rebin_impl(Ctx& c, bool check, bool proj, bool from_advect) {
   const int* nc_arr = from_advect ? c.newcell : c.pcell[c.cur];
-  const size_t smem = (size_t)kRebinWarps * (c.list_cap + kMaxBuckets) * sizeof(int);
-  auto set_attr = [&](const void* f) { cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); };
-  if (check && proj) {
-    set_attr((const void*)k_rebin<DIM, R, true, true>);
-    rebin_launch<DIM, R, true, true>(c, nc_arr);
-  } else if (check) {
-    set_attr((const void*)k_rebin<DIM, R, true, false>);
-    rebin_launch<DIM, R, true, false>(c, nc_arr);
-  } else if (proj) {
-    set_attr((const void*)k_rebin<DIM, R, false, true>);
-    rebin_launch<DIM, R, false, true>(c, nc_arr);
-  } else {
-    set_attr((const void*)k_rebin<DIM, R, false, false>);
-    rebin_launch<DIM, R, false, false>(c, nc_arr);
-  }
-  return PFEM2_OK;
+  if (check) return proj ? rebin_launch<DIM, R, true, true>(c, nc_arr) : rebin_launch<DIM, R, true, false>(c, nc_arr);
+  return proj ? rebin_launch<DIM, R, false, true>(c, nc_arr) : rebin_launch<DIM, R, false, false>(c, nc_arr);
 }
 
 pfem2_status launch_rebin(Ctx& c, bool check, bool proj, bool from_advect) {
   if (!from_advect) {
-    // no movers: make sure the far list is empty
+    // no movers: make sure their lists are empty
     PFEM2_CUDA(cudaMemsetAsync(c.d_counters + CNT_FAR, 0, sizeof(int), c.stream));
+    PFEM2_CUDA(cudaMemsetAsync(c.movers.cnt, 0, sizeof(int) * c.nc, c.stream));
   }
   if (c.dim == 2) return c.pmixed ? rebin_impl<2, float>(c, check, proj, from_advect) : rebin_impl<2, double>(c, check, proj, from_advect);
   return c.pmixed ? rebin_impl<3, float>(c, check, proj, from_advect) : rebin_impl<3, double>(c, check, proj, from_advect);
