@@ -8,6 +8,7 @@
 // smoothed-aggregation transfers is applied in its additive form
 //   M_l^-1 = J_l + Pt_l M_{l+1}^-1 Pt_l^T,
 //   J_l  = 2 w D^-1 - w^2 D^-1 A_l D^-1,  Pt_l = (I - w D^-1 A_l) P_l,
+// D the smoother's diagonal (the absolute row sums on level 0 of a fixed mesh),
 // which is algebraically the same V-cycle: the pre- and post-smoothing of a
 // level are folded into J_l and into the post-smoothed prolongator Pt_l, so
 // a level costs one sparse product each way and no extra synchronisation.
@@ -51,7 +52,8 @@ struct MgHost {
   std::vector<int> blk_s1, s1_lk, j1_ptr, j1_col, p1_ptr, p1_col;
   std::vector<double> j1_val, p1_val;
   std::vector<int> sys_n2, sys_off2;      // level-2 size and first level-2 dof per system
-  std::vector<double> w0;                 // level-0 smoother weight per system (at most 0.49 on a moving mesh)
+  std::vector<double> w0;                 // level-0 smoother weight per system
+  std::vector<double> d0;                 // [nv] level-0 smoother diagonal D^-1 (1 / a_ii on a moving mesh)
   int s1max = 0;
   int b2max = 0;                          // level-2 dofs of the local systems of a block
 };

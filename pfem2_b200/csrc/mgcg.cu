@@ -629,6 +629,7 @@ struct MgWs {
   int *r1_ptr, *r1_col, *q2_ptr, *q2_col, *m2_off, *p0_ptr, *p0_len, *p0_col;
   int *blk_s1, *s1_lk, *j1_ptr, *j1_col, *p1_ptr, *p1_col, *sys_n2, *sys_off2;
   double* sys_w;
+  void* d0 = nullptr;  // level-0 smoother diagonal (fixed mesh)
   long long* blk_m2;
   void *r1_val, *q2_val, *m2, *p0_val, *j1_val, *p1_val;
   void *z, *dq, *jr, *c1, *b1, *x1, *b2, *x2;
@@ -841,6 +842,7 @@ pfem2_status mg_setup(Ctx& c) {
   PFEM2_TRY(ws_upload(w, &m->sys_n2, H.sys_n2));
   PFEM2_TRY(ws_upload(w, &m->sys_off2, H.sys_off2));
   PFEM2_TRY(ws_upload(w, &m->sys_w, H.w0));
+  if (!c.moving) PFEM2_TRY(ws_upload_r(w, c.kmixed, &m->d0, H.d0));
   void** vec[] = {&m->z, &m->dq, &m->jr, &m->c1, &m->b1, &m->x1, &m->b2, &m->x2};
   const size_t nv = c.nv, n1 = H.n[1], n2 = H.n[2], nvec[] = {nv, nv, nv, n1, n1, n1, n2, n2};
   for (int k = 0; k < 8; ++k) {
@@ -878,7 +880,7 @@ pfem2_status mg_solve_impl(Ctx& c) {
   a.sl_col = c.sl_col;
   a.A64 = c.A64[3];
   a.A = c.kmixed ? (const R*)c.A32[3] : (const R*)c.A64[3];
-  a.dinv = c.kmixed ? (const R*)c.dinv32[3] : (const R*)c.dinv64[3];
+  a.dinv = !c.moving ? (const R*)m->d0 : c.kmixed ? (const R*)c.dinv32[3] : (const R*)c.dinv64[3];
   a.r1_wide = m->wide;
   a.raw = c.moving;
   a.xsplit = m->xsplit;
