@@ -30,7 +30,7 @@
 // publishing and 2 us of work), on the 131k-cell pipe the gathers and the
 // matrix from L2. A block owns a contiguous run of slices with all their
 // components, cut to equal lengths, and a warp takes one (slice, component)
-// at a time. Measured against tiles of 8 slices per component (some blocks
+// at a time (where warps would be left over, several share one). Measured against tiles of 8 slices per component (some blocks
 // held two, others one), separate vectors, generic pointers and three phases
 // per restart, prediction and correction take per step: 52k channel FP32 0.45
 // ms instead of 0.86, FP64 0.59 instead of 1.03; 16 channels 1.38 instead of
@@ -49,6 +49,10 @@
 #include "krylov_ws.h"
 
 namespace pfem2 {
+
+// entries of a SELL row whose loads are issued together: a Q1 row of 9 (2D)
+// in one round, one of 27 (3D) in three; with FP64 the registers hold five
+template <typename R> struct Chunk { static constexpr int value = sizeof(R) == 8 ? 5 : 9; };
 
 template <int MINB> struct SolveThreads { static constexpr int value = MINB == 1 ? 768 : 384; };
 static int solve_threads(int minb) { return minb == 1 ? SolveThreads<1>::value : SolveThreads<2>::value; }
@@ -119,6 +123,7 @@ template <typename R> struct SolveArgs {
   const R* dinv[3];
   int share;              // the components share one matrix
   int items_max;
+  int split;              // warps that share an item's entries
   double* x[3];
   const double* b[3];
   const unsigned char* isd[3];
@@ -149,6 +154,7 @@ template <typename R> struct SolveArgs {
 struct LocalSys {
   int sys, state, act, it, outer, par, first, pend, maxit, slot;
   int s0, s1;                       // partial slots of the system
+  int j0, j1;                       // its slices in the block
   double tol, rtol, intol, res, rz_prev, alpha, beta, omega, irv;
   double sum[kMaxSums];
 };
@@ -291,9 +297,7 @@ template <typename R, int MINB, int SM, bool CL>
 __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(SolveArgs<R> a) {
   constexpr int kSolveThreads = SolveThreads<MINB>::value, kWarps = kSolveThreads / 32;
   extern __shared__ __align__(16) unsigned char dyn_smem[];
-  // entries of a SELL row whose loads are issued together: a Q1 row of 9 (2D)
-  // in one round, one of 27 (3D) in three; with FP64 the registers hold five
-  constexpr int CH = sizeof(R) == 8 ? 5 : 9;
+  constexpr int CH = Chunk<R>::value;
   __shared__ LocalSys ls[kMaxLocalSys];
   __shared__ int s_err;
   __shared__ double s_pub[CL ? 2 * 3 * kMaxSums * kClusterMax : 1];  // [parity][system][sum][block]
@@ -305,11 +309,14 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
   const int bs0 = a.blk_sl[blockIdx.x], bs1 = a.blk_sl[blockIdx.x + 1];
   const int nitems = (bs1 - bs0) * NC, own0 = bs0 * 32;
   const int NS = a.bicg ? kMaxSums : 3;
+  const int split = a.split, group = warp / split, part = warp - group * split, ngroups = kWarps / split;
   unsigned bar_gen = 0;
 
-  // ---- shared memory: the items' partial sums, then the staged static data
-  double* spart = reinterpret_cast<double*>(dyn_smem);
-  unsigned char* cur = dyn_smem + al16_dev((size_t)a.items_max * NS * sizeof(double));
+  // ---- shared memory: partial products of split items, the items' partial
+  // sums, then the staged static data
+  double* const s_dot = reinterpret_cast<double*>(dyn_smem);
+  double* spart = s_dot + (split > 1 ? kWarps * 32 : 0);
+  unsigned char* cur = reinterpret_cast<unsigned char*>(spart) + al16_dev((size_t)a.items_max * NS * sizeof(double));
   // own rows of the vectors that no product gathers: by item in shared memory
   R *ve, *vr, *vs, *vt, *vv, *vh;
   const int *SLp, *SLl, *SLk, *SLc;  // by slice - bs0; columns by entry - e0
@@ -363,6 +370,10 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
     L.s0 = a.sys_slot0[s];
     L.s1 = a.sys_slot0[s + 1];
     L.slot = L.s0 + a.blk_slot[io + l / NC];
+    L.j0 = 0;
+    while (L.j0 < bs1 - bs0 && a.slk[bs0 + L.j0] != l / NC) ++L.j0;
+    L.j1 = L.j0;
+    while (L.j1 < bs1 - bs0 && a.slk[bs0 + L.j1] == l / NC) ++L.j1;
     L.maxit = a.maxit_i[inst];
     L.tol = a.tol_i[inst];
     L.rtol = a.rtol_i[inst];
@@ -431,8 +442,9 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
     bool any = false;
     for (int l = 0; l < nls; ++l) any |= ls[l].act != ACT_NONE;
     if (!any) break;  // every local system is done
-    // ---- the block's (slice, component) items, a warp per item
-    for (int it = warp; it < nitems; it += kWarps) {
+    // ---- the block's (slice, component) items, `split` warps per item: each
+    // takes a run of the row's entries, the first adds up their products
+    for (int it = group < ngroups ? group : nitems; it < nitems; it += ngroups) {
       const int sl = bs0 + it / NC, k = it % NC;
       const LocalSys& L = ls[SLk[sl - bs0] * NC + k];
       const int act = L.act;
@@ -440,7 +452,24 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
       double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0, v4 = 0.0;
       const int row = sl * 32 + lane;
       const size_t g0 = k * nv + row, o = SM >= 1 ? (size_t)(it * 32 + lane) : g0;
-      const int p0 = SLp[sl - bs0] - e0, len = SLl[sl - bs0];
+      int nj = SLl[sl - bs0], p0 = SLp[sl - bs0] - e0;
+      if (split > 1) {
+        const int j0 = nj * part / split;
+        nj = nj * (part + 1) / split - j0;
+        p0 += 32 * j0;
+      }
+      const auto row_dot = [&](auto zero, const auto& val, const auto& gx) {
+        using T = decltype(zero);
+        T acc = sell_dot<T, CH>(zero, SLc, p0, nj, lane, val, gx);
+        if (split > 1) {  // (a group has one item per phase: its slots are free)
+          T* const d = reinterpret_cast<T*>(s_dot + 32 * warp);
+          d[lane] = acc;
+          asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(32 * split) : "memory");
+          if (part == 0)
+            for (int u = 1; u < split; ++u) acc += reinterpret_cast<const T*>(s_dot + 32 * (warp + u))[lane];
+        }
+        return acc;
+      };
       const R* dinv = a.dinv[k];
       const R* A = k == 0 ? A0 : (k == 1 ? A1 : A2);
       const auto aval = [&](int ei) { return A[ei]; };
@@ -454,7 +483,7 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
         const bool pend = L.pend != 0;
         const R al = R(L.alpha), om = R(L.omega);
         const double bb = a.b[k][row];
-        const double acc = sell_dot<double, CH>(0.0, SLc, p0, len, lane, [&](int ei) { return A64[ei]; }, [&](int j) {
+        const double acc = row_dot(0.0, [&](int ei) { return A64[ei]; }, [&](int j) {
           R ee = __ldcg(e + j);
           if (pend) {
             R zr, w;
@@ -463,11 +492,13 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
           }
           return __ldcg(xk + j) + (double)ee;
         });
+        if (part) continue;
         const double rr = bb - acc;
         a.r64[g0] = rr;
         v0 = rr * rr;
         v1 = bb * bb;
       } else if (act == ACT_FINISH) {
+        if (part) continue;
         R ee = ve[o];
         if (L.pend) {
           R zr, w;
@@ -490,7 +521,8 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
           const double xo = a.x[k][row];
           R zr = R(0), w = R(0);
           if (L.pend) ld2(pk + row, zr, w);
-          acc = sell_dot<R, CH>(R(0), SLc, p0, len, lane, aval, [&](int j) { return R(__ldcg(r64 + j)) * dinv[j]; });
+          acc = row_dot(R(0), aval, [&](int j) { return R(__ldcg(r64 + j)) * dinv[j]; });
+          if (part) continue;
           const R ee = L.pend ? fma_r(R(L.omega), fma_r(-R(L.alpha), w, zr), e_old) : e_old;
           a.x[k][row] = xo + (double)ee;
           ve[o] = R(0);
@@ -507,7 +539,8 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
           };
           const V4<R> g = ld4(pk + row);
           const R t_old = vt[o], s_old = vs[o], rh = vh[o];
-          acc = sell_dot<R, CH>(R(0), SLc, p0, len, lane, aval, [&](int j) { return ynew(ld4(pk + j)); });
+          acc = row_dot(R(0), aval, [&](int j) { return ynew(ld4(pk + j)); });
+          if (part) continue;
           const R zs = fma_r(-al, g.b, g.a);
           const R ee = fma_r(om, zs, e_old);
           ve[o] = ee;
@@ -525,11 +558,12 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
         const R al = R(L.alpha);
         const R y = pk[row].c, e_old = ve[o], v_old = vv[o], r_old = vr[o], di = dinv[row];
         const double rh = (double)vh[o];
-        const R tv = sell_dot<R, CH>(R(0), SLc, p0, len, lane, aval, [&](int j) {
+        const R tv = row_dot(R(0), aval, [&](int j) {
           R zr, w;
           ld2(pk + j, zr, w);
           return fma_r(-al, w, zr);
         });
+        if (part) continue;
         const R sv = fma_r(-al, v_old, r_old);
         const R ee = fma_r(al, y, e_old);
         ve[o] = ee;
@@ -546,7 +580,8 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
         // restart: u = K^-1 r64, w = A u, wh = K^-1 w; (r, u), (w, u), (r, r)
         const R e_old = ve[o], rr = R(__ldcg(r64 + row)), di = dinv[row], u = rr * di;
         const double xo = a.x[k][row];
-        const R w = sell_dot<R, CH>(R(0), SLc, p0, len, lane, aval, [&](int j) { return R(__ldcg(r64 + j)) * dinv[j]; });
+        const R w = row_dot(R(0), aval, [&](int j) { return R(__ldcg(r64 + j)) * dinv[j]; });
+        if (part) continue;
         a.x[k][row] = xo + (double)e_old;
         ve[o] = R(0);
         if (SM >= 1) a.e[g0] = R(0);
@@ -566,10 +601,11 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
         const auto shn = [&](const V4<R>& g) { return first ? g.b : fma_r(be, g.c, g.b); };
         const V4<R> g = ld4(pk + row);
         const R p_old = vt[o], s_old = vs[o], w_old = vv[o], e_old = ve[o], r_old = vr[o], di = dinv[row];
-        const R w = sell_dot<R, CH>(R(0), SLc, p0, len, lane, aval, [&](int j) {
+        const R w = row_dot(R(0), aval, [&](int j) {
           const V4<R> h = ld4(pk + j);
           return fma_r(-al, shn(h), h.a);
         });
+        if (part) continue;
         const R sh = shn(g), un = fma_r(-al, sh, g.a);
         const R pp = first ? g.a : fma_r(be, p_old, g.a);
         const R ss = first ? w_old : fma_r(be, s_old, w_old);
@@ -610,12 +646,18 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
     // write of the block's phase
     for (int l = warp; l < nls; l += kWarps) {
       LocalSys& L = ls[l];
-      const int act = L.act, k = l % NC, il = l / NC;
+      const int act = L.act, k = l % NC;
       const int ns = act == ACT_P2 ? kMaxSums : act == ACT_P1 ? 1 : act == ACT_NONE || act == ACT_FINISH ? 0 : 3;
       double s = 0.0;
-      if (lane < ns)  // lane q adds up sum q
-        for (int j = 0; j < bs1 - bs0; ++j)
-          if (SLk[j] == il) s += spart[(size_t)NS * (j * NC + k) + lane];
+      {
+        // lanes q, q + 8, q + 16 and q + 24 add up sum q
+        const int q = lane & 7;
+        if (q < ns)
+#pragma unroll 4
+          for (int j = L.j0 + (lane >> 3); j < L.j1; j += 4) s += spart[NS * (j * NC + k) + q];
+        s += __shfl_xor_sync(PFEM2_FULL_MASK, s, 8);
+        s += __shfl_xor_sync(PFEM2_FULL_MASK, s, 16);
+      }
       if constexpr (CL) {
         for (int q = 0; q < ns; ++q) {
           const double v = __shfl_sync(PFEM2_FULL_MASK, s, q);
@@ -700,7 +742,8 @@ static bool cluster_fits(bool mixed, int sm, int grid, size_t smem) {
 
 // shared memory of a block and what it holds; sm < 0: not even its partial sums fit
 static size_t plan_smem(const JacobiPlan& P, size_t rs, int minb, int nmat, int& sm) {
-  size_t smem = al16(sizeof(double) * (P.bicg ? kMaxSums : 3) * (size_t)P.items_max);
+  size_t smem = al16(sizeof(double) * (P.bicg ? kMaxSums : 3) * (size_t)P.items_max) +
+                (P.split > 1 ? sizeof(double) * solve_threads(minb) : 0);
   const size_t level[3] = {al16(6 * 32 * rs * (size_t)P.items_max) + P.st_meta, al16(4 * P.st_entries),
                            nmat * al16(rs * P.st_entries)};
   sm = 0;
@@ -759,28 +802,48 @@ static pfem2_status plan_build(Ctx& c, KrylovWs* w, JacobiPlan& P, bool mixed, c
   const int ni = (int)ioff.size() - 1, ns = ioff.back();
   const size_t rs = mixed ? sizeof(float) : sizeof(double);
   std::vector<int> up[6];
+  int len = 0;  // the longest row, and the rounds of loads it takes
+  for (int sl = 0; sl < ns; ++sl) len = std::max(len, (slp[sl + 1] - slp[sl]) / kSlice);
+  const int ch = mixed ? Chunk<float>::value : Chunk<double>::value, rounds = (len + ch - 1) / ch;
+  // warps that would have no item share the others': as many as shorten a row's
+  // rounds of loads, each group of warps with one item at most. An iteration of
+  // the mesh elasticity (17k rows of 18 entries, FP64) takes 6.0 us instead of
+  // 8.5 with four warps to an item; 10k-cell pipe (27 entries, FP64), prediction
+  // and correction 1.42 ms instead of 1.65 with two; 13k-cell channel, FP64,
+  // 0.41 instead of 0.45.
+  const auto set_split = [&] {
+    const auto rounds_of = [&](int n) { return ((len + n - 1) / n + ch - 1) / ch; };
+    const int most = std::min(solve_threads(P.minb) / 32 / std::max(1, P.items_max), rounds);
+    P.split = 1;
+    for (int k = 2; k <= most; ++k)
+      if (rounds_of(k) < rounds_of(P.split)) P.split = k;
+  };
   P.cluster = false;
   if (try_cluster && ni == 1 && ns * ncomp <= kClusterItems) {
     int G = 1;
     while (2 * G <= kClusterMax && 4 * G <= ns) G *= 2;
     PFEM2_TRY(plan_runs(P, up, ioff, slp, ncomp, G));
+    P.minb = 1;
+    set_split();
     const size_t smem = plan_smem(P, rs, 1, nmat, P.sm);
     if (P.sm >= 2 && cluster_fits(mixed, P.sm, G, smem)) {
       P.cluster = true;
-      P.minb = 1;
     }
   }
   if (!P.cluster) {
-    // one block per SM, but at least four slices in each (channel of 1k rows,
-    // FP64: 0.49 ms per step with four, 0.53 with six, 0.48 with two; 13k
-    // rows: 0.48 with four, 0.53 with two)
-    const int ts_auto = std::max(4, (ns + c.num_sms - 1) / c.num_sms);
+    // one block per SM, but at least four slices in each where a row is one
+    // round of loads (13k rows, FP32: 0.39 ms per step with four, 0.40 with
+    // two, 0.42 with six), three with two rounds (FP64: 0.41 with three, 0.42
+    // with four, 0.46 with six), two with more (10k-cell pipe, FP64: 1.42 with
+    // two, 1.46 with three, 1.57 with four)
+    const int ts_auto = std::max(std::max(2, 5 - rounds), (ns + c.num_sms - 1) / c.num_sms);
     // one system: a block of 768 threads per SM, so that few blocks are waited
     // for (52k channel: prediction and correction 0.45 ms per step against
     // 0.55 with two blocks of 384; 131k pipe 3.58 against 3.77), unless 12
-    // warps hold its items in one round; a batch takes two of 384, whose
+    // warps hold its items in one round of loads (13k rows: one round, FP32; two,
+    // FP64, where 768 threads take 0.42 ms and 384 take 0.45); a batch takes two of 384, whose
     // instances wait less for each other (16 channels: 1.38 against 1.44 ms)
-    P.minb = minb ? minb : (ni > 1 || ts_auto * ncomp <= 12 ? 2 : 1);
+    P.minb = minb ? minb : (ni > 1 || ts_auto * ncomp * rounds <= 12 ? 2 : 1);
     if (!ts) ts = ni > 1 ? 4 : ts_auto;
     const int occ = std::min(P.minb, occupancy(mixed, P.minb, 0, 0));
     if (occ < 1) {
@@ -788,6 +851,7 @@ static pfem2_status plan_build(Ctx& c, KrylovWs* w, JacobiPlan& P, bool mixed, c
       return PFEM2_CUDA_ERROR;
     }
     PFEM2_TRY(plan_runs(P, up, ioff, slp, ncomp, std::max(1, std::min(occ * c.num_sms, (ns + ts - 1) / ts))));
+    set_split();
   }
   P.ts = (ns + P.grid - 1) / P.grid;
   int** dst[6] = {&P.blk_sl, &P.blk_inst, &P.blk_inst_off, &P.blk_slot, &P.sys_slot0, &P.slk};
@@ -804,6 +868,7 @@ static void plan_args(const KrylovWs* w, const JacobiPlan& P, SolveArgs<R>& a) {
   a.blk_sl = P.blk_sl;
   a.slk = P.slk;
   a.items_max = P.items_max;
+  a.split = P.split;
   a.nslots = P.nslots;
   a.bicg = P.bicg;
   a.scount = w->scount;
