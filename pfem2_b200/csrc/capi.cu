@@ -516,7 +516,7 @@ static pfem2_status do_setup(Ctx& c) {
   PFEM2_TRY(dalloc(&c.rebin_tiles, (size_t)nc / kScanTile + 4));
   PFEM2_TRY(dalloc(&c.rebin_cnt, (size_t)nc));
   PFEM2_TRY(dalloc(&c.rebin_pos, (size_t)nc));
-  PFEM2_TRY(dalloc(&c.movers.cnt, (size_t)nc));
+  PFEM2_TRY(dalloc(&c.movers.cnt, (size_t)nc + 1));
   PFEM2_TRY(dalloc(&c.d_np, 2));
   PFEM2_TRY(dalloc(&c.d_counters, CNT_N));
   // far movers are sorted by one CTA in shared memory (8 B per key)

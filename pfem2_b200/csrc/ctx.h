@@ -50,7 +50,7 @@ struct Tile {
 // particles that changed cell within the 1-ring of their old cell, by new
 // cell, in no order: a cell's list holds the first cap, cnt counts them all
 struct Movers {
-  int* cnt = nullptr;   // [nc], reset before each advection
+  int* cnt = nullptr;   // [nc], then the units of leavers; reset before each advection
   int* list = nullptr;  // [nc][cap]
   int cap = 0;
 };
@@ -144,7 +144,7 @@ struct Ctx {
   void* pu[2] = {};
   int cur = 0;
   int* newcell = nullptr;
-  // particle capacity from which the advection runs in two phases per warp
+  // particle capacity from which the advection runs as two kernels
   // (stayers, then the warp's queued leavers; measured faster than the
   // one-pass kernel on every bench workload, the smallest 1.3M particles);
   // the environment variable PFEM2_ADVECT_SPLIT_MIN overrides it at creation

@@ -8,12 +8,12 @@
 //   k_seed          seed_particles / seed_particles_into_cell
 //                   (TurekBenchmark/pfem2particle.cpp:701-721,774-790)
 //   k_correct       correct_particles_velocities (:792-811)
-//   k_advect_q,     move_particles sub-steps (:813-848) + point location
-//   k_advect_one
+//   k_advect_stay,  move_particles sub-steps (:813-848) + point location
+//   k_advect_leave, (k_advect_one: the same in one kernel)
 //                   sort_particles_into_subdomains_and_cells (:276-507),
 //                   find_closest_vertex_of_cell (:142-166),
 //                   compare_particle_association (:268-274)
-//   k_rebin         the re-sort by cell plus check_cell_for_empty_parts
+//   k_rebin_*       the re-sort by cell plus check_cell_for_empty_parts
 //                   (:723-772), with the projection partials fused in
 //   k_project_*     distribute_particle_velocities_to_grid (:858-918)
 #include <algorithm>
@@ -196,7 +196,7 @@ pfem2_status launch_correct(Ctx& c) {
 // sub-step the particle is located like the reference does: current cell
 // first, then the patch of the "closest" vertex in alignment order; a
 // particle found nowhere is deleted (newcell = -1).
-// resident 256-thread blocks per SM the advection kernel is compiled for:
+// resident 256-thread blocks per SM the one-kernel advection is compiled for:
 // it is latency-bound, so the FP32 2D variant trades its few extra
 // registers for four blocks (32 warps) per SM, and the FP64 3D variant
 // (240 registers uncapped, one block) runs two at 128 registers in spite of
@@ -207,6 +207,21 @@ struct AdvectMinBlocks {
   static constexpr int value = DIM == 2 ? (sizeof(R) == 4 ? 4 : 2) : 2;
 };
 
+
+// Resident blocks per SM of the two-kernel form (stay: 256 threads, leave: 128),
+// measured as advection per step. Stay, without the point location's registers:
+// 1M-cell FP32 mesh 1.04 ms with 6 (5: 1.07, 7: more spills, 1.39); 131k-cell
+// pipe, FP64, 0.86 ms with 2 (3: 1.13, 1: 1.04). Leave: 16 channels, FP64, 0.57 ms
+// with 6 (4: 0.67, 8: 0.68); 1M cells FP32 1.04 with 8 (7: 1.22, 10: 1.34);
+// 10k-cell pipe, FP64, 0.128 with 3 (4: 0.134).
+template <int DIM, typename R>
+struct StayMinBlocks {
+  static constexpr int value = sizeof(R) == 4 ? (DIM == 2 ? 6 : 3) : (DIM == 2 ? 4 : 2);
+};
+template <int DIM, typename R>
+struct LeaveMinBlocks {
+  static constexpr int value = sizeof(R) == 4 ? (DIM == 2 ? 8 : 4) : (DIM == 2 ? 6 : 3);
+};
 
 constexpr int kAdvLeft = -2;  // advect_steps<.., false>: the particle left its cell
 
@@ -476,127 +491,109 @@ __global__ void __launch_bounds__(256, AdvectMinBlocks<DIM, R>::value) k_advect_
   }
 }
 
-// Advection in two phases per warp (large particle sets): a warp walks its
-// 32-particle slices of the block's contiguous chunk; every particle is
-// corrected (FUSE) and takes the lean sub-steps while it stays in its cell,
-// and one that leaves is appended to the warp's queue in shared memory with
-// its state (slot, old cell, the sub-step it left in, its reference
-// coordinates at the start of that sub-step). Whenever the queue holds 32
-// particles the warp resumes them with the full point location, so that the
-// divergent patch search runs on full warps, the leavers' state never goes
-// back to memory and the warps stay independent of each other (no block
-// barrier). The arithmetic is that of k_advect_one (bitwise equal results).
-constexpr int kAdvThreads = 256;
+// Advection in two kernels. k_advect_stay: a block walks the 32-particle slices
+// of a contiguous chunk; every particle is corrected (FUSE) and takes the lean
+// sub-steps while it stays in its cell; one that leaves goes to the chunk's part
+// of the queue, with its reference coordinates at the start of the sub-step it
+// left in xi and that sub-step's index in newcell. k_advect_leave: a warp takes
+// units of up to 32 leavers of one chunk and resumes them with the full point
+// location, so that the divergent patch search runs on full warps.
+//
+// Both are bound by dependent loads, the FP64 3D form by the FP64 pipe. In one
+// kernel (a queue per warp, resumed in place) the point location's registers
+// held every warp to its occupancy: 131k-cell pipe, 3.5M FP64 particles, 1.28
+// ms against 0.86 now; 16 channels, 8.7M, FP64, 0.70 against 0.57; 52k cells,
+// 1.7M, FP64, 0.164 against 0.149; 13k cells, FP64, 0.074 against 0.058; 1M
+// cells, 28M, FP32, 1.10 against 1.04. Units keep a chunk's leavers together:
+// one queue over all chunks lost the cell data's L1 hits (1M cells 1.19 ms, 16
+// channels 0.64), a block per chunk waited for the fastest region (16 channels
+// 0.78). The arithmetic is that of k_advect_one (bitwise equal results).
+constexpr int kAdvThreads = 256, kLeaveThreads = 128;
 
 template <int DIM, typename R, bool FUSE>
-__global__ void __launch_bounds__(kAdvThreads, AdvectMinBlocks<DIM, R>::value) k_advect_q(
+__global__ void __launch_bounds__(kAdvThreads, StayMinBlocks<DIM, R>::value) k_advect_stay(
     const int* __restrict__ cell, R* __restrict__ xi, R* __restrict__ u, int* __restrict__ newcell, size_t cap,
     const int* __restrict__ d_np, const CellGeo<DIM, R>* __restrict__ geo, const int* __restrict__ cv,
     const R* __restrict__ Vr, const R* __restrict__ dVr, int nv, int S, const DevInst* __restrict__ inst,
-    const int* __restrict__ cell_inst, const int* __restrict__ v2c_ptr, const int* __restrict__ v2c_cell,
-    const R* __restrict__ v2c_dir, const int* __restrict__ ring_ptr, const int* __restrict__ ring_cell,
-    unsigned long long* __restrict__ far_keys, int far_cap, int* __restrict__ counters, const Movers mv) {
+    const int* __restrict__ cell_inst, int* __restrict__ queue, int2* __restrict__ units, int* __restrict__ n_units) {
   constexpr int NV = Dims<DIM>::NV;
-  constexpr int NW = kAdvThreads / 32;
-  constexpr int QN = 64;  // below 32 left over + 32 appended
-  __shared__ int q_p[NW][QN], q_c[NW][QN];
-  __shared__ R q_x[NW][DIM][QN];
-  __shared__ unsigned short q_s[NW][QN];  // sub-step index (movement_steps <= 65535)
+  __shared__ int s_n, s_at;
   const int n = min(*d_np, (int)cap);
   const int chunk = (n + gridDim.x - 1) / gridDim.x;
-  const int lo = min(n, (int)blockIdx.x * chunk), hi = min(n, lo + chunk);
+  const int lo = (int)min((long long)n, (long long)blockIdx.x * chunk), hi = min(n, lo + chunk);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int nq = 0;  // the warp's queued particles (uniform over the warp)
-  // 2D: a slice's records are loaded while the one before it is worked on
-  // (32M FP32 particles: 1.16 -> 1.09 ms; the FP64 3D kernel, at its register
-  // limit, 1.27 -> 1.31 ms on the 131k-cell pipe)
-  constexpr bool AHEAD = DIM == 2;
-  int c_next = 0;
-  R x_next[DIM], u_next[DIM];
-  const auto fetch = [&](int p) {
+  if (threadIdx.x == 0) s_n = 0;
+  __syncthreads();
+  for (int base = lo + warp * 32; base < hi; base += kAdvThreads) {
+    const int p = base + lane;
+    bool leave = false;
     if (p < hi) {
-      c_next = cell[p];
+      const int c0 = cell[p];
+      R x[DIM];
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) {
-        x_next[d] = xi[d * cap + p];
-        if (FUSE) u_next[d] = u[d * cap + p];
+      for (int d = 0; d < DIM; ++d) x[d] = xi[d * cap + p];
+      if (FUSE) {
+        R N[NV], up[DIM];
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) up[d] = u[d * cap + p];
+        shape_values<DIM, R>(x, N);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          const int g = __ldg(cv + (size_t)c0 * NV + v);
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) up[d] = up[d] + N[v] * __ldg(dVr + (size_t)d * nv + g);
+        }
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) u[d * cap + p] = up[d];
       }
-    }
-  };
-  if (AHEAD) fetch(lo + warp * 32 + lane);
-  for (int base = lo + warp * 32;; base += kAdvThreads) {
-    const bool more = base < hi;  // uniform over the warp
-    if (more) {
-      const int p = base + lane;
-      bool leave = false;
+      const R dts = R(inst[__ldg(cell_inst + c0)].dt_sub);
       int s_left = 0;
-      if (!AHEAD) fetch(p);
-      const int c0 = c_next;
-      R x[DIM], up[DIM];
+      const int c = advect_steps<DIM, R, false>(c0, x, dts, 0, s_left, S, geo, cv, Vr, nv, nullptr, nullptr, nullptr);
+      leave = c == kAdvLeft;
+      newcell[p] = leave ? s_left : c;
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) {
-        x[d] = x_next[d];
-        up[d] = u_next[d];
-      }
-      if (AHEAD) fetch(p + kAdvThreads);
-      if (p < hi) {
-        if (FUSE) {
-          R N[NV];
-          shape_values<DIM, R>(x, N);
-#pragma unroll
-          for (int v = 0; v < NV; ++v) {
-            const int g = __ldg(cv + (size_t)c0 * NV + v);
-#pragma unroll
-            for (int d = 0; d < DIM; ++d) up[d] = up[d] + N[v] * __ldg(dVr + (size_t)d * nv + g);
-          }
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) u[d * cap + p] = up[d];
-        }
-        const R dts = R(inst[__ldg(cell_inst + c0)].dt_sub);
-        const int c = advect_steps<DIM, R, false>(c0, x, dts, 0, s_left, S, geo, cv, Vr, nv, nullptr, nullptr, nullptr);
-        if (c == kAdvLeft) {
-          leave = true;
-        } else {
-          newcell[p] = c;
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) xi[d * cap + p] = x[d];
-        }
-      }
-      const unsigned m = __ballot_sync(PFEM2_FULL_MASK, leave);
-      if (leave) {
-        const int k = nq + __popc(m & lanemask_lt());
-        q_p[warp][k] = p;
-        q_c[warp][k] = c0;
-        q_s[warp][k] = (unsigned short)s_left;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) q_x[warp][d][k] = x[d];
-      }
-      nq += __popc(m);
+      for (int d = 0; d < DIM; ++d) xi[d * cap + p] = x[d];
     }
-    __syncwarp();
-    // resume 32 queued particles at a time (after the last slice: all),
-    // from the top of the queue; the order does not change any result
-    while (nq >= 32 || (!more && nq > 0)) {
-      const int k = nq - 32 + lane;
-      if (k >= 0) {
-        const int p = q_p[warp][k], c0 = q_c[warp][k];
-        R x[DIM];
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) x[d] = q_x[warp][d][k];
-        const R dts = R(inst[__ldg(cell_inst + c0)].dt_sub);
-        int s_left = 0;
-        int c = advect_steps<DIM, R, true>(c0, x, dts, (int)q_s[warp][k], s_left, S, geo, cv, Vr, nv, v2c_ptr,
-                                           v2c_cell, v2c_dir);
-        if (c < 0) c = -1;
-        advect_record(p, c0, c, ring_ptr, ring_cell, far_keys, far_cap, counters, mv);
-        newcell[p] = c;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) xi[d * cap + p] = x[d];
-      }
-      nq = nq > 32 ? nq - 32 : 0;
-      __syncwarp();  // the resumed entries are read before the next slice appends over them
+    const unsigned m = __ballot_sync(PFEM2_FULL_MASK, leave);
+    if (m) {
+      int k = 0;
+      if (lane == 0) k = atomicAdd(&s_n, __popc(m));
+      k = __shfl_sync(PFEM2_FULL_MASK, k, 0);
+      if (leave) queue[lo + k + __popc(m & lanemask_lt())] = p;
     }
-    if (!more) break;
+  }
+  __syncthreads();
+  const int left = s_n, nu = (left + 31) / 32;
+  if (threadIdx.x == 0) s_at = atomicAdd(n_units, nu);
+  __syncthreads();
+  for (int j = threadIdx.x; j < nu; j += kAdvThreads) units[s_at + j] = make_int2(lo + 32 * j, min(32, left - 32 * j));
+}
+
+template <int DIM, typename R>
+__global__ void __launch_bounds__(kLeaveThreads, LeaveMinBlocks<DIM, R>::value) k_advect_leave(
+    const int* __restrict__ cell, R* __restrict__ xi, int* __restrict__ newcell, size_t cap,
+    const CellGeo<DIM, R>* __restrict__ geo, const int* __restrict__ cv,
+    const R* __restrict__ Vr, int nv, int S, const DevInst* __restrict__ inst, const int* __restrict__ cell_inst,
+    const int* __restrict__ v2c_ptr, const int* __restrict__ v2c_cell, const R* __restrict__ v2c_dir,
+    const int* __restrict__ ring_ptr, const int* __restrict__ ring_cell, unsigned long long* __restrict__ far_keys,
+    int far_cap, int* __restrict__ counters, const Movers mv, const int* __restrict__ queue,
+    const int2* __restrict__ units, const int* __restrict__ n_units) {
+  const int nu = *n_units, lane = threadIdx.x & 31;
+  for (int i = (blockIdx.x * kLeaveThreads + threadIdx.x) >> 5; i < nu; i += gridDim.x * (kLeaveThreads / 32)) {
+    const int2 unit = units[i];
+    if (lane >= unit.y) continue;
+    const int p = queue[unit.x + lane], c0 = cell[p];
+    R x[DIM];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) x[d] = xi[d * cap + p];
+    const R dts = R(inst[__ldg(cell_inst + c0)].dt_sub);
+    int s_left = 0;
+    int c = advect_steps<DIM, R, true>(c0, x, dts, newcell[p], s_left, S, geo, cv, Vr, nv, v2c_ptr, v2c_cell, v2c_dir);
+    if (c < 0) c = -1;
+    advect_record(p, c0, c, ring_ptr, ring_cell, far_keys, far_cap, counters, mv);
+    newcell[p] = c;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) xi[d * cap + p] = x[d];
   }
 }
 
@@ -831,20 +828,20 @@ static pfem2_status advect_impl(Ctx& c, bool fuse) {
           c.movers);
     c.launches++;
   } else {
-    // the queue kernel's blocks walk contiguous chunks
+    // every resident block walks one contiguous chunk
     const int grid = grid_for(c, c.pcap, kAdvThreads, c.tune.advect_blocks_per_sm);
-    if (fuse)
-      k_advect_q<DIM, R, true><<<grid, kAdvThreads, 0, c.stream>>>(
-          c.pcell[b], (R*)c.pxi[b], (R*)c.pu[b], c.newcell, (size_t)c.pcap, c.d_np + b,
-          (const CellGeo<DIM, R>*)c.cell_geo, c.cv, (const R*)c.Vr, (const R*)c.dVr, c.nv, S, c.d_inst, c.cell_inst,
-          c.v2c_ptr, c.v2c_cell, (const R*)c.v2c_dir_r, c.ring_ptr, c.ring_cell, c.far_keys, c.far_cap, c.d_counters,
-          c.movers);
-    else
-      k_advect_q<DIM, R, false><<<grid, kAdvThreads, 0, c.stream>>>(
-          c.pcell[b], (R*)c.pxi[b], (R*)c.pu[b], c.newcell, (size_t)c.pcap, c.d_np + b,
-          (const CellGeo<DIM, R>*)c.cell_geo, c.cv, (const R*)c.Vr, (const R*)c.dVr, c.nv, S, c.d_inst, c.cell_inst,
-          c.v2c_ptr, c.v2c_cell, (const R*)c.v2c_dir_r, c.ring_ptr, c.ring_cell, c.far_keys, c.far_cap, c.d_counters,
-          c.movers);
+    int* const queue = c.rebin_list + (size_t)c.nc * kListStride;  // the re-sort's overflow part, free until then
+    int* const n_units = c.movers.cnt + c.nc;
+    int2* const units = (int2*)c.pu[1 - b];  // filled by the re-sort later
+    const auto stay = fuse ? k_advect_stay<DIM, R, true> : k_advect_stay<DIM, R, false>;
+    stay<<<grid, kAdvThreads, 0, c.stream>>>(
+        c.pcell[b], (R*)c.pxi[b], (R*)c.pu[b], c.newcell, (size_t)c.pcap, c.d_np + b,
+        (const CellGeo<DIM, R>*)c.cell_geo, c.cv, (const R*)c.Vr, (const R*)c.dVr, c.nv, S, c.d_inst, c.cell_inst,
+        queue, units, n_units);
+    k_advect_leave<DIM, R><<<grid, kLeaveThreads, 0, c.stream>>>(
+        c.pcell[b], (R*)c.pxi[b], c.newcell, (size_t)c.pcap, (const CellGeo<DIM, R>*)c.cell_geo, c.cv, (const R*)c.Vr, c.nv, S, c.d_inst, c.cell_inst, c.v2c_ptr, c.v2c_cell, (const R*)c.v2c_dir_r, c.ring_ptr,
+        c.ring_cell, c.far_keys, c.far_cap, c.d_counters, c.movers, queue, units, n_units);
+    c.launches++;
     c.launches++;
   }
   k_far_sort<<<1, 1024, sizeof(unsigned long long) * c.far_cap, c.stream>>>(c.far_keys, c.d_counters, c.far_cap);
@@ -854,7 +851,7 @@ static pfem2_status advect_impl(Ctx& c, bool fuse) {
 
 pfem2_status launch_advect(Ctx& c, bool fuse) {
   PFEM2_CUDA(cudaMemsetAsync(c.d_counters, 0, sizeof(int) * CNT_N_STATS, c.stream));
-  PFEM2_CUDA(cudaMemsetAsync(c.movers.cnt, 0, sizeof(int) * c.nc, c.stream));
+  PFEM2_CUDA(cudaMemsetAsync(c.movers.cnt, 0, sizeof(int) * (c.nc + 1), c.stream));
   if (c.dim == 2) return c.pmixed ? advect_impl<2, float>(c, fuse) : advect_impl<2, double>(c, fuse);
   return c.pmixed ? advect_impl<3, float>(c, fuse) : advect_impl<3, double>(c, fuse);
 }

@@ -62,3 +62,28 @@ def test_resort(dim, q, scale, crowd):
     gs, os_ = g.stats(), o.stats()
     for k in ("deleted", "removed", "reseeded"):
         assert gs[k] == os_[k]
+
+
+@pytest.mark.parametrize("dim,q,scale,blocks,prec", [
+    (2, (1, 1), 1.0, 32, "fp64"),   # chunks of a few particles, units of one
+    (2, (5, 5), 1.0, 1, "fp64"),    # several slices a warp, full units
+    (2, (5, 5), 4.0, 4, "fp32"),    # far movers, FP32 storage
+    (3, (3, 3, 3), 1.0, 2, "fp64"),
+    (3, (2, 2, 2), 1.0, 32, "fp32"),
+])
+def test_advection_forms(dim, q, scale, blocks, prec):
+    """the two-kernel advection moves every particle bit for bit as the
+    one-kernel form does, for chunks from below a warp to many slices"""
+    out = []
+    for split in (1, 2):
+        sp = spec_2d() if dim == 2 else spec_3d()
+        g, o = make_pair(sp, prec, tuning={"advect_split": split, "advect_blocks_per_sm": blocks})
+        set_vel(g, o, sp, smooth_field(sp.mesh.vertices, scale))
+        g.seed_particles(q, seed=5, jitter=0.1)
+        for _ in range(3):
+            g.advect()
+        out.append((g.particles(), g.stats()["deleted"], g.stats()["far"]))
+    (a, da, fa), (b, db, fb) = out
+    assert da == db and fa == fb
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y)
