@@ -215,7 +215,12 @@ __device__ __forceinline__ void decide(LocalSys& L, bool bicg, bool trust, doubl
       const double rho = s[2] - om * s[3];
       L.omega = om;
       L.it += 1;
-      if (!(om != 0.0) || !(rho != 0.0) || rr <= L.intol * L.intol || L.it >= L.maxit || !(rr == rr)) {
+      // a rho that is mostly the rounding of its sum is no direction: the solve
+      // would wander, up to max_iter on the rounding-sized cross components of a
+      // pipe, so the next cycle takes a new shadow residual (1e-12 |rh| |r|: at
+      // most 83 iterations over 8 steps of the 442k-cell pipe, FP64, where 1e-13
+      // had 163, an exact zero 10,000)
+      if (!(om != 0.0) || !(fabs(rho) > 1e-12 * L.res * sqrt(rr)) || rr <= L.intol * L.intol || L.it >= L.maxit || !(rr == rr)) {
         L.pend = 1;  // x += omega K^-1 s is folded into the FP64 residual
         L.act = ACT_OUT_A;
         L.state = S_OUT_B;

@@ -52,3 +52,20 @@ def test_fem_step_partitions(monkeypatch, size, prec, kind, tuning, wide):
     for fld in [A.FIELD_PRED_VX + d for d in range(dim)] + [A.FIELD_P] + [A.FIELD_VX + d for d in range(dim)]:
         e = rel_l2(g.field(fld), o.field(fld))
         assert e <= 1e-8, (fld, e)
+
+
+def test_bicgstab_of_rounding_sized_components():
+    """a pipe whose cross components are rounding noise, every solve to 1e-11
+    of its right-hand side: no BiCGStab solve loses its direction and runs on
+    towards max_iter (the solves that do not take 30 to 90 iterations)"""
+    sp = cases.pipe_3d(nx=48, ny=12, nz=12)
+    sp.case.vel_solver = BICG
+    sp.case.vel_tol = sp.case.p_tol = 0.0
+    sp.case.vel_rtol = sp.case.p_rtol = 1e-11
+    g, _ = make_pair(sp, "fp64")
+    g.seed_particles(sp.q, seed=sp.seed, jitter=sp.jitter)
+    for _ in range(8):
+        g.step()
+        st = g.stats()
+        it = st["iters"]
+        assert st["status"] == A.OK and max(it[:3] + it[4:7]) <= 500
