@@ -172,15 +172,17 @@ def pressure_solve_bytes(s, iters, outer):
     """Algorithmic bytes of the pressure solves with the multigrid operators.
     One inner CG iteration (inner type R: FP32 for the mixed path) reads
     every operator once with its column indices and streams the vectors:
-        A   q = A (z + beta p)         nnz*(R+4) + n*(z, p in; p, q out)
-        B   e, r' update; b1, b2       n*(e, p, q, r in; e, r' out) + (R01 + R02 + C3)*(R+4) + (n1 + n2)*R
-        UZ  z = J0 r + Pt0 x1, coarse  nnz*(R+4) + P0*(R+4) + (J1+P1+J2+P2)*(R+4) + n*(r in, z out) + n2*R
+        A   q = A z + beta q, p, dq    nnz*(R+4) + n*(z, q, p in; q, p, dq out)
+        B   c1 = Pt0^T q               R01*(R+4)
+        B2  e, r; b2; J0 q             R02*(R+4) + nnz*(R+4) + n*(e, p, r, q, dq, jr in; e, r, jr out)
+        X2  x2 = M2 b2 (dense)         M2*R
+        UZ  z = J0 r + Pt0 x1          (J1 + P1 + P0)*(R+4) + n*(jr in, z out)
     FP64 refinement sweep: nnz*(8+4) + n*(x64 + e + b + r64) bytes."""
     info = s.sizes()
     n, nnz, rb = info["rows"], info["nnz"], info["real_bytes"]
     mg = s.solver_sizes()
-    ops = mg["r01"] + mg["r02"] + mg["c3"] + mg["p0"] + mg["j1"] + mg["p1"] + mg["j2"] + mg["p2"]
-    inner = 2 * nnz * (rb + 4) + ops * (rb + 4) + 12 * n * rb + (mg["n1"] + 2 * mg["n2"]) * rb
+    ops = mg["r01"] + mg["r02"] + mg["p0"] + mg["j1"] + mg["p1"]
+    inner = 2 * nnz * (rb + 4) + ops * (rb + 4) + mg["j2"] * rb + 17 * n * rb + 3 * (mg["n1"] + mg["n2"]) * rb
     outerb = nnz * 12 + n * (8 + rb + 8 + 8)
     return iters * inner + outer * outerb
 
@@ -333,7 +335,7 @@ def run_ours(args, rank, world, local):
         "cell_updates_per_s": cells * value,
         "stage_ms_per_step": {n: stages[i] / args.steps for i, n in enumerate(STAGE_NAMES)},
         "pressure_cg_iters_per_step": it_p / args.steps,
-        "roofline": {"bound": "hbm", "kernel": "k_krylov<float, MG> (pressure solve: CG, multigrid preconditioner)",
+        "roofline": {"bound": "hbm", "kernel": "k_mgcg<float> (pressure solve: CG, multigrid preconditioner)",
                      "achieved": gbs(cgb), "peak": hbm, "peak_kind": peak_kind, "unit": "GB/s",
                      "frac": (gbs(cgb) / hbm) if gbs(cgb) else None,
                      "algorithmic_bytes_per_step": cgb / args.steps,
@@ -372,7 +374,7 @@ def run_ours(args, rank, world, local):
 # cold read of the solve's working set, which then stays in L2: it does
 # not grow with the iteration count.
 KRYLOV_TRAFFIC_PER_LAUNCH = 0.5 * ((27532032 + 54272) + (27526400 + 10240))
-KRYLOV_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the k_krylov<float, MG> launches "
+KRYLOV_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the k_mgcg<float> launches "
                          "of steps 5-6 (31 and 30 iterations) of `bench.py --only channel --steps 3 --warmup 4`; "
                          "per launch = per step")
 
