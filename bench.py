@@ -367,15 +367,15 @@ def run_ours(args, rank, world, local):
 
 
 # DRAM bytes (read + write) of one pressure-solve launch of the channel in
-# the timed window (steps 5 and 6 after 4 warm-up steps, 31 and 30 CG
-# iterations, rtol 1e-8): ncu dram__bytes_read.sum + dram__bytes_write.sum
+# the timed window (steps 5 and 6 after 4 warm-up steps, 25 CG
+# iterations each, rtol 1e-8): ncu dram__bytes_read.sum + dram__bytes_write.sum
 # of `bench.py --only channel --steps 3 --warmup 4`, mean of the two
 # launches. Under ncu every launch starts with a flushed L2, so this is one
 # cold read of the solve's working set, which then stays in L2: it does
 # not grow with the iteration count.
-KRYLOV_TRAFFIC_PER_LAUNCH = 0.5 * ((27532032 + 54272) + (27526400 + 10240))
+KRYLOV_TRAFFIC_PER_LAUNCH = 0.5 * ((23025920 + 23296) + (23028480 + 1536))
 KRYLOV_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the k_mgcg<float> launches "
-                         "of steps 5-6 (31 and 30 iterations) of `bench.py --only channel --steps 3 --warmup 4`; "
+                         "of steps 5-6 (about 25 iterations each) of `bench.py --only channel --steps 3 --warmup 4`; "
                          "per launch = per step")
 
 
