@@ -286,8 +286,9 @@ typedef struct {
  * system sum_q [lambda d_ci N_a d_cj N_b + mu d_cj N_a d_ci N_b
  * + delta_ci,cj mu grad N_a . grad N_b] JxW on the current mesh, u = 0 on
  * fixed_mask, u = body_disp on body_id, solved by CG (Jacobi) into
- * PFEM2_FIELD_DISP_X/Y; iterations and the final residual norm out
- * (either may be NULL). NOT_CONVERGED past max_iter. */
+ * PFEM2_FIELD_DISP_X/Y; iterations and the final residual norm |b - K u|
+ * out (either may be NULL). A tolerance below the rounding of b - K u is met
+ * at that rounding. NOT_CONVERGED past max_iter. */
 pfem2_status pfem2_mesh_elasticity(pfem2_ctx* ctx, int32_t instance, const pfem2_elasticity* e,
                                    const double body_disp[3], int32_t* iterations, double* residual);
 /* reinterpolate_fields + transform_grid + sort_particles_into_subdomains_and_
