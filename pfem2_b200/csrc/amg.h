@@ -67,8 +67,8 @@ pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vec
                       const std::vector<int>& len, const std::vector<Tile>& tiles, const std::vector<int>& st0,
                       const std::vector<int>& bt0, int coarse_max, MgHost& out);
 
-// In-place inverse of an SPD matrix (Cholesky, then L^-T L^-1); false if
-// the matrix is not SPD.
-bool spd_inverse(std::vector<double>& M, int n);
+// In-place inverse of an SPD matrix (Cholesky, then L^-T L^-1); false if the
+// matrix is not SPD, a pivot being pivot_min times its diagonal entry or less.
+bool spd_inverse(std::vector<double>& M, int n, double pivot_min);
 
 }  // namespace pfem2

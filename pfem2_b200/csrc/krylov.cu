@@ -918,6 +918,22 @@ void krylov_free(Ctx& c) {
   c.kws = nullptr;
 }
 
+// whether the grid of a flow solve is resident with its shared memory (a
+// cluster's is checked with its plan)
+static pfem2_status plan_resident(Ctx& c, int which) {
+  const KrylovWs* w = (const KrylovWs*)c.kws;
+  const JacobiPlan& P = w->plan[which == 1 ? 0 : 1];
+  if (P.cluster) return PFEM2_OK;
+  int sm = 0;
+  const size_t smem = plan_smem(P, c.kmixed ? sizeof(float) : sizeof(double), P.minb,
+                                which == 1 || (which == 2 && w->mass_share) ? 1 : c.dim, sm);
+  if (occupancy(c.kmixed, P.minb, sm, smem) * c.num_sms < P.grid) {
+    set_error("krylov: the solver grid cannot be resident");
+    return PFEM2_CUDA_ERROR;
+  }
+  return PFEM2_OK;
+}
+
 pfem2_status krylov_setup(Ctx& c) {
   KrylovWs* w = new KrylovWs();
   c.kws = w;
@@ -926,8 +942,9 @@ pfem2_status krylov_setup(Ctx& c) {
   std::vector<int> ioff(1, 0);
   for (const HostInst& in : c.inst) ioff.push_back((in.v_off + in.nv_pad) / kSlice);
   int maxslots = 0;
-  // plan 0: the pressure systems where the multigrid is not used
-  for (int ph = c.two_level ? 1 : 0; ph < 2; ++ph) {
+  // plan 0: the pressure systems where the multigrid is not used, or may turn
+  // out not to be (moving meshes)
+  for (int ph = c.two_level && !c.moving ? 1 : 0; ph < 2; ++ph) {
     JacobiPlan& P = w->plan[ph];
     P.bicg = ph == 0 ? c.p_bicg : c.vel_bicg;
     const bool tuned = ph == 1 && (c.tune.vel_blocks_per_sm || c.tune.vel_tile_slices);
@@ -963,18 +980,9 @@ pfem2_status krylov_setup(Ctx& c) {
     PFEM2_TRY(ws_alloc(w, &w->out_tol[k], dim * ni));
     PFEM2_TRY(ws_alloc(w, &w->out_outer[k], dim * ni));
   }
-  // residency of the grids with their shared memory (a cluster's is checked with its plan)
-  for (int which = 0; which < 3; ++which) {
-    const JacobiPlan& P = w->plan[which == 1 ? 0 : 1];
-    if ((which == 1 && c.two_level) || P.cluster) continue;
-    int sm = 0;
-    const size_t smem = plan_smem(P, rs, P.minb, which == 1 || (which == 2 && w->mass_share) ? 1 : dim, sm);
-    if (occupancy(c.kmixed, P.minb, sm, smem) * c.num_sms < P.grid) {
-      set_error("krylov: the solver grid cannot be resident");
-      return PFEM2_CUDA_ERROR;
-    }
-  }
   // (a cluster keeps the same operands in shared memory in every solve)
+  for (int which = 0; which < 3; ++which)
+    if (which != 1 || !c.two_level) PFEM2_TRY(plan_resident(c, which));
   return PFEM2_OK;
 }
 
@@ -1065,8 +1073,17 @@ pfem2_status krylov_elastic_read(Ctx& c, int* it, double* res, double* tol) {
   return PFEM2_OK;
 }
 
-// The multigrid of the pressure matrix (after Dirichlet elimination).
-pfem2_status krylov_setup_precond(Ctx& c) { return c.two_level ? mg_setup(c) : PFEM2_OK; }
+// The multigrid of the pressure matrix (after Dirichlet elimination). A moving
+// mesh that has none (too small to coarsen, or a pressure without a Dirichlet
+// boundary) is solved by the Jacobi CG.
+pfem2_status krylov_setup_precond(Ctx& c) {
+  if (!c.two_level) return PFEM2_OK;
+  const pfem2_status st = mg_setup(c);
+  if (st == PFEM2_OK || st == PFEM2_CUDA_ERROR || !c.moving) return st;
+  mg_free((KrylovWs*)c.kws);
+  c.two_level = false;
+  return plan_resident(c, 1);
+}
 
 // resets the solve's state; the previous solve's exit code (1 timeout,
 // 2 iteration cap) is kept as bit (1 << code) in *sticky until the host
