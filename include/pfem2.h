@@ -366,7 +366,10 @@ typedef struct {
  * (written by the autotuner, pfem2_b200/autotune.py) when it holds an entry
  * for this context's key, else chosen by size. */
 pfem2_status pfem2_set_tuning(pfem2_ctx* ctx, const pfem2_tuning* t);
-/* The launch shapes in use (after pfem2_setup: every field resolved). */
+/* The launch shapes in use (after pfem2_setup: every field resolved; the
+ * velocity fields are 0 where one thread-block cluster solves, the automatic
+ * form of small single systems). A context of the same instances that is given
+ * them runs the same shapes. */
 pfem2_status pfem2_get_tuning(pfem2_ctx* ctx, pfem2_tuning* t);
 /* The key of the tuning cache for this context (after pfem2_add_instance):
  * "<device name> <dim> <fp32 stages, -1 for FP64> <log2 cells> <log2 instances>". */

@@ -4,8 +4,8 @@ The particle kernels and the persistent Krylov solver have shapes that the
 best choice of depends on the GPU and the mesh size: the advection grid
 (particles per block) and whether advection runs in one pass or in two
 phases (stayers, then queued leavers), the re-sort grid, the velocity
-solves' tile size (SELL slices per tile) and blocks per SM, and the blocks
-per SM of a single pressure system's multigrid solve. `tune` times whole
+solves' SELL slices per block and blocks per SM, and the blocks per SM of a
+single pressure system's multigrid solve. `tune` times whole
 steps (the device time of every stage,
 CUDA events inside the library) for candidate shapes by coordinate descent
 (coupled knobs, such as the advection grid and its one- or two-phase form,
@@ -113,7 +113,9 @@ def _tune(specs, space, steps, warmup, cache, rounds, prepare, solver_kw):
     probe = Solver(specs, use_graph=True, **solver_kw)
     key = probe.tuning_key()
     probe.close()
-    best = {k: v for k, v in best.items() if k in space or v}
+    # (velocity shapes that are not searched stay automatic: their best form
+    # changes within a key's range of sizes)
+    best = {k: v for k, v in best.items() if k in space or (v and not k.startswith("vel_"))}
     best_t = t0
     trials = [({k: best[k] for k in best}, t0)]
     for _ in range(rounds):

@@ -857,6 +857,7 @@ static pfem2_status plan_build(Ctx& c, KrylovWs* w, JacobiPlan& P, bool mixed, c
     // instances wait less for each other (16 channels: 1.38 against 1.44 ms)
     P.minb = minb ? minb : (ni > 1 || ts_auto * ncomp * rounds <= 12 ? 2 : 1);
     if (!ts) ts = ni > 1 ? 4 : ts_auto;
+    P.ts = ts;
     const int occ = std::min(P.minb, occupancy(mixed, P.minb, 0, 0));
     if (occ < 1) {
       set_error("krylov: the solver kernel cannot be resident");
@@ -865,7 +866,6 @@ static pfem2_status plan_build(Ctx& c, KrylovWs* w, JacobiPlan& P, bool mixed, c
     PFEM2_TRY(plan_runs(P, up, ioff, slp, ncomp, std::max(1, std::min(occ * c.num_sms, (ns + ts - 1) / ts))));
     set_split();
   }
-  P.ts = (ns + P.grid - 1) / P.grid;
   int** dst[6] = {&P.blk_sl, &P.blk_inst, &P.blk_inst_off, &P.blk_slot, &P.sys_slot0, &P.slk};
   for (int k = 0; k < 6; ++k) PFEM2_TRY(ws_upload(w, dst[k], up[k]));
   return PFEM2_OK;
@@ -951,7 +951,9 @@ pfem2_status krylov_setup(Ctx& c) {
     PFEM2_TRY(plan_build(c, w, P, c.kmixed, ioff, c.h_sl_ptr, ph == 0 ? 1 : dim, ph == 0 ? 1 : dim,
                          ph == 0 ? 0 : c.tune.vel_blocks_per_sm, ph == 0 ? 0 : c.tune.vel_tile_slices, !tuned));
     maxslots = std::max(maxslots, P.nslots);
-    if (ph == 1) {
+    // (the shape that makes this partition again when it is set; with a cluster
+    // both fields stay automatic: any value would rule it out)
+    if (ph == 1 && !P.cluster) {
       if (!c.tune.vel_blocks_per_sm) c.tune.vel_blocks_per_sm = P.minb;
       if (!c.tune.vel_tile_slices) c.tune.vel_tile_slices = P.ts;
     }

@@ -100,7 +100,8 @@ struct MgWs;  // mgcg.cu
 struct JacobiPlan {
   int *blk_inst = nullptr, *blk_inst_off = nullptr, *blk_slot = nullptr, *blk_sl = nullptr, *sys_slot0 = nullptr,
       *slk = nullptr;
-  int grid = 0, nslots = 0, items_max = 0, minb = 2, ts = 0, split = 1;
+  int grid = 0, nslots = 0, items_max = 0, minb = 2, split = 1;
+  int ts = 0;                                      // no cluster: least slices of a block
   int sm = 0;                                      // cluster: what a block keeps in shared memory
   bool cluster = false, bicg = false;
   size_t st_meta = 0, st_entries = 0;              // per block: static index bytes, SELL entries
