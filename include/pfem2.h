@@ -364,7 +364,8 @@ typedef struct {
 /* Sets the launch shapes (before pfem2_setup). Fields left at 0 are taken
  * from the tuning cache named by the environment variable PFEM2_TUNING_CACHE
  * (written by the autotuner, pfem2_b200/autotune.py) when it holds an entry
- * for this context's key, else chosen by size. */
+ * for this context's key, timed with this version of the kernels, else chosen
+ * by size. */
 pfem2_status pfem2_set_tuning(pfem2_ctx* ctx, const pfem2_tuning* t);
 /* The launch shapes in use (after pfem2_setup: every field resolved; the
  * velocity fields are 0 where one thread-block cluster solves, the automatic

@@ -69,9 +69,13 @@ def measure(specs, tuning, steps=5, warmup=2, seed_q=None, prepare=None, **solve
         s.close()
 
 
+# of the kernels that the shapes were timed with: the library passes over lines of another one
+CACHE_VERSION = "v2"
+
+
 def cache_line(key, tuning, ms):
     vals = " ".join(str(int(tuning[k])) for k in A.TUNING_FIELDS)
-    return f"{key} {vals} {ms:.4f}\n"
+    return f"{key} {vals} {ms:.4f} {CACHE_VERSION}\n"
 
 
 def tune(specs, space=None, steps=5, warmup=2, cache=None, rounds=1, prepare=None, **solver_kw):

@@ -142,11 +142,16 @@ static std::string tuning_key(const Ctx& c) {
 
 // The tuning cache (PFEM2_TUNING_CACHE): one entry per line,
 //   <device> <dim> <stages> <log2 cells> <log2 instances>
-//   <advect bps> <advect split> <rebin bps> <vel tile slices> <p bps> [<vel bps>] [ms per step]
+//   <advect bps> <advect split> <rebin bps> <vel tile slices> <p bps> [<vel bps>] <ms per step> <version>
 // (the launch-shape values are integers, the time has a decimal point; a
 // missing value is automatic). '#' starts a comment; the last entry with
 // this context's key wins. Its values fill the fields the caller left at 0.
+// Lines of another version, or of none, were timed with kernels that shared
+// their work out differently and are passed over: the shapes found for the
+// velocity solves' former partition made the 52k channel 13% slower than the
+// automatic ones (1.32 against 1.17 ms per step).
 constexpr int kTuneVals = 6;
+constexpr char kTuneVersion[] = "v2";
 
 static void apply_tuning_cache(Ctx& c) {
   c.tune = c.tune_req;
@@ -167,7 +172,7 @@ static void apply_tuning_cache(Ctx& c) {
       tok.emplace_back(t);
     if (tok.size() < 5 + 5) continue;
     const std::string k = tok[0] + " " + tok[1] + " " + tok[2] + " " + tok[3] + " " + tok[4];
-    if (key != k) continue;
+    if (key != k || tok.back() != kTuneVersion) continue;
     int v[kTuneVals] = {};
     bool ok = true;
     int nv = 0;

@@ -49,3 +49,21 @@ def test_reported_shapes_reproduce_the_run(sizes, prec, kind):
     assert t2 == t
     for x, y in zip(a, b):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("end,advect,vel", [
+    ("1.2345", 16, 0),      # written for the kernels before: automatic shapes
+    ("1.2345 v2", 3, 7),
+])
+def test_cache_lines_of_former_kernels_are_passed_over(tmp_path, monkeypatch, end, advect, vel):
+    sp = cases.poiseuille_2d(nx=32, ny=12)
+    s = Solver(sp, precision=A.PREC_FP64)
+    key = s.tuning_key()
+    s.close()
+    path = tmp_path / "tuning.txt"
+    path.write_text(f"{key} 3 1 2 7 1 1 {end}\n")
+    monkeypatch.setenv("PFEM2_TUNING_CACHE", str(path))
+    s = Solver(sp, precision=A.PREC_FP64)
+    t = s.tuning()
+    s.close()
+    assert t["advect_blocks_per_sm"] == advect and t["vel_tile_slices"] == vel
