@@ -71,6 +71,11 @@ enum {
 // residual phase |r|^2 and |b|^2)
 constexpr int kMaxSums = 5;
 constexpr int kClusterMax = 16;  // blocks of a cluster
+// systems (components x instances) a block may own parts of: a run of slices
+// that cuts an instance at either end touches up to two instances more than
+// its length holds, so that 1,570 instances in 3D and 2,360 in 2D, the smallest
+// at one slice each, fit two blocks on each of 148 SMs
+constexpr int kMaxRunSys = 24;
 // items (slices x components) up to which one cluster solves: above, the 16
 // SMs' work outweighs the cheaper barrier (1k channel FP64, 70 items:
 // prediction and correction 0.49 -> 0.38 ms per step; 8k cells, 520 items:
@@ -310,14 +315,14 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
   constexpr int kSolveThreads = SolveThreads<MINB>::value, kWarps = kSolveThreads / 32;
   extern __shared__ __align__(16) unsigned char dyn_smem[];
   constexpr int CH = Chunk<R>::value;
-  __shared__ LocalSys ls[kMaxLocalSys];
+  __shared__ LocalSys ls[kMaxRunSys];
   __shared__ int s_err;
   __shared__ double s_pub[CL ? 2 * 3 * kMaxSums * kClusterMax : 1];  // [parity][system][sum][block]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t nv = (size_t)a.nv;
   const int NC = a.ncomp;
   const int io = a.blk_inst_off[blockIdx.x];
-  const int nls = min((a.blk_inst_off[blockIdx.x + 1] - io) * NC, kMaxLocalSys);
+  const int nls = min((a.blk_inst_off[blockIdx.x + 1] - io) * NC, kMaxRunSys);
   const int bs0 = a.blk_sl[blockIdx.x], bs1 = a.blk_sl[blockIdx.x + 1];
   const int nitems = (bs1 - bs0) * NC, own0 = bs0 * 32;
   const int NS = a.bicg ? kMaxSums : 3;
@@ -793,8 +798,8 @@ static pfem2_status plan_runs(JacobiPlan& P, std::vector<int> (&up)[6], const st
       slk[sl] = j - i;
     }
     binst_off.push_back((int)binst.size());
-    if ((binst_off[b + 1] - binst_off[b]) * ncomp > kMaxLocalSys) {
-      set_error("krylov: more than 16 systems would share one block (instances too small for the batch)");
+    if ((binst_off[b + 1] - binst_off[b]) * ncomp > kMaxRunSys) {
+      set_error("krylov: more than 24 systems would share one block (instances too small for the batch)");
       return PFEM2_INVALID_ARG;
     }
     P.items_max = std::max(P.items_max, (s1 - s0) * ncomp);
@@ -863,7 +868,12 @@ static pfem2_status plan_build(Ctx& c, KrylovWs* w, JacobiPlan& P, bool mixed, c
       set_error("krylov: the solver kernel cannot be resident");
       return PFEM2_CUDA_ERROR;
     }
-    PFEM2_TRY(plan_runs(P, up, ioff, slp, ncomp, std::max(1, std::min(occ * c.num_sms, (ns + ts - 1) / ts))));
+    // (more blocks than ts asks for where such a run would touch too many instances)
+    const int most = std::max(1, std::min(occ * c.num_sms, ns));
+    int G = std::max(1, std::min(most, (ns + ts - 1) / ts));
+    pfem2_status st;
+    while ((st = plan_runs(P, up, ioff, slp, ncomp, G)) != PFEM2_OK && G < most) G = std::min(most, 2 * G);
+    PFEM2_TRY(st);
     set_split();
   }
   int** dst[6] = {&P.blk_sl, &P.blk_inst, &P.blk_inst_off, &P.blk_slot, &P.sys_slot0, &P.slk};

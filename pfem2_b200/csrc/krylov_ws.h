@@ -9,7 +9,7 @@
 
 namespace pfem2 {
 
-constexpr int kMaxLocalSys = 16;  // systems a block of a solver grid may own parts of
+constexpr int kMaxLocalSys = 16;  // systems a block of the multigrid's grid may own parts of
 
 __device__ __forceinline__ float fma_r(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double fma_r(double a, double b, double c) { return fma(a, b, c); }
