@@ -227,10 +227,21 @@ __global__ void k_v2c_dir(int nv, const double* __restrict__ X, const int* __res
     }
 }
 
-static pfem2_status ale_alloc(Ctx& c) {
-  if (c.ale_x) return PFEM2_OK;
+// the tables and vectors that ale_alloc makes
+static void ale_free_tables(Ctx& c) {
+  void** p[] = {(void**)&c.ale_K,   (void**)&c.ale_fix, (void**)&c.ale_g,   (void**)&c.ale_rhs,
+                (void**)&c.ale_dinv, (void**)&c.ale_x,  (void**)&c.ale_new, (void**)&c.ale_flag,
+                (void**)&c.ale_slp, (void**)&c.ale_sll, (void**)&c.ale_slc};
+  for (void** q : p) {
+    if (*q) cudaFree(*q);
+    *q = nullptr;
+  }
+}
+
+static pfem2_status ale_alloc_tables(Ctx& c) {
   const size_t nv = c.nv, dim = c.dim;
   auto al = [&](void** p, size_t bytes) -> pfem2_status {
+    *p = nullptr;
     PFEM2_CUDA(cudaMalloc(p, bytes));
     PFEM2_CUDA(cudaMemset(*p, 0, bytes));
     return PFEM2_OK;
@@ -266,6 +277,15 @@ static pfem2_status ale_alloc(Ctx& c) {
   return PFEM2_OK;
 }
 
+// on the first use; a call that fails half-way leaves nothing behind
+static pfem2_status ale_alloc(Ctx& c) {
+  if (c.ale_ready) return PFEM2_OK;
+  const pfem2_status st = ale_alloc_tables(c);
+  c.ale_ready = st == PFEM2_OK;
+  if (!c.ale_ready) ale_free_tables(c);
+  return st;
+}
+
 // boundary vertices (on any boundary face) of the mesh, once at setup
 pfem2_status ale_setup(Ctx& c) {
   const int NV = 1 << c.dim, NF = 2 * c.dim;
@@ -283,10 +303,9 @@ pfem2_status ale_setup(Ctx& c) {
 }
 
 void ale_free(Ctx& c) {
-  void* p[] = {c.ale_bnd, c.ale_fix, c.ale_g,     c.ale_rhs, c.ale_dinv, c.ale_x,   c.ale_K,
-               c.ale_slp, c.ale_sll, c.ale_slc, c.ale_xphys, c.ale_new, c.ale_flag};
-  for (void* q : p)
-    if (q) cudaFree(q);
+  ale_free_tables(c);
+  if (c.ale_bnd) cudaFree(c.ale_bnd);
+  if (c.ale_xphys) cudaFree(c.ale_xphys);
 }
 
 pfem2_status ale_elasticity(Ctx& c, const pfem2_elasticity& e, const double* body_disp, int* iters, double* res) {

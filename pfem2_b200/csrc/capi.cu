@@ -21,6 +21,7 @@ static thread_local std::string g_last_error;
 void set_error(const std::string& s) { g_last_error = s; }
 
 pfem2_status cuda_status(cudaError_t e, const char* where) {
+  cudaGetLastError();  // reported here: the next call's check of its launches must not see it again
   set_error(std::string(where) + ": " + cudaGetErrorString(e));
   return PFEM2_CUDA_ERROR;
 }

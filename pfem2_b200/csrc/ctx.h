@@ -202,6 +202,7 @@ struct Ctx {
   size_t ale_xphys_cap = 0;
   double* ale_new = nullptr;   // [4][nv]
   int* ale_flag = nullptr;
+  bool ale_ready = false;      // all of the elasticity's tables and vectors are there
 
   // launch shapes: as set by the caller (0 = automatic) and as resolved at
   // setup (caller, else the tuning cache, else by size)

@@ -1001,7 +1001,7 @@ pfem2_status krylov_setup(Ctx& c) {
 // Plan and vectors of the mesh elasticity (moving contexts, first use): one
 // FP64 system of dim x nv rows whose components follow each other, on slices
 // of its own (ale.cu).
-pfem2_status krylov_elastic_setup(Ctx& c, const std::vector<int>& slp) {
+static pfem2_status elastic_setup(Ctx& c, const std::vector<int>& slp) {
   KrylovWs* w = (KrylovWs*)c.kws;
   JacobiPlan& P = w->elastic;
   const std::vector<int> ioff = {0, (int)slp.size() - 1};
@@ -1019,6 +1019,18 @@ pfem2_status krylov_elastic_setup(Ctx& c, const std::vector<int>& slp) {
     return PFEM2_CUDA_ERROR;
   }
   return PFEM2_OK;
+}
+
+pfem2_status krylov_elastic_setup(Ctx& c, const std::vector<int>& slp) {
+  KrylovWs* w = (KrylovWs*)c.kws;
+  const size_t before = w->allocs.size();
+  const pfem2_status st = elastic_setup(c, slp);
+  if (st != PFEM2_OK) {  // another call starts over
+    for (size_t k = before; k < w->allocs.size(); ++k) cudaFree(w->allocs[k]);
+    w->allocs.resize(before);
+    w->elastic = JacobiPlan();
+  }
+  return st;
 }
 
 // CG (Jacobi, FP64) on that system. Its residual, s and u all follow by
