@@ -550,28 +550,45 @@ static pfem2_status do_setup(Ctx& c) {
   return PFEM2_OK;
 }
 
+static void free_particles(Ctx& c) {
+  void** p[] = {(void**)&c.pcell[0], (void**)&c.pcell[1], (void**)&c.pxi[0], (void**)&c.pxi[1], (void**)&c.pu[0],
+                (void**)&c.pu[1],    (void**)&c.newcell,  (void**)&c.rebin_list, (void**)&c.movers.list};
+  for (void** q : p) {
+    if (*q) cudaFree(*q);
+    *q = nullptr;
+  }
+  c.pcap = 0;
+}
+
+static pfem2_status alloc_particle_buffers(Ctx& c, size_t seeded, size_t cap) {
+  const size_t rs = c.pmixed ? 4 : 8;
+  for (int b = 0; b < 2; ++b) {
+    PFEM2_CUDA(cudaMalloc(&c.pcell[b], sizeof(int) * cap));
+    PFEM2_CUDA(cudaMalloc(&c.pxi[b], rs * c.dim * cap));
+    PFEM2_CUDA(cudaMalloc(&c.pu[b], rs * c.dim * cap));
+  }
+  PFEM2_CUDA(cudaMalloc(&c.newcell, sizeof(int) * cap));
+  PFEM2_CUDA(cudaMalloc(&c.rebin_list, sizeof(int) * ((size_t)c.nc * kListStride + cap)));
+  // room for twice a cell's mean share of particles to arrive in one move
+  c.movers.cap = (int)std::min<size_t>(kMoverMax, (2 * seeded / (size_t)c.nc + 32) / 32 * 32);
+  PFEM2_CUDA(cudaMalloc((void**)&c.movers.list, sizeof(int) * (size_t)c.movers.cap * c.nc));
+  return PFEM2_OK;
+}
+
+// Storage for `seeded` particles and more. Without enough memory the context
+// is left without particles: what needs them returns PFEM2_BAD_STATE.
 static pfem2_status alloc_particles(Ctx& c, size_t seeded) {
   double f = c.cfg.particle_capacity_factor > 0 ? c.cfg.particle_capacity_factor : 2.0;
   size_t cap = (size_t)std::ceil(seeded * f) + 1024;
   if (cap > (size_t)2000000000) cap = 2000000000;
   if ((int)cap <= c.pcap) return PFEM2_OK;
-  const size_t rs = c.pmixed ? 4 : 8;
-  for (int b = 0; b < 2; ++b) {
-    if (c.pcell[b]) cudaFree(c.pcell[b]);
-    if (c.pxi[b]) cudaFree(c.pxi[b]);
-    if (c.pu[b]) cudaFree(c.pu[b]);
-    PFEM2_CUDA(cudaMalloc(&c.pcell[b], sizeof(int) * cap));
-    PFEM2_CUDA(cudaMalloc(&c.pxi[b], rs * c.dim * cap));
-    PFEM2_CUDA(cudaMalloc(&c.pu[b], rs * c.dim * cap));
+  free_particles(c);
+  const pfem2_status st = alloc_particle_buffers(c, seeded, cap);
+  if (st != PFEM2_OK) {
+    free_particles(c);
+    c.seeded = false;
+    return st;
   }
-  if (c.newcell) cudaFree(c.newcell);
-  PFEM2_CUDA(cudaMalloc(&c.newcell, sizeof(int) * cap));
-  if (c.rebin_list) cudaFree(c.rebin_list);
-  PFEM2_CUDA(cudaMalloc(&c.rebin_list, sizeof(int) * ((size_t)c.nc * kListStride + cap)));
-  // room for twice a cell's mean share of particles to arrive in one move
-  c.movers.cap = (int)std::min<size_t>(kMoverMax, (2 * seeded / (size_t)c.nc + 32) / 32 * 32);
-  if (c.movers.list) cudaFree(c.movers.list);
-  PFEM2_CUDA(cudaMalloc((void**)&c.movers.list, sizeof(int) * (size_t)c.movers.cap * c.nc));
   c.pcap = (int)cap;
   c.graph_valid = false;
   return PFEM2_OK;
@@ -787,10 +804,9 @@ pfem2_status pfem2_destroy(pfem2_ctx* x) {
   // device memory is released with the context's allocations; free the big ones
   void* ptrs[] = {c.cell_geo, c.X, c.cv, c.fb, c.cell_inst, c.vert_inst, c.v2c_ptr, c.v2c_cell, c.v2c_loc, c.v2c_dir,
                   c.ring_ptr, c.ring_cell, c.sl_ptr, c.sl_len, c.sl_col, c.inc_slot, c.zero_flag, c.wall_dv,
-                  c.wall_cells, c.movers.cnt, c.movers.list, c.d_inst,
+                  c.wall_cells, c.movers.cnt, c.d_inst,
                   c.sys_scalars, c.d_sysinfo, c.Vr, c.dVr, c.partial, c.rebin_tiles, c.rebin_cnt,
-                  c.rebin_pos, c.rebin_list, c.d_np, c.d_counters,
-                  c.far_keys, c.barrier, c.d_err, c.d_err_sticky, c.newcell};
+                  c.rebin_pos, c.d_np, c.d_counters, c.far_keys, c.barrier, c.d_err, c.d_err_sticky};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c.pmixed && c.v2c_dir_r) cudaFree(c.v2c_dir_r);
@@ -800,9 +816,8 @@ pfem2_status pfem2_destroy(pfem2_ctx* x) {
   for (int f = 0; f < 4; ++f) { cudaFree(c.isdir[f]); cudaFree(c.dirval[f]); cudaFree(c.shift[f]); }
   for (int f = 0; f < PFEM2_N_FIELDS; ++f) cudaFree(c.F[f]);
   for (int k = 0; k < 3; ++k) { cudaFree(c.corr[k]); cudaFree(c.rhs[k]); }
-  for (int b = 0; b < 2; ++b) {
-    cudaFree(c.pcell[b]); cudaFree(c.pxi[b]); cudaFree(c.pu[b]); cudaFree(c.cell_start[b]);
-  }
+  free_particles(c);
+  for (int b = 0; b < 2; ++b) cudaFree(c.cell_start[b]);
   for (int k = 0; k < 8; ++k) cudaEventDestroy(c.ev[k]);
   for (const Ctx::LoadFaces& e : c.load_faces) cudaFree(e.d);
   cudaFree(c.loads_dev);

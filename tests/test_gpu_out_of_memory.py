@@ -63,3 +63,35 @@ def test_mesh_elasticity():
         s.close()
     first.close()
     assert len(failed) >= 2, failed  # at more than one of the call's allocations
+
+
+def test_seed():
+    """a context that cannot hold the particles asked for has none"""
+    sp = cases.channel_disk(h=float(np.sqrt(4.0 / 30000)))
+    kw = dict(precision=A.PREC_FP64, particles_only=True)
+    first = Solver(sp, **kw)
+    first.seed_particles((5, 5), 1, 0.1)
+    first.step()
+    want = first.particles()
+    failed = []
+    for left in range(6, 166, 20):
+        s = Solver(sp, **kw)
+        s.seed_particles((1, 1), 1, 0.1)
+        s.step()
+        with NoMemory(left * MB):
+            try:
+                s.seed_particles((5, 5), 1, 0.1)
+            except Pfem2Error as e:
+                assert e.status == A.CUDA_ERROR
+                failed.append(left)
+                for call in (s.step, s.move_particles, s.particles):
+                    with pytest.raises(Pfem2Error) as e:
+                        call()
+                    assert e.value.status == A.BAD_STATE
+        s.seed_particles((5, 5), 1, 0.1)
+        s.step()
+        for x, y in zip(s.particles(), want):
+            assert np.array_equal(x, y), left
+        s.close()
+    first.close()
+    assert len(failed) >= 2, failed
