@@ -887,6 +887,7 @@ pfem2_status pfem2_seed(pfem2_ctx* x, int32_t instance, const uint32_t q[3], uin
   for (auto& in : c.inst) total += (size_t)in.nc * in.q[0] * in.q[1] * in.q[2];
   PFEM2_TRY(alloc_particles(c, total));
   c.cur = 0;
+  c.seeded = false;  // until they are there
   PFEM2_TRY(launch_seed(c, instance, q, seed, jitter));
   c.seeded = true;
   c.stats.n_particles = (int)total;
@@ -1150,8 +1151,12 @@ pfem2_status pfem2_set_particles(pfem2_ctx* x, const int32_t* counts, const int3
   for (size_t i = 0; i < c.inst.size(); ++i) total += counts[i];
   for (auto& in : c.inst)
     if (in.q[0] == 0) { set_error("seed (to set q) before set_particles"); return PFEM2_BAD_STATE; }
+  // a refused call leaves the particles as they are (the idle half of their
+  // storage holds nothing that could be stepped: reads pack into it)
+  PFEM2_TRY(check_set_particles(c, counts, cell, xi, u));
   PFEM2_TRY(alloc_particles(c, total));
   c.cur = 0;
+  c.seeded = false;  // until they are there
   PFEM2_TRY(launch_set_particles(c, counts, cell, xi, u));
   c.seeded = true;
   for (int k = 0; k < 2; ++k)

@@ -270,6 +270,7 @@ pfem2_status launch_advect(Ctx& c, bool fuse_correct);
 pfem2_status launch_rebin(Ctx& c, bool do_check, bool fuse_project, bool from_advect);
 pfem2_status launch_project(Ctx& c, bool partials_ready);
 pfem2_status launch_sync_real_fields(Ctx& c);
+pfem2_status check_set_particles(const Ctx& c, const int* counts, const int* cell, const double* xi, const double* u);
 pfem2_status launch_set_particles(Ctx& c, const int* counts, const int* cell, const double* xi, const double* u);
 pfem2_status read_particles(Ctx& c, int instance, int* cell, double* xi, double* u, int* n);
 

@@ -1606,6 +1606,24 @@ __global__ void k_unpack_in(int n, const int* __restrict__ pos, const int* __res
   }
 }
 
+// refused before anything of the context changes
+pfem2_status check_set_particles(const Ctx& c, const int* counts, const int* cell, const double* xi, const double* u) {
+  size_t k = 0;
+  for (size_t i = 0; i < c.inst.size(); ++i)
+    for (int j = 0; j < counts[i]; ++j, ++k) {
+      if (cell[k] < 0 || cell[k] >= c.inst[i].nc) {
+        set_error("set_particles: cell out of range");
+        return PFEM2_INVALID_ARG;
+      }
+      for (int d = 0; d < c.dim; ++d)
+        if (!std::isfinite(xi[k * c.dim + d]) || !std::isfinite(u[k * c.dim + d])) {
+          set_error("set_particles: a coordinate or velocity is not finite");
+          return PFEM2_INVALID_ARG;
+        }
+    }
+  return PFEM2_OK;
+}
+
 template <int DIM, typename R>
 static pfem2_status set_impl(Ctx& c, const int* counts, const int* cell, const double* xi, const double* u) {
   // host-side stable placement by cell (a state-loading utility, not the step)
@@ -1619,17 +1637,7 @@ static pfem2_status set_impl(Ctx& c, const int* counts, const int* cell, const d
   size_t k = 0;
   for (size_t i = 0; i < c.inst.size(); ++i)
     for (int j = 0; j < counts[i]; ++j, ++k) {
-      int lc = cell[k];
-      if (lc < 0 || lc >= c.inst[i].nc) {
-        set_error("set_particles: cell out of range");
-        return PFEM2_INVALID_ARG;
-      }
-      for (int d = 0; d < DIM; ++d)
-        if (!std::isfinite(xi[k * DIM + d]) || !std::isfinite(u[k * DIM + d])) {
-          set_error("set_particles: a coordinate or velocity is not finite");
-          return PFEM2_INVALID_ARG;
-        }
-      gcell[k] = lc + c.inst[i].c_off;
+      gcell[k] = cell[k] + c.inst[i].c_off;
       cnt[gcell[k] + 1]++;
     }
   for (int i = 0; i < c.nc; ++i) cnt[i + 1] += cnt[i];
