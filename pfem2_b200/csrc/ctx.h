@@ -179,6 +179,9 @@ struct Ctx {
   // return PFEM2_BAD_STATE until the context is destroyed
   bool failed = false;
   long long mg_wide_min = 262144;  // rows from which one pressure system runs two blocks per SM
+  // bytes of partial sums up to which a block of a Jacobi solve keeps them in
+  // shared memory (where they fit); PFEM2_PARTIALS_MAX lowers it at creation
+  long long partials_max = 1 << 30;
   bool two_level = true;        // pressure: multigrid preconditioner (else Jacobi)
   bool vel_bicg = false;        // velocity systems solved by BiCGStab (else CG)
   bool p_bicg = false;          // pressure solved by BiCGStab with Jacobi (else CG with multigrid)

@@ -143,6 +143,7 @@ template <typename R> struct SolveArgs {
   R *e, *r;
   double* r64;
   double* part;          // [2 parities][kMaxSums][nslots]
+  double* item_part;     // [blocks][items_max][sums] where they do not fit shared memory, else null
   int nslots;
   unsigned* scount;      // [nsys][32]: per-system count of block phases published (one 128-byte line each, zeroed per launch)
   int* active;
@@ -334,6 +335,7 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
   double* const s_dot = reinterpret_cast<double*>(dyn_smem);
   double* spart = s_dot + (split > 1 ? kWarps * 32 : 0);
   unsigned char* cur = reinterpret_cast<unsigned char*>(spart) + al16_dev((size_t)a.items_max * NS * sizeof(double));
+  if (SM == 0 && a.item_part) spart = a.item_part + (size_t)blockIdx.x * a.items_max * NS;
   // own rows of the vectors that no product gathers: by item in shared memory
   R *ve, *vr, *vs, *vt, *vv, *vh;
   const int *SLp, *SLl, *SLk, *SLc;  // by slice - bs0; columns by entry - e0
@@ -757,13 +759,18 @@ static bool cluster_fits(bool mixed, int sm, int grid, size_t smem) {
   return ok;
 }
 
-// shared memory of a block and what it holds; sm < 0: not even its partial sums fit
+// the items' partial sums of a block
+static size_t plan_partials(const JacobiPlan& P) {
+  return al16(sizeof(double) * (P.bicg ? kMaxSums : 3) * (size_t)P.items_max);
+}
+
+// shared memory of a block and what it holds
 static size_t plan_smem(const JacobiPlan& P, size_t rs, int minb, int nmat, int& sm) {
-  size_t smem = al16(sizeof(double) * (P.bicg ? kMaxSums : 3) * (size_t)P.items_max) +
-                (P.split > 1 ? sizeof(double) * solve_threads(minb) : 0);
+  sm = 0;
+  if (P.item_part) return 0;
+  size_t smem = plan_partials(P) + (P.split > 1 ? sizeof(double) * solve_threads(minb) : 0);
   const size_t level[3] = {al16(6 * 32 * rs * (size_t)P.items_max) + P.st_meta, al16(4 * P.st_entries),
                            nmat * al16(rs * P.st_entries)};
-  sm = 0;
   while (sm < 3 && smem + level[sm] <= smem_budget(minb)) smem += level[sm++];
   return smem;
 }
@@ -876,6 +883,11 @@ static pfem2_status plan_build(Ctx& c, KrylovWs* w, JacobiPlan& P, bool mixed, c
     PFEM2_TRY(st);
     set_split();
   }
+  // Blocks of very long runs (3D BiCGStab from 8M rows on, 13M with CG) keep
+  // their items' partial sums in global memory: 40 of the some 10,000 bytes
+  // that a phase moves per item. Such a block has more items than warps (split 1).
+  if (!P.cluster && plan_partials(P) > std::min((size_t)c.partials_max, smem_budget(P.minb)) && P.split == 1)
+    PFEM2_TRY(ws_alloc(w, &P.item_part, (size_t)P.grid * plan_partials(P) / sizeof(double)));
   int** dst[6] = {&P.blk_sl, &P.blk_inst, &P.blk_inst_off, &P.blk_slot, &P.sys_slot0, &P.slk};
   for (int k = 0; k < 6; ++k) PFEM2_TRY(ws_upload(w, dst[k], up[k]));
   return PFEM2_OK;
@@ -890,6 +902,7 @@ static void plan_args(const KrylovWs* w, const JacobiPlan& P, SolveArgs<R>& a) {
   a.blk_sl = P.blk_sl;
   a.slk = P.slk;
   a.items_max = P.items_max;
+  a.item_part = P.item_part;
   a.split = P.split;
   a.nslots = P.nslots;
   a.bicg = P.bicg;

@@ -105,6 +105,7 @@ struct JacobiPlan {
   int sm = 0;                                      // cluster: what a block keeps in shared memory
   bool cluster = false, bicg = false;
   size_t st_meta = 0, st_entries = 0;              // per block: static index bytes, SELL entries
+  double* item_part = nullptr;                     // the items' partial sums, where they do not fit shared memory
 };
 
 struct KrylovWs {
