@@ -235,7 +235,8 @@ int tile_aggregate(const Csr& A, const std::vector<int>& tile, int t0, int per, 
 }
 
 // aggregates of aggregates: the graph of the tentative (piecewise-constant)
-// coarse operator aggregated again inside the tiles; the new count
+// coarse operator aggregated again inside the tiles, those without neighbours
+// (parts of the mesh by themselves) kept, numbered in tile order; the new count
 int merge_aggregates(const Csr& A, const std::vector<int>& tile, int na, std::vector<int>& agg) {
   Csr P;
   P.n = A.n;
@@ -251,11 +252,19 @@ int merge_aggregates(const Csr& A, const std::vector<int>& tile, int na, std::ve
     P.ptr[i + 1] = (int)P.col.size();
   }
   const Csr Ac = spgemm(transpose(P), spgemm(A, P));
-  const int nc = aggregate(Ac, ctile, cagg);
+  int nc = aggregate(Ac, ctile, cagg);
+  std::vector<int> order(na), newid(na, -1);
   for (int k = 0; k < na; ++k)
-    if (cagg[k] < 0) return na;  // an aggregate without neighbours: keep the finer ones
+    if (cagg[k] < 0) cagg[k] = nc++;
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    return ctile[a] != ctile[b] ? ctile[a] < ctile[b] : cagg[a] < cagg[b];
+  });
+  int next = 0;
+  for (int k : order)
+    if (newid[cagg[k]] < 0) newid[cagg[k]] = next++;
   for (int i = 0; i < A.n; ++i)
-    if (agg[i] >= 0) agg[i] = cagg[agg[i]];
+    if (agg[i] >= 0) agg[i] = newid[cagg[agg[i]]];
   return nc;
 }
 
