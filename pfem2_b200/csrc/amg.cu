@@ -312,7 +312,7 @@ bool spd_inverse(std::vector<double>& M, int n, double pivot_min) {
 
 pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vector<int>& col,
                       const std::vector<int>& len, const std::vector<Tile>& tiles, const std::vector<int>& st0,
-                      const std::vector<int>& bt0, int coarse_max, MgHost& H) {
+                      const std::vector<int>& bt0, int coarse_max, size_t b2_max, MgHost& H) {
   const int ni = (int)c.inst.size(), T = (int)tiles.size(), G = (int)bt0.size() - 1;
   // M2 is dense: level 2 is coarsened further where a system would have more
   // dofs than this (151 MB of FP32 rows per system, 4 GB over a batch)
@@ -466,6 +466,19 @@ pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vec
     for (int t = 0; t < T; ++t) H.toff[l][t + 1] += H.toff[l][t];
   }
   H.n[0] = c.nv;
+  std::vector<int> sys_of_tile(T);
+  for (int s = 0; s < ni; ++s)
+    for (int t = st0[s]; t < st0[s + 1]; ++t) sys_of_tile[t] = s;
+  // what a block holds of level 2, before the dense matrices of that size are made
+  for (int b = 0; b < G; ++b)
+    if (bt0[b + 1] > bt0[b]) {
+      const int s0 = sys_of_tile[bt0[b]], s1 = sys_of_tile[bt0[b + 1] - 1];
+      H.b2max = std::max(H.b2max, goff[2][s1 + 1] - goff[2][s0]);
+    }
+  if ((size_t)H.b2max > b2_max) {
+    set_error("krylov: the pressure multigrid's per-block data exceed shared memory");
+    return PFEM2_INVALID_ARG;
+  }
   // ---- restrictions
   auto append_rows = [](const Csr& M, int coff, std::vector<int>& ptr, std::vector<int>& cl, std::vector<double>& vl) {
     if (ptr.empty()) ptr.push_back(0);
@@ -509,9 +522,6 @@ pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vec
     }
   }
   // ---- per-block lists
-  std::vector<int> sys_of_tile(T);
-  for (int s = 0; s < ni; ++s)
-    for (int t = st0[s]; t < st0[s + 1]; ++t) sys_of_tile[t] = s;
   std::vector<int> loc1(H.n[1], -1);
   // the level-1 halo each block's rows prolong from, and the entries of its
   // J_1 and Pt_1 rows
@@ -556,11 +566,6 @@ pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vec
     const int sys_first = t_hi > t_lo ? sys_of_tile[t_lo] : 0;
     for (int l = 1; l <= 2; ++l)
       for (int g = H.toff[l][t_lo]; g < H.toff[l][t_hi]; ++g) H.lk[l][g] = H.lsys[l][g] - sys_first;
-    if (t_hi > t_lo) {
-      int n2 = 0;
-      for (int s = sys_of_tile[t_lo]; s <= sys_of_tile[t_hi - 1]; ++s) n2 += sysL[s][2].A.n;
-      H.b2max = std::max(H.b2max, n2);
-    }
     long long mo = 0;
     for (int g = H.toff[2][t_lo]; g < H.toff[2][t_hi]; ++g) {
       H.m2_off[g] = (int)mo;

@@ -62,10 +62,11 @@ struct MgHost {
 // the eliminated FP64 pressure matrix in the context's SELL layout; tiles,
 // st0: the pressure solve's tiles and first tile per system; bt0: first
 // tile per block of the persistent grid; coarse_max: level-3 unknowns per
-// system at most (groups of tiles share one).
+// system at most (groups of tiles share one); b2_max: level-2 unknowns of a
+// block's systems at most (PFEM2_INVALID_ARG above).
 pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vector<int>& col,
                       const std::vector<int>& len, const std::vector<Tile>& tiles, const std::vector<int>& st0,
-                      const std::vector<int>& bt0, int coarse_max, MgHost& out);
+                      const std::vector<int>& bt0, int coarse_max, size_t b2_max, MgHost& out);
 
 // In-place inverse of an SPD matrix (Cholesky, then L^-T L^-1); false if the
 // matrix is not SPD, a pivot being pivot_min times its diagonal entry or less.

@@ -735,7 +735,8 @@ pfem2_status mg_setup(Ctx& c) {
   PFEM2_CUDA(cudaMemcpy(col.data(), c.sl_col, sizeof(int) * c.nell, cudaMemcpyDeviceToHost));
   PFEM2_CUDA(cudaMemcpy(len.data(), c.sl_len, sizeof(int) * c.nslices, cudaMemcpyDeviceToHost));
   MgHost H;
-  PFEM2_TRY(mg_build(c, A, col, len, tiles, st0, bt0, m->minb == 1 ? 160 : 128, H));
+  const size_t rs = c.kmixed ? sizeof(float) : sizeof(double), budget = smem_budget(m->minb);
+  PFEM2_TRY(mg_build(c, A, col, len, tiles, st0, bt0, m->minb == 1 ? 160 : 128, budget / rs, H));
   m->wide = H.r1_col.size() >= 64 * (size_t)std::max(1, H.n[1]);
   m->xsplit = H.xsplit;
   m->s1max = H.s1max;
@@ -747,7 +748,7 @@ pfem2_status mg_setup(Ctx& c) {
   }
   // ---- shared memory: the vectors, then the static data per category while
   // the budget lasts (maximum over blocks; the kernel stages the same pieces)
-  const size_t rs = c.kmixed ? sizeof(float) : sizeof(double), i4 = 4;
+  const size_t i4 = 4;
   size_t smem = al16(sizeof(double) * kMgSums * m->items_max) + al16(rs * m->s1max) + al16(rs * m->b2max);
   constexpr int NC = 9;
   size_t cat[NC] = {};
@@ -772,7 +773,6 @@ pfem2_status mg_setup(Ctx& c) {
                           al16(i4 * nr) + al16(rs * nr)};
     for (int k = 0; k < NC; ++k) cat[k] = std::max(cat[k], v[k]);
   }
-  const size_t budget = smem_budget(m->minb);
   if (smem > budget) {
     set_error("krylov: the pressure multigrid's per-block data exceed shared memory");
     return PFEM2_INVALID_ARG;

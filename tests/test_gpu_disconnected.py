@@ -1,11 +1,13 @@
 """The pressure hierarchy of a large mesh with a small part by itself."""
+import resource
+
 import numpy as np
 import pytest
 
 from pfem2_b200 import _abi as A
 from pfem2_b200 import cases
 from pfem2_b200 import meshes as M
-from pfem2_b200.solver import Solver
+from pfem2_b200.solver import Pfem2Error, Solver
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +54,24 @@ def test_solution_beside_a_small_part():
         s.close()
     for x, y in zip(*out):
         assert np.linalg.norm(x - y) <= 1e-7 * max(1.0, np.linalg.norm(x))
+
+
+def test_more_parts_than_a_block_holds_is_refused():
+    """each of 30,000 parts has a level-2 unknown at least, 240 KB in FP64: the
+    refusal comes before a dense matrix of that size (7.2 GB) is made, and
+    leaves the process able to make another context"""
+    part = M.rect_mesh(5, 5)
+    k = 30000
+    sp = cases.poiseuille_2d(nx=4, ny=2)
+    shift = np.stack([2.0 * (np.arange(k) % 200), 2.0 * (np.arange(k) // 200)], 1)
+    nv = part.n_vertices
+    sp.mesh = M.Mesh((part.vertices[None] + shift[:, None]).reshape(-1, 2),
+                     (part.cells[None] + nv * np.arange(k)[:, None, None]).reshape(-1, 4).astype(part.cells.dtype),
+                     np.tile(part.face_bid, (k, 1)))
+    before = resource.getrusage(resource.RUSAGE_SELF).ru_maxrss
+    with pytest.raises(Pfem2Error) as e:
+        Solver(sp, precision=A.PREC_FP64)
+    assert e.value.status == A.INVALID_ARG and "shared memory" in str(e.value)
+    assert resource.getrusage(resource.RUSAGE_SELF).ru_maxrss - before < 5_000_000  # kB
+    s = Solver(cases.poiseuille_2d(nx=32, ny=12), precision=A.PREC_FP64)
+    s.close()
