@@ -630,10 +630,14 @@ static pfem2_status check_counters(Ctx& c, bool sync) {
 }
 
 // ------------------------------------------------------------ FEM step
-// stage boundary event; external so that it becomes a timing node when the
-// step is being captured into a CUDA graph
+// stage boundary event; external, so that it becomes a timing node, when the
+// step is being captured into a CUDA graph (an error outside a capture)
 static void mark(Ctx& c, int k) {
-  if (c.timing) cudaEventRecordWithFlags(c.ev[k], c.stream, cudaEventRecordExternal);
+  if (!c.timing) return;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(c.stream, &st);
+  cudaEventRecordWithFlags(c.ev[k], c.stream,
+                           st == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault);
 }
 
 static pfem2_status fem_step_launch(Ctx& c) {
