@@ -1217,6 +1217,16 @@ pfem2_status pfem2_solver_sizes(pfem2_ctx* x, int64_t* out) {
   return PFEM2_OK;
 }
 
+pfem2_status pfem2_solver_forms(pfem2_ctx* x, int32_t* out) {
+  CTX_CHECK(x);
+  if (!out) {
+    set_error("pfem2_solver_forms: null output");
+    return PFEM2_INVALID_ARG;
+  }
+  krylov_forms(x->c, out);
+  return PFEM2_OK;
+}
+
 pfem2_status pfem2_enable_stage_timing(pfem2_ctx* x, int32_t on) {
   CTX_CHECK(x);
   PFEM2_TRY(collect_stage_times(x->c));

@@ -306,6 +306,7 @@ void krylov_free(Ctx& c);
 pfem2_status krylov_solve(Ctx& c, int which);
 pfem2_status krylov_read_stats(Ctx& c);
 void krylov_sizes(Ctx& c, long long* out12);
+void krylov_forms(const Ctx& c, int* out12);
 // the mesh elasticity's system (FP64): dim x nv rows, components one after the other
 struct ElasticSystem {
   const int *sl_ptr, *sl_len, *sl_col;

@@ -790,7 +790,7 @@ static pfem2_status plan_runs(JacobiPlan& P, std::vector<int> (&up)[6], const st
   slk.assign(ns, 0);
   for (int b = 0; b <= G; ++b) bsl[b] = (int)((long long)ns * b / G);
   P.grid = G;
-  P.items_max = 0;
+  P.items_max = P.sys_max = 0;
   P.st_meta = P.st_entries = 0;
   for (int b = 0, i = 0; b < G; ++b) {
     const int s0 = bsl[b], s1 = bsl[b + 1];
@@ -810,6 +810,7 @@ static pfem2_status plan_runs(JacobiPlan& P, std::vector<int> (&up)[6], const st
       return PFEM2_INVALID_ARG;
     }
     P.items_max = std::max(P.items_max, (s1 - s0) * ncomp);
+    P.sys_max = std::max(P.sys_max, (binst_off[b + 1] - binst_off[b]) * ncomp);
     P.st_meta = std::max(P.st_meta, 3 * al16(4 * (size_t)(s1 - s0)));
     P.st_entries = std::max(P.st_entries, (size_t)(slp[s1] - slp[s0]));
   }
@@ -1253,6 +1254,18 @@ static pfem2_status read_stats_phase(Ctx& c, int which) {
 void krylov_sizes(Ctx& c, long long* out12) {
   for (int k = 0; k < 12; ++k) out12[k] = 0;
   if (c.kws) mg_sizes((KrylovWs*)c.kws, out12);
+}
+
+void krylov_forms(const Ctx& c, int* out12) {
+  for (int k = 0; k < 12; ++k) out12[k] = 0;
+  const KrylovWs* w = (const KrylovWs*)c.kws;
+  if (!w) return;
+  const JacobiPlan& P = w->plan[1];
+  int sm = 0;
+  plan_smem(P, c.kmixed ? sizeof(float) : sizeof(double), P.minb, c.dim, sm);
+  const int f[6] = {P.grid, P.minb, P.cluster, P.split, sm, P.sys_max};
+  std::copy(f, f + 6, out12);
+  mg_forms(w, out12 + 6);
 }
 
 pfem2_status krylov_read_stats(Ctx& c) {

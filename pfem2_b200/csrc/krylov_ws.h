@@ -100,7 +100,7 @@ struct MgWs;  // mgcg.cu
 struct JacobiPlan {
   int *blk_inst = nullptr, *blk_inst_off = nullptr, *blk_slot = nullptr, *blk_sl = nullptr, *sys_slot0 = nullptr,
       *slk = nullptr;
-  int grid = 0, nslots = 0, items_max = 0, minb = 2, split = 1;
+  int grid = 0, nslots = 0, items_max = 0, sys_max = 0, minb = 2, split = 1;
   int ts = 0;                                      // no cluster: least slices of a block
   int sm = 0;                                      // cluster: what a block keeps in shared memory
   bool cluster = false, bicg = false;
@@ -175,5 +175,6 @@ pfem2_status mg_setup(Ctx& c);
 pfem2_status mg_solve(Ctx& c);
 void mg_free(KrylovWs* w);
 void mg_sizes(const KrylovWs* w, long long* out12);
+void mg_forms(const KrylovWs* w, int* out6);
 
 }  // namespace pfem2

@@ -623,7 +623,7 @@ struct MgWs {
   int minb = 1, grid = 0, nsys = 0, nslots = 0, mask = 0;  // mask: index into kMgMask
   size_t smem = 0;
   bool wide = false, xsplit = false;
-  int items_max = 0, s1max = 0, b2max = 0;
+  int items_max = 0, s1max = 0, b2max = 0, sys_max = 0;
   long long sizes[12] = {};
   int *blk_sys, *blk_sys_off, *blk_sl, *blk_slot, *sys_slot0, *blk_o1, *blk_o2, *slk, *lk1, *lk2;
   int *r1_ptr, *r1_col, *q2_ptr, *q2_col, *m2_off, *p0_ptr, *p0_len, *p0_col;
@@ -643,6 +643,13 @@ void mg_free(KrylovWs* w) {
 
 void mg_sizes(const KrylovWs* w, long long* out12) {
   for (int k = 0; k < 12; ++k) out12[k] = w->mg ? w->mg->sizes[k] : 0;
+}
+
+void mg_forms(const KrylovWs* w, int* out6) {
+  const MgWs* m = w->mg;
+  const int f[6] = {m ? m->grid : 0, m ? m->minb : 0,         m ? m->mask : 0,
+                    m ? (m->wide ? 32 : 8) : 0, m ? m->xsplit : 0, m ? m->sys_max : 0};
+  std::copy(f, f + 6, out6);
 }
 
 namespace {
@@ -716,6 +723,7 @@ pfem2_status mg_setup(Ctx& c) {
       set_error("krylov: more than 16 systems would share one block (instances too small for the batch)");
       return PFEM2_INVALID_ARG;
     }
+    m->sys_max = std::max(m->sys_max, s1 - s0 + 1);
     for (int s = s0; s <= s1; ++s) bsys.push_back(s);
     bsys_off.push_back((int)bsys.size());
     bsl[2 * b] = tiles[bt0[b]].s0;

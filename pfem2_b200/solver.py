@@ -38,7 +38,7 @@ EXPORTS = [
     "pfem2_launch_count", "pfem2_stage_times", "pfem2_enable_stage_timing", "pfem2_get_stream",
     "pfem2_last_error", "pfem2_abi_version", "pfem2_project_noalloc", "pfem2_solver_sizes",
     "pfem2_calculate_vorticity", "pfem2_set_tuning", "pfem2_get_tuning", "pfem2_tuning_key",
-    "pfem2_mesh_elasticity", "pfem2_move_mesh", "pfem2_get_vertices",
+    "pfem2_mesh_elasticity", "pfem2_move_mesh", "pfem2_get_vertices", "pfem2_solver_forms",
 ]
 
 
@@ -75,6 +75,7 @@ def load_library(path=LIB_PATH):
         "pfem2_launch_count": [vp, C.POINTER(C.c_int64)],
         "pfem2_stage_times": [vp, dp, C.c_int32],
         "pfem2_solver_sizes": [vp, C.POINTER(C.c_int64)],
+        "pfem2_solver_forms": [vp, ip],
         "pfem2_calculate_vorticity": [vp],
         "pfem2_enable_stage_timing": [vp, C.c_int32],
         "pfem2_get_stream": [vp, C.POINTER(vp)],
@@ -336,6 +337,14 @@ class Solver:
         self._check(self.L.pfem2_solver_sizes(self.h, out))
         keys = ("n0", "n1", "n2", "n3", "r01", "r02", "c3", "p0", "j1", "p1", "j2", "p2")
         return dict(zip(keys, (int(v) for v in out)))
+
+    def solver_forms(self):
+        """Forms that the velocity and pressure solvers took (pfem2_solver_forms)."""
+        out = (C.c_int32 * 12)()
+        self._check(self.L.pfem2_solver_forms(self.h, out))
+        vel = ("blocks", "blocks_per_sm", "cluster", "warps_per_slice", "staged", "systems_per_block")
+        p = ("blocks", "blocks_per_sm", "staged", "restriction_lanes", "level1_published", "systems_per_block")
+        return dict(zip(vel, out[:6])), dict(zip(p, out[6:]))
 
     def stage_times(self, reset=False):
         ms = np.zeros(N_STAGES)
