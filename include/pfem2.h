@@ -346,7 +346,7 @@ pfem2_status pfem2_solver_sizes(pfem2_ctx* ctx, int64_t* out);
 /* Forms that the solvers took after pfem2_setup (diagnostics; no counterpart
  * in the reference). Velocity prediction: out[0] blocks, [1] blocks per SM,
  * [2] 1 if they are one thread-block cluster, [3] warps that share a row
- * slice, [4] what a block keeps in shared memory (0 nothing .. 3 own rows,
+ * slice, [4] what a block keeps in shared memory (-1 nothing .. 3 own rows,
  * columns and values), [5] systems (components x instances) of a block at
  * most. Pressure multigrid, all 0 without one: [6] blocks, [7] blocks per SM,
  * [8] the same for it (0 everything .. 3 nothing), [9] lanes per restriction

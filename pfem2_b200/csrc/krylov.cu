@@ -86,6 +86,9 @@ constexpr int kClusterItems = 300;
 // fits; every phase start's GPU-scope acquire invalidates L1, so what is read
 // from global memory costs an L2 round trip per phase). Known at compile time:
 // generic pointers made the solves 15-20% slower.
+//   -1 nothing, the items' partial sums in global memory: their pointer alone,
+//      left generic, cost the 1.05M-cell pipe 3 to 6% of its velocity solves
+//   0  those sums
 //   1  the own rows of the vectors that no product gathers, the slices' pointers
 //   2  and the SELL columns
 //   3  and the SELL values of every component (once where they share a matrix)
@@ -143,7 +146,7 @@ template <typename R> struct SolveArgs {
   R *e, *r;
   double* r64;
   double* part;          // [2 parities][kMaxSums][nslots]
-  double* item_part;     // [blocks][items_max][sums] where they do not fit shared memory, else null
+  double* item_part;     // [blocks][items_max][sums] where they do not fit shared memory
   int nslots;
   unsigned* scount;      // [nsys][32]: per-system count of block phases published (one 128-byte line each, zeroed per launch)
   int* active;
@@ -333,9 +336,14 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
   // ---- shared memory: partial products of split items, the items' partial
   // sums, then the staged static data
   double* const s_dot = reinterpret_cast<double*>(dyn_smem);
-  double* spart = s_dot + (split > 1 ? kWarps * 32 : 0);
-  unsigned char* cur = reinterpret_cast<unsigned char*>(spart) + al16_dev((size_t)a.items_max * NS * sizeof(double));
-  if (SM == 0 && a.item_part) spart = a.item_part + (size_t)blockIdx.x * a.items_max * NS;
+  double* spart;
+  unsigned char* cur = dyn_smem;
+  if constexpr (SM < 0) {
+    spart = a.item_part + (size_t)blockIdx.x * a.items_max * NS;
+  } else {
+    spart = s_dot + (split > 1 ? kWarps * 32 : 0);
+    cur = reinterpret_cast<unsigned char*>(spart) + al16_dev((size_t)a.items_max * NS * sizeof(double));
+  }
   // own rows of the vectors that no product gathers: by item in shared memory
   R *ve, *vr, *vs, *vt, *vv, *vh;
   const int *SLp, *SLl, *SLk, *SLc;  // by slice - bs0; columns by entry - e0
@@ -706,7 +714,8 @@ __global__ void __launch_bounds__(SolveThreads<MINB>::value, MINB) k_krylov(Solv
 // ------------------------------------------------------------------ host
 template <typename R, int MINB>
 static const void* kernel_of(int sm) {
-  return sm == 0   ? (const void*)k_krylov<R, MINB, 0, false>
+  return sm < 0    ? (const void*)k_krylov<R, MINB, -1, false>
+         : sm == 0 ? (const void*)k_krylov<R, MINB, 0, false>
          : sm == 1 ? (const void*)k_krylov<R, MINB, 1, false>
          : sm == 2 ? (const void*)k_krylov<R, MINB, 2, false>
                    : (const void*)k_krylov<R, MINB, 3, false>;
@@ -766,8 +775,8 @@ static size_t plan_partials(const JacobiPlan& P) {
 
 // shared memory of a block and what it holds
 static size_t plan_smem(const JacobiPlan& P, size_t rs, int minb, int nmat, int& sm) {
-  sm = 0;
-  if (P.item_part) return 0;
+  sm = P.item_part ? -1 : 0;
+  if (sm < 0) return 0;
   size_t smem = plan_partials(P) + (P.split > 1 ? sizeof(double) * solve_threads(minb) : 0);
   const size_t level[3] = {al16(6 * 32 * rs * (size_t)P.items_max) + P.st_meta, al16(4 * P.st_entries),
                            nmat * al16(rs * P.st_entries)};
