@@ -895,6 +895,7 @@ pfem2_status pfem2_seed(pfem2_ctx* x, int32_t instance, const uint32_t q[3], uin
   c.seeded = false;  // until they are there
   PFEM2_TRY(launch_seed(c, instance, q, seed, jitter));
   c.seeded = true;
+  c.n_seeded = total;
   c.stats.n_particles = (int)total;
   x->graph_failed = false;
   for (int k = 0; k < 2; ++k)
@@ -1164,6 +1165,7 @@ pfem2_status pfem2_set_particles(pfem2_ctx* x, const int32_t* counts, const int3
   c.seeded = false;  // until they are there
   PFEM2_TRY(launch_set_particles(c, counts, cell, xi, u));
   c.seeded = true;
+  c.n_seeded = total;
   for (int k = 0; k < 2; ++k)
     if (x->graph[k]) { cudaGraphExecDestroy(x->graph[k]); x->graph[k] = nullptr; }
   return PFEM2_OK;
@@ -1294,7 +1296,7 @@ pfem2_status pfem2_get_tuning(pfem2_ctx* x, pfem2_tuning* t) {
   if (!t) { set_error("pfem2_get_tuning: null argument"); return PFEM2_INVALID_ARG; }
   const Ctx& c = x->c;
   *t = c.setup_done ? c.tune : c.tune_req;
-  if (c.setup_done && !t->advect_split) t->advect_split = (long long)c.pcap >= c.adv_split_min ? 2 : 1;
+  if (c.setup_done && !t->advect_split) t->advect_split = advect_split(c) ? 2 : 1;
   return PFEM2_OK;
 }
 

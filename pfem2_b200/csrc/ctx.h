@@ -144,11 +144,11 @@ struct Ctx {
   void* pu[2] = {};
   int cur = 0;
   int* newcell = nullptr;
-  // particle capacity from which the advection runs as two kernels
-  // (stayers, then leavers; faster than the one-kernel form on every workload
-  // measured, from 0.3M particles on, and within 3 us of it on 20k);
-  // the environment variable PFEM2_ADVECT_SPLIT_MIN overrides it at creation
-  long long adv_split_min = 0;
+  // particle capacity from which the advection runs as two kernels (stayers,
+  // then leavers), set by the environment variable PFEM2_ADVECT_SPLIT_MIN at
+  // creation; < 0: by dimension and particles (advect_split)
+  long long adv_split_min = -1;
+  size_t n_seeded = 0;  // particles of the last seeding or setting
   int* cell_start[2] = {};
   unsigned long long* rebin_tiles = nullptr;  // ticket + status words of the re-sort's scan, overflow fill count
   int* rebin_cnt = nullptr;                   // [nc] particles of each cell after the re-sort
@@ -270,6 +270,7 @@ inline int grid_for(const Ctx& c, long long n, int threads, int per_sm = 8) {
 pfem2_status launch_seed(Ctx& c, int instance, const uint32_t q[3], uint64_t seed, double jitter);
 pfem2_status launch_correct(Ctx& c);
 pfem2_status launch_advect(Ctx& c, bool fuse_correct);
+bool advect_split(const Ctx& c);  // whether it runs as two kernels
 pfem2_status launch_rebin(Ctx& c, bool do_check, bool fuse_project, bool from_advect);
 pfem2_status launch_project(Ctx& c, bool partials_ready);
 pfem2_status launch_sync_real_fields(Ctx& c);

@@ -448,9 +448,9 @@ __device__ __forceinline__ void advect_record(int p, int c0, int c, const int* _
   }
 }
 
-// Advection in one pass (selectable with advect_split = 1 or below
-// PFEM2_ADVECT_SPLIT_MIN slots): correction, every sub-step with the full
-// point location in line. Same arithmetic as the two-phase form.
+// Advection in one kernel (small 2D sets, see advect_split): correction, every
+// sub-step with the full point location in line. Same arithmetic as the
+// two-kernel form.
 template <int DIM, typename R, bool FUSE>
 __global__ void __launch_bounds__(256, AdvectMinBlocks<DIM, R>::value) k_advect_one(
     const int* __restrict__ cell, R* __restrict__ xi, R* __restrict__ u, int* __restrict__ newcell, size_t cap,
@@ -807,12 +807,27 @@ pfem2_status far_sort_setup(Ctx& c) {
   return PFEM2_OK;
 }
 
+// One kernel or two. In 2D the second kernel's launch and its own chain of
+// point locations pay from about 130k particles on. Move (advection and
+// re-sort), FP64, one / two kernels, at a third and at four fifths of a cell
+// per step: 28k particles 0.038 / 0.042 and 0.050 / 0.063 ms, 83k 0.050 / 0.049
+// and 0.050 / 0.058, 171k 0.065 / 0.060 and 0.065 / 0.073, 398k 0.099 / 0.089
+// and 0.156 / 0.168, 1.0M 0.206 / 0.157 and 0.215 / 0.229. In 3D the one kernel's
+// registers leave it half the warps: 0.7k particles, FP64, 0.129
+// / 0.107 ms, 46k 0.190 / 0.141, 0.6M 0.905 / 0.538.
+constexpr size_t kSplitMin2D = 131072;
+
+bool advect_split(const Ctx& c) {
+  if (c.tune.advect_split) return c.tune.advect_split == 2;
+  if (c.adv_split_min >= 0) return (long long)c.pcap >= c.adv_split_min;
+  return c.dim == 3 || c.n_seeded >= kSplitMin2D;
+}
+
 template <int DIM, typename R>
 static pfem2_status advect_impl(Ctx& c, bool fuse) {
   int b = c.cur;
   int S = c.cfg.movement_steps;
-  const bool split = c.tune.advect_split ? c.tune.advect_split == 2 : (long long)c.pcap >= c.adv_split_min;
-  if (!split) {
+  if (!advect_split(c)) {
     const int grid = grid_for(c, c.pcap, 256, c.tune.advect_blocks_per_sm);
     if (fuse)
       k_advect_one<DIM, R, true><<<grid, 256, 0, c.stream>>>(
