@@ -769,13 +769,7 @@ def run_reference(args, rank, world):
     print(json.dumps(res), flush=True)
 
 
-# the launch shapes the autotuner chose for these workloads on a B200
-# (pfem2_b200/autotune.py); a tuning cache named in the environment wins
-TUNING_CACHE = os.path.join(ROOT, "pfem2_b200", "tuning", "b200.txt")
-
-
 def main():
-    os.environ.setdefault("PFEM2_TUNING_CACHE", TUNING_CACHE)
     args = parse()
     rank, world, local = dist_info()
     if args.impl == "reference":

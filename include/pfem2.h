@@ -366,7 +366,7 @@ int32_t pfem2_abi_version(void);
  * solver tolerance. */
 typedef struct {
   int32_t advect_blocks_per_sm;  /* advection grid in 256-thread blocks per SM (sets particles per block) */
-  int32_t advect_split;          /* 1: one advection pass, 2: stayers, then each block's queued leavers */
+  int32_t advect_split;          /* 1: one advection kernel, 2: the particles that stay in their cell, then the others */
   int32_t rebin_blocks_per_sm;   /* re-sort grids in 256-thread blocks per SM, at most those that fit */
   int32_t vel_tile_slices;       /* velocity solves: SELL slices of 32 rows per block at least */
   int32_t p_blocks_per_sm;       /* pressure multigrid of a single system: 1 or 2 blocks per SM */

@@ -2,13 +2,13 @@
 
 The particle kernels and the persistent Krylov solver have shapes that the
 best choice of depends on the GPU and the mesh size: the advection grid
-(particles per block) and whether advection runs in one pass or in two
-phases (stayers, then queued leavers), the re-sort grid, the velocity
-solves' SELL slices per block and blocks per SM, and the blocks per SM of a
+(particles per block) and whether advection runs as one kernel or as two
+(particles that stay in their cell, then the others), the re-sort grid, the
+velocity solves' SELL slices per block and blocks per SM, and the blocks per SM of a
 single pressure system's multigrid solve. `tune` times whole
 steps (the device time of every stage,
 CUDA events inside the library) for candidate shapes by coordinate descent
-(coupled knobs, such as the advection grid and its one- or two-phase form,
+(coupled knobs, such as the advection grid and its one- or two-kernel form,
 over all their combinations) and appends the fastest to a cache file under the context's key: device
 name, dim, FP32 stages, log2 cells, log2 instances (pfem2_tuning_key). A
 later context with the same key reads the entry at pfem2_setup when the

@@ -21,10 +21,12 @@ namespace pfem2 {
 
 namespace {
 
-// entries of J_1 and Pt_1 rows that a block may read for its level-1 halo per
-// iteration; above, x1 is formed by the owners in a phase of its own (about 3
-// us an iteration): 2D channels read 1.5-2k (no gain), the 10k-cell pipe 13k
-// (pressure solve 1.47 -> 1.01 ms) and the 131k-cell pipe 23k (4.85 -> 3.47 ms)
+// Entries of J_1 and Pt_1 rows that a block may read for its level-1 halo per
+// iteration; above, x1 is formed by the owners in a phase of its own. Pressure
+// solve with halo rows / with the phase: channels of 8k to 52k cells (1 to 1.5k
+// entries) 0.43 / 0.46 and 0.79 / 0.85 ms; pipes of 1.5k cells (7k) 0.56 / 0.49,
+// 3k (13k) 0.99 / 0.52, 12k (12k) 1.31 / 0.73, 131k (23k) 4.2 / 3.4 FP64 and
+// 2.8 / 1.8 FP32
 constexpr size_t kHaloMax = 4096;
 
 struct Csr {
@@ -315,7 +317,12 @@ pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vec
                       const std::vector<int>& bt0, int coarse_max, size_t b2_max, MgHost& H) {
   const int ni = (int)c.inst.size(), T = (int)tiles.size(), G = (int)bt0.size() - 1;
   // M2 is dense: level 2 is coarsened further where a system would have more
-  // dofs than this (151 MB of FP32 rows per system, 4 GB over a batch)
+  // dofs than this. The line bounds memory (151 MB of FP32 rows per system, 4 GB
+  // over a batch), not time: every iteration reads M2, and large 2D channels
+  // solve faster with fewer dofs in spite of more iterations (144k cells: 2,609
+  // dofs 2.8 ms FP64 and 2.6 FP32, 608 dofs 1.3 and 1.6; 262k cells: 4,160 dofs
+  // 7.6 and 10.5 ms, 1,196 dofs 4.4 and 3.9). 3D pipes of up to 0.5M cells have
+  // 1,700 at most
   const int n2_max = std::max(512, std::min(6144, (int)std::sqrt(1.0e9 / ni)));
   const std::vector<int>& sp = c.h_sl_ptr;
   std::vector<std::vector<Level>> sysL(ni);
@@ -417,10 +424,13 @@ pfem2_status mg_build(const Ctx& c, const std::vector<double>& A, const std::vec
       // 37 -> 32 (solve 0.77 -> 0.67 ms, FP64), 13k 30 -> 25, 131k-cell pipe
       // 46 -> 42, 16 channels 44 -> 37; 1.8 / rho took 17 instead of 14 on a
       // uniform channel. The coarse levels' weights and an exact level 1 change
-      // none of these by more than one. Contexts that round P or V to FP32 for the
-      // right-hand sides keep 4 / (3 rho) (34k-cell channel 0.66 ms per solve, 0.60
-      // with the row sums): rounding turns any other iterate within the solver's
-      // tolerance, 1e-11 of P, into last-bit flips and 1e-6 in the loads.
+      // none of these by more than one. (1.6 / rho stays below 1.7 / lambda_max on
+      // the coarse levels of graded, stretched, sheared and randomly distorted
+      // channels.) Contexts that round P or V to FP32 for the right-hand sides keep
+      // 4 / (3 rho) (34k-cell channel 0.66 ms per solve, 0.60 with the row sums).
+      // That is for the same results, not for better ones: the rounding turns
+      // differences far below the solver's tolerance into last-bit flips and 1e-6
+      // in the loads, whose error against FP64 is 5e-5 with either weight.
       if (c.amixed || c.prmixed) {
         V.w = 4.0 / (3.0 * rho);
         if (l == 0 && c.moving) V.w = std::min(V.w, 0.49);

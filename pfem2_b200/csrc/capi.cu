@@ -750,7 +750,7 @@ pfem2_status pfem2_create(const pfem2_config* cfg, pfem2_ctx** out) {
     set_error("movement_steps and max_particles_per_cell_part must be >= 1");
     return PFEM2_INVALID_ARG;
   }
-  if (cfg->movement_steps > 65535) {
+  if (cfg->movement_steps > 65535) {  // (no storage depends on it any more)
     set_error("movement_steps must be <= 65535");
     return PFEM2_INVALID_ARG;
   }

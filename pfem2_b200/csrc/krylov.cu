@@ -76,10 +76,16 @@ constexpr int kClusterMax = 16;  // blocks of a cluster
 // its length holds, so that 1,570 instances in 3D and 2,360 in 2D, the smallest
 // at one slice each, fit two blocks on each of 148 SMs
 constexpr int kMaxRunSys = 24;
-// items (slices x components) up to which one cluster solves: above, the 16
-// SMs' work outweighs the cheaper barrier (1k channel FP64, 70 items:
-// prediction and correction 0.49 -> 0.38 ms per step; 8k cells, 520 items:
-// 0.45 -> 0.63)
+// Items (slices x components) up to which one cluster solves: above, the 16
+// SMs' work outweighs the cheaper barrier. Prediction and correction of uniform
+// channels, cluster / grid, ms per step:
+//   items            70          150         240         300         350         400         520
+//   FP64 BiCGStab  .38 / .47   .42 / .45   .41 / .42   .44 / .41   .45 / .41   .56 / .40   .57 / .38
+//   FP64 CG        .33 / .41   .35 / .40   .36 / .39   .38 / .38   .40 / .37   .51 / .37   .51 / .36
+//   FP32 BiCGStab  .31 / .39   .32 / .38   .32 / .36   .33 / .37   .35 / .37   .42 / .34   .43 / .34
+//   FP32 CG        .40 / .49   .39 / .49   .38 / .46   .38 / .45   .39 / .46   .51 / .44   .52 / .44
+// (from 385 items on a warp takes two). One line for all: FP64 crosses between
+// 270 and 300, FP32 at 385.
 constexpr int kClusterItems = 300;
 
 // What a block keeps in shared memory (template parameter SM, the most that
@@ -1215,7 +1221,8 @@ static pfem2_status solve_impl(Ctx& c, int which) {
   a.out_tol = w->out_tol[which];
   a.out_outer = w->out_outer[which];
   a.eta = c.kmixed ? c.refine_eta : 0.0;
-  // phases per iteration, and the restarts (one phase more, at most max_iter)
+  // CG: a phase per iteration, and the restarts (two more, at most one per
+  // iteration); BiCGStab: two, and the same
   a.iter_cap = (a.bicg ? 5 : 4) * krylov_max_iter(c) + 256;
   PFEM2_TRY(krylov_init_solve(c, ncomp * ni));
   return plan_launch(c, P, a, P.cluster || !a.share ? ncomp : 1);
